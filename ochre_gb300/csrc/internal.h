@@ -296,7 +296,9 @@ namespace ochre {
 int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uint32_t* n_lines);
 int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaStream_t s, uint64_t* n_entries,
               uint32_t* key_bits);
-int stage_sort(ochre_gpu_ctx* ctx, uint64_t n_entries, uint32_t key_bits, cudaStream_t s, uint32_t* passes);
+// Sorts by key bits first_bit .. first_bit + key_bits - 1.
+int stage_sort(ochre_gpu_ctx* ctx, uint64_t n_entries, uint32_t key_bits, cudaStream_t s, uint32_t* passes,
+               uint32_t first_bit = 0);
 int stage_tiles(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t n_entries, cudaStream_t s, uint32_t* n_tiles,
                 uint32_t* n_spans);
 // Rewrites stroked fills into plain fills (stroke.cu); *out views device memory.

@@ -266,7 +266,8 @@ __global__ void __launch_bounds__(SORT_BLOCK, RB <= 8 ? 3 : 2) k_onesweep(
 }
 
 template <class K, int RB>
-static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStream_t s, uint32_t* passes_done) {
+static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStream_t s, uint32_t* passes_done,
+                     uint32_t first_bit) {
     constexpr int RADIX = 1 << RB;
     DevScalars* ds = dev_scalars(ctx);
     // graph replays: n is the capacity, the count is on the device, and every
@@ -276,7 +277,7 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
     const uint32_t kb = std::max<uint32_t>(key_bits, 1u);
     plan.passes = (int)((kb + RB - 1) / RB);
     if (plan.passes > SORT_MAX_PASSES) return OCHRE_E_INVALID;
-    for (int p = 0, at = 0; p < plan.passes; p++) {
+    for (int p = 0, at = (int)first_bit; p < plan.passes; p++) {
         // balanced widths: the first kb % passes passes take one bit more
         const int w = (int)(kb / plan.passes) + (p < (int)(kb % plan.passes) ? 1 : 0);
         plan.shift[p] = (uint8_t)at;
@@ -337,14 +338,15 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
     return OCHRE_OK;
 }
 
-int stage_sort(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStream_t s, uint32_t* passes) {
+int stage_sort(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStream_t s, uint32_t* passes,
+               uint32_t first_bit) {
     *passes = 0;
     if (n <= 1) return OCHRE_OK;
     if (ctx->tune_sort_digit_bits == 11)
-        return ctx->keys64 ? sort_impl<uint64_t, 11>(ctx, n, key_bits, s, passes)
-                           : sort_impl<uint32_t, 11>(ctx, n, key_bits, s, passes);
-    return ctx->keys64 ? sort_impl<uint64_t, 8>(ctx, n, key_bits, s, passes)
-                       : sort_impl<uint32_t, 8>(ctx, n, key_bits, s, passes);
+        return ctx->keys64 ? sort_impl<uint64_t, 11>(ctx, n, key_bits, s, passes, first_bit)
+                           : sort_impl<uint32_t, 11>(ctx, n, key_bits, s, passes, first_bit);
+    return ctx->keys64 ? sort_impl<uint64_t, 8>(ctx, n, key_bits, s, passes, first_bit)
+                       : sort_impl<uint32_t, 8>(ctx, n, key_bits, s, passes, first_bit);
 }
 
 }  // namespace ochre
