@@ -42,32 +42,89 @@ __device__ __forceinline__ void bbox_add(BBoxAcc& b, int x, int y) {
     b.y1 = max(b.y1, ty);
 }
 
-// Count bins, crossings and increment cells of a line; extend its raster's
-// tile bbox; sum the crossing signs.
-__device__ __forceinline__ uint32_t count_line(V2 a, V2 p, BBoxAcc& bb, bool* capped, int* wsum, uint32_t* cells) {
-    *wsum = 0;
-    *cells = 0;
-    if (veq(a, p)) return 0u;
-    uint32_t nb = 0, nc = 0, nx = 0, run = 0;
-    int ws = 0;
-    int ptx = 0x7fffffff, pty = 0x7fffffff;
+// What a line's walk leaves: sort entries (bins and crossings), increment
+// cells, the sum of its crossing signs, the tile box of its visited cells.
+struct LineCount {
+    uint32_t ent, cells;
+    int wsum;
+    BBoxAcc box;
+};
+
+// The same by walking (a line that reaches WALK_CAP).
+__device__ __noinline__ LineCount count_by_walking(V2 a, V2 p, uint32_t* err) {
+    uint32_t ent = 0, cells = 0;
+    int ws = 0, ptx = 0x7fffffff, pty = 0x7fffffff;
+    BBoxAcc box{0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000};
     const bool ok = walk_line(
         a, p,
         [&](const Walk&, const WalkState& s) {
             const int tx = div8(s.x), ty = div8(s.y);
-            if (tx != ptx || ty != pty || run == BIN_MAX_CELLS) { nb++; ptx = tx; pty = ty; run = 0; }
-            run++;
-            nx++;
+            if (tx != ptx || ty != pty) { ent++; ptx = tx; pty = ty; }
+            cells++;
         },
         [&](int, int, int sign) {
-            nc++;
+            ent++;
             ws += sign;
         },
-        [&](int x, int y) { bbox_add(bb, x, y); });
-    if (!ok) *capped = true;
-    *wsum = ws;
-    *cells = nx;
-    return nb + nc;
+        [&](int x, int y) { bbox_add(box, x, y); });
+    if (!ok) atomicOr(err, ERR_LIMIT);
+    return LineCount{ent, cells, ws, box};
+}
+
+// Counts of a line without walking it.  The walk takes the row and column
+// steps in order of their parameters and ends with the first at 1, so it
+// takes every step below 1 of either axis whatever their order, then one
+// more: the numbers of row and column steps below 1 (two independent
+// recurrences, each two operations a step) give the last cell, and with it
+//   * cells: every step below 1 leads to a cell, and there is the first one;
+//   * bins: each step moves along one axis, so a new bin opens exactly where
+//     a step leaves a tile column or a tile row;
+//   * crossings: the tile rows left that way, and the snapped end cell's.
+// Cells wrap at the i16 limits, which are tile boundaries too: a step across
+// one leaves a tile like any other, in the walk's direction (the sign byte of
+// -8191 is +1, of 8191 -1).  Bound by instruction issue: eight instructions
+// per step of the longer axis, where walking took about 25 per cell.  20,000
+// uneven paths (60 M lines, 689 M cells): 2.55 ms (walked, ordered by length,
+// the long lines beside) -> 1.08 ms, the lines in their own order.
+__device__ __forceinline__ LineCount count_line(V2 a, V2 p, uint32_t* err) {
+    LineCount n{0u, 0u, 0, {0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000}};
+    if (veq(a, p)) return n;
+    Walk w;
+    WalkState s;
+    walk_setup(a, p, w, s);
+    uint32_t rows = 0, cols = 0;
+    float rt = s.row_t1, ct = s.col_t1;
+    while (rt < 1.0f || ct < 1.0f) {
+#pragma unroll
+        for (int k = 0; k < 4; k++) {   // (past 1 nothing more is counted)
+            if (rt < 1.0f) rows++;
+            if (ct < 1.0f) cols++;
+            rt = rmin(__fadd_rn(rt, w.y_step), 1.0f);
+            ct = rmin(__fadd_rn(ct, w.x_step), 1.0f);
+        }
+        if (rows + cols >= WALK_CAP) {
+            return count_by_walking(a, p, err);
+        }
+    }
+    // the last cell, not wrapped
+    const int lx = s.x + w.x_dir * (int)cols, ly = s.y + w.y_dir * (int)rows;
+    const int left_x = abs(div8(lx) - div8(s.x)), left_y = abs(div8(ly) - div8(s.y));
+    const int end_ty = div8(w.end_y), last_ty = div8(wrap16(ly));
+    n.cells = rows + cols + 1u;
+    n.ent = 1u + (uint32_t)left_x + 2u * (uint32_t)left_y + (end_ty != last_ty ? 1u : 0u);
+    n.wsum = w.y_dir * left_y + (int)(int8_t)(int16_t)(end_ty - last_ty);
+    bbox_add(n.box, s.x, s.y);
+    bbox_add(n.box, wrap16(lx), wrap16(ly));
+    bbox_add(n.box, w.end_x, w.end_y);
+    if (lx != wrap16(lx)) {   // past an i16 limit: every column of the range's ends
+        n.box.x0 = min(n.box.x0, -4096);
+        n.box.x1 = max(n.box.x1, 4095);
+    }
+    if (ly != wrap16(ly)) {
+        n.box.y0 = min(n.box.y0, -4096);
+        n.box.y1 = max(n.box.y1, 4095);
+    }
+    return n;
 }
 
 // Block-local work order by walk length: the BLOCK items of a block are
@@ -98,56 +155,11 @@ __device__ __forceinline__ uint32_t order_by_length(uint32_t cells, uint32_t* s_
     return s_item[threadIdx.x];
 }
 
-// Persistent count walks of short lines.  A warp takes windows of WIN
-// consecutive lines by ticket and walks each window's lines 32 at a time in
-// order of length (grouped by log2 of their cell count, unstable within a
-// group), so a warp's lanes walk lines of about the same length; no warp
-// waits on another, so an SM stays full until the last window (a block of
-// lines ordered in the block holds its SM slot until its slowest warp ends:
-// count 1.87 -> 1.71 ms on the 20,000-path uneven mix, 0.169 -> 0.143 ms on
-// 100,000 glyphs).  The emit walk keeps the block form: there, each group's
-// set-up loads (line, offsets, raster box and key base) waited behind the
-// previous group of the warp, 9.8 against 7.9 ms.
-constexpr int WIN = 256;
-constexpr int WIN_PER_LANE = WIN / 32;
-constexpr int WALK_BLOCK = 128;
-constexpr int LEN_GROUPS = 17;
-
-// Orders this warp's window: item WIN_PER_LANE * ... of lane k is
-// k + 32 * j (j < WIN_PER_LANE) with `cells[j]` cells; fills s_item[0..WIN)
-// with the items grouped by length.  s_cnt: LEN_GROUPS words of the warp.
-__device__ __forceinline__ void order_window(const uint32_t (&cells)[WIN_PER_LANE], uint32_t* s_cnt,
-                                             uint16_t* s_item) {
-    const uint32_t lane = threadIdx.x & 31u;
-    if (lane < LEN_GROUPS) s_cnt[lane] = 0u;
-    __syncwarp();
-    uint32_t g[WIN_PER_LANE], k[WIN_PER_LANE];
-#pragma unroll
-    for (int j = 0; j < WIN_PER_LANE; j++) {
-        g[j] = min(31u - (uint32_t)__clz(max(cells[j], 1u)), (uint32_t)LEN_GROUPS - 1u);
-        k[j] = atomicAdd(&s_cnt[g[j]], 1u);
-    }
-    __syncwarp();
-    const uint32_t c = lane < LEN_GROUPS ? s_cnt[lane] : 0u;
-    uint32_t inc = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= (uint32_t)o) inc += t;
-    }
-    __syncwarp();
-    if (lane < LEN_GROUPS) s_cnt[lane] = inc - c;
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < WIN_PER_LANE; j++) s_item[s_cnt[g[j]] + k[j]] = (uint16_t)(j * 32 + lane);
-    __syncwarp();
-}
-
-// The next window of a warp (lane 0 takes the ticket); WIN * it is its first line.
+// The next window of a warp (lane 0 takes the ticket).
 __device__ __forceinline__ uint64_t next_window(uint32_t* ticket) {
     uint32_t w = 0;
     if ((threadIdx.x & 31u) == 0u) w = atomicAdd(ticket, 1u);
-    return (uint64_t)__shfl_sync(0xffffffffu, w, 0) * WIN;
+    return (uint64_t)__shfl_sync(0xffffffffu, w, 0);
 }
 
 // A raster's global tile box grows by atomics only where it grows.
@@ -159,41 +171,15 @@ __device__ __forceinline__ void box_grow(int4* d, int x0, int y0, int x1, int y1
     if (y1 > cur.w) atomicMax(&d->w, y1);
 }
 
-// ---------------------------------------------------------------------
-// Long lines: persistent walkers with per-lane refill.
-//
-// Walk lengths run from one cell to thousands (a path's long edges).  One
-// thread per line, as the count and emit kernels walk most lines, would give
-// a long line's warp one busy lane for thousands of steps.  The flatten
-// stage queues every line of more than `long_cells` (estimated) cells, and
-// the first blocks of the count and emit kernels walk that queue this way:
-// every lane of a warp makes one DDA step per loop iteration; a lane whose
-// line has ended takes the next line from the warp's pool of WALK_POOL
-// queued lines, and the warp takes a new pool from a global ticket when its
-// pool runs out.  A refill waits until at least `refill` lanes are idle (a
-// refill costs the new lines' set-up loads).  Outputs go to the per-line
-// offsets of the count scan, so they do not depend on which lane walks which
-// line.  (For short lines the per-line set-up, run by the few lanes that
-// refill at a time, costs more than the idle lanes it saves: measured
-// slower on every configuration, so short lines stay one per thread.)
-//
-// Job interface (per lane): bool begin(queue index, Walk&, WalkState&) sets
-// the walk up (false: the line has no walk); cell(w, s) for every increment
-// cell; visit(x, y) for every visited cell; cross(tx, ty, sign) for every
-// tile-row crossing; end(capped) when the line's walk is over.  The step
-// sequence is walk_line's (common.cuh), including its WALK_CAP.
-// ---------------------------------------------------------------------
-constexpr uint32_t WALK_POOL = 32;
-
-// The rest of a line's walk from its current state (it steps taken):
-// walk_line's loop with the job's callbacks, then job.end.
+// The rest of a line's walk from its current state: walk_line's loop with
+// the job's callbacks, then job.end.
 template <class Job>
-__device__ __forceinline__ void walk_rest(const Walk& w, WalkState& s, int ty_prev, uint32_t it, Job& job) {
+__device__ __forceinline__ void walk_one(const Walk& w, WalkState& s, Job& job) {
+    int ty_prev = div8(s.y);
     bool capped = false;
-    for (;;) {
+    for (uint32_t it = 0;;) {
         job.cell(w, s);
         const bool done = walk_step(w, s);
-        job.visit(s.x, s.y);
         const int ty = div8(s.y);
         if (ty != ty_prev) {
             job.cross(div8(s.x), min(ty_prev, ty), (int)(int8_t)(int16_t)(ty - ty_prev));
@@ -208,249 +194,191 @@ __device__ __forceinline__ void walk_rest(const Walk& w, WalkState& s, int ty_pr
     job.end(capped);
 }
 
-template <class Job>
-__device__ __forceinline__ void walk_refill(uint64_t n_lines, const uint32_t* __restrict__ queue, uint32_t* ticket,
-                                            uint32_t refill, Job& job) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t below = (1u << lane) - 1u;
-    uint64_t pool = 0, pool_end = 0;   // warp-uniform
-    bool more = true;                  // warp-uniform
-    bool live = false;
-    Walk w;
-    WalkState s;
-    int ty_prev = 0;
-    uint32_t it = 0;
-    for (;;) {
-        uint32_t idle = __ballot_sync(0xffffffffu, !live);
-        if (more && (uint32_t)__popc(idle) >= refill) {
-            while (idle != 0u) {
-                if (pool == pool_end) {
-                    uint32_t b = 0;
-                    if (lane == 0) b = atomicAdd(ticket, 1u);
-                    const uint64_t first = (uint64_t)__shfl_sync(0xffffffffu, b, 0) * WALK_POOL;
-                    if (first >= n_lines) {
-                        more = false;
-                        break;
-                    }
-                    pool = first;
-                    pool_end = min(first + WALK_POOL, n_lines);
-                }
-                const uint32_t avail = (uint32_t)(pool_end - pool);
-                const uint32_t rank = (uint32_t)__popc(idle & below);
-                if (((idle >> lane) & 1u) && rank < avail) {
-                    live = job.begin(queue[pool + rank], w, s);
-                    if (live) {
-                        ty_prev = div8(s.y);
-                        it = 0;
-                        job.visit(s.x, s.y);
-                    }
-                }
-                pool += min((uint32_t)__popc(idle), avail);
-                idle = __ballot_sync(0xffffffffu, !live);
-            }
-        }
-        if (!more) {
-            // nothing left to take: the live lanes finish their lines without
-            // the per-step votes (the last, longest walks set the kernel's end)
-            if (live) walk_rest(w, s, ty_prev, it, job);
-            break;
-        }
-        if (__ballot_sync(0xffffffffu, live) == 0u) continue;
-        if (live) {
-            job.cell(w, s);
-            bool done = walk_step(w, s);
-            job.visit(s.x, s.y);
-            const int ty = div8(s.y);
-            if (ty != ty_prev) {
-                job.cross(div8(s.x), min(ty_prev, ty), (int)(int8_t)(int16_t)(ty - ty_prev));
-                ty_prev = ty;
-            }
-            bool capped = false;
-            if (!done && ++it >= WALK_CAP) {
-                capped = true;
-                done = true;
-            }
-            if (done) {
-                job.end(capped);
-                live = false;
-            }
-        }
-    }
-}
+// ---------------------------------------------------------------------
+// Long lines: a group of G lanes per line.
+//
+// Walk lengths run from one cell to thousands (a path's long edges).  One
+// thread per line, as the count and emit kernels walk most lines, would give
+// a long line's warp one busy lane for thousands of steps, every cell's work
+// (two points on the line, area, tile, entry, stores) in one dependent chain.
+// The flatten stage queues every line of more than `long_cells` (estimated)
+// cells, and the walkers below take G cells of a line per round: only the
+// reference's two recurrences are serial (row_t1 and col_t1, one compare, one
+// add and one min per step, run alike by every lane of the group), each lane
+// keeps the parameter of its own step, and the work of the G cells is then
+// done side by side.  Where a cell lies follows from the row steps before it
+// (a bit mask of the round).
+//
+// Against one thread per line with idle lanes refilled: a document of 415
+// paths (65,417 lines) 285 -> 42 us, one path of 2,093 lines 54 -> 15 us.
+// ---------------------------------------------------------------------
+template <int G>
+struct GroupLine {
+    // the line, the same in every lane of the group
+    V2 a, p;
+    int x_dir, y_dir, end_x, end_y;
+    float x_step, y_step;
+    // the walk before the round's first cell
+    float row, col;      // row_t1, col_t1
+    float t;             // where that cell begins
+    int x, y;            // that cell
+    bool seen_row, seen_col;   // a row / column step was taken
+    uint32_t it;         // cells walked
+    bool live;
 
-// One line whose walk job.begin has set up.
-template <class Job>
-__device__ __forceinline__ void walk_one(Walk& w, WalkState& s, Job& job) {
-    job.visit(s.x, s.y);
-    walk_rest(w, s, div8(s.y), 0u, job);
-}
-
-// Counts of the count pass (see k_line_count) for a queued line, per lane.
-// The raster boxes and crossing-sign sums gather over the lane's lines of one
-// raster and go to memory when the lane moves to another raster.
-struct CountJob {
-    const float4* lines;
-    const uint32_t* line_raster;
-    uint32_t* counts;
-    uint32_t* inc_counts;
-    int4* bbox;
-    int* raster_wsum;
-    uint32_t* err;
-    // the line
-    uint32_t line, nb, nc, nx, run;
-    int ptx, pty, ws;
-    // the lane's current raster
-    uint32_t r;
-    BBoxAcc bb;
-    int wsr;
-    uint64_t incs;   // increments of the lane's lines
-
-    __device__ __forceinline__ void flush() {
-        if (r == 0xffffffffu) return;
-        if (bb.x0 <= bb.x1) box_grow(bbox + r, bb.x0, bb.y0, bb.x1, bb.y1);
-        if (wsr) atomicAdd(raster_wsum + r, wsr);
-    }
-    __device__ __forceinline__ bool begin(uint32_t i, Walk& w, WalkState& s) {
-        const float4 l = lines[i];
-        const uint32_t ri = line_raster[i];
-        if (ri != r) {
-            flush();
-            r = ri;
-            bb = BBoxAcc{0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000};
-            wsr = 0;
-        }
-        const V2 a = v2(l.x, l.y), p = v2(l.z, l.w);
-        if (veq(a, p)) {
-            counts[i] = 0u;
-            inc_counts[i] = 0u;
-            return false;
-        }
-        walk_setup(a, p, w, s);
-        line = i;
-        nb = nc = nx = run = 0u;
-        ptx = pty = 0x7fffffff;
-        ws = 0;
-        return true;
-    }
-    __device__ __forceinline__ void cell(const Walk&, const WalkState& s) {
-        const int tx = div8(s.x), ty = div8(s.y);
-        if (tx != ptx || ty != pty || run == BIN_MAX_CELLS) {
-            nb++;
-            ptx = tx;
-            pty = ty;
-            run = 0;
-        }
-        run++;
-        nx++;
-    }
-    __device__ __forceinline__ void visit(int x, int y) { bbox_add(bb, x, y); }
-    __device__ __forceinline__ void cross(int, int, int sign) {
-        nc++;
-        ws += sign;
-    }
-    __device__ __forceinline__ void end(bool capped) {
-        counts[line] = nb + nc;
-        inc_counts[line] = nx;
-        incs += nx;
-        wsr += ws;
-        if (capped) atomicOr(err, ERR_LIMIT);
+    __device__ __forceinline__ void begin(V2 from, V2 to) {
+        Walk w;
+        WalkState s;
+        walk_setup(from, to, w, s);
+        a = from;
+        p = to;
+        x_dir = w.x_dir;
+        y_dir = w.y_dir;
+        end_x = w.end_x;
+        end_y = w.end_y;
+        x_step = w.x_step;
+        y_step = w.y_step;
+        row = s.row_t1;
+        col = s.col_t1;
+        t = 0.0f;
+        x = s.x;
+        y = s.y;
+        seen_row = seen_col = false;
+        it = 0;
+        live = true;
     }
 };
+// What a round leaves in each lane (cell c = lane within the group), and its
+// totals for the group.
+struct GroupCell {
+    bool valid;          // the cell exists
+    float t0, t1;        // where the line enters and leaves it
+    int x, y;            // the cell
+    int nx, ny;          // the cell visited next (the snapped end cell after the last one)
+    uint32_t row_bits;   // bit k: the step out of cell k went to another row (group)
+    uint32_t m;          // cells of the round (group)
+    bool fin;            // the walk ends in this round (group)
+    bool capped;         // ... because it reached WALK_CAP (group)
+};
 
-// The queued long lines' counts (see k_line_count): persistent blocks of
-// refilled lanes (walk_refill).
+// The next G cells of every group's line (walk_line's steps, common.cuh; all
+// lanes of the warp call it, dead groups get no valid cell).
+template <int G>
+__device__ __forceinline__ void group_round(GroupLine<G>& L, GroupCell& q) {
+    const uint32_t lane = threadIdx.x & 31u, c = lane & (G - 1), gshift = lane & ~(uint32_t)(G - 1);
+    constexpr uint32_t ALL = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+    float mine = 0.0f;
+    uint32_t rows = 0;
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+        const bool r = L.row < L.col;   // ties step x
+        const float t = r ? L.row : L.col;
+        if (c == (uint32_t)k) mine = t;
+        if (r) rows |= 1u << k;
+        const float rn = rmin(__fadd_rn(L.row, L.y_step), 1.0f), cn = rmin(__fadd_rn(L.col, L.x_step), 1.0f);
+        L.row = r ? rn : L.row;
+        L.col = r ? L.col : cn;
+    }
+    // the walk ends with the first step at t == 1 (steps past it are not used)
+    const uint32_t ends = (__ballot_sync(0xffffffffu, mine == 1.0f) >> gshift) & ALL;
+    q.m = L.live ? (ends ? (uint32_t)__ffs(ends) : (uint32_t)G) : 0u;
+    q.capped = !ends && L.it + q.m >= WALK_CAP;
+    q.fin = ends != 0u || q.capped;
+    q.valid = c < q.m;
+    q.row_bits = rows;
+    const uint32_t lt = (1u << c) - 1u;
+    const int steps_y = __popc(rows & lt), steps_x = (int)c - steps_y;
+    q.x = wrap16(L.x + L.x_dir * steps_x);
+    q.y = wrap16(L.y + L.y_dir * steps_y);
+    q.t1 = mine;
+    const float before = __shfl_up_sync(0xffffffffu, mine, 1, G);
+    // max(row_t0, col_t0): the last step's parameter, and 0 for an axis not
+    // stepped along yet
+    q.t0 = c == 0 ? L.t : before;
+    if (!((L.seen_row || (rows & lt)) && (L.seen_col || (~rows & lt)))) q.t0 = rmax(q.t0, 0.0f);
+    const bool r = (rows >> c) & 1u;
+    q.nx = r ? q.x : wrap16(q.x + L.x_dir);
+    q.ny = r ? wrap16(q.y + L.y_dir) : q.y;
+    if (mine == 1.0f) {
+        q.nx = L.end_x;
+        q.ny = L.end_y;
+    }
+}
+// The line after the round.
+template <int G>
+__device__ __forceinline__ void group_advance(GroupLine<G>& L, const GroupCell& q) {
+    const int last = (int)q.m - 1;
+    L.t = __shfl_sync(0xffffffffu, q.t1, max(last, 0), G);
+    L.x = __shfl_sync(0xffffffffu, q.nx, max(last, 0), G);
+    L.y = __shfl_sync(0xffffffffu, q.ny, max(last, 0), G);
+    if (q.m) {
+        L.seen_row = L.seen_row || q.row_bits != 0u;
+        L.seen_col = L.seen_col || q.row_bits != (G == 32 ? 0xffffffffu : (1u << G) - 1u);
+    }
+    L.it += q.m;
+    if (q.fin) L.live = false;
+}
+// Lanes per line: a line alone in its warp takes the fewest cycles a cell
+// (its recurrences plus 1/32 of the cells' work), which is what counts while
+// warps are idle; where there are more lines than warps, four share one and
+// the warp does less work per cell.
+__device__ __forceinline__ bool long_lines_share(uint32_t n_queue) {
+    return n_queue > gridDim.x * (blockDim.x >> 5);
+}
+
 constexpr int LONG_THREADS = 128;
 constexpr uint32_t LONG_BLOCKS_PER_SM = 2;
-__global__ void __launch_bounds__(LONG_THREADS) k_line_count_long(
-    const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster, uint32_t n_cap, const uint32_t* n_dev,
-    int4* bbox, int* raster_wsum, uint32_t* __restrict__ counts, uint32_t* __restrict__ inc_counts,
-    unsigned long long* inc_total, const uint32_t* __restrict__ queue, const uint32_t* n_queue, uint32_t* ticket,
-    uint32_t refill, uint32_t* err) {
-    // (a line count zeroed on the device, after an overflow of a graph's
-    // plan, stops these walks too)
-    if (dev_count(n_cap, n_dev) == 0) return;
-    CountJob job;
-    job.lines = lines;
-    job.line_raster = line_raster;
-    job.counts = counts;
-    job.inc_counts = inc_counts;
-    job.bbox = bbox;
-    job.raster_wsum = raster_wsum;
-    job.err = err;
-    job.r = 0xffffffffu;
-    job.bb = BBoxAcc{0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000};
-    job.wsr = 0;
-    job.incs = 0;
-    walk_refill(*n_queue, queue, ticket, refill, job);
-    job.flush();
-    unsigned long long t = job.incs;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if ((threadIdx.x & 31u) == 0u && t) atomicAdd(inc_total, t);
-}
 
 // Entry counts per line (written in place of the offsets, then scanned)
 // and the raster tile boxes.  Counting is a separate kernel, not folded into
-// the offset scan: a walk's length varies from one cell to thousands, and a
-// single-pass scan would hold every later block behind the slowest walk.
-// Persistent warps over windows (see order_window); lines of more than
-// long_cells cells are left to k_line_count_long.  Boxes (and the rasters'
-// crossing-sign sums) are reduced before any global atomic: lanes of one
-// raster by warp reductions, then the window's first BOX_SLOTS rasters (lines
-// of a raster are contiguous) in the warp's shared slots; each global box is
-// then updated only where it grows.
+// the offset scan: a count's length varies from no step to thousands, and a
+// single-pass scan would hold every later block behind the slowest one.
+// Persistent warps take windows of `groups` times 32 consecutive lines by
+// ticket (more than one group only where there are lines enough to fill the
+// GPU).  Boxes (and the rasters' crossing-sign sums) are reduced before any
+// global atomic: lanes of one raster by warp reductions, then the window's
+// first BOX_SLOTS rasters (lines of a raster are contiguous) in the warp's
+// shared slots; each global box is then updated only where it grows.
+constexpr int COUNT_GROUPS_MAX = 8;
+constexpr int WALK_BLOCK = 128;
 constexpr int BOX_SLOTS = 8;
 __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restrict__ lines,
                                                            const uint32_t* __restrict__ line_raster, uint32_t n_cap,
-                                                           const uint32_t* n_dev, int4* bbox, int* raster_wsum,
-                                                           uint32_t* __restrict__ counts,
+                                                           const uint32_t* n_dev, uint32_t groups, int4* bbox,
+                                                           int* raster_wsum, uint32_t* __restrict__ counts,
                                                            uint32_t* __restrict__ inc_counts,
-                                                           unsigned long long* inc_total, uint32_t long_cells,
-                                                           uint32_t* ticket, uint32_t* err) {
+                                                           unsigned long long* inc_total, uint32_t* ticket,
+                                                           uint32_t* err) {
     constexpr int WARPS = WALK_BLOCK / 32;
     __shared__ int4 s_box[WARPS][BOX_SLOTS];
     __shared__ int s_ws[WARPS][BOX_SLOTS];
-    __shared__ uint32_t s_cnt[WARPS][LEN_GROUPS];
-    __shared__ uint16_t s_item[WARPS][WIN];
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint64_t n_lines = dev_count(n_cap, n_dev);
     unsigned long long incs = 0;   // the warp's increments (lane 0)
     for (;;) {
-        const uint64_t i0 = next_window(ticket);
+        const uint64_t i0 = next_window(ticket) * (32u * groups);
         if (i0 >= n_lines) break;
-        uint32_t cells[WIN_PER_LANE];
-#pragma unroll
-        for (int j = 0; j < WIN_PER_LANE; j++) {
-            const uint64_t i = i0 + j * 32 + lane;
-            cells[j] = i < n_lines ? walk_cells(lines[i]) : 0u;
-        }
-        order_window(cells, s_cnt[wid], s_item[wid]);
         if (lane < BOX_SLOTS) {
             s_box[wid][lane] = make_int4(0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000);
             s_ws[wid][lane] = 0;
         }
         const uint32_t r0 = line_raster[i0];
         __syncwarp();
-        for (int j = 0; j < WIN_PER_LANE; j++) {
-            const uint64_t i = i0 + s_item[wid][j * 32 + lane];
-            BBoxAcc bb{0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000};
+        for (uint32_t j = 0; j < groups; j++) {
+            const uint64_t i = i0 + j * 32u + lane;
+            LineCount n{0u, 0u, 0, {0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000}};
             uint32_t r = r0;
-            int ws = 0;
-            uint32_t nc = 0;
             if (i < n_lines) {
                 const float4 l = lines[i];
-                if (!(long_cells && walk_cells(l) > long_cells)) {
-                    bool capped = false;
-                    counts[i] = count_line(v2(l.x, l.y), v2(l.z, l.w), bb, &capped, &ws, &nc);
-                    inc_counts[i] = nc;
-                    if (capped) atomicOr(err, ERR_LIMIT);
-                    r = line_raster[i];
-                }
+                r = line_raster[i];
+                n = count_line(v2(l.x, l.y), v2(l.z, l.w), err);
+                counts[i] = n.ent;
+                inc_counts[i] = n.cells;
             }
             const unsigned grp = __match_any_sync(0xffffffffu, r);
-            const int x0 = __reduce_min_sync(grp, bb.x0), y0 = __reduce_min_sync(grp, bb.y0);
-            const int x1 = __reduce_max_sync(grp, bb.x1), y1 = __reduce_max_sync(grp, bb.y1);
-            const int wsg = __reduce_add_sync(grp, ws);
+            const int x0 = __reduce_min_sync(grp, n.box.x0), y0 = __reduce_min_sync(grp, n.box.y0);
+            const int x1 = __reduce_max_sync(grp, n.box.x1), y1 = __reduce_max_sync(grp, n.box.y1);
+            const int wsg = __reduce_add_sync(grp, n.wsum);
             if ((int)lane == __ffs(grp) - 1) {
                 if (r - r0 < (uint32_t)BOX_SLOTS) {
                     if (x0 <= x1) {
@@ -467,7 +395,7 @@ __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restr
                 }
             }
             // (at most 32 capped walks: 32 bits hold it)
-            incs += __reduce_add_sync(0xffffffffu, nc);
+            incs += __reduce_add_sync(0xffffffffu, n.cells);
         }
         __syncwarp();
         if (lane < BOX_SLOTS) {
@@ -642,7 +570,6 @@ struct EmitJob {
         prev_x = s.x;
         bcount++;
     }
-    __device__ __forceinline__ void visit(int, int) {}
     __device__ __forceinline__ void cross(int tx, int ty, int sign) {
         const uint32_t c = e++;
         keys[c] = make_key<K>(base, bb, tx, ty, 0u);
@@ -654,36 +581,155 @@ struct EmitJob {
     }
 };
 
-// The queued long lines' entries and increments (see k_line_emit):
-// persistent blocks of refilled lanes (walk_refill).
+// Entries and increments of queued lines (see k_line_emit and EmitJob, whose
+// entries in the same order these are).
+template <int G, class K>
+__device__ __forceinline__ void emit_long(const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster,
+                                          const uint32_t* __restrict__ ent_off, const uint32_t* __restrict__ inc_off,
+                                          const int4* __restrict__ bbox, const uint64_t* __restrict__ key_base,
+                                          K* __restrict__ keys, uint32_t* __restrict__ vals, BinRec* __restrict__ bins,
+                                          float2* __restrict__ incs, const uint32_t* __restrict__ queue,
+                                          uint32_t n_queue, uint32_t* ticket) {
+    const uint32_t lane = threadIdx.x & 31u, c = lane & (G - 1), gshift = lane & ~(uint32_t)(G - 1);
+    constexpr uint32_t ALL = G == 32 ? 0xffffffffu : (1u << G) - 1u;
+    const uint32_t lt = (1u << c) - 1u;
+    GroupLine<G> L;
+    L.begin(v2(0.0f, 0.0f), v2(1.0f, 1.0f));
+    L.live = false;
+    bool more = true;
+    // the group's line: raster, key of tile (0, 0) and tile columns, next entry, next increment
+    uint32_t r = 0, e = 0, inc = 0;
+    K key0 = 0, cols = 0;
+    // the bin left open by the round before: its entry, first increment, first
+    // cell, cells and steps so far (n 0: none; else the next cell is in it)
+    uint32_t o_entry = 0, o_inc = 0, o_xy = 0, o_n = 0, o_steps = 0;
+    for (;;) {
+        if (more && !L.live) {
+            more = false;   // until a line is taken
+            const uint32_t gmask = ALL << gshift;
+            uint32_t k = 0;
+            // (lanes of a group agree on more and live)
+            if (c == 0) k = atomicAdd(ticket, 1u);
+            k = __shfl_sync(gmask, k, 0, G);
+            if (k < n_queue) {
+                more = true;
+                const uint32_t i = queue[k];
+                const float4 l = lines[i];
+                r = line_raster[i];
+                e = ent_off[i];
+                inc = inc_off[i];
+                const int4 bb = bbox[r];
+                cols = (K)(bb.z - bb.x + 1);
+                key0 = (K)key_base[r] - (((K)(int64_t)bb.y * cols + (K)(int64_t)bb.x) << 1);
+                L.begin(v2(l.x, l.y), v2(l.z, l.w));
+                o_n = 0;
+            }
+        }
+        __syncwarp();
+        if (__ballot_sync(0xffffffffu, L.live) == 0u) {
+            if (__ballot_sync(0xffffffffu, more) == 0u) break;
+            continue;
+        }
+        GroupCell q;
+        group_round<G>(L, q);
+        if (q.valid) {
+            // walk_increment (rasterizer.rs:98-106)
+            const V2 p0 = vlerp(q.t0, L.a, L.p), p1 = vlerp(q.t1, L.a, L.p);
+            const float height = __fsub_rn(p1.y, p0.y);
+            const float right = (float)wrap16(q.x + 1);
+            const float area =
+                __fmul_rn(__fmul_rn(0.5f, height), __fadd_rn(__fsub_rn(right, p0.x), __fsub_rn(right, p1.x)));
+            incs[inc + c] = make_float2(area, height);
+        }
+        const int tx = div8(q.x), ty = div8(q.y), nty = div8(q.ny);
+        const int tile = (int)(((uint32_t)ty << 16) | ((uint32_t)tx & 0xffffu));
+        const int before = __shfl_up_sync(0xffffffffu, tile, 1, G);
+        const bool new_bin = q.valid && (c == 0 ? o_n == 0 : tile != before);
+        const bool cross = q.valid && nty != ty;
+        const uint32_t B = (__ballot_sync(0xffffffffu, new_bin) >> gshift) & ALL;
+        const uint32_t X = (__ballot_sync(0xffffffffu, cross) >> gshift) & ALL;
+        // a cell's bin opens before its crossing
+        const uint32_t mine = e + (uint32_t)__popc(B & lt) + (uint32_t)__popc(X & lt);
+        auto key_of = [&](int kx, int ky, K kind) {
+            return key0 + (((K)(int64_t)ky * cols + (K)(int64_t)kx) << 1) + kind;
+        };
+        if (cross) {
+            const uint32_t x = mine + (new_bin ? 1u : 0u);
+            keys[x] = key_of(div8(q.nx), min(ty, nty), (K)0);
+            vals[x] = CROSS_TAG | (r << 8) | ((uint32_t)(nty - ty) & 0xffu);
+        }
+        // runs: a lane that opens a bin owns it, and lane 0 the one left open
+        // by the round before; the round's last run stays open if the walk
+        // goes on in its tile
+        // (the shuffle is every lane's, ended groups' too)
+        const int next_same = __shfl_sync(0xffffffffu, div8(q.nx) == tx && nty == ty ? 1 : 0, (int)max(q.m, 1u) - 1, G);
+        const bool goes_on = !q.fin && next_same != 0;
+        const uint32_t cells = q.m == 32u ? 0xffffffffu : (1u << q.m) - 1u;
+        const uint32_t xsteps = ~q.row_bits & cells;
+        const bool carried = c == 0 && o_n != 0;
+        const uint32_t after = (B >> c) >> 1;   // bins opened by later cells
+        const uint32_t run = after ? (uint32_t)__ffs(after) : q.m - c;
+        const bool owner = q.valid && (new_bin || carried);
+        const bool stays = owner && !after && goes_on;
+        const uint32_t have = carried ? o_n : 0u;
+        const uint32_t n = have + run;
+        const uint32_t in_run = run >= 32u ? 0xffffffffu : (1u << run) - 1u;
+        // steps out of the run's cells; the last one leaves the bin unless it stays open
+        const uint32_t steps = (carried ? o_steps : 0u) | (((xsteps >> c) & (stays ? in_run : in_run >> 1)) << have);
+        const uint32_t xy = carried ? o_xy : ((uint32_t)(uint16_t)(int16_t)q.x | ((uint32_t)(uint16_t)(int16_t)q.y << 16));
+        const uint32_t at = carried ? o_entry : mine, first = carried ? o_inc : inc + c;
+        if (owner && !stays) {
+            BinRec rec;
+            rec.inc = first;
+            rec.raster = r;
+            rec.x = (int16_t)(xy & 0xffffu);
+            rec.y = (int16_t)(xy >> 16);
+            rec.steps = (uint16_t)steps;
+            rec.n = (uint8_t)n;
+            rec.dirs = (uint8_t)((L.x_dir < 0 ? 1u : 0u) | (L.y_dir < 0 ? 2u : 0u));
+            *reinterpret_cast<uint4*>(bins + at) = *reinterpret_cast<const uint4*>(&rec);
+            keys[at] = key_of(tx, ty, (K)1);   // (the owner's cell lies in the bin's tile)
+            vals[at] = at;
+        }
+        const uint32_t open = (__ballot_sync(0xffffffffu, stays) >> gshift) & ALL;   // at most one
+        const int src = open ? __ffs(open) - 1 : 0;
+        o_entry = __shfl_sync(0xffffffffu, at, src, G);
+        o_inc = __shfl_sync(0xffffffffu, first, src, G);
+        o_xy = __shfl_sync(0xffffffffu, xy, src, G);
+        o_steps = __shfl_sync(0xffffffffu, steps, src, G);
+        o_n = __shfl_sync(0xffffffffu, n, src, G);
+        if (!open) o_n = 0;
+        e += (uint32_t)__popc(B) + (uint32_t)__popc(X);
+        inc += q.m;
+        group_advance<G>(L, q);
+        __syncwarp();
+    }
+}
+
+// The queued long lines' entries and increments (see k_line_emit).
 template <class K>
 __global__ void __launch_bounds__(LONG_THREADS) k_line_emit_long(
     const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster, const uint32_t* __restrict__ ent_off,
     const uint32_t* __restrict__ inc_off, uint64_t n_cap, const uint32_t* n_dev, const int4* __restrict__ bbox,
     const uint64_t* __restrict__ key_base, K* __restrict__ keys, uint32_t* __restrict__ vals,
     BinRec* __restrict__ bins, float2* __restrict__ incs, const uint32_t* __restrict__ queue, const uint32_t* n_queue,
-    uint32_t* ticket, uint32_t refill) {
+    uint32_t* ticket) {
     // (a line count zeroed on the device, after an overflow of a graph's
     // plan, stops these walks too: their offsets were not written)
     if (dev_count(n_cap, n_dev) == 0) return;
-    EmitJob<K> job;
-    job.lines = lines;
-    job.line_raster = line_raster;
-    job.ent_off = ent_off;
-    job.inc_off = inc_off;
-    job.bbox = bbox;
-    job.key_base = key_base;
-    job.keys = keys;
-    job.vals = vals;
-    job.bins = bins;
-    job.incs = incs;
-    job.r = 0xffffffffu;
-    walk_refill(*n_queue, queue, ticket, refill, job);
+    const uint32_t n = *n_queue;
+    if (long_lines_share(n))
+        emit_long<8, K>(lines, line_raster, ent_off, inc_off, bbox, key_base, keys, vals, bins, incs, queue, n, ticket);
+    else
+        emit_long<32, K>(lines, line_raster, ent_off, inc_off, bbox, key_base, keys, vals, bins, incs, queue, n, ticket);
 }
 
 // Every thread walks one line, the lines of a block in order of length
 // (order_by_length) so a warp's lanes walk lines of about the same length.
-// Lines of more than long_cells cells are left to k_line_emit_long.
+// Lines of more than long_cells cells are left to k_line_emit_long (default
+// 96: on 20,000 strokes a call takes 4.93 / 4.84 / 4.79 / 4.79 / 4.84 ms at 48 /
+// 64 / 96 / 128 / 192, a document of 415 paths 0.824 .. 0.828 ms up to 96 and
+// 0.852 at 192; one path, shapes and the uneven mix do not care).
 template <class K>
 __global__ void __launch_bounds__(256) k_line_emit(const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster,
                             const uint32_t* __restrict__ ent_off, const uint32_t* __restrict__ inc_off, uint64_t n_cap,
@@ -771,19 +817,21 @@ static cudaError_t join_walks(ochre_gpu_ctx* ctx, cudaStream_t side, cudaStream_
     return e;
 }
 
-// Persistent grid of a windowed walk kernel: the blocks the GPU keeps
-// resident, or fewer when there are fewer windows than warps.
-template <class Kernel>
-static unsigned window_grid(ochre_gpu_ctx* ctx, Kernel kernel, uint64_t n_lines) {
+// Persistent grid of the count kernel and the 32-line groups of its windows:
+// the blocks the GPU keeps resident, with larger windows (fewer updates of
+// the rasters' boxes) only where every resident warp still gets one.
+static void count_shape(ochre_gpu_ctx* ctx, uint64_t n_lines, unsigned* grid, uint32_t* groups) {
     int sms = 152, occ = 1;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, WALK_BLOCK, 0) != cudaSuccess || occ < 1) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_line_count, WALK_BLOCK, 0) != cudaSuccess || occ < 1) {
         cudaGetLastError();
         occ = 1;
     }
-    const uint64_t windows = (n_lines + WIN - 1) / WIN;
+    const uint64_t warps = (uint64_t)sms * (uint64_t)occ * (WALK_BLOCK / 32);
+    *groups = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(COUNT_GROUPS_MAX, n_lines / (32 * warps)));
+    const uint64_t windows = (n_lines + 32ull * *groups - 1) / (32ull * *groups);
     const uint64_t blocks = (windows + WALK_BLOCK / 32 - 1) / (WALK_BLOCK / 32);
-    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)sms * (uint64_t)occ));
+    *grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, warps / (WALK_BLOCK / 32)));
 }
 
 int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaStream_t s, uint64_t* n_entries,
@@ -808,10 +856,9 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
                   "layout");
     OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->line_ent_total, 0, 24, s));
     OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->line_ticket, 0, 4, s));
-    // long-line walkers: persistent, LONG_BLOCKS_PER_SM blocks per SM (each
-    // refills its lanes from the queue)
+    // long-line walkers: persistent, LONG_BLOCKS_PER_SM blocks per SM (their
+    // groups take lines from the queue)
     const uint32_t long_cells = (uint32_t)ctx->tune_chain_long_cells;
-    const uint32_t refill = (uint32_t)ctx->tune_chain_walk_refill;
     uint32_t long_blocks = 0;
     if (long_cells) {
         int sms = 152;
@@ -826,22 +873,15 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
         OCHRE_CUDA_TRY(ctx->line_ent_off.ensure((size_t)n_lines * 4));
         OCHRE_CUDA_TRY(ctx->line_inc_off.ensure((size_t)n_lines * 4));
         OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(n_lines) * sizeof(ScanStatus<LinePair>)));
-        cudaStream_t side = s;
-        if (long_blocks) {
-            OCHRE_CUDA_TRY(fork_walks(ctx, s, &side));
-            OCHRE_LAUNCH(ctx, "dda_count_long", side, k_line_count_long<<<long_blocks, LONG_THREADS, 0, side>>>(
-                ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), n_lines, lines_dev,
-                ctx->raster_bbox.as<int4>(), ctx->raster_wsum.as<int>(), ctx->line_ent_off.as<uint32_t>(),
-                ctx->line_inc_off.as<uint32_t>(), reinterpret_cast<unsigned long long*>(&ds->inc_total), queue,
-                &ds->n_long, &ds->walk_ticket[0], refill, &ds->err));
-            OCHRE_CUDA_TRY(cudaGetLastError());
-        }
-        OCHRE_LAUNCH(ctx, "dda_count", s, k_line_count<<<window_grid(ctx, k_line_count, n_lines), WALK_BLOCK, 0, s>>>(
-            ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
+        unsigned count_grid = 1;
+        uint32_t groups = 1;
+        count_shape(ctx, n_lines, &count_grid, &groups);
+        OCHRE_LAUNCH(ctx, "dda_count", s, k_line_count<<<count_grid, WALK_BLOCK, 0, s>>>(
+            ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), n_lines, lines_dev, groups,
+            ctx->raster_bbox.as<int4>(),
             ctx->raster_wsum.as<int>(), ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>(),
-            reinterpret_cast<unsigned long long*>(&ds->inc_total), long_cells, &ds->line_ticket, &ds->err));
+            reinterpret_cast<unsigned long long*>(&ds->inc_total), &ds->line_ticket, &ds->err));
         OCHRE_CUDA_TRY(cudaGetLastError());
-        OCHRE_CUDA_TRY(join_walks(ctx, side, s));
         // in place: every count is read by the thread that writes its offset
         OCHRE_LAUNCH(ctx, "dda_offset_scan", s, OCHRE_CUDA_TRY(launch_scan<LinePair>(
             n_lines, LinePairIn{ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>()},
@@ -902,13 +942,13 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint64_t>(), ctx->vals.as<uint32_t>(),
-                ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), queue, &ds->n_long, &ds->walk_ticket[1], refill));
+                ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), queue, &ds->n_long, &ds->walk_ticket));
         else if (long_blocks)
             OCHRE_LAUNCH(ctx, "dda_emit_long", side, k_line_emit_long<uint32_t><<<long_blocks, LONG_THREADS, 0, side>>>(
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),
-                ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), queue, &ds->n_long, &ds->walk_ticket[1], refill));
+                ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), queue, &ds->n_long, &ds->walk_ticket));
         if (ctx->keys64)
             OCHRE_LAUNCH(ctx, "dda_emit", s, k_line_emit<uint64_t><<<(unsigned)((n_lines + 255) / 256), 256, 0, s>>>(
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) k_count_each(uint64_t n, In in, uint32_t*
 constexpr uint64_t SPLIT_COUNT_TILES = 256;
 
 // Lines of more than long_cells cells (walk_cells) are also queued for the
-// long-line walkers of the DDA stage (long_cells 0: none are).
+// long-line emit walk of the DDA stage (long_cells 0: none are).
 __global__ void k_cmd_emit(BatchView b, const uint32_t* __restrict__ line_off, uint32_t n_lines_cap,
                            float4* __restrict__ lines, uint32_t* __restrict__ line_raster, uint32_t long_cells,
                            uint32_t* __restrict__ long_lines, uint32_t* n_long, uint32_t* err) {

@@ -74,7 +74,8 @@ struct DevScalars {
     uint32_t n_incs;          // chain: pixel-cell increments of the lines } pair total)
     uint64_t inc_total;       // the same increment count summed in 64 bits (the pair
                               // total wraps above 2^32; this one says when it did)
-    uint32_t walk_ticket[2];  // long-line pools handed out in the count and emit walks
+    uint32_t walk_ticket;     // long lines handed out in the emit walk
+    uint32_t pad6;
     uint32_t n_long;          // lines queued for the long-line walkers (flatten)
     uint32_t pad4;
     uint32_t line_ticket;     // line windows handed out in the count walk
@@ -257,8 +258,8 @@ struct ochre_gpu_ctx {
     int tune_chain_tiles_per_warp = 8;
     int tune_chain_coverage_form = 0;   // 0: by row count, 1: block form, 2: row form
     int tune_sort_digit_bits = 8;       // radix sort digit width: 8 or 11
-    int tune_chain_long_cells = 192;    // lines of more (estimated) cells go to the long-line walkers; 0: none
-    int tune_chain_walk_refill = 8;     // idle lanes of a long-line warp that trigger a refill (1..32)
+    int tune_chain_long_cells = 96;     // lines of more (estimated) cells go to the long-line walkers; 0: none
+    int tune_chain_walk_refill = 8;     // accepted and kept for callers that set it; nothing reads it
 
     // Host-batch entry: a large point array is copied on copy_stream while
     // the first stages run; pts_pending until a stage that reads points has
@@ -267,7 +268,7 @@ struct ochre_gpu_ctx {
     cudaEvent_t ev_prior = nullptr, ev_pts = nullptr;
     bool pts_pending = false;
     // The chain's long-line walkers run on walk_stream beside the per-line
-    // walks (forked from and joined to the run's stream by the two events),
+    // emit walk (forked from and joined to the run's stream by the two events),
     // or on the run's stream itself when no_side_stream is set.
     cudaStream_t walk_stream = nullptr;
     cudaEvent_t ev_walk_fork = nullptr, ev_walk_join = nullptr;
