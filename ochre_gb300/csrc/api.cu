@@ -163,7 +163,48 @@ int read_scalars(ochre_gpu_ctx* ctx, cudaStream_t s) {
     const int st = copy_scalars_async(ctx, s);
     if (st != OCHRE_OK) return st;
     OCHRE_CUDA_TRY(cudaStreamSynchronize(s));
+    if (host_scalars(ctx)->err & ERR_TIMEOUT) ctx->scan_dirty = true;   // blocks left without taking tickets
     return OCHRE_OK;
+}
+
+// Modes: eager on a context of its own: cleared when the buffer is new (or a
+// wait gave up), else not at all.  In a launch chain captured into a graph the
+// tag and the tickets are fixed arguments, so every scan clears its words and
+// its own ticket word; in an arena (no allocation) the words lie where
+// anything may have lain, and the ticket is the run's.
+cudaError_t scan_space(ochre_gpu_ctx* ctx, size_t status_bytes, uint32_t tiles, uint32_t first_ticket, cudaStream_t s,
+                       ScanSpace* out) {
+    constexpr size_t HEAD = 4 * sizeof(uint32_t);   // eager ticket, unused, planned ticket, unused
+    DevBuf& b = ctx->scan_status;
+    constexpr uint32_t PLANNED = (1u << 30) - 1u;   // a tag no eager scan uses
+    out->tag = PLANNED;
+    out->ticket_base = 0u - first_ticket;
+    cudaError_t e;
+    if (b.arena != nullptr) {
+        if ((e = b.ensure(status_bytes)) != cudaSuccess) return e;
+        out->status = b.p;
+        out->ticket = &dev_scalars(ctx)->sort_ticket;   // (.ticket counts the fused kernel's rasters)
+        if ((e = cudaMemsetAsync(b.p, 0, status_bytes, s)) != cudaSuccess) return e;
+        return cudaMemsetAsync(out->ticket, 0, sizeof(uint32_t), s);
+    }
+    void* const before = b.p;
+    if ((e = b.ensure(HEAD + status_bytes)) != cudaSuccess) return e;
+    if (b.p != before || ctx->scan_dirty || ctx->scan_tag + 1u >= PLANNED) {
+        if ((e = cudaMemsetAsync(b.p, 0, b.cap, s)) != cudaSuccess) return e;
+        ctx->scan_tag = 0;
+        ctx->scan_tickets = 0;
+        ctx->scan_dirty = false;
+    }
+    out->status = static_cast<char*>(b.p) + HEAD;
+    if (ctx->plan) {
+        out->ticket = b.as<uint32_t>() + 2;
+        return cudaMemsetAsync(out->ticket, 0, HEAD / 2 + status_bytes, s);
+    }
+    out->ticket = b.as<uint32_t>();
+    out->tag = ++ctx->scan_tag;
+    out->ticket_base = ctx->scan_tickets - first_ticket;
+    ctx->scan_tickets += tiles;
+    return cudaSuccess;
 }
 
 void prof_begin(ochre_gpu_ctx* ctx, const char* name, cudaStream_t s) {

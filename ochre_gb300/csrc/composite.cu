@@ -320,11 +320,9 @@ extern "C" int ochre_gpu_composite(ochre_gpu_ctx* ctx, const ochre_result* res, 
     const PieceItems items{res->tile_xy, res->span_xy, res->span_width, res->raster_tile_off, res->raster_span_off,
                            T, N, n_rasters, (int)w, (int)h, (int)w8};
     OCHRE_CUDA_TRY(ctx->line_ent_off.ensure(S * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(S) * sizeof(ScanStatus<uint32_t>)));
     OCHRE_CUDA_TRY(reset_scalars(ctx, s));
     OCHRE_LAUNCH(ctx, "composite_count", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-        S, PieceCount{items}, PieceOff{ctx->line_ent_off.as<uint32_t>()}, OpSumU32{}, 0u, ctx->scan_status.p,
-        &ds->ticket, &ds->n_line_ent, &ds->err, s)));
+        ctx, S, PieceCount{items}, PieceOff{ctx->line_ent_off.as<uint32_t>()}, OpSumU32{}, 0u, &ds->n_line_ent, s)));
     int st = read_scalars(ctx, s);
     if (st != OCHRE_OK) return st;
     st = check_device_error(ctx);

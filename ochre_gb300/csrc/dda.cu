@@ -872,7 +872,6 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
     if (n_lines) {
         OCHRE_CUDA_TRY(ctx->line_ent_off.ensure((size_t)n_lines * 4));
         OCHRE_CUDA_TRY(ctx->line_inc_off.ensure((size_t)n_lines * 4));
-        OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(n_lines) * sizeof(ScanStatus<LinePair>)));
         unsigned count_grid = 1;
         uint32_t groups = 1;
         count_shape(ctx, n_lines, &count_grid, &groups);
@@ -884,18 +883,15 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
         OCHRE_CUDA_TRY(cudaGetLastError());
         // in place: every count is read by the thread that writes its offset
         OCHRE_LAUNCH(ctx, "dda_offset_scan", s, OCHRE_CUDA_TRY(launch_scan<LinePair>(
-            n_lines, LinePairIn{ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>()},
+            ctx, n_lines, LinePairIn{ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>()},
             LinePairOut{ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>()}, OpLinePair{},
-            LinePair{0u, 0u}, ctx->scan_status.p, &ds->ticket, reinterpret_cast<LinePair*>(&ds->line_ent_total),
-            &ds->err, s, lines_dev)));
+            LinePair{0u, 0u}, reinterpret_cast<LinePair*>(&ds->line_ent_total), s, lines_dev)));
     }
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(R) * sizeof(ScanStatus<RasterScan>)));
     OCHRE_LAUNCH(ctx, "raster_key_scan", s, OCHRE_CUDA_TRY(launch_scan<RasterScan>(
-        R, RasterIn{ctx->raster_bbox.as<int4>(), ctx->raster_wsum.as<int>()},
+        ctx, R, RasterIn{ctx->raster_bbox.as<int4>(), ctx->raster_wsum.as<int>()},
         RasterOut{ctx->raster_bbox.as<int4>(), ctx->raster_keybase.as<uint64_t>(), ctx->raster_empty.as<uint32_t>(),
                   ctx->raster_wbase.as<int>()},
-        OpRaster{}, RasterScan{0, 0, 0}, ctx->scan_status.p, &ds->ticket,
-        reinterpret_cast<RasterScan*>(&ds->keyspace), &ds->err, s)));
+        OpRaster{}, RasterScan{0, 0, 0}, reinterpret_cast<RasterScan*>(&ds->keyspace), s)));
     uint64_t E;
     uint32_t bits;
     uint32_t first_entry = 0;

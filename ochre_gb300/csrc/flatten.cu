@@ -162,14 +162,12 @@ int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uin
     OCHRE_CUDA_TRY(ctx->cmd_mv.ensure(n * 4));
     OCHRE_CUDA_TRY(ctx->cmd_ep.ensure(n * 4));
     OCHRE_CUDA_TRY(ctx->cmd_line_off.ensure(n * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(n) * sizeof(ScanStatus<CmdScan>)));
 
     CmdScan total_id{0, 0, 0};
-    OCHRE_LAUNCH(ctx, "cmd_scan", s, OCHRE_CUDA_TRY(launch_scan<CmdScan>(n, CmdIn{in->verbs, &ds->err},
+    OCHRE_LAUNCH(ctx, "cmd_scan", s, OCHRE_CUDA_TRY(launch_scan<CmdScan>(ctx, n, CmdIn{in->verbs, &ds->err},
                                         CmdOut{ctx->cmd_foff.as<uint32_t>(), ctx->cmd_mv.as<uint32_t>(),
                                                ctx->cmd_ep.as<uint32_t>()},
-                                        OpCmd{}, total_id, ctx->scan_status.p, &ds->ticket,
-                                        reinterpret_cast<CmdScan*>(&ds->n_floats), &ds->err, s)));
+                                        OpCmd{}, total_id, reinterpret_cast<CmdScan*>(&ds->n_floats), s)));
 
     // A command whose points lie beyond the point array is flagged invalid
     // by the kernels that read it (load_cmd), reported at the next read-back.
@@ -187,12 +185,11 @@ int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uin
             n, CountIn{b, &ds->err}, ctx->cmd_line_off.as<uint32_t>()));
         OCHRE_CUDA_TRY(cudaGetLastError());
         OCHRE_LAUNCH(ctx, "flatten_count_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-            n, Load32{ctx->cmd_line_off.as<uint32_t>()}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u,
-            ctx->scan_status.p, &ds->ticket, &ds->n_lines, &ds->err, s)));
+            ctx, n, Load32{ctx->cmd_line_off.as<uint32_t>()}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u,
+            &ds->n_lines, s)));
     } else {
         OCHRE_LAUNCH(ctx, "flatten_count_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-            n, CountIn{b, &ds->err}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u, ctx->scan_status.p,
-            &ds->ticket, &ds->n_lines, &ds->err, s)));
+            ctx, n, CountIn{b, &ds->err}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u, &ds->n_lines, s)));
     }
     uint32_t L;
     if (plan) {

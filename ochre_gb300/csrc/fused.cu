@@ -675,7 +675,6 @@ static int run_fused(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, 
     // float offset of every command (the kernel reads its points there)
     const uint64_t n_cmds = in->n_cmds;
     OCHRE_CUDA_TRY(ctx->cmd_foff.ensure((size_t)std::max<uint64_t>(n_cmds, 1) * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(n_cmds) * sizeof(ScanStatus<uint32_t>)));
     // capacity guess: the last run's totals, else 48 tiles per raster; with
     // caller-provided (fixed) outputs, their capacity
     const bool fixed_out = ctx->out_tile_xy.fixed;
@@ -704,8 +703,8 @@ static int run_fused(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, 
         OCHRE_CUDA_TRY(reset_scalars(ctx, s));
         if (n_cmds)
             OCHRE_LAUNCH(ctx, "fused_float_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-                n_cmds, VerbFloats{in->verbs}, FloatOff{ctx->cmd_foff.as<uint32_t>()}, OpSumU32{}, 0u,
-                ctx->scan_status.p, &ds->sort_ticket, &ds->n_floats, &ds->err, s, nullptr,
+                ctx, n_cmds, VerbFloats{in->verbs}, FloatOff{ctx->cmd_foff.as<uint32_t>()}, OpSumU32{}, 0u,
+                &ds->n_floats, s, nullptr,
                 ctx->test_skip_first_ticket ? 1u : 0u)));
         FusedArgs a{};
         a.verbs = in->verbs;

@@ -196,8 +196,12 @@ struct ochre_gpu_ctx {
     ochre::DevBuf tile_head, tile_info, tile_row_start, tile_state, span_flag, span_val;   // tile_state: TileBlockState
     // per tile: bins and crossing-sign sum of all entries before its head
     ochre::DevBuf tile_head_bins, tile_head_wind;
-    // scan workspace
+    // scan workspace: four ticket words, then look-back words (scan_space).
+    // scan_tag: the last eager scan's; scan_tickets: tickets taken so far;
+    // scan_dirty: a wait gave up, so tickets and words may be anything.
     ochre::DevBuf scan_status;
+    uint32_t scan_tag = 0, scan_tickets = 0;
+    bool scan_dirty = false;
     ochre::DevBuf scalars;   // DevScalars
     ochre::DevBuf fused_chain;   // fused path: the rasters' and blocks' look-back words
     ochre::DevBuf fused_stage;   // fused path: per-CTA staged alpha (and coverage) of its raster

@@ -9,15 +9,18 @@
 #pragma once
 
 #include "common.cuh"
+#include "internal.h"
 
 namespace ochre {
 
 // A tile's aggregate and inclusive prefix, every 32-bit word of each in a
-// 64-bit word whose high half is its flag (1: aggregate, 2: inclusive; 0:
-// not yet).  One naturally aligned 64-bit access reads or writes a word with
+// 64-bit word whose high half is its flag: the scan's tag (see ScanSpace) and
+// SCAN_AGG or SCAN_INC.  Anything else there (zero, or the tag of an earlier
+// scan that used the same memory) means not yet.  One naturally aligned 64-bit access reads or writes a word with
 // its flag, so a reader takes a value once all its words carry the flag, with
 // relaxed accesses only, and one round of loads reads a predecessor's flags
 // and values together.
+constexpr uint32_t SCAN_AGG = 1u, SCAN_INC = 2u;
 template <class T>
 struct ScanStatus {
     static constexpr int W = (int)(sizeof(T) / 4);
@@ -46,8 +49,8 @@ __device__ __forceinline__ bool ld_flagged(const uint64_t* src, uint32_t flag, T
 
 template <int BLOCK, int ITEMS, class T, class Op, class In, class Out>
 __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_dev, In in, Out out, Op op,
-                                                 T identity, ScanStatus<T>* status, uint32_t* ticket, T* total,
-                                                 uint32_t* err) {
+                                                 T identity, ScanStatus<T>* status, uint32_t* ticket,
+                                                 uint32_t ticket_base, uint32_t tag, T* total, uint32_t* err) {
     constexpr int WARPS = BLOCK / 32;
     __shared__ uint32_t s_tile;
     __shared__ T s_warp[WARPS];
@@ -59,7 +62,8 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
     // an earlier wait of the run gave up: its outputs (this scan's inputs) are
     // not valid; every block ends here, before publishing
     if (run_aborted(err)) return;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+    if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u) - ticket_base;
+    const uint32_t f_agg = tag << 2 | SCAN_AGG, f_inc = tag << 2 | SCAN_INC;
     __syncthreads();
     const uint32_t tile = s_tile;
     if ((uint64_t)tile * (BLOCK * ITEMS) >= n) return;
@@ -100,9 +104,9 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
         T prefix = identity;
         ScanStatus<T>* me = status + tile;
         if (tile == 0) {
-            if (lane == 0) st_flagged(me->inc, tile_agg, 2u);
+            if (lane == 0) st_flagged(me->inc, tile_agg, f_inc);
         } else {
-            if (lane == 0) st_flagged(me->agg, tile_agg, 1u);
+            if (lane == 0) st_flagged(me->agg, tile_agg, f_agg);
             int64_t top = (int64_t)tile - 1;
             long long spins = 0;
             const long long poll_limit = spin_limit(err);
@@ -112,8 +116,8 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
                 bool has_inc = true, has_agg = true;   // before tile 0: an inclusive identity
                 T vi = identity, va = identity;
                 if (j >= 0) {
-                    has_inc = ld_flagged(status[j].inc, 2u, vi);
-                    has_agg = ld_flagged(status[j].agg, 1u, va);
+                    has_inc = ld_flagged(status[j].inc, f_inc, vi);
+                    has_agg = ld_flagged(status[j].agg, f_agg, va);
                 }
                 const uint32_t m2 = __ballot_sync(0xffffffffu, has_inc);
                 const int limit = m2 ? __ffs(m2) - 1 : 31;   // lanes [0, limit] are needed
@@ -134,7 +138,7 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
                 if (m2) break;
                 top -= 32;
             }
-            if (lane == 0) st_flagged(me->inc, op(prefix, tile_agg), 2u);
+            if (lane == 0) st_flagged(me->inc, op(prefix, tile_agg), f_inc);
         }
         if (lane == 0) {
             s_prefix = prefix;
@@ -159,31 +163,36 @@ struct OpSumU32 {
     __device__ __forceinline__ uint32_t operator()(uint32_t a, uint32_t b) const { return a + b; }
 };
 
-// Launch helper.  `status` must hold at least scan_tiles(n) entries and,
-// together with `ticket`, be zeroed on `stream` before the launch (done here).
 constexpr int SCAN_BLOCK = 256;
 constexpr int SCAN_ITEMS = 8;
 inline uint64_t scan_tiles(uint64_t n) { return (n + SCAN_BLOCK * SCAN_ITEMS - 1) / (SCAN_BLOCK * SCAN_ITEMS); }
 
+// Look-back memory of one scan (scan_space, api.cu).  An eager scan clears
+// nothing: its flags carry a tag no earlier scan of the context used, and its
+// tickets go on from the last scan's (ticket_base).  Two clears before each of
+// a call's eight scans had cost more than a small batch's scans themselves.
+struct ScanSpace {
+    void* status;
+    uint32_t* ticket;
+    uint32_t ticket_base, tag;
+};
+cudaError_t scan_space(ochre_gpu_ctx* ctx, size_t status_bytes, uint32_t tiles, uint32_t first_ticket, cudaStream_t s,
+                       ScanSpace* out);
+
+// Launch helper.
 // `n_dev` (optional): the count lives on the device and `n` is its capacity.
 // `first_ticket` (a test hook, else 0): tiles below it are never taken.
 template <class T, class Op, class In, class Out>
-cudaError_t launch_scan(uint64_t n, In in, Out out, Op op, T identity, void* status, uint32_t* ticket, T* total,
-                        uint32_t* err, cudaStream_t stream, const uint32_t* n_dev = nullptr,
-                        uint32_t first_ticket = 0u) {
+cudaError_t launch_scan(ochre_gpu_ctx* ctx, uint64_t n, In in, Out out, Op op, T identity, T* total, cudaStream_t stream,
+                        const uint32_t* n_dev = nullptr, uint32_t first_ticket = 0u) {
     const uint64_t tiles = scan_tiles(n);
     if (tiles == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(status, 0, tiles * sizeof(ScanStatus<T>), stream);
-    if (e != cudaSuccess) return e;
-    if (first_ticket == 0u) {
-        e = cudaMemsetAsync(ticket, 0, sizeof(uint32_t), stream);
-    } else {
-        static const uint32_t one = 1u;
-        e = cudaMemcpyAsync(ticket, &one, sizeof(uint32_t), cudaMemcpyHostToDevice, stream);
-    }
+    ScanSpace sp;
+    const cudaError_t e = scan_space(ctx, tiles * sizeof(ScanStatus<T>), (uint32_t)tiles, first_ticket, stream, &sp);
     if (e != cudaSuccess) return e;
     k_scan<SCAN_BLOCK, SCAN_ITEMS, T, Op, In, Out><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(
-        n, n_dev, in, out, op, identity, reinterpret_cast<ScanStatus<T>*>(status), ticket, total, err);
+        n, n_dev, in, out, op, identity, reinterpret_cast<ScanStatus<T>*>(sp.status), sp.ticket, sp.ticket_base, sp.tag,
+        total, &dev_scalars(ctx)->err);
     return cudaGetLastError();
 }
 

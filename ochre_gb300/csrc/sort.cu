@@ -8,8 +8,8 @@
 // Digits are 8 bits wide, or up to 11 (the tunable sort_digit_bits: fewer
 // passes, larger per-tile histograms and look-back rows); a sort of k key bits
 // takes ceil(k / width) passes of balanced widths.
-// One upfront kernel histograms every digit of every pass; each pass
-// then ranks a tile of keys in shared memory (per-warp counters with
+// One upfront kernel histograms every digit of every pass (and scans the
+// counts); each pass then ranks a tile of keys in shared memory (per-warp counters with
 // __match_any_sync for stable ranks), publishes its per-digit counts and
 // resolves its global offsets by decoupled look-back over earlier tiles
 // (bounded spins; a look-back word holds its flag and count together, so
@@ -20,7 +20,6 @@
 
 #include <algorithm>
 #include <utility>
-#include <vector>
 
 namespace ochre {
 
@@ -40,12 +39,17 @@ struct SortPlan {
     uint8_t width[SORT_MAX_PASSES];
 };
 
+// Histograms of every pass's digits; the block that adds its counts last turns
+// them into each digit's first output place (`done` counts the blocks).
 template <class K, int RB>
 __global__ void __launch_bounds__(256) k_sort_hist(const K* __restrict__ keys, uint64_t n, const uint32_t* n_dev,
-                                                   SortPlan plan, uint32_t* __restrict__ hist) {
+                                                   SortPlan plan, uint32_t* hist, uint32_t* __restrict__ off,
+                                                   uint32_t* done) {
     constexpr int RADIX = 1 << RB;
     constexpr int MAXP = (64 + RB - 1) / RB;
+    constexpr int PER = RADIX / 256;   // consecutive digits per thread
     __shared__ uint32_t sh[MAXP][RADIX];
+    uint32_t* s_scan = &sh[0][0];   // the last block's scan, once the counts have left
     n = dev_count(n, n_dev);
     for (int i = threadIdx.x; i < MAXP * RADIX; i += blockDim.x) (&sh[0][0])[i] = 0u;
     __syncthreads();
@@ -60,34 +64,36 @@ __global__ void __launch_bounds__(256) k_sort_hist(const K* __restrict__ keys, u
         const uint32_t v = (&sh[0][0])[i];
         if (v) atomicAdd(hist + i, v);
     }
-}
-
-// Exclusive scan of each pass's RADIX counts (one block per pass).
-template <int RB>
-__global__ void k_sort_offsets(const uint32_t* __restrict__ hist, uint32_t* __restrict__ off) {
-    constexpr int RADIX = 1 << RB;
-    constexpr int PER = RADIX / 256;   // consecutive digits per thread
-    __shared__ uint32_t s[256];
-    const int p = blockIdx.x, t = threadIdx.x;
-    uint32_t v[PER], sum = 0;
-#pragma unroll
-    for (int q = 0; q < PER; q++) {
-        v[q] = hist[p * RADIX + t * PER + q];
-        sum += v[q];
-    }
-    s[t] = sum;
+    __threadfence();
     __syncthreads();
-    for (int k = 1; k < 256; k <<= 1) {
-        const uint32_t a = t >= k ? s[t - k] : 0u;
-        __syncthreads();
-        s[t] += a;
-        __syncthreads();
-    }
-    uint32_t run = s[t] - sum;
+    if (threadIdx.x == 0) s_scan[0] = atomicAdd(done, 1u);
+    __syncthreads();
+    if (s_scan[0] + 1u != gridDim.x) return;
+    __threadfence();
+    __syncthreads();
+    const int t = threadIdx.x;
+    for (int p = 0; p < plan.passes; p++) {
+        uint32_t v[PER], sum = 0;
 #pragma unroll
-    for (int q = 0; q < PER; q++) {
-        off[p * RADIX + t * PER + q] = run;
-        run += v[q];
+        for (int q = 0; q < PER; q++) {
+            v[q] = __ldcg(hist + p * RADIX + t * PER + q);
+            sum += v[q];
+        }
+        s_scan[t] = sum;
+        __syncthreads();
+        for (int k = 1; k < 256; k <<= 1) {
+            const uint32_t a = t >= k ? s_scan[t - k] : 0u;
+            __syncthreads();
+            s_scan[t] += a;
+            __syncthreads();
+        }
+        uint32_t run = s_scan[t] - sum;
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            off[p * RADIX + t * PER + q] = run;
+            run += v[q];
+        }
+        __syncthreads();
     }
 }
 
@@ -270,8 +276,7 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
                      uint32_t first_bit) {
     constexpr int RADIX = 1 << RB;
     DevScalars* ds = dev_scalars(ctx);
-    // graph replays: n is the capacity, the count is on the device, and every
-    // pass runs (no read-back to skip passes whose digit is constant)
+    // graph replays: n is the capacity, the count is on the device
     const uint32_t* n_dev = ctx->plan ? &ds->n_entries : nullptr;
     SortPlan plan{};
     const uint32_t kb = std::max<uint32_t>(key_bits, 1u);
@@ -286,11 +291,28 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
     }
     const int passes = plan.passes;
     const uint64_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
+    // The counts, the tickets and every pass's look-back words lie together
+    // and are cleared once.  In an arena (no allocation) the passes share one
+    // pass's words, cleared before each, so that the sort takes no more of it.
+    // No count is read back: a pass whose digit is the same in all keys runs
+    // like any other (the read-back that found it out took longer than most
+    // calls' passes: 15 to 20 us of every call).
+    const bool shared = ctx->sort_lookback.arena != nullptr;
+    constexpr size_t TICKETS = 16;   // one per pass, the last one counts k_sort_hist's blocks
+    const size_t rows = (size_t)tiles * RADIX;
     OCHRE_CUDA_TRY(ctx->sort_hist.ensure((size_t)passes * RADIX * 4 * 2));
-    OCHRE_CUDA_TRY(ctx->sort_lookback.ensure((size_t)tiles * RADIX * 4));
-    uint32_t* hist = ctx->sort_hist.as<uint32_t>();
-    uint32_t* off = hist + passes * RADIX;
-    OCHRE_CUDA_TRY(cudaMemsetAsync(hist, 0, (size_t)passes * RADIX * 4, s));
+    const size_t head = shared ? 0 : (size_t)passes * RADIX + TICKETS;
+    const size_t words = head + rows * (shared ? 1 : passes);
+    OCHRE_CUDA_TRY(ctx->sort_lookback.ensure(words * 4));
+    uint32_t* off = ctx->sort_hist.as<uint32_t>();
+    uint32_t* hist = shared ? off + passes * RADIX : ctx->sort_lookback.as<uint32_t>();
+    uint32_t* tickets = shared ? &ds->sort_ticket : hist + passes * RADIX;
+    if (shared) {
+        OCHRE_CUDA_TRY(cudaMemsetAsync(hist, 0, (size_t)passes * RADIX * 4, s));
+        OCHRE_CUDA_TRY(cudaMemsetAsync(tickets, 0, 4, s));
+    } else {
+        OCHRE_CUDA_TRY(cudaMemsetAsync(hist, 0, words * 4, s));
+    }
     K* kin = ctx->keys.as<K>();
     uint32_t* vin = ctx->vals.as<uint32_t>();
     K* kout = ctx->keys_alt.as<K>();
@@ -299,42 +321,32 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         int blocks = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)std::max(sms, 1) * 8);
-        OCHRE_LAUNCH(ctx, "sort_hist", s, k_sort_hist<K, RB><<<blocks, 256, 0, s>>>(kin, n, n_dev, plan, hist));
-        OCHRE_CUDA_TRY(cudaGetLastError());
-        OCHRE_LAUNCH(ctx, "sort_offsets", s, k_sort_offsets<RB><<<passes, 256, 0, s>>>(hist, off));
+        OCHRE_LAUNCH(ctx, "sort_hist", s, k_sort_hist<K, RB><<<blocks, 256, 0, s>>>(
+            kin, n, n_dev, plan, hist, off, shared ? tickets : tickets + TICKETS - 1));
         OCHRE_CUDA_TRY(cudaGetLastError());
     }
     const size_t smem = onesweep_smem<K, RB>();
     OCHRE_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<K, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // Skip passes whose digit is constant over all keys (one bucket holds n).
-    std::vector<uint32_t> h_hist;
-    if (!n_dev) {
-        h_hist.resize((size_t)passes * RADIX);
-        OCHRE_CUDA_TRY(cudaMemcpyAsync(h_hist.data(), hist, (size_t)passes * RADIX * 4, cudaMemcpyDeviceToHost, s));
-        OCHRE_CUDA_TRY(cudaStreamSynchronize(s));
-    }
-    uint32_t done = 0;
     for (int p = 0; p < passes; p++) {
-        bool trivial = false;
-        for (int d = 0; d < RADIX && !n_dev; d++)
-            if (h_hist[(size_t)p * RADIX + d] == n) trivial = true;
-        if (trivial) continue;
-        OCHRE_CUDA_TRY(cudaMemsetAsync(ctx->sort_lookback.p, 0, (size_t)tiles * RADIX * 4, s));
-        OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->sort_ticket, 0, 4, s));
+        uint32_t* lookback = ctx->sort_lookback.as<uint32_t>() + head + (shared ? 0 : p * rows);
+        uint32_t* ticket = shared ? tickets : tickets + p;
+        if (shared) {
+            OCHRE_CUDA_TRY(cudaMemsetAsync(lookback, 0, rows * 4, s));
+            OCHRE_CUDA_TRY(cudaMemsetAsync(ticket, 0, 4, s));
+        }
         OCHRE_LAUNCH(ctx, "sort_onesweep", s, k_onesweep<K, RB><<<(unsigned)tiles, SORT_BLOCK, smem, s>>>(
-            kin, vin, kout, vout, n, n_dev, plan.shift[p], (1u << plan.width[p]) - 1u, off + p * RADIX,
-            ctx->sort_lookback.as<uint32_t>(), &ds->sort_ticket, &ds->err));
+            kin, vin, kout, vout, n, n_dev, plan.shift[p], (1u << plan.width[p]) - 1u, off + p * RADIX, lookback,
+            ticket, &ds->err));
         OCHRE_CUDA_TRY(cudaGetLastError());
-        K* tk = kin; kin = kout; kout = tk;
-        uint32_t* tv = vin; vin = vout; vout = tv;
-        done++;
+        std::swap(kin, kout);
+        std::swap(vin, vout);
     }
     if (kin != ctx->keys.as<K>()) {
         // leave the sorted result in ctx->keys / ctx->vals
         std::swap(ctx->keys, ctx->keys_alt);
         std::swap(ctx->vals, ctx->vals_alt);
     }
-    *passes_done = done;
+    *passes_done = (uint32_t)passes;
     return OCHRE_OK;
 }
 

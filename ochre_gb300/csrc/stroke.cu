@@ -491,13 +491,11 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     OCHRE_CUDA_TRY(ctx->sk_cmd_foff.ensure(n * 4));
     OCHRE_CUDA_TRY(ctx->sk_cmd_mv.ensure(n * 4));
     OCHRE_CUDA_TRY(ctx->sk_cmd_ep.ensure(n * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(n) * sizeof(ScanStatus<CmdScan>)));
     if (!plan) OCHRE_CUDA_TRY(reset_scalars(ctx, s));
     OCHRE_LAUNCH(ctx, "stroke_cmd_scan", s, OCHRE_CUDA_TRY(launch_scan<CmdScan>(
-        n, CmdIn{in->verbs, &ds->err},
+        ctx, n, CmdIn{in->verbs, &ds->err},
         CmdOut{ctx->sk_cmd_foff.as<uint32_t>(), ctx->sk_cmd_mv.as<uint32_t>(), ctx->sk_cmd_ep.as<uint32_t>()},
-        OpCmd{}, CmdScan{0, 0, 0}, ctx->scan_status.p, &ds->ticket, reinterpret_cast<CmdScan*>(&ds->n_floats),
-        &ds->err, s)));
+        OpCmd{}, CmdScan{0, 0, 0}, reinterpret_cast<CmdScan*>(&ds->n_floats), s)));
     if (!plan) {
         st = read_scalars(ctx, s);
         if (st != OCHRE_OK) return st;
@@ -509,7 +507,6 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     wait_inputs(ctx, s);   // path-space flatten counts read points
     OCHRE_CUDA_TRY(ctx->sk_poly_off.ensure((n + 1) * 4));
     OCHRE_CUDA_TRY(ctx->sk_poly_foff.ensure((n + 1) * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(n) * sizeof(ScanStatus<Pair>)));
     OCHRE_LAUNCH(ctx, "stroke_poly_count", s, k_pair_count<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(
         n, nullptr,
         PolyCount{in->verbs, in->pts, in->fill_cmd_off, F, in->fill_flags, ctx->sk_cmd_foff.as<uint32_t>(),
@@ -517,9 +514,9 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
         ctx->sk_poly_off.as<uint32_t>(), ctx->sk_poly_foff.as<uint32_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());
     OCHRE_LAUNCH(ctx, "stroke_poly_scan", s, OCHRE_CUDA_TRY(launch_scan<Pair>(
-        n, PairIn{ctx->sk_poly_off.as<uint32_t>(), ctx->sk_poly_foff.as<uint32_t>()},
+        ctx, n, PairIn{ctx->sk_poly_off.as<uint32_t>(), ctx->sk_poly_foff.as<uint32_t>()},
         PairOut{ctx->sk_poly_off.as<uint32_t>(), ctx->sk_poly_foff.as<uint32_t>()}, OpPair{}, Pair{0u, 0u},
-        ctx->scan_status.p, &ds->ticket, reinterpret_cast<Pair*>(&ds->n_lines), &ds->err, s)));
+        reinterpret_cast<Pair*>(&ds->n_lines), s)));
     // (n_lines, n_line_ent) hold the polyline totals here; the fill chain resets them
     uint32_t P, PF;   // polyline commands and floats (planned: the capacities)
     if (plan) {
@@ -564,10 +561,9 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
         return OCHRE_OK;
     }
     // float offset of every polyline command: an exclusive scan of its float counts
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(P) * sizeof(ScanStatus<uint32_t>)));
     OCHRE_LAUNCH(ctx, "stroke_pfoff_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-        P, PolyFloats{ctx->sk_pverbs.as<uint8_t>()}, OffOutU32{ctx->sk_pfoff.as<uint32_t>()}, OpSumU32{}, 0u,
-        ctx->scan_status.p, &ds->ticket, static_cast<uint32_t*>(nullptr), &ds->err, s, p_dev)));
+        ctx, P, PolyFloats{ctx->sk_pverbs.as<uint8_t>()}, OffOutU32{ctx->sk_pfoff.as<uint32_t>()}, OpSumU32{}, 0u,
+        static_cast<uint32_t*>(nullptr), s, p_dev)));
     OCHRE_LAUNCH(ctx, "stroke_first_close", s, k_first_close<<<(P + 255) / 256, 256, 0, s>>>(
         ctx->sk_pverbs.as<uint8_t>(), P, p_dev, ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
         ctx->sk_first_close.as<uint32_t>()));
@@ -575,9 +571,8 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     // 3. units
     OCHRE_CUDA_TRY(ctx->sk_unit_start.ensure((size_t)P * 4));
     OCHRE_LAUNCH(ctx, "stroke_unit_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-        P, UnitIn{ctx->sk_pverbs.as<uint8_t>(), ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags},
-        UnitOut{ctx->sk_unit_start.as<uint32_t>()}, OpSumU32{}, 0u, ctx->scan_status.p, &ds->ticket,
-        &ds->n_tiles, &ds->err, s, p_dev)));
+        ctx, P, UnitIn{ctx->sk_pverbs.as<uint8_t>(), ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags},
+        UnitOut{ctx->sk_unit_start.as<uint32_t>()}, OpSumU32{}, 0u, &ds->n_tiles, s, p_dev)));
     uint32_t U;   // units (planned: at most P, the count stays on the device)
     if (plan) {
         U = P;
@@ -593,7 +588,6 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     OCHRE_CUDA_TRY(ctx->sk_out_off.ensure(((size_t)U + 1) * 4));
     OCHRE_CUDA_TRY(ctx->sk_out_foff.ensure(((size_t)U + 1) * 4));
     OCHRE_CUDA_TRY(ctx->sk_unit_fill.ensure(((size_t)U + 1) * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(U ? U : 1) * sizeof(ScanStatus<Pair>)));
     // the output totals: a scan that covers no unit writes none
     OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->n_lines, 0, 8, s));
     if (U) {
@@ -604,9 +598,9 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
             ctx->sk_out_foff.as<uint32_t>()));
         OCHRE_CUDA_TRY(cudaGetLastError());
         OCHRE_LAUNCH(ctx, "stroke_out_scan", s, OCHRE_CUDA_TRY(launch_scan<Pair>(
-            U, PairIn{ctx->sk_out_off.as<uint32_t>(), ctx->sk_out_foff.as<uint32_t>()},
+            ctx, U, PairIn{ctx->sk_out_off.as<uint32_t>(), ctx->sk_out_foff.as<uint32_t>()},
             PairOut{ctx->sk_out_off.as<uint32_t>(), ctx->sk_out_foff.as<uint32_t>()}, OpPair{}, Pair{0u, 0u},
-            ctx->scan_status.p, &ds->ticket, reinterpret_cast<Pair*>(&ds->n_lines), &ds->err, s, u_dev)));
+            reinterpret_cast<Pair*>(&ds->n_lines), s, u_dev)));
     }
     uint32_t ON, OF;   // output commands and floats (planned: the capacities)
     if (plan) {

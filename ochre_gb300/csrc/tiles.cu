@@ -634,17 +634,15 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
     OCHRE_CUDA_TRY(ctx->tile_head.ensure(E * 4));
     OCHRE_CUDA_TRY(ctx->tile_head_bins.ensure(E * 4));
     OCHRE_CUDA_TRY(ctx->tile_head_wind.ensure(E * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(E) * sizeof(ScanStatus<HeadScan>)));
     // graph replays: E and T are capacities, the counts stay on the device
     const GraphPlan* plan = ctx->plan;
     const uint32_t* t_dev = plan ? &ds->n_tiles : nullptr;
     OCHRE_LAUNCH(ctx, "tile_head_scan", s,
                  OCHRE_CUDA_TRY(launch_scan<HeadScan>(
-                     E, HeadIn<K>{ctx->keys.as<K>(), ctx->vals.as<uint32_t>()},
+                     ctx, E, HeadIn<K>{ctx->keys.as<K>(), ctx->vals.as<uint32_t>()},
                      HeadOut{ctx->tile_head.as<uint32_t>(), ctx->tile_head_bins.as<uint32_t>(),
                              ctx->tile_head_wind.as<int32_t>()},
-                     OpHead{}, HeadScan{0u, 0u, 0, 0u}, ctx->scan_status.p, &ds->ticket,
-                     reinterpret_cast<HeadScan*>(&ds->n_tiles), &ds->err, s, plan ? &ds->n_entries : nullptr)));
+                     OpHead{}, HeadScan{0u, 0u, 0, 0u}, reinterpret_cast<HeadScan*>(&ds->n_tiles), s, plan ? &ds->n_entries : nullptr)));
     int st = OCHRE_OK;
     uint32_t T;
     if (plan) {
@@ -678,11 +676,10 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
                          ctx->out_raster_tile_off.as<uint32_t>(), &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
     if (T) {
-        OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(T) * sizeof(ScanStatus<uint32_t>)));
         OCHRE_LAUNCH(ctx, "tile_row_scan", s,
                      OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-                         T, RowIn{ctx->tile_info.as<TileInfo>()}, RowOut{ctx->tile_row_start.as<uint32_t>()},
-                         OpSumU32{}, 0u, ctx->scan_status.p, &ds->ticket, &ds->n_rows, &ds->err, s, t_dev)));
+                         ctx, T, RowIn{ctx->tile_info.as<TileInfo>()}, RowOut{ctx->tile_row_start.as<uint32_t>()},
+                         OpSumU32{}, 0u, &ds->n_rows, s, t_dev)));
     }
     uint32_t n_rows;
     if (plan) {
@@ -705,14 +702,13 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
     OCHRE_CUDA_TRY(ctx->out_span_xy.ensure((size_t)T * 4));
     OCHRE_CUDA_TRY(ctx->out_span_w.ensure((size_t)T * 2));
     OCHRE_CUDA_TRY(ctx->out_span_tile.ensure((size_t)T * 4));
-    OCHRE_CUDA_TRY(ctx->scan_status.ensure(scan_tiles(T) * sizeof(ScanStatus<uint32_t>)));
     OCHRE_LAUNCH(ctx, "span_scan", s,
                  OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-                     T, SpanIn{ctx->span_flag.as<uint32_t>()},
+                     ctx, T, SpanIn{ctx->span_flag.as<uint32_t>()},
                      SpanOut{ctx->span_val.as<uint64_t>(), ctx->tile_info.as<TileInfo>(), T, R, t_dev,
                              ctx->out_span_xy.as<uint32_t>(), ctx->out_span_w.as<uint16_t>(),
                              ctx->out_span_tile.as<uint32_t>(), ctx->out_raster_span_off.as<uint32_t>()},
-                     OpSumU32{}, 0u, ctx->scan_status.p, &ds->ticket, &ds->n_spans, &ds->err, s, t_dev)));
+                     OpSumU32{}, 0u, &ds->n_spans, s, t_dev)));
     if (plan) {
         *n_spans_out = 0;   // on the device; read after the replay
         return OCHRE_OK;
