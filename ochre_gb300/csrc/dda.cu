@@ -42,17 +42,17 @@ __device__ __forceinline__ void bbox_add(BBoxAcc& b, int x, int y) {
     b.y1 = max(b.y1, ty);
 }
 
-// What a line's walk leaves: sort entries (bins and crossings), increment
-// cells, the sum of its crossing signs, the tile box of its visited cells.
+// What a line's walk leaves: sort entries (bins and crossings), crossings
+// alone, increment cells, the sum of its crossing signs, the tile box of its visited cells.
 struct LineCount {
-    uint32_t ent, cells;
+    uint32_t ent, cross, cells;
     int wsum;
     BBoxAcc box;
 };
 
 // The same by walking (a line that reaches WALK_CAP).
 __device__ __noinline__ LineCount count_by_walking(V2 a, V2 p, uint32_t* err) {
-    uint32_t ent = 0, cells = 0;
+    uint32_t ent = 0, cross = 0, cells = 0;
     int ws = 0, ptx = 0x7fffffff, pty = 0x7fffffff;
     BBoxAcc box{0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000};
     const bool ok = walk_line(
@@ -64,11 +64,12 @@ __device__ __noinline__ LineCount count_by_walking(V2 a, V2 p, uint32_t* err) {
         },
         [&](int, int, int sign) {
             ent++;
+            cross++;
             ws += sign;
         },
         [&](int x, int y) { bbox_add(box, x, y); });
     if (!ok) atomicOr(err, ERR_LIMIT);
-    return LineCount{ent, cells, ws, box};
+    return LineCount{ent, cross, cells, ws, box};
 }
 
 // Counts of a line without walking it.  The walk takes the row and column
@@ -87,7 +88,7 @@ __device__ __noinline__ LineCount count_by_walking(V2 a, V2 p, uint32_t* err) {
 // uneven paths (60 M lines, 689 M cells): 2.55 ms (walked, ordered by length,
 // the long lines beside) -> 1.08 ms, the lines in their own order.
 __device__ __forceinline__ LineCount count_line(V2 a, V2 p, uint32_t* err) {
-    LineCount n{0u, 0u, 0, {0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000}};
+    LineCount n{0u, 0u, 0u, 0, {0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000}};
     if (veq(a, p)) return n;
     Walk w;
     WalkState s;
@@ -111,7 +112,8 @@ __device__ __forceinline__ LineCount count_line(V2 a, V2 p, uint32_t* err) {
     const int left_x = abs(div8(lx) - div8(s.x)), left_y = abs(div8(ly) - div8(s.y));
     const int end_ty = div8(w.end_y), last_ty = div8(wrap16(ly));
     n.cells = rows + cols + 1u;
-    n.ent = 1u + (uint32_t)left_x + 2u * (uint32_t)left_y + (end_ty != last_ty ? 1u : 0u);
+    n.cross = (uint32_t)left_y + (end_ty != last_ty ? 1u : 0u);
+    n.ent = 1u + (uint32_t)left_x + (uint32_t)left_y + n.cross;
     n.wsum = w.y_dir * left_y + (int)(int8_t)(int16_t)(end_ty - last_ty);
     bbox_add(n.box, s.x, s.y);
     bbox_add(n.box, wrap16(lx), wrap16(ly));
@@ -347,14 +349,15 @@ __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restr
                                                            const uint32_t* n_dev, uint32_t groups, int4* bbox,
                                                            int* raster_wsum, uint32_t* __restrict__ counts,
                                                            uint32_t* __restrict__ inc_counts,
-                                                           unsigned long long* inc_total, uint32_t* ticket,
-                                                           uint32_t* err) {
+                                                           unsigned long long* inc_total, uint32_t* n_cross,
+                                                           uint32_t* ticket, uint32_t* err) {
     constexpr int WARPS = WALK_BLOCK / 32;
     __shared__ int4 s_box[WARPS][BOX_SLOTS];
     __shared__ int s_ws[WARPS][BOX_SLOTS];
     const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
     const uint64_t n_lines = dev_count(n_cap, n_dev);
     unsigned long long incs = 0;   // the warp's increments (lane 0)
+    uint32_t crosses = 0;          // this lane's crossings
     for (;;) {
         const uint64_t i0 = next_window(ticket) * (32u * groups);
         if (i0 >= n_lines) break;
@@ -366,7 +369,7 @@ __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restr
         __syncwarp();
         for (uint32_t j = 0; j < groups; j++) {
             const uint64_t i = i0 + j * 32u + lane;
-            LineCount n{0u, 0u, 0, {0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000}};
+            LineCount n{0u, 0u, 0u, 0, {0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000}};
             uint32_t r = r0;
             if (i < n_lines) {
                 const float4 l = lines[i];
@@ -396,6 +399,7 @@ __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restr
             }
             // (at most 32 capped walks: 32 bits hold it)
             incs += __reduce_add_sync(0xffffffffu, n.cells);
+            crosses += n.cross;
         }
         __syncwarp();
         if (lane < BOX_SLOTS) {
@@ -405,7 +409,9 @@ __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restr
         }
         __syncwarp();
     }
+    crosses = __reduce_add_sync(0xffffffffu, crosses);
     if (lane == 0 && incs) atomicAdd(inc_total, incs);
+    if (lane == 0 && crosses) atomicAdd(n_cross, crosses);
 }
 // Entry and increment offsets of every line, one scan of the pair (in place:
 // every count is read by the thread that writes its offset).
@@ -850,7 +856,8 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
     OCHRE_LAUNCH(ctx, "bbox_init", s, k_bbox_init<<<(R + 255) / 256, 256, 0, s>>>(ctx->raster_bbox.as<int4>(),
                                                                                  ctx->raster_wsum.as<int>(), R));
     OCHRE_CUDA_TRY(cudaGetLastError());
-    // the line pair's totals, the 64-bit increment count and the walks' tickets
+    // the line pair's totals, the 64-bit increment count, the long lines' ticket
+    // and the crossing count
     static_assert(offsetof(DevScalars, inc_total) == offsetof(DevScalars, line_ent_total) + 8 &&
                       offsetof(DevScalars, walk_ticket) == offsetof(DevScalars, line_ent_total) + 16,
                   "layout");
@@ -879,7 +886,8 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
             ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), n_lines, lines_dev, groups,
             ctx->raster_bbox.as<int4>(),
             ctx->raster_wsum.as<int>(), ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>(),
-            reinterpret_cast<unsigned long long*>(&ds->inc_total), &ds->line_ticket, &ds->err));
+            reinterpret_cast<unsigned long long*>(&ds->inc_total), &ds->n_cross, &ds->line_ticket,
+            &ds->err));
         OCHRE_CUDA_TRY(cudaGetLastError());
         // in place: every count is read by the thread that writes its offset
         OCHRE_LAUNCH(ctx, "dda_offset_scan", s, OCHRE_CUDA_TRY(launch_scan<LinePair>(

@@ -233,7 +233,7 @@ void fill_result(ochre_graph* g, ochre_result* out) {
         st.n_entries = hs->n_entries;
         st.n_tiles = hs->n_tiles;
         st.n_spans = hs->n_spans;
-        st.n_bins = hs->n_bins;
+        st.n_bins = hs->n_entries - hs->n_cross;
         st.key_bits = g->plan.key_bits;
         st.sort_passes = (g->plan.key_bits + 7) / 8;
     }

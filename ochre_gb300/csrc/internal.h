@@ -58,16 +58,16 @@ struct DevScalars {
     uint64_t keyspace;     // total key space (raster scan .ks)
     uint32_t n_empty;      // rasters without increments (raster scan .ne)
     uint32_t pad1;
-    uint32_t n_tiles;      // tile-head scan total .heads   }
-    uint32_t n_bins;       // tile-head scan total .bins    } (HeadScan layout)
-    int32_t head_wind;     // sum of all crossing signs     }
-    uint32_t pad2;         //                               }
+    uint32_t n_tiles;      // tiles                         }
+    int32_t head_wind;     // sum of all crossing signs     } (HeadScan layout)
+    uint32_t n_rows;       // tile rows (raster, tile_y)
+    uint32_t pad2;
     uint32_t n_spans;
     uint32_t sort_ticket;
     uint32_t fused_fallback;  // fused path: some raster did not fit
     uint32_t fused_tiles;     // fused path totals
     uint32_t fused_spans;
-    uint32_t n_rows;          // tile rows (raster, tile_y) of the general chain
+    uint32_t pad1b;
     uint32_t spin_log2;       // poll limit of the run's bounded waits, log2 (0: SPIN_LIMIT)
     uint32_t pad3;
     uint32_t line_ent_total;  // chain: sort entries the lines produce   } (line scan
@@ -75,7 +75,7 @@ struct DevScalars {
     uint64_t inc_total;       // the same increment count summed in 64 bits (the pair
                               // total wraps above 2^32; this one says when it did)
     uint32_t walk_ticket;     // long lines handed out in the emit walk
-    uint32_t pad6;
+    uint32_t n_cross;         // sort entries that are tile-row crossings
     uint32_t n_long;          // lines queued for the long-line walkers (flatten)
     uint32_t pad4;
     uint32_t line_ticket;     // line windows handed out in the count walk
@@ -158,17 +158,6 @@ struct TileBlockState {
     float inc[8];
 };
 
-struct TileInfo {
-    int32_t raster;
-    int32_t tx, ty;
-    uint32_t head;       // first bin entry of the tile in the sorted entries
-    uint32_t nbins;
-    int32_t wind;        // tile-row crossing winding at this tile (inclusive, per raster)
-    uint32_t row_head;   // 1 if the tile starts its (raster, tile_y) row
-    uint32_t pad;
-};
-
-
 }  // namespace ochre
 
 struct ochre_gpu_ctx {
@@ -192,10 +181,8 @@ struct ochre_gpu_ctx {
     // sort entries
     ochre::DevBuf keys, vals, keys_alt, vals_alt, bins;
     ochre::DevBuf sort_hist, sort_lookback;
-    // tiles
-    ochre::DevBuf tile_head, tile_info, tile_row_start, tile_state, span_flag, span_val;   // tile_state: TileBlockState
-    // per tile: bins and crossing-sign sum of all entries before its head
-    ochre::DevBuf tile_head_bins, tile_head_wind;
+    // tile metadata (tiles.cu), and the coverage block form's TileBlockState
+    ochre::DevBuf tile_head, tile_xy, tile_rf, tile_state;
     // scan workspace: four ticket words, then look-back words (scan_space).
     // scan_tag: the last eager scan's; scan_tickets: tickets taken so far;
     // scan_dirty: a wait gave up, so tickets and words may be anything.

@@ -98,9 +98,9 @@ extern "C" int ochre_gpu_rasterize_noalloc(const ochre_batch* in, ochre_output_b
                                  &ctx.cmd_line_off, &ctx.lines, &ctx.line_raster, &ctx.line_ent_off, &ctx.line_inc_off,
                                  &ctx.long_lines, &ctx.incs,
                                  &ctx.raster_bbox, &ctx.raster_keybase, &ctx.raster_empty,
-                                 &ctx.raster_wsum, &ctx.raster_wbase, &ctx.tile_head_bins, &ctx.tile_head_wind, &ctx.keys, &ctx.vals,
+                                 &ctx.raster_wsum, &ctx.raster_wbase, &ctx.keys, &ctx.vals,
                                  &ctx.keys_alt, &ctx.vals_alt, &ctx.bins, &ctx.sort_hist, &ctx.sort_lookback,
-                                 &ctx.tile_head, &ctx.tile_info, &ctx.tile_row_start, &ctx.tile_state, &ctx.span_flag, &ctx.span_val,
+                                 &ctx.tile_head, &ctx.tile_xy, &ctx.tile_rf, &ctx.tile_state,
                                  &ctx.scan_status, &ctx.scalars, &ctx.fused_chain, &ctx.fused_stage, &ctx.out_tile_cov,
                                  &ctx.grad_g, &ctx.grad_gs, &ctx.grad_left, &ctx.grad_line, &ctx.grad_pts,
                                  &ctx.sk_cmd_foff, &ctx.sk_cmd_mv, &ctx.sk_cmd_ep, &ctx.sk_poly_off,

@@ -47,6 +47,57 @@ __device__ __forceinline__ bool ld_flagged(const uint64_t* src, uint32_t flag, T
     return ok;
 }
 
+// The prefix of a tile with aggregate tile_agg: decoupled look-back by one
+// whole warp, 32 predecessors per round: lane k inspects tile top - k; the
+// window up to the nearest inclusive value is combined in tile order (earlier
+// tiles on the left).  Publishes the tile's aggregate and inclusive prefix.
+template <class T, class Op>
+__device__ __forceinline__ T scan_lookback(uint32_t tile, const T& tile_agg, Op op, const T& identity,
+                                           ScanStatus<T>* status, uint32_t tag, uint32_t* err) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t f_agg = tag << 2 | SCAN_AGG, f_inc = tag << 2 | SCAN_INC;
+    T prefix = identity;
+    ScanStatus<T>* me = status + tile;
+    if (tile == 0) {
+        if (lane == 0) st_flagged(me->inc, tile_agg, f_inc);
+        return prefix;
+    }
+    if (lane == 0) st_flagged(me->agg, tile_agg, f_agg);
+    int64_t top = (int64_t)tile - 1;
+    long long spins = 0;
+    const long long poll_limit = spin_limit(err);
+    while (top >= 0) {
+        const int64_t j = top - lane;
+        // the predecessor's inclusive prefix and aggregate, read together
+        bool has_inc = true, has_agg = true;   // before tile 0: an inclusive identity
+        T vi = identity, va = identity;
+        if (j >= 0) {
+            has_inc = ld_flagged(status[j].inc, f_inc, vi);
+            has_agg = ld_flagged(status[j].agg, f_agg, va);
+        }
+        const uint32_t m2 = __ballot_sync(0xffffffffu, has_inc);
+        const int limit = m2 ? __ffs(m2) - 1 : 31;   // lanes [0, limit] are needed
+        const uint32_t need = limit == 31 ? 0xffffffffu : ((1u << (limit + 1)) - 1u);
+        if (__ballot_sync(0xffffffffu, !has_inc && !has_agg) & need) {
+            if (wait_give_up_warp(spins, poll_limit, err)) break;
+            if (spins > 64) __nanosleep(64);
+            continue;
+        }
+        T v = identity;
+        if (lane <= limit && j >= 0) v = has_inc ? vi : va;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const T o = shfl_down_T(v, d);
+            if (lane + d < 32) v = op(o, v);
+        }
+        prefix = op(shfl_idx_T(v, 0), prefix);
+        if (m2) break;
+        top -= 32;
+    }
+    if (lane == 0) st_flagged(me->inc, op(prefix, tile_agg), f_inc);
+    return prefix;
+}
+
 template <int BLOCK, int ITEMS, class T, class Op, class In, class Out>
 __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_dev, In in, Out out, Op op,
                                                  T identity, ScanStatus<T>* status, uint32_t* ticket,
@@ -63,7 +114,6 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
     // not valid; every block ends here, before publishing
     if (run_aborted(err)) return;
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u) - ticket_base;
-    const uint32_t f_agg = tag << 2 | SCAN_AGG, f_inc = tag << 2 | SCAN_INC;
     __syncthreads();
     const uint32_t tile = s_tile;
     if ((uint64_t)tile * (BLOCK * ITEMS) >= n) return;
@@ -98,48 +148,7 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
         const T ex = shfl_up_T(w, 1);
         const T tile_agg = shfl_idx_T(w, WARPS - 1);
         if (lane < WARPS) s_warp[lane] = lane == 0 ? identity : ex;
-        // Decoupled look-back by the whole warp, 32 predecessors per round:
-        // lane k inspects tile top - k; the window up to the nearest inclusive
-        // value is combined in tile order (earlier tiles on the left).
-        T prefix = identity;
-        ScanStatus<T>* me = status + tile;
-        if (tile == 0) {
-            if (lane == 0) st_flagged(me->inc, tile_agg, f_inc);
-        } else {
-            if (lane == 0) st_flagged(me->agg, tile_agg, f_agg);
-            int64_t top = (int64_t)tile - 1;
-            long long spins = 0;
-            const long long poll_limit = spin_limit(err);
-            while (top >= 0) {
-                const int64_t j = top - lane;
-                // the predecessor's inclusive prefix and aggregate, read together
-                bool has_inc = true, has_agg = true;   // before tile 0: an inclusive identity
-                T vi = identity, va = identity;
-                if (j >= 0) {
-                    has_inc = ld_flagged(status[j].inc, f_inc, vi);
-                    has_agg = ld_flagged(status[j].agg, f_agg, va);
-                }
-                const uint32_t m2 = __ballot_sync(0xffffffffu, has_inc);
-                const int limit = m2 ? __ffs(m2) - 1 : 31;   // lanes [0, limit] are needed
-                const uint32_t need = limit == 31 ? 0xffffffffu : ((1u << (limit + 1)) - 1u);
-                if (__ballot_sync(0xffffffffu, !has_inc && !has_agg) & need) {
-                    if (wait_give_up_warp(spins, poll_limit, err)) break;
-                    if (spins > 64) __nanosleep(64);
-                    continue;
-                }
-                T v = identity;
-                if (lane <= limit && j >= 0) v = has_inc ? vi : va;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const T o = shfl_down_T(v, d);
-                    if (lane + d < 32) v = op(o, v);
-                }
-                prefix = op(shfl_idx_T(v, 0), prefix);
-                if (m2) break;
-                top -= 32;
-            }
-            if (lane == 0) st_flagged(me->inc, op(prefix, tile_agg), f_inc);
-        }
+        const T prefix = scan_lookback(tile, tile_agg, op, identity, status, tag, err);
         if (lane == 0) {
             s_prefix = prefix;
             const uint64_t tile_end = (uint64_t)(tile + 1) * (BLOCK * ITEMS);

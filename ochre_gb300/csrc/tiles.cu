@@ -10,8 +10,9 @@
 //     prefix over the whole raster) is nonzero (:252-265).
 //
 // Tiles are numbered in sorted order, which is the reference's callback
-// order.  The tile-head scan also counts bins and sums crossing signs, so
-// each tile's metadata and winding follow without a per-tile search.
+// order.  One scan over the sorted entries numbers the tiles and their rows and
+// sums the crossing signs, and writes each tile's metadata at its head; the
+// spans follow from it by a scan over the tiles.
 // Coverage (row form) runs one warp per whole tile row (raster, tile_y) at a
 // time, taken by ticket: chunk by chunk of TILES_PER_WARP tiles it adds the
 // increments the emit walk stored for the chunk's bins into shared-memory
@@ -27,79 +28,231 @@
 
 namespace ochre {
 
-// Tile heads: the first bin entry of every run of equal keys.  The same
-// scan counts bin entries and sums the crossing signs, so that every tile
-// learns, at its head, how many bins and how much winding precede it.
+// Tile metadata, three words per tile: the first bin entry of the tile in
+// the sorted entries (its bins run to the next tile's first, crossing entries
+// between), its tile coordinates, and its raster with two flags.
+constexpr uint32_t RF_RASTER = MAX_RASTERS - 1u;
+constexpr uint32_t RF_WIND = 1u << 30;   // the crossings of its raster sorted before it sum to a nonzero winding
+constexpr uint32_t RF_ROW = 1u << 31;    // it starts its (raster, tile_y) row
+__device__ __forceinline__ uint32_t pack_tile(int tx, int ty) {
+    return (uint32_t)(uint16_t)(int16_t)tx | ((uint32_t)(uint16_t)(int16_t)ty << 16);
+}
+__device__ __forceinline__ int tile_tx(uint32_t xy) { return (int)(int16_t)(xy & 0xffffu); }
+__device__ __forceinline__ int tile_ty(uint32_t xy) { return (int)(int16_t)(xy >> 16); }
+struct TileView {
+    const uint32_t* head;
+    const uint32_t* xy;
+    const uint32_t* rf;
+    uint32_t n_entries;          // sorted entries: the end of the last tile's bins
+    const uint32_t* entries_dev; // the same held on the device (graph replays), else null
+    __device__ __forceinline__ uint32_t end() const { return (uint32_t)dev_count(n_entries, entries_dev); }
+};
+
+// Tile heads: the first bin entry of every run of equal keys.  One single-pass
+// scan numbers the tiles and sums the crossing signs; a tile's winding
+// (rasterizer.rs:219, 253-258: the signs of all crossings of its raster sorted
+// before it, never reset) is the sum before its head minus that of all earlier
+// rasters.
 struct HeadScan {
     uint32_t heads;
-    uint32_t bins;
     int32_t w;
-    uint32_t pad;
 };
 struct OpHead {
     __device__ __forceinline__ HeadScan operator()(HeadScan a, HeadScan b) const {
-        return HeadScan{a.heads + b.heads, a.bins + b.bins, a.w + b.w, 0u};
+        return HeadScan{a.heads + b.heads, a.w + b.w};
     }
 };
-template <class K>
-struct HeadIn {
-    const K* keys;
+// The value of the last bin entry before entry i (false: there is none).  The
+// entries between are the crossings of the tile that starts at or after i: its
+// bins are as many, so the search never costs more than they do.
+__device__ __forceinline__ bool bin_before(const uint32_t* __restrict__ vals, uint64_t i, uint32_t& value) {
+    for (int64_t j = (int64_t)i - 1; j >= 0; j--) {
+        value = vals[j];
+        if (!(value & CROSS_TAG)) return true;
+    }
+    return false;
+}
+
+// A warp takes HEAD_ITEMS steps of 32 consecutive entries, so every load is
+// one segment of 128 bytes, a head's number is a count of ballot bits, and so
+// is the sum of the signs before it (they are +-1 but for walks that snap far,
+// which take a shuffle scan).  Each head then gathers its bin record once; a
+// row starts where raster or tile row differ from the head before, a shuffle
+// away.  Bound by those gathers.  For the 178 M entries and 70 M tiles of
+// 20,000 uneven paths a generic scan (threads own 8 consecutive entries), the
+// metadata gathered by a kernel of its own and a scan for the rows took 3.40
+// ms; 1.33 ms here (the coverage kernel finds the rows itself).  Few entries
+// take 4 steps a warp instead of 16, so that more warps share the gathers'
+// latency: one path's 6,339 entries 16 us at 16 steps, 10 us at 4.
+constexpr int HEAD_BLOCK = 256;
+struct HeadArgs {
     const uint32_t* vals;
-    __device__ __forceinline__ HeadScan operator()(uint64_t i) const {
-        const uint32_t v = vals[i];
-        if (v & CROSS_TAG) return HeadScan{0u, 0u, (int32_t)(int8_t)(v & 0xffu), 0u};
-        return HeadScan{(i == 0 || keys[i] != keys[i - 1]) ? 1u : 0u, 1u, 0, 0u};
-    }
-};
-struct HeadOut {
+    const BinRec* bins;
+    const int32_t* raster_wbase;
+    uint64_t n;
+    const uint32_t* n_dev;   // device-held entry count (graph replays), else null
+    uint32_t n_rasters;
     uint32_t* head;
-    uint32_t* head_bins;
-    int32_t* head_wind;
-    __device__ __forceinline__ void operator()(uint64_t i, HeadScan ex, HeadScan v) const {
-        if (v.heads) {
-            head[ex.heads] = (uint32_t)i;
-            head_bins[ex.heads] = ex.bins;
-            head_wind[ex.heads] = ex.w;
+    uint32_t* xy;
+    uint32_t* rf;
+    uint32_t* raster_tile_off;
+    HeadScan* total;
+    uint32_t* n_rows;        // zero before the launch
+};
+template <class K, int HEAD_ITEMS>
+__global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__ keys, HeadArgs A,
+                                                           ScanStatus<HeadScan>* status, uint32_t* ticket,
+                                                           uint32_t ticket_base, uint32_t tag, uint32_t* err) {
+    constexpr int WARPS = HEAD_BLOCK / 32, HEAD_TILE = HEAD_BLOCK * HEAD_ITEMS;
+    constexpr uint32_t FULL = 0xffffffffu;
+    __shared__ uint32_t s_tile, s_rows;
+    __shared__ HeadScan s_warp[WARPS];
+    __shared__ HeadScan s_prefix;
+    const uint64_t n = dev_count(A.n, A.n_dev);
+    if (run_aborted(err)) return;   // a wait of the sort gave up: the values are not valid indices
+    if (threadIdx.x == 0) {
+        s_tile = atomicAdd(ticket, 1u) - ticket_base;
+        s_rows = 0u;
+    }
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if ((uint64_t)tile * HEAD_TILE >= n) return;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint64_t base = (uint64_t)tile * HEAD_TILE + (uint64_t)warp * (32 * HEAD_ITEMS);
+
+    // heads and signs of the warp's entries
+    uint32_t val[HEAD_ITEMS];
+    uint32_t heads = 0;   // bit k: this lane's entry of step k is a head
+    int32_t w = 0;
+    uint32_t n_heads = 0;
+    {
+        K key[HEAD_ITEMS];
+        K before = 0;     // the key before the warp's first entry
+#pragma unroll
+        for (int k = 0; k < HEAD_ITEMS; k++) {
+            const uint64_t i = base + k * 32 + lane;
+            val[k] = i < n ? A.vals[i] : CROSS_TAG;   // (past the end: a crossing without a sign)
+            key[k] = i < n ? keys[i] : (K)0;
+        }
+        if (base > 0 && base < n) before = keys[base - 1];
+#pragma unroll
+        for (int k = 0; k < HEAD_ITEMS; k++) {
+            K left = shfl_up_T(key[k], 1);
+            if (lane == 0) left = before;
+            before = shfl_idx_T(key[k], 31);
+            const uint64_t i = base + k * 32 + lane;
+            const bool bin = !(val[k] & CROSS_TAG);
+            const bool is = bin && (i == 0 || key[k] != left);
+            if (is) heads |= 1u << k;
+            n_heads += (uint32_t)__popc(__ballot_sync(FULL, is));
+            if (!bin) w += (int32_t)(int8_t)(val[k] & 0xffu);
         }
     }
-};
-
-// Tile metadata, one thread per tile.  The tile's bins are the bins between
-// its head and the next tile's head; its winding (rasterizer.rs:219, 253-258:
-// the signs of all crossings of its raster sorted before it, never reset)
-// is the crossing-sign sum before its head minus that of all earlier
-// rasters.
-__global__ void k_tile_info(const uint32_t* __restrict__ vals, const BinRec* __restrict__ bins,
-                            const uint32_t* __restrict__ head, const uint32_t* __restrict__ head_bins,
-                            const int32_t* __restrict__ head_wind, const int32_t* __restrict__ raster_wbase,
-                            const uint32_t* __restrict__ total_bins, uint32_t n_tiles, const uint32_t* n_dev,
-                            uint32_t n_rasters, TileInfo* __restrict__ info, uint32_t* __restrict__ raster_tile_off,
-                            const uint32_t* err) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    n_tiles = (uint32_t)dev_count(n_tiles, n_dev);
-    // a wait of the sort gave up: the sorted entries are not valid indices
-    if (t >= n_tiles || run_aborted(err)) return;
-    const uint32_t h = head[t];
-    const BinRec* rec = bins + vals[h];
-    const int r = (int)rec->raster;
-    TileInfo ti;
-    ti.raster = r;
-    ti.tx = div8((int)rec->x);
-    ti.ty = div8((int)rec->y);
-    ti.head = h;
-    ti.nbins = (t + 1 < n_tiles ? head_bins[t + 1] : *total_bins) - head_bins[t];
-    ti.wind = head_wind[t] - raster_wbase[r];
-    bool ras_head = t == 0, row_head = t == 0;
-    if (t > 0) {
-        const BinRec* pr = bins + vals[head[t - 1]];
-        ras_head = (int)pr->raster != r;
-        row_head = ras_head || div8((int)pr->y) != ti.ty;
+    const int32_t warp_w = __reduce_add_sync(FULL, w);
+    if (lane == 0) s_warp[warp] = HeadScan{n_heads, warp_w};
+    // raster and tile row of the last bin before the warp's entries
+    uint32_t prev_r = 0xffffffffu;
+    int prev_ty = 0;
+    if (lane == 0 && heads + n_heads != 0u && base < n) {
+        uint32_t pv;
+        if (bin_before(A.vals, base, pv)) {
+            prev_r = A.bins[pv].raster;
+            prev_ty = div8((int)A.bins[pv].y);
+        }
     }
-    ti.row_head = row_head ? 1u : 0u;
-    ti.pad = 0;
-    info[t] = ti;
-    if (ras_head) raster_tile_off[r] = t;
-    if (t + 1 == n_tiles) raster_tile_off[n_rasters] = n_tiles;
+    prev_r = __shfl_sync(FULL, prev_r, 0);
+    prev_ty = __shfl_sync(FULL, prev_ty, 0);
+    __syncthreads();
+    if (warp == 0) {
+        HeadScan v = lane < (uint32_t)WARPS ? s_warp[lane] : HeadScan{0u, 0};
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const HeadScan o = shfl_up_T(v, d);
+            if (lane >= (uint32_t)d) v = OpHead{}(o, v);
+        }
+        HeadScan ex = shfl_up_T(v, 1);
+        if (lane == 0) ex = HeadScan{0u, 0};
+        const HeadScan agg = shfl_idx_T(v, WARPS - 1);
+        if (lane < (uint32_t)WARPS) s_warp[lane] = ex;
+        const HeadScan prefix = scan_lookback(tile, agg, OpHead{}, HeadScan{0u, 0}, status, tag, err);
+        if (lane == 0) {
+            s_prefix = prefix;
+            if ((uint64_t)(tile + 1) * HEAD_TILE >= n) {
+                const HeadScan t = OpHead{}(prefix, agg);
+                *A.total = t;
+                A.raster_tile_off[A.n_rasters] = t.heads;
+            }
+        }
+    }
+    __syncthreads();
+    uint32_t t0 = s_prefix.heads + s_warp[warp].heads;   // tiles before the step
+    int32_t w0 = s_prefix.w + s_warp[warp].w;            // signs before the step
+    uint32_t rows = 0;
+#pragma unroll 4
+    for (int k = 0; k < HEAD_ITEMS; k++) {
+        const bool is = (heads >> k) & 1u;
+        const bool cross = (val[k] & CROSS_TAG) != 0u;
+        const int sign = cross ? (int)(int8_t)(val[k] & 0xffu) : 0;
+        const uint32_t hm = __ballot_sync(FULL, is);
+        const uint32_t pos = __ballot_sync(FULL, sign == 1), neg = __ballot_sync(FULL, sign == -1);
+        int wb = __popc(pos & lt) - __popc(neg & lt), wt = __popc(pos) - __popc(neg);
+        if (__any_sync(FULL, sign > 1 || sign < -1)) {
+            int inc = sign;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int o = __shfl_up_sync(FULL, inc, d);
+                if (lane >= (uint32_t)d) inc += o;
+            }
+            wb = inc - sign;
+            wt = __shfl_sync(FULL, inc, 31);
+        }
+        if (hm) {
+            uint32_t r = 0;
+            int tx = 0, ty = 0;
+            if (is) {
+                const BinRec rec = A.bins[val[k]];
+                r = rec.raster;
+                tx = div8((int)rec.x);
+                ty = div8((int)rec.y);
+            }
+            // the head before: in this step, else the last one so far (or the
+            // last bin before the warp: the same tile as the head before)
+            const uint32_t below = hm & lt;
+            const int src = below ? 31 - __clz(below) : 0;
+            const uint32_t sr = __shfl_sync(FULL, r, src);
+            const int sy = __shfl_sync(FULL, ty, src);
+            const uint32_t pr = below ? sr : prev_r;
+            const int py = below ? sy : prev_ty;
+            const bool row = is && (pr != r || py != ty);
+            if (is) {
+                const uint32_t t = t0 + (uint32_t)__popc(below);
+                A.head[t] = (uint32_t)(base + k * 32 + lane);
+                A.xy[t] = pack_tile(tx, ty);
+                A.rf[t] = r | (w0 + wb != A.raster_wbase[r] ? RF_WIND : 0u) | (row ? RF_ROW : 0u);
+                if (pr != r) A.raster_tile_off[r] = t;
+            }
+            rows += (uint32_t)__popc(__ballot_sync(FULL, row));
+            const int last = 31 - __clz(hm);
+            prev_r = __shfl_sync(FULL, r, last);
+            prev_ty = __shfl_sync(FULL, ty, last);
+        }
+        t0 += (uint32_t)__popc(hm);
+        w0 += wt;
+    }
+    if (lane == 0 && rows) atomicAdd(&s_rows, rows);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_rows) atomicAdd(A.n_rows, s_rows);
+}
+
+// Graph replays: the tile count against its capacity; above it there is no
+// tile, no row and no span to work on.
+__global__ void k_plan_tiles(DevScalars* ds, uint32_t cap) {
+    if (ds->n_tiles > cap) {
+        ds->n_tiles = 0u;
+        ds->n_rows = 0u;
+        atomicOr(&ds->err, ERR_CAPACITY);
+    }
 }
 
 // Shared-memory accumulators of one tile: 64 area cells, then 64 height
@@ -226,9 +379,9 @@ __device__ __forceinline__ void add_chunk_increments(const uint32_t* __restrict_
 template <int CH>
 __global__ void __launch_bounds__(128) k_tile_cov_blocks(
     const uint32_t* __restrict__ vals, const BinRec* __restrict__ bins, const float2* __restrict__ incs,
-    const TileInfo* __restrict__ info, uint32_t n_tiles, const uint32_t* n_dev, TileBlockState* state,
-    uint32_t* ticket, uint32_t* __restrict__ out_xy, uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov,
-    uint32_t* __restrict__ span_flag, uint64_t* __restrict__ span_val, uint32_t* err, bool cov_signed) {
+    TileView tiles, uint32_t n_tiles, const uint32_t* n_dev, TileBlockState* state, uint32_t* ticket,
+    uint32_t* __restrict__ out_xy, uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov, uint32_t* err,
+    bool cov_signed) {
     constexpr int WARPS = 4;
     // device-held count (graph replays): blocks past it end before publishing
     n_tiles = (uint32_t)dev_count(n_tiles, n_dev);
@@ -237,8 +390,8 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
     if (run_aborted(err)) return;
     // [tile][area cells | height cells], ACC_STRIDE floats per tile; see acc_idx
     __shared__ __align__(16) float s_acc[WARPS][CH][ACC_STRIDE];
-    __shared__ uint32_t s_head[WARPS][CH];
-    __shared__ TileInfo s_info[WARPS][CH + 1];
+    __shared__ uint32_t s_head[WARPS][CH + 1];   // (and the end of the block's entries)
+    __shared__ uint32_t s_xy[WARPS][CH], s_rf[WARPS][CH];
     __shared__ BinStage s_stage[WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t blk = 0;
@@ -249,22 +402,22 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
     const int nt = (int)min((uint32_t)CH, n_tiles - t0);
     float (*acc)[ACC_STRIDE] = s_acc[wid];
 
-    // tile metadata (one extra for the span test of the last tile)
+    // tile metadata
     for (int i = lane; i <= nt; i += 32) {
-        if (t0 + i < n_tiles) s_info[wid][i] = info[t0 + i];
-        else s_info[wid][i].raster = -1;
+        s_head[wid][i] = t0 + i < n_tiles ? tiles.head[t0 + i] : tiles.end();
+        if (i < nt) {
+            s_xy[wid][i] = tiles.xy[t0 + i];
+            s_rf[wid][i] = tiles.rf[t0 + i];
+        }
     }
     for (int k = lane; k < nt * (ACC_STRIDE / 4); k += 32)
         reinterpret_cast<float4*>(acc[0])[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    __syncwarp();
-    if (lane < nt) s_head[wid][lane] = s_info[wid][lane].head;
     __syncwarp();
 
     // The stored increments of every bin of the block (rasterizer.rs:97-106,
     // 223-228).  The block's entries are contiguous; crossing entries in
     // between are skipped.
-    const uint32_t e0 = s_info[wid][0].head;
-    const uint32_t e1 = s_info[wid][nt - 1].head + s_info[wid][nt - 1].nbins;
+    const uint32_t e0 = s_head[wid][0], e1 = s_head[wid][nt];
     add_chunk_increments<CH>(vals, bins, incs, e0, e1, s_head[wid], nt, acc, s_stage[wid]);
 
     // Each lane owns one pixel row of one tile: lane = 8 * g + y, four tiles
@@ -274,8 +427,8 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
     // Row sums of the block's last row segment -> publish (decoupled).
     int last_seg = 0;
     for (int i = nt - 1; i > 0; i--)
-        if (s_info[wid][i].row_head) { last_seg = i; break; }
-    const bool starts_mid_row = !s_info[wid][0].row_head;
+        if (s_rf[wid][i] & RF_ROW) { last_seg = i; break; }
+    const bool starts_mid_row = !(s_rf[wid][0] & RF_ROW);
     const bool one_segment = last_seg == 0 && starts_mid_row;
     float part = 0.0f;
     for (int i = last_seg + g; i < nt; i += 4) {
@@ -366,7 +519,7 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
             for (int c = 0; c < 8; c++) a[c] = h[c] = 0.0f;
         }
         const float rs = ((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]));
-        const bool head = valid && i > 0 && s_info[wid][i].row_head;
+        const bool head = valid && i > 0 && (s_rf[wid][i] & RF_ROW);
         // segmented inclusive scan of rs over g (lanes 8 apart), then shifted
         // by one tile: ex = the sum of rs since the last row start before g
         float v = rs;
@@ -409,182 +562,158 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
                 o[1] = make_float4(cv[4], cv[5], cv[6], cv[7]);
             }
             if (y == 0) {
-                const TileInfo& ti = s_info[wid][i];
-                out_xy[t] = (uint32_t)(uint16_t)(int16_t)(ti.tx * 8) |
-                            ((uint32_t)(uint16_t)(int16_t)(ti.ty * 8) << 16);
-                const TileInfo& nx = s_info[wid][i + 1];
-                uint32_t has_span = 0;
-                if (nx.raster == ti.raster && nx.ty == ti.ty && nx.tx > ti.tx + 1 && ti.wind != 0) {
-                    has_span = 1;
-                    const uint32_t x = (uint16_t)(int16_t)((ti.tx + 1) * 8);
-                    const uint32_t yy = (uint16_t)(int16_t)(ti.ty * 8);
-                    const uint32_t wd = (uint16_t)((uint16_t)(nx.tx - ti.tx - 1) * 8u);
-                    span_val[t] = (uint64_t)x | ((uint64_t)yy << 16) | ((uint64_t)wd << 32);
-                }
-                span_flag[t] = has_span;
+                const uint32_t xy = s_xy[wid][i];
+                out_xy[t] = pack_tile(tile_tx(xy) * 8, tile_ty(xy) * 8);
             }
         }
     }
 }
 
 // Coverage, row form: one warp per tile row (see the file comment).
+constexpr uint32_t ROW_RANGE = 32;   // tiles per ticket
 template <int CH>
 __global__ void __launch_bounds__(128) k_tile_cov(
     const uint32_t* __restrict__ vals, const BinRec* __restrict__ bins, const float2* __restrict__ incs,
-    const TileInfo* __restrict__ info, uint32_t n_tiles, const uint32_t* n_dev, const uint32_t* __restrict__ row_start,
-    const uint32_t* __restrict__ n_rows_p, uint32_t* ticket, uint32_t* __restrict__ out_xy,
-    uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov, uint32_t* __restrict__ span_flag,
-    uint64_t* __restrict__ span_val, const uint32_t* err, bool cov_signed) {
+    TileView tiles, uint32_t n_tiles, const uint32_t* n_dev, uint32_t* ticket, uint32_t* __restrict__ out_xy,
+    uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov, const uint32_t* err, bool cov_signed) {
     constexpr int WARPS = 4;
     // an earlier wait of the run gave up: the tile data is not valid
     if (run_aborted(err)) return;
     __shared__ __align__(16) float s_acc[WARPS][CH][ACC_STRIDE];
-    __shared__ uint32_t s_head[WARPS][CH];
-    __shared__ TileInfo s_info[WARPS][CH + 1];
+    __shared__ uint32_t s_head[WARPS][CH + 1];   // (and the end of the chunk's entries)
+    __shared__ uint32_t s_xy[WARPS][CH];
     __shared__ BinStage s_stage[WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     // lane = 8 * g + y: pixel row y of the g-th tile of a pass of four
     const int y = lane & 7, g = lane >> 3;
-    const uint32_t n_rows = *n_rows_p;
     n_tiles = (uint32_t)dev_count(n_tiles, n_dev);
     float (*acc)[ACC_STRIDE] = s_acc[wid];
 
     for (;;) {
         // one tile row (raster, tile_y) per warp at a time: the row carry
-        // (rasterizer.rs:243-250) never leaves the warp
-        uint32_t k = 0;
-        if (lane == 0) k = atomicAdd(ticket, 1u);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= n_rows) return;
-        const uint32_t tb = row_start[k];
-        const uint32_t te = k + 1 < n_rows ? row_start[k + 1] : n_tiles;
-        float carry_row = 0.0f;   // carry into the next tile, pixel row y
-        for (uint32_t t0 = tb; t0 < te; t0 += CH) {
-            const int nt = (int)min((uint32_t)CH, te - t0);
-            // tile metadata (one extra for the span test of the last tile)
-            for (int i = lane; i <= nt; i += 32) {
-                if (t0 + i < n_tiles) s_info[wid][i] = info[t0 + i];
-                else s_info[wid][i].raster = -1;
-            }
-            for (int q = lane; q < nt * (ACC_STRIDE / 4); q += 32)
-                reinterpret_cast<float4*>(acc[0])[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            __syncwarp();
-            if (lane < nt) s_head[wid][lane] = s_info[wid][lane].head;
-            __syncwarp();
-
-            // The stored increments of every bin of the chunk
-            // (rasterizer.rs:97-106, 223-228).  The chunk's entries are
-            // contiguous; crossing entries in between are skipped.
-            const uint32_t e0 = s_info[wid][0].head;
-            const uint32_t e1 = s_info[wid][nt - 1].head + s_info[wid][nt - 1].nbins;
-            add_chunk_increments<CH>(vals, bins, incs, e0, e1, s_head[wid], nt, acc, s_stage[wid]);
-
-            // Tiles left to right (rasterizer.rs:232-250): along its row a lane
-            // adds the cells in the reference's order; the carry into a tile is
-            // the carry into the previous tile plus that tile's row sum.
-            for (int i0 = 0; i0 < nt; i0 += 4) {
-                const int i = i0 + g;
-                const bool valid = i < nt;
-                float a[8], h[8];
-                if (valid) {
-                    const float4 a0 = *reinterpret_cast<const float4*>(&acc[i][acc_idx(8 * y)]);
-                    const float4 a1 = *reinterpret_cast<const float4*>(&acc[i][acc_idx(8 * y + 4)]);
-                    const float4 h0 = *reinterpret_cast<const float4*>(&acc[i][ACC_H + acc_idx(8 * y)]);
-                    const float4 h1 = *reinterpret_cast<const float4*>(&acc[i][ACC_H + acc_idx(8 * y + 4)]);
-                    a[0] = a0.x; a[1] = a0.y; a[2] = a0.z; a[3] = a0.w; a[4] = a1.x; a[5] = a1.y; a[6] = a1.z; a[7] = a1.w;
-                    h[0] = h0.x; h[1] = h0.y; h[2] = h0.z; h[3] = h0.w; h[4] = h1.x; h[5] = h1.y; h[6] = h1.z; h[7] = h1.w;
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 8; c++) a[c] = h[c] = 0.0f;
+        // (rasterizer.rs:243-250) never leaves the warp.  A ticket is a range
+        // of tiles; its warp takes the rows that start there.
+        uint32_t range = 0;
+        if (lane == 0) range = atomicAdd(ticket, 1u);
+        range = __shfl_sync(0xffffffffu, range, 0) * ROW_RANGE;
+        if (range >= n_tiles) return;
+        uint32_t starts = __ballot_sync(0xffffffffu, range + lane < n_tiles && (tiles.rf[range + lane] & RF_ROW));
+        for (; starts; starts &= starts - 1u) {
+            float carry_row = 0.0f;   // carry into the next tile, pixel row y
+            bool more = true;
+            for (uint32_t t0 = range + (uint32_t)__ffs(starts) - 1u; more; t0 += CH) {
+                // tile metadata, and where the row ends
+                const uint32_t ti = t0 + lane;
+                const bool ends = lane > 0 && lane <= CH && (ti >= n_tiles || (tiles.rf[ti] & RF_ROW));
+                const uint32_t em = __ballot_sync(0xffffffffu, ends);
+                const int nt = em ? __ffs(em) - 1 : CH;
+                more = em == 0u;
+                if (lane <= nt) {
+                    s_head[wid][lane] = ti < n_tiles ? tiles.head[ti] : tiles.end();
+                    if (lane < nt) s_xy[wid][lane] = tiles.xy[ti];
                 }
-                const float rs = ((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]));
-                // exclusive sum of rs over the tiles of the pass before this one
-                float v = rs;
+                for (int q = lane; q < nt * (ACC_STRIDE / 4); q += 32)
+                    reinterpret_cast<float4*>(acc[0])[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                __syncwarp();
+
+                // The stored increments of every bin of the chunk
+                // (rasterizer.rs:97-106, 223-228).  The chunk's entries are
+                // contiguous; crossing entries in between are skipped.
+                const uint32_t e0 = s_head[wid][0], e1 = s_head[wid][nt];
+                add_chunk_increments<CH>(vals, bins, incs, e0, e1, s_head[wid], nt, acc, s_stage[wid]);
+
+                // Tiles left to right (rasterizer.rs:232-250): along its row a lane
+                // adds the cells in the reference's order; the carry into a tile is
+                // the carry into the previous tile plus that tile's row sum.
+                for (int i0 = 0; i0 < nt; i0 += 4) {
+                    const int i = i0 + g;
+                    const bool valid = i < nt;
+                    float a[8], h[8];
+                    if (valid) {
+                        const float4 a0 = *reinterpret_cast<const float4*>(&acc[i][acc_idx(8 * y)]);
+                        const float4 a1 = *reinterpret_cast<const float4*>(&acc[i][acc_idx(8 * y + 4)]);
+                        const float4 h0 = *reinterpret_cast<const float4*>(&acc[i][ACC_H + acc_idx(8 * y)]);
+                        const float4 h1 = *reinterpret_cast<const float4*>(&acc[i][ACC_H + acc_idx(8 * y + 4)]);
+                        a[0] = a0.x; a[1] = a0.y; a[2] = a0.z; a[3] = a0.w; a[4] = a1.x; a[5] = a1.y; a[6] = a1.z; a[7] = a1.w;
+                        h[0] = h0.x; h[1] = h0.y; h[2] = h0.z; h[3] = h0.w; h[4] = h1.x; h[5] = h1.y; h[6] = h1.z; h[7] = h1.w;
+                    } else {
 #pragma unroll
-                for (int d = 8; d < 32; d <<= 1) {
-                    const float vo = __shfl_up_sync(0xffffffffu, v, d);
-                    if (lane >= d) v = vo + v;
-                }
-                float ex = __shfl_up_sync(0xffffffffu, v, 8);
-                if (g == 0) ex = 0.0f;
-                const float carry = carry_row + ex;
-                carry_row = __shfl_sync(0xffffffffu, carry + rs, 24 + y);
-                if (valid) {
-                    const uint32_t t = t0 + i;
-                    float accum = carry;
-                    uint32_t lo = 0, hi = 0;
-                    float cv[8];
+                        for (int c = 0; c < 8; c++) a[c] = h[c] = 0.0f;
+                    }
+                    const float rs = ((h[0] + h[1]) + (h[2] + h[3])) + ((h[4] + h[5]) + (h[6] + h[7]));
+                    // exclusive sum of rs over the tiles of the pass before this one
+                    float v = rs;
 #pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        const float sum = accum + a[c];
-                        const float cov = fabsf(sum);
-                        cv[c] = cov_signed ? sum : cov;
-                        const uint32_t al = f2u8(rmin(cov * 256.0f, 255.0f));
-                        if (c < 4) lo |= al << (8 * c); else hi |= al << (8 * (c - 4));
-                        accum = accum + h[c];
+                    for (int d = 8; d < 32; d <<= 1) {
+                        const float vo = __shfl_up_sync(0xffffffffu, v, d);
+                        if (lane >= d) v = vo + v;
                     }
-                    reinterpret_cast<uint2*>(out_alpha + (size_t)t * 64)[y] = make_uint2(lo, hi);
-                    if (out_cov) {
-                        float4* o = reinterpret_cast<float4*>(out_cov + (size_t)t * 64 + 8 * y);
-                        o[0] = make_float4(cv[0], cv[1], cv[2], cv[3]);
-                        o[1] = make_float4(cv[4], cv[5], cv[6], cv[7]);
-                    }
-                    if (y == 0) {
-                        const TileInfo& ti = s_info[wid][i];
-                        out_xy[t] = (uint32_t)(uint16_t)(int16_t)(ti.tx * 8) |
-                                    ((uint32_t)(uint16_t)(int16_t)(ti.ty * 8) << 16);
-                        const TileInfo& nx = s_info[wid][i + 1];
-                        uint32_t has_span = 0;
-                        if (nx.raster == ti.raster && nx.ty == ti.ty && nx.tx > ti.tx + 1 && ti.wind != 0) {
-                            has_span = 1;
-                            const uint32_t x = (uint16_t)(int16_t)((ti.tx + 1) * 8);
-                            const uint32_t yy = (uint16_t)(int16_t)(ti.ty * 8);
-                            const uint32_t wd = (uint16_t)((uint16_t)(nx.tx - ti.tx - 1) * 8u);
-                            span_val[t] = (uint64_t)x | ((uint64_t)yy << 16) | ((uint64_t)wd << 32);
+                    float ex = __shfl_up_sync(0xffffffffu, v, 8);
+                    if (g == 0) ex = 0.0f;
+                    const float carry = carry_row + ex;
+                    carry_row = __shfl_sync(0xffffffffu, carry + rs, 24 + y);
+                    if (valid) {
+                        const uint32_t t = t0 + i;
+                        float accum = carry;
+                        uint32_t lo = 0, hi = 0;
+                        float cv[8];
+#pragma unroll
+                        for (int c = 0; c < 8; c++) {
+                            const float sum = accum + a[c];
+                            const float cov = fabsf(sum);
+                            cv[c] = cov_signed ? sum : cov;
+                            const uint32_t al = f2u8(rmin(cov * 256.0f, 255.0f));
+                            if (c < 4) lo |= al << (8 * c); else hi |= al << (8 * (c - 4));
+                            accum = accum + h[c];
                         }
-                        span_flag[t] = has_span;
+                        reinterpret_cast<uint2*>(out_alpha + (size_t)t * 64)[y] = make_uint2(lo, hi);
+                        if (out_cov) {
+                            float4* o = reinterpret_cast<float4*>(out_cov + (size_t)t * 64 + 8 * y);
+                            o[0] = make_float4(cv[0], cv[1], cv[2], cv[3]);
+                            o[1] = make_float4(cv[4], cv[5], cv[6], cv[7]);
+                        }
+                        if (y == 0) {
+                            const uint32_t xy = s_xy[wid][i];
+                            out_xy[t] = pack_tile(tile_tx(xy) * 8, tile_ty(xy) * 8);
+                        }
                     }
                 }
+                __syncwarp();
             }
-            __syncwarp();
         }
     }
 }
 
-// Row starts: the tiles that begin a (raster, tile_y) row, compacted.
-struct RowIn {
-    const TileInfo* info;
-    __device__ __forceinline__ uint32_t operator()(uint64_t t) const { return info[t].row_head; }
-};
-struct RowOut {
-    uint32_t* row_start;
-    __device__ __forceinline__ void operator()(uint64_t t, uint32_t ex, uint32_t v) const {
-        if (v) row_start[ex] = (uint32_t)t;
+// Spans (rasterizer.rs:252-265): a tile is followed by one when the next tile
+// of its row leaves a gap and its winding is nonzero.
+struct SpanIn {
+    const uint32_t* xy;
+    const uint32_t* rf;
+    uint32_t n_tiles;
+    const uint32_t* n_dev;   // device-held tile count (graph replays), else null
+    __device__ __forceinline__ uint32_t operator()(uint64_t t) const {
+        if (t + 1 >= dev_count(n_tiles, n_dev) || (rf[t + 1] & RF_ROW) || !(rf[t] & RF_WIND)) return 0u;
+        return tile_tx(xy[t + 1]) > tile_tx(xy[t]) + 1 ? 1u : 0u;
     }
 };
-
-struct SpanIn {
-    const uint32_t* flag;
-    __device__ __forceinline__ uint32_t operator()(uint64_t t) const { return flag[t]; }
-};
 struct SpanOut {
-    const uint64_t* val;
-    const TileInfo* info;
+    const uint32_t* xy;
+    const uint32_t* rf;
     uint32_t n_tiles, n_rasters;
-    const uint32_t* n_dev;   // device-held tile count (graph replays), else null
-    uint32_t* xy;
+    const uint32_t* n_dev;
+    uint32_t* out_xy;
     uint16_t* w;
     uint32_t* tile;
     uint32_t* raster_span_off;
     __device__ __forceinline__ void operator()(uint64_t t, uint32_t ex, uint32_t v) const {
         if (v) {
-            const uint64_t s = val[t];
-            xy[ex] = (uint32_t)(s & 0xffffffffu);
-            w[ex] = (uint16_t)(s >> 32);
+            const int tx = tile_tx(xy[t]), ty = tile_ty(xy[t]);
+            out_xy[ex] = pack_tile((tx + 1) * 8, ty * 8);
+            w[ex] = (uint16_t)((uint16_t)(tile_tx(xy[t + 1]) - tx - 1) * 8u);
             tile[ex] = (uint32_t)t;
         }
-        const int r = info[t].raster;
-        if (t == 0 || info[t - 1].raster != r) raster_span_off[r] = ex;
+        const uint32_t r = rf[t] & RF_RASTER;
+        if ((rf[t] & RF_ROW) && (t == 0 || (rf[t - 1] & RF_RASTER) != r)) raster_span_off[r] = ex;
         if (t + 1 == dev_count(n_tiles, n_dev)) raster_span_off[n_rasters] = ex + v;
     }
 };
@@ -596,7 +725,8 @@ struct SpanOut {
 constexpr uint32_t ROW_FORM_MIN_ROWS_PER_SM = 64;
 
 template <int TPW>
-static void launch_tile_cov(ochre_gpu_ctx* ctx, uint32_t T, uint32_t n_rows, bool want_cov, cudaStream_t s) {
+static void launch_tile_cov(ochre_gpu_ctx* ctx, const TileView& tiles, uint32_t T, uint32_t n_rows, bool want_cov,
+                            cudaStream_t s) {
     DevScalars* ds = dev_scalars(ctx);
     int sms = 152;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
@@ -611,18 +741,16 @@ static void launch_tile_cov(ochre_gpu_ctx* ctx, uint32_t T, uint32_t n_rows, boo
         // no more warps than rows, nor than the GPU keeps resident (16 CTAs of 4 warps per SM)
         const uint32_t ctas = (uint32_t)std::min<uint64_t>(((uint64_t)n_rows + 3) / 4, (uint64_t)sms * 16);
         k_tile_cov<TPW><<<ctas, 128, 0, s>>>(
-            ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), ctx->tile_info.as<TileInfo>(),
-            T, t_dev, ctx->tile_row_start.as<uint32_t>(), &ds->n_rows, &ds->ticket, ctx->out_tile_xy.as<uint32_t>(),
-            ctx->out_tile_alpha.as<uint8_t>(), cov, ctx->span_flag.as<uint32_t>(), ctx->span_val.as<uint64_t>(),
+            ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), tiles, T, t_dev,
+            &ds->ticket, ctx->out_tile_xy.as<uint32_t>(), ctx->out_tile_alpha.as<uint8_t>(), cov,
             &ds->err, ctx->cov_signed);
     } else {
         const uint32_t blocks = (T + TPW - 1) / TPW;
         cudaMemsetAsync(ctx->tile_state.p, 0, (size_t)blocks * sizeof(TileBlockState), s);
         k_tile_cov_blocks<TPW><<<(blocks + 3) / 4, 128, 0, s>>>(
-            ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), ctx->tile_info.as<TileInfo>(),
-            T, t_dev, ctx->tile_state.as<TileBlockState>(), &ds->ticket, ctx->out_tile_xy.as<uint32_t>(),
-            ctx->out_tile_alpha.as<uint8_t>(), cov, ctx->span_flag.as<uint32_t>(), ctx->span_val.as<uint64_t>(),
-            &ds->err, ctx->cov_signed);
+            ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), tiles, T, t_dev,
+            ctx->tile_state.as<TileBlockState>(), &ds->ticket, ctx->out_tile_xy.as<uint32_t>(),
+            ctx->out_tile_alpha.as<uint8_t>(), cov, &ds->err, ctx->cov_signed);
     }
 }
 
@@ -631,84 +759,77 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
                       uint32_t* n_spans_out) {
     DevScalars* ds = dev_scalars(ctx);
     const uint32_t R = in->n_rasters;
+    // tile metadata: no more tiles than entries
     OCHRE_CUDA_TRY(ctx->tile_head.ensure(E * 4));
-    OCHRE_CUDA_TRY(ctx->tile_head_bins.ensure(E * 4));
-    OCHRE_CUDA_TRY(ctx->tile_head_wind.ensure(E * 4));
+    OCHRE_CUDA_TRY(ctx->tile_xy.ensure(E * 4));
+    OCHRE_CUDA_TRY(ctx->tile_rf.ensure(E * 4));
+    OCHRE_CUDA_TRY(ctx->out_raster_tile_off.ensure((size_t)(R + 1) * 4));
+    OCHRE_CUDA_TRY(ctx->out_raster_span_off.ensure((size_t)(R + 1) * 4));
     // graph replays: E and T are capacities, the counts stay on the device
     const GraphPlan* plan = ctx->plan;
     const uint32_t* t_dev = plan ? &ds->n_tiles : nullptr;
-    OCHRE_LAUNCH(ctx, "tile_head_scan", s,
-                 OCHRE_CUDA_TRY(launch_scan<HeadScan>(
-                     ctx, E, HeadIn<K>{ctx->keys.as<K>(), ctx->vals.as<uint32_t>()},
-                     HeadOut{ctx->tile_head.as<uint32_t>(), ctx->tile_head_bins.as<uint32_t>(),
-                             ctx->tile_head_wind.as<int32_t>()},
-                     OpHead{}, HeadScan{0u, 0u, 0, 0u}, reinterpret_cast<HeadScan*>(&ds->n_tiles), s, plan ? &ds->n_entries : nullptr)));
-    int st = OCHRE_OK;
-    uint32_t T;
-    if (plan) {
-        OCHRE_LAUNCH(ctx, "plan_tiles", s, OCHRE_CUDA_TRY(launch_plan_cap(ctx, &ds->n_tiles, plan->tiles, s)));
-        T = plan->tiles;
-    } else {
-        st = read_scalars(ctx, s);
-        if (st != OCHRE_OK) return st;
-        st = check_device_error(ctx);
-        if (st != OCHRE_OK) return st;
-        T = host_scalars(ctx)->n_tiles;
-    }
-    *n_tiles_out = T;
-    OCHRE_CUDA_TRY(ctx->tile_info.ensure((size_t)T * sizeof(TileInfo)));
-    OCHRE_CUDA_TRY(ctx->tile_row_start.ensure((size_t)T * 4));
-    OCHRE_CUDA_TRY(ctx->tile_state.ensure((size_t)((T + 3) / 4) * sizeof(TileBlockState)));
-    OCHRE_CUDA_TRY(ctx->span_flag.ensure((size_t)T * 4));
-    OCHRE_CUDA_TRY(ctx->span_val.ensure((size_t)T * 8));
-    OCHRE_CUDA_TRY(ctx->out_tile_xy.ensure((size_t)T * 4));
-    OCHRE_CUDA_TRY(ctx->out_tile_alpha.ensure((size_t)T * 64));
-    const bool want_cov = (ctx->flags & OCHRE_CTX_WANT_COV) != 0;
-    if (want_cov) OCHRE_CUDA_TRY(ctx->out_tile_cov.ensure((size_t)T * 64 * 4));
-    OCHRE_CUDA_TRY(ctx->out_raster_tile_off.ensure((size_t)(R + 1) * 4));
-    OCHRE_CUDA_TRY(ctx->out_raster_span_off.ensure((size_t)(R + 1) * 4));
-    if (T)
-        OCHRE_LAUNCH(ctx, "tile_info", s,
-                     k_tile_info<<<(T + 255) / 256, 256, 0, s>>>(
-                         ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->tile_head.as<uint32_t>(),
-                         ctx->tile_head_bins.as<uint32_t>(), ctx->tile_head_wind.as<int32_t>(),
-                         ctx->raster_wbase.as<int32_t>(), &ds->n_bins, T, t_dev, R, ctx->tile_info.as<TileInfo>(),
-                         ctx->out_raster_tile_off.as<uint32_t>(), &ds->err));
+    const uint32_t* e_dev = plan ? &ds->n_entries : nullptr;
+    const TileView tiles{ctx->tile_head.as<uint32_t>(), ctx->tile_xy.as<uint32_t>(), ctx->tile_rf.as<uint32_t>(),
+                         (uint32_t)E, e_dev};
+    static_assert(offsetof(DevScalars, head_wind) == offsetof(DevScalars, n_tiles) + 4, "HeadScan layout");
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    const int steps = E < (uint64_t)sms * 2 * HEAD_BLOCK * 16 ? 4 : 16;
+    const uint32_t blocks = (uint32_t)((E + HEAD_BLOCK * steps - 1) / (HEAD_BLOCK * steps));
+    ScanSpace sp;
+    OCHRE_CUDA_TRY(scan_space(ctx, blocks * sizeof(ScanStatus<HeadScan>), blocks, 0u, s, &sp));
+    const HeadArgs args{ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->raster_wbase.as<int32_t>(), E, e_dev, R,
+                        ctx->tile_head.as<uint32_t>(), ctx->tile_xy.as<uint32_t>(), ctx->tile_rf.as<uint32_t>(),
+                        ctx->out_raster_tile_off.as<uint32_t>(), reinterpret_cast<HeadScan*>(&ds->n_tiles),
+                        &ds->n_rows};
+    auto* status = reinterpret_cast<ScanStatus<HeadScan>*>(sp.status);
+    if (steps == 4)
+        OCHRE_LAUNCH(ctx, "tile_heads", s, k_tile_heads<K, 4><<<blocks, HEAD_BLOCK, 0, s>>>(
+            ctx->keys.as<K>(), args, status, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
+    else
+        OCHRE_LAUNCH(ctx, "tile_heads", s, k_tile_heads<K, 16><<<blocks, HEAD_BLOCK, 0, s>>>(
+            ctx->keys.as<K>(), args, status, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
-    if (T) {
-        OCHRE_LAUNCH(ctx, "tile_row_scan", s,
-                     OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-                         ctx, T, RowIn{ctx->tile_info.as<TileInfo>()}, RowOut{ctx->tile_row_start.as<uint32_t>()},
-                         OpSumU32{}, 0u, &ds->n_rows, s, t_dev)));
-    }
-    uint32_t n_rows;
+    int st = OCHRE_OK;
+    uint32_t T, n_rows;
     if (plan) {
+        OCHRE_LAUNCH(ctx, "plan_tiles", s, k_plan_tiles<<<1, 1, 0, s>>>(ds, plan->tiles));
+        OCHRE_CUDA_TRY(cudaGetLastError());
+        T = plan->tiles;
         n_rows = plan->rows;
     } else {
         st = read_scalars(ctx, s);
         if (st != OCHRE_OK) return st;
         st = check_device_error(ctx);
         if (st != OCHRE_OK) return st;
+        T = host_scalars(ctx)->n_tiles;
         n_rows = host_scalars(ctx)->n_rows;
     }
-    switch (ctx->tune_chain_tiles_per_warp) {
-    case 4: OCHRE_LAUNCH(ctx, "tile_coverage", s, launch_tile_cov<4>(ctx, T, n_rows, want_cov, s)); break;
-    case 8: OCHRE_LAUNCH(ctx, "tile_coverage", s, launch_tile_cov<8>(ctx, T, n_rows, want_cov, s)); break;
-    case 16: OCHRE_LAUNCH(ctx, "tile_coverage", s, launch_tile_cov<16>(ctx, T, n_rows, want_cov, s)); break;
-    default: return OCHRE_E_INVALID;
-    }
-    OCHRE_CUDA_TRY(cudaGetLastError());
+    *n_tiles_out = T;
+    const uint32_t tpw = (uint32_t)ctx->tune_chain_tiles_per_warp;
+    OCHRE_CUDA_TRY(ctx->tile_state.ensure((size_t)((T + tpw - 1) / tpw) * sizeof(TileBlockState)));
+    OCHRE_CUDA_TRY(ctx->out_tile_xy.ensure((size_t)T * 4));
+    OCHRE_CUDA_TRY(ctx->out_tile_alpha.ensure((size_t)T * 64));
+    const bool want_cov = (ctx->flags & OCHRE_CTX_WANT_COV) != 0;
+    if (want_cov) OCHRE_CUDA_TRY(ctx->out_tile_cov.ensure((size_t)T * 64 * 4));
     // Spans: compact in tile order.  Capacity: at most one span per tile.
     OCHRE_CUDA_TRY(ctx->out_span_xy.ensure((size_t)T * 4));
     OCHRE_CUDA_TRY(ctx->out_span_w.ensure((size_t)T * 2));
     OCHRE_CUDA_TRY(ctx->out_span_tile.ensure((size_t)T * 4));
     OCHRE_LAUNCH(ctx, "span_scan", s,
                  OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-                     ctx, T, SpanIn{ctx->span_flag.as<uint32_t>()},
-                     SpanOut{ctx->span_val.as<uint64_t>(), ctx->tile_info.as<TileInfo>(), T, R, t_dev,
-                             ctx->out_span_xy.as<uint32_t>(), ctx->out_span_w.as<uint16_t>(),
-                             ctx->out_span_tile.as<uint32_t>(), ctx->out_raster_span_off.as<uint32_t>()},
+                     ctx, T, SpanIn{tiles.xy, tiles.rf, T, t_dev},
+                     SpanOut{tiles.xy, tiles.rf, T, R, t_dev, ctx->out_span_xy.as<uint32_t>(),
+                             ctx->out_span_w.as<uint16_t>(), ctx->out_span_tile.as<uint32_t>(),
+                             ctx->out_raster_span_off.as<uint32_t>()},
                      OpSumU32{}, 0u, &ds->n_spans, s, t_dev)));
+    switch (tpw) {
+    case 4: OCHRE_LAUNCH(ctx, "tile_coverage", s, launch_tile_cov<4>(ctx, tiles, T, n_rows, want_cov, s)); break;
+    case 8: OCHRE_LAUNCH(ctx, "tile_coverage", s, launch_tile_cov<8>(ctx, tiles, T, n_rows, want_cov, s)); break;
+    case 16: OCHRE_LAUNCH(ctx, "tile_coverage", s, launch_tile_cov<16>(ctx, tiles, T, n_rows, want_cov, s)); break;
+    default: return OCHRE_E_INVALID;
+    }
+    OCHRE_CUDA_TRY(cudaGetLastError());
     if (plan) {
         *n_spans_out = 0;   // on the device; read after the replay
         return OCHRE_OK;
@@ -716,7 +837,7 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
     st = read_scalars(ctx, s);
     if (st != OCHRE_OK) return st;
     *n_spans_out = host_scalars(ctx)->n_spans;
-    ctx->stats.n_bins = host_scalars(ctx)->n_bins;
+    ctx->stats.n_bins = E - host_scalars(ctx)->n_cross;
     return check_device_error(ctx);
 }
 
