@@ -97,11 +97,13 @@ void HostBuf::release() {
 }
 
 __global__ void k_copy_words(const uint32_t* __restrict__ src, uint32_t n, uint32_t* dst) {
+    dependent_start();
     const uint32_t i = threadIdx.x;
     if (i < n) dst[i] = src[i];
 }
 
 __global__ void k_plan_cap(uint32_t* count, uint32_t cap, uint32_t* err) {
+    dependent_start();
     if (*count > cap) {
         *count = 0u;
         atomicOr(err, ERR_CAPACITY);
@@ -109,6 +111,7 @@ __global__ void k_plan_cap(uint32_t* count, uint32_t cap, uint32_t* err) {
 }
 
 __global__ void k_plan_entries(DevScalars* ds, uint32_t cap, uint32_t key_bits, uint32_t inc_cap) {
+    dependent_start();
     const uint64_t e = (uint64_t)ds->line_ent_total + ds->n_empty;
     const uint64_t k = ds->keyspace;
     const bool keys_fit = key_bits >= 64 || k == 0 || ((k - 1) >> key_bits) == 0;
@@ -122,13 +125,13 @@ __global__ void k_plan_entries(DevScalars* ds, uint32_t cap, uint32_t key_bits, 
 }
 
 cudaError_t launch_plan_cap(ochre_gpu_ctx* ctx, uint32_t* count, uint32_t cap, cudaStream_t s) {
-    k_plan_cap<<<1, 1, 0, s>>>(count, cap, &dev_scalars(ctx)->err);
+    launch_after(k_plan_cap, 1, 1, 0, s, count, cap, &dev_scalars(ctx)->err);
     return cudaGetLastError();
 }
 
 cudaError_t launch_plan_entries(ochre_gpu_ctx* ctx, uint32_t cap, uint32_t key_bits, uint32_t inc_cap,
                                 cudaStream_t s) {
-    k_plan_entries<<<1, 1, 0, s>>>(dev_scalars(ctx), cap, key_bits, inc_cap);
+    launch_after(k_plan_entries, 1, 1, 0, s, dev_scalars(ctx), cap, key_bits, inc_cap);
     return cudaGetLastError();
 }
 
@@ -141,7 +144,7 @@ void wait_inputs(ochre_gpu_ctx* ctx, cudaStream_t s) {
 int copy_scalars_async(ochre_gpu_ctx* ctx, cudaStream_t s) {
     static_assert(sizeof(DevScalars) / 4 <= 64, "one word per thread of k_copy_words");
     if (ctx->h_scalars_dev) {
-        k_copy_words<<<1, 64, 0, s>>>(ctx->scalars.as<uint32_t>(), (uint32_t)(sizeof(DevScalars) / 4),
+        launch_after(k_copy_words, 1, 64, 0, s, ctx->scalars.as<uint32_t>(), (uint32_t)(sizeof(DevScalars) / 4),
                                        static_cast<uint32_t*>(ctx->h_scalars_dev));
         OCHRE_CUDA_TRY(cudaGetLastError());
     } else {

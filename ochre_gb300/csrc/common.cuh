@@ -46,6 +46,18 @@ constexpr long long SPIN_LIMIT = 1ll << 21;  // polls of a look-back flag (about
 // holds both (internal.h checks the layout).
 constexpr int SPIN_LOG2_WORD = 22;
 
+// First statement of every kernel.  Kernels that follow one another on a
+// stream are launched so that the next one's blocks may be placed while this
+// one still runs (launch_after, internal.h): every block says at once that it
+// has started, which lets the next kernel in when the last block has, and waits
+// for the kernels before it to finish before it reads or writes anything.  No
+// block of a kernel waits on a block not yet placed: the next kernel's blocks
+// come only when all of this one's have.
+__device__ __forceinline__ void dependent_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // The count a kernel works on: its launch-time value, or, when the count is
 // held on the device (launch chains replayed from a CUDA graph), the device
 // value, never more than the launch-time capacity.

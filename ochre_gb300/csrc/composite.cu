@@ -88,6 +88,7 @@ struct PieceOff {
 template <class K>
 __global__ void k_piece_emit(PieceItems items, uint32_t rbits, const uint32_t* __restrict__ off, K* __restrict__ keys,
                              uint32_t* __restrict__ vals) {
+    dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= (uint64_t)items.T + items.N) return;
     const PieceItems::Item it = items((uint32_t)i);
@@ -107,6 +108,7 @@ constexpr uint32_t NO_PIECE = 0xffffffffu;
 template <class K>
 __global__ void k_piece_heads(const K* __restrict__ keys, uint32_t E, uint32_t rbits, uint32_t n_tiles,
                               uint32_t* __restrict__ head, const uint32_t* err) {
+    dependent_start();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= E || run_aborted(err)) return;   // a wait of the sort gave up: the sorted pieces are not valid
     const K st = keys[e] >> rbits;
@@ -189,6 +191,7 @@ __global__ void __launch_bounds__(128) k_composite(const K* __restrict__ keys, c
                                                    const uint32_t* __restrict__ colors, uint32_t n_rasters, uint32_t w,
                                                    uint32_t h, uint32_t w8, uint32_t h8, uint32_t* __restrict__ canvas,
                                                    float neg_zero, const uint32_t* err) {
+    dependent_start();
     const uint32_t st = (uint32_t)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5);
     const uint32_t lane = threadIdx.x & 31u;
     // a wait of the sort gave up: the sorted pieces are not valid
@@ -275,7 +278,7 @@ static int composite_pieces(ochre_gpu_ctx* ctx, const PieceItems& items, uint32_
     OCHRE_CUDA_TRY(ctx->keys_alt.ensure((size_t)E * sizeof(K)));
     OCHRE_CUDA_TRY(ctx->vals_alt.ensure((size_t)E * 4));
     OCHRE_CUDA_TRY(ctx->tile_head.ensure((size_t)screen * 4));
-    OCHRE_LAUNCH(ctx, "composite_pieces", s, k_piece_emit<K><<<(unsigned)((S + 255) / 256), 256, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "composite_pieces", s, launch_after(k_piece_emit<K>, (unsigned)((S + 255) / 256), 256, 0, s, 
         items, rbits, ctx->line_ent_off.as<uint32_t>(), ctx->keys.as<K>(), ctx->vals.as<uint32_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());
     uint32_t passes = 0;
@@ -283,10 +286,10 @@ static int composite_pieces(ochre_gpu_ctx* ctx, const PieceItems& items, uint32_
     if (st != OCHRE_OK) return st;
     uint32_t* head = ctx->tile_head.as<uint32_t>();
     OCHRE_CUDA_TRY(cudaMemsetAsync(head, 0xff, (size_t)screen * 4, s));
-    OCHRE_LAUNCH(ctx, "composite_heads", s, k_piece_heads<K><<<(E + 255) / 256, 256, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "composite_heads", s, launch_after(k_piece_heads<K>, (E + 255) / 256, 256, 0, s, 
         ctx->keys.as<K>(), E, rbits, screen, head, &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
-    OCHRE_LAUNCH(ctx, "composite", s, k_composite<K><<<(unsigned)(((uint64_t)screen * 32 + 127) / 128), 128, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "composite", s, launch_after(k_composite<K>, (unsigned)(((uint64_t)screen * 32 + 127) / 128), 128, 0, s, 
         ctx->keys.as<K>(), ctx->vals.as<uint32_t>(), E, head, rbits, items.T, tile_alpha,
         reinterpret_cast<const uint32_t*>(colors), items.R, (uint32_t)items.w, (uint32_t)items.h, w8, h8,
         reinterpret_cast<uint32_t*>(canvas), -0.0f, &ds->err));

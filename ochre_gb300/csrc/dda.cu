@@ -351,6 +351,7 @@ __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restr
                                                            uint32_t* __restrict__ inc_counts,
                                                            unsigned long long* inc_total, uint32_t* n_cross,
                                                            uint32_t* ticket, uint32_t* err) {
+    dependent_start();
     constexpr int WARPS = WALK_BLOCK / 32;
     __shared__ int4 s_box[WARPS][BOX_SLOTS];
     __shared__ int s_ws[WARPS][BOX_SLOTS];
@@ -438,6 +439,7 @@ struct LinePairOut {
 };
 
 __global__ void k_bbox_init(int4* bbox, int* wsum, uint32_t n) {
+    dependent_start();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         bbox[i] = make_int4(0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000);
@@ -720,6 +722,7 @@ __global__ void __launch_bounds__(LONG_THREADS) k_line_emit_long(
     const uint64_t* __restrict__ key_base, K* __restrict__ keys, uint32_t* __restrict__ vals,
     BinRec* __restrict__ bins, float2* __restrict__ incs, const uint32_t* __restrict__ queue, const uint32_t* n_queue,
     uint32_t* ticket) {
+    dependent_start();
     // (a line count zeroed on the device, after an overflow of a graph's
     // plan, stops these walks too: their offsets were not written)
     if (dev_count(n_cap, n_dev) == 0) return;
@@ -742,6 +745,7 @@ __global__ void __launch_bounds__(256) k_line_emit(const float4* __restrict__ li
                             const uint32_t* n_dev, const int4* __restrict__ bbox, const uint64_t* __restrict__ key_base,
                             K* __restrict__ keys, uint32_t* __restrict__ vals, BinRec* __restrict__ bins,
                             float2* __restrict__ incs, uint32_t long_cells) {
+    dependent_start();
     __shared__ uint32_t s_cnt[17];
     __shared__ uint16_t s_item[256];
     const uint64_t n_lines = dev_count(n_cap, n_dev);
@@ -773,6 +777,7 @@ __global__ void k_empty_emit(const uint32_t* __restrict__ empty, uint32_t n_rast
                              const uint32_t* first_dev, const uint32_t* n_ent_dev,
                              const uint64_t* __restrict__ key_base, K* __restrict__ keys,
                              uint32_t* __restrict__ vals, BinRec* __restrict__ bins) {
+    dependent_start();
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n_rasters) return;
     const uint32_t rank = empty[r];
@@ -853,7 +858,7 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
     OCHRE_CUDA_TRY(ctx->raster_empty.ensure((size_t)R * 4));
     OCHRE_CUDA_TRY(ctx->raster_wsum.ensure((size_t)R * 4));
     OCHRE_CUDA_TRY(ctx->raster_wbase.ensure((size_t)R * 4));
-    OCHRE_LAUNCH(ctx, "bbox_init", s, k_bbox_init<<<(R + 255) / 256, 256, 0, s>>>(ctx->raster_bbox.as<int4>(),
+    OCHRE_LAUNCH(ctx, "bbox_init", s, launch_after(k_bbox_init, (R + 255) / 256, 256, 0, s, ctx->raster_bbox.as<int4>(),
                                                                                  ctx->raster_wsum.as<int>(), R));
     OCHRE_CUDA_TRY(cudaGetLastError());
     // the line pair's totals, the 64-bit increment count, the long lines' ticket
@@ -882,7 +887,7 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
         unsigned count_grid = 1;
         uint32_t groups = 1;
         count_shape(ctx, n_lines, &count_grid, &groups);
-        OCHRE_LAUNCH(ctx, "dda_count", s, k_line_count<<<count_grid, WALK_BLOCK, 0, s>>>(
+        OCHRE_LAUNCH(ctx, "dda_count", s, launch_after(k_line_count, count_grid, WALK_BLOCK, 0, s, 
             ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), n_lines, lines_dev, groups,
             ctx->raster_bbox.as<int4>(),
             ctx->raster_wsum.as<int>(), ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>(),
@@ -954,13 +959,13 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), queue, &ds->n_long, &ds->walk_ticket));
         if (ctx->keys64)
-            OCHRE_LAUNCH(ctx, "dda_emit", s, k_line_emit<uint64_t><<<(unsigned)((n_lines + 255) / 256), 256, 0, s>>>(
+            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint64_t>, (unsigned)((n_lines + 255) / 256), 256, 0, s, 
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint64_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), long_cells));
         else
-            OCHRE_LAUNCH(ctx, "dda_emit", s, k_line_emit<uint32_t><<<(unsigned)((n_lines + 255) / 256), 256, 0, s>>>(
+            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint32_t>, (unsigned)((n_lines + 255) / 256), 256, 0, s, 
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),
@@ -972,12 +977,12 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
         const uint32_t* first_dev = plan ? &ds->line_ent_total : nullptr;
         const uint32_t* ent_dev = plan ? &ds->n_entries : nullptr;
         if (ctx->keys64)
-            OCHRE_LAUNCH(ctx, "empty_emit", s, k_empty_emit<uint64_t><<<(R + 255) / 256, 256, 0, s>>>(
+            OCHRE_LAUNCH(ctx, "empty_emit", s, launch_after(k_empty_emit<uint64_t>, (R + 255) / 256, 256, 0, s, 
                 ctx->raster_empty.as<uint32_t>(), R, first_entry, first_dev, ent_dev,
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint64_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>()));
         else
-            OCHRE_LAUNCH(ctx, "empty_emit", s, k_empty_emit<uint32_t><<<(R + 255) / 256, 256, 0, s>>>(
+            OCHRE_LAUNCH(ctx, "empty_emit", s, launch_after(k_empty_emit<uint32_t>, (R + 255) / 256, 256, 0, s, 
                 ctx->raster_empty.as<uint32_t>(), R, first_entry, first_dev, ent_dev,
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>()));

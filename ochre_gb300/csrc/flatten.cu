@@ -124,6 +124,7 @@ struct Load32 {
 // (a scan would give each of a handful of threads eight serial t loops).
 template <class In>
 __global__ void __launch_bounds__(128) k_count_each(uint64_t n, In in, uint32_t* __restrict__ out) {
+    dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i < n) out[i] = in(i);
 }
@@ -135,6 +136,7 @@ constexpr uint64_t SPLIT_COUNT_TILES = 256;
 __global__ void k_cmd_emit(BatchView b, const uint32_t* __restrict__ line_off, uint32_t n_lines_cap,
                            float4* __restrict__ lines, uint32_t* __restrict__ line_raster, uint32_t long_cells,
                            uint32_t* __restrict__ long_lines, uint32_t* n_long, uint32_t* err) {
+    dependent_start();
     const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (c >= b.n_cmds) return;
     const CmdCtx k = load_cmd(b, (uint32_t)c);
@@ -181,7 +183,7 @@ int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uin
                 ctx->cmd_ep.as<uint32_t>(), in->n_floats};
     if (scan_tiles(n) < SPLIT_COUNT_TILES) {
         // counts first (one thread per command), then the offsets in place
-        OCHRE_LAUNCH(ctx, "flatten_count", s, k_count_each<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(
+        OCHRE_LAUNCH(ctx, "flatten_count", s, launch_after(k_count_each<CountIn>, (unsigned)((n + 127) / 128), 128, 0, s, 
             n, CountIn{b, &ds->err}, ctx->cmd_line_off.as<uint32_t>()));
         OCHRE_CUDA_TRY(cudaGetLastError());
         OCHRE_LAUNCH(ctx, "flatten_count_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
@@ -212,7 +214,7 @@ int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uin
     if (long_cells) OCHRE_CUDA_TRY(ctx->long_lines.ensure((size_t)L * 4));
     OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->n_long, 0, 4, s));
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    OCHRE_LAUNCH(ctx, "flatten_emit", s, k_cmd_emit<<<blocks, 256, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "flatten_emit", s, launch_after(k_cmd_emit, blocks, 256, 0, s, 
         b, ctx->cmd_line_off.as<uint32_t>(), L, ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), long_cells,
         long_cells ? ctx->long_lines.as<uint32_t>() : nullptr, &ds->n_long, &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());

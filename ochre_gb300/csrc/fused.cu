@@ -148,6 +148,7 @@ __device__ __forceinline__ void block_excl_max2(int a, int b, int& a_ex, int& b_
 
 template <int THREADS, int CHUNK>
 __global__ void __launch_bounds__(THREADS, fused_min_ctas(THREADS)) k_raster_fused(FusedArgs A) {
+    dependent_start();
     constexpr int FUSED_THREADS = THREADS;
     constexpr int F_WARPS = THREADS / 32;
     constexpr int F_CMAX = THREADS;   // commands per raster
@@ -623,7 +624,7 @@ static int fused_shape(ochre_gpu_ctx* ctx, const FusedArgs* a, int* grid, cudaSt
             *grid = fused_full_grid<T, C>();                                          \
             return OCHRE_OK;                                                          \
         }                                                                             \
-        OCHRE_LAUNCH(ctx, "raster_fused", s, k_raster_fused<T, C><<<*grid, T, 0, s>>>(*a)); \
+        OCHRE_LAUNCH(ctx, "raster_fused", s, launch_after(k_raster_fused<T, C>, *grid, T, 0, s, *a)); \
         OCHRE_CUDA_TRY(cudaGetLastError());                                           \
         return OCHRE_OK;
     switch (ctx->tune_fused_threads * 1000 + ctx->tune_fused_chunk) {

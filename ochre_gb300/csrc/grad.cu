@@ -44,6 +44,7 @@ __device__ __forceinline__ int tile_y_of(uint32_t xy) { return (int)(int16_t)(xy
 __global__ void k_composite_tiles(const uint32_t* __restrict__ tile_xy, const float* __restrict__ tile_sum,
                                   uint32_t T, const uint32_t* t_dev, const uint32_t* __restrict__ raster_tile_off,
                                   uint32_t R, uint32_t W, uint32_t H, float* __restrict__ cov) {
+    dependent_start();
     const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint32_t t = (uint32_t)(idx >> 6), c = (uint32_t)(idx & 63u);
     if (t >= dev_count(T, t_dev)) return;
@@ -57,6 +58,7 @@ __global__ void k_composite_tiles(const uint32_t* __restrict__ tile_xy, const fl
 __global__ void k_composite_spans(const uint32_t* __restrict__ span_xy, const uint16_t* __restrict__ span_w,
                                   uint32_t N, const uint32_t* n_dev, const uint32_t* __restrict__ raster_span_off,
                                   uint32_t R, uint32_t W, uint32_t H, float* __restrict__ cov) {
+    dependent_start();
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (warp >= dev_count(N, n_dev)) return;
@@ -78,6 +80,7 @@ __global__ void k_composite_spans(const uint32_t* __restrict__ span_xy, const ui
 // the block reduction.  16-byte accesses when all three arrays allow.
 __global__ void k_l2(const float* __restrict__ cov, const float* __restrict__ target, uint64_t n,
                      double* __restrict__ loss, float* __restrict__ dl) {
+    dependent_start();
     float sum = 0.0f, comp = 0.0f;
     auto add = [&](float d) {
         const float y = d * d - comp;
@@ -127,6 +130,7 @@ __global__ void k_l2(const float* __restrict__ cov, const float* __restrict__ ta
 __global__ void k_gsigma(const uint32_t* __restrict__ tile_xy, const float* __restrict__ tile_sum, uint32_t T,
                          const uint32_t* t_dev, const uint32_t* __restrict__ raster_tile_off, uint32_t R, uint32_t W,
                          uint32_t H, const float* __restrict__ dl_dcov, float* __restrict__ gsig) {
+    dependent_start();
     const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint32_t t = (uint32_t)(idx >> 6), c = (uint32_t)(idx & 63u);
     if (t >= dev_count(T, t_dev)) return;
@@ -143,6 +147,7 @@ __global__ void k_gsigma(const uint32_t* __restrict__ tile_xy, const float* __re
 // ---- backward 2: exclusive suffix sums of dL/dS along every canvas row ----
 __global__ void k_row_suffix(const float* __restrict__ gsig, uint64_t rows, uint32_t W, float* __restrict__ gs,
                              float* __restrict__ row_total) {
+    dependent_start();
     const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
@@ -224,6 +229,7 @@ __global__ void k_line_grad(const float4* __restrict__ lines, const uint32_t* __
                             const uint32_t* l_dev, uint32_t W, uint32_t H, const float* __restrict__ gsig,
                             const float* __restrict__ gs, const float* __restrict__ row_total,
                             LineGrad* __restrict__ out) {
+    dependent_start();
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l >= dev_count(L, l_dev)) return;
     const float4 ln = lines[l];
@@ -341,6 +347,7 @@ __global__ void k_cmd_grad(BatchView b, const uint32_t* __restrict__ line_off, u
                            const uint32_t* err, const LineGrad* __restrict__ lg, float* __restrict__ gp, uint32_t W,
                            uint32_t H, const float* __restrict__ gsig, const float* __restrict__ gs,
                            const float* __restrict__ row_total) {
+    dependent_start();
     const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (c >= b.n_cmds) return;
     if (err != nullptr && (ld_relaxed(err) & ERR_CAPACITY)) return;
@@ -513,6 +520,7 @@ __global__ void k_cmd_grad(BatchView b, const uint32_t* __restrict__ line_off, u
 // ---- backward 5: device-space point gradients -> input points and transforms ----
 __global__ void k_fill_grad(BatchView b, const float* __restrict__ gp, float* __restrict__ dl_dpts,
                             float* __restrict__ dl_dxf) {
+    dependent_start();
     const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const bool valid = c < b.n_cmds;
@@ -599,10 +607,10 @@ int stage_diff_tail(ochre_gpu_ctx* ctx, const ochre_batch* in, const DiffStep& d
     if (npx) OCHRE_CUDA_TRY(cudaMemsetAsync(d.cov, 0, npx * sizeof(float), s));
     if (npx && T) {
         OCHRE_LAUNCH(ctx, "composite_tiles", s,
-                     k_composite_tiles<<<(unsigned)(((uint64_t)T * 64 + 255) / 256), 256, 0, s>>>(
+                     launch_after(k_composite_tiles, (unsigned)(((uint64_t)T * 64 + 255) / 256), 256, 0, s, 
                          tile_xy, tile_sum, T, t_dev, tile_off, R, w, h, d.cov));
         OCHRE_LAUNCH(ctx, "composite_spans", s,
-                     k_composite_spans<<<(unsigned)(((uint64_t)T * 32 + 255) / 256), 256, 0, s>>>(
+                     launch_after(k_composite_spans, (unsigned)(((uint64_t)T * 32 + 255) / 256), 256, 0, s, 
                          ctx->out_span_xy.as<uint32_t>(), ctx->out_span_w.as<uint16_t>(), T, n_dev,
                          ctx->out_raster_span_off.as<uint32_t>(), R, w, h, d.cov));
     }
@@ -610,7 +618,7 @@ int stage_diff_tail(ochre_gpu_ctx* ctx, const ochre_batch* in, const DiffStep& d
     OCHRE_CUDA_TRY(cudaMemsetAsync(d.loss, 0, sizeof(double), s));
     if (npx) {
         const int blocks = (int)std::min<uint64_t>((npx + 255) / 256, 152u * 16u);
-        OCHRE_LAUNCH(ctx, "l2_loss", s, k_l2<<<blocks, 256, 0, s>>>(d.cov, d.target, npx, d.loss, d.dl_dcov));
+        OCHRE_LAUNCH(ctx, "l2_loss", s, launch_after(k_l2, blocks, 256, 0, s, d.cov, d.target, npx, d.loss, d.dl_dcov));
     }
     OCHRE_CUDA_TRY(cudaGetLastError());
     // backward (ochre_gpu_fill_backward) on this run's lines and tiles
@@ -626,24 +634,24 @@ int stage_diff_tail(ochre_gpu_ctx* ctx, const ochre_batch* in, const DiffStep& d
     OCHRE_CUDA_TRY(cudaMemsetAsync(gsig, 0, npx * 4, s));
     if (T)
         OCHRE_LAUNCH(ctx, "grad_sigma", s,
-                     k_gsigma<<<(unsigned)(((uint64_t)T * 64 + 255) / 256), 256, 0, s>>>(
+                     launch_after(k_gsigma, (unsigned)(((uint64_t)T * 64 + 255) / 256), 256, 0, s, 
                          tile_xy, tile_sum, T, t_dev, tile_off, R, w, h, d.dl_dcov, gsig));
     const uint64_t rows = (uint64_t)R * h;
     OCHRE_LAUNCH(ctx, "grad_row_suffix", s,
-                 k_row_suffix<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, s>>>(
+                 launch_after(k_row_suffix, (unsigned)((rows * 32 + 255) / 256), 256, 0, s, 
                      gsig, rows, w, ctx->grad_gs.as<float>(), ctx->grad_left.as<float>()));
     OCHRE_LAUNCH(ctx, "grad_lines", s,
-                 k_line_grad<<<(L + 127) / 128, 128, 0, s>>>(ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(),
+                 launch_after(k_line_grad, (L + 127) / 128, 128, 0, s, ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(),
                                                              L, l_dev, w, h, gsig, ctx->grad_gs.as<float>(),
                                                              ctx->grad_left.as<float>(), ctx->grad_line.as<LineGrad>()));
     OCHRE_CUDA_TRY(cudaMemsetAsync(ctx->grad_pts.p, 0, in->n_floats * 4, s));
     const BatchView b = view_of(ctx, in);
     const unsigned cb = (unsigned)((in->n_cmds + 127) / 128);
     OCHRE_LAUNCH(ctx, "grad_commands", s,
-                 k_cmd_grad<<<cb, 128, 0, s>>>(b, ctx->cmd_line_off.as<uint32_t>(), L, l_dev, &ds->err,
+                 launch_after(k_cmd_grad, cb, 128, 0, s, b, ctx->cmd_line_off.as<uint32_t>(), L, l_dev, &ds->err,
                                                ctx->grad_line.as<LineGrad>(), ctx->grad_pts.as<float>(), w, h, gsig,
                                                ctx->grad_gs.as<float>(), ctx->grad_left.as<float>()));
-    OCHRE_LAUNCH(ctx, "grad_fills", s, k_fill_grad<<<cb, 128, 0, s>>>(b, ctx->grad_pts.as<float>(), d.dl_dpts, d.dl_dxf));
+    OCHRE_LAUNCH(ctx, "grad_fills", s, launch_after(k_fill_grad, cb, 128, 0, s, b, ctx->grad_pts.as<float>(), d.dl_dpts, d.dl_dxf));
     OCHRE_CUDA_TRY(cudaGetLastError());
     return OCHRE_OK;
 }
@@ -670,14 +678,14 @@ int ochre_gpu_render_coverage(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_
     if (res.n_tiles) {
         const uint64_t threads = (uint64_t)res.n_tiles * 64;
         OCHRE_LAUNCH(ctx, "composite_tiles", s,
-                     k_composite_tiles<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+                     launch_after(k_composite_tiles, (unsigned)((threads + 255) / 256), 256, 0, s, 
                          reinterpret_cast<const uint32_t*>(res.tile_xy), res.tile_cov, res.n_tiles, nullptr,
                          res.raster_tile_off, in->n_rasters, w, h, cov));
     }
     if (res.n_spans) {
         const uint64_t threads = (uint64_t)res.n_spans * 32;
         OCHRE_LAUNCH(ctx, "composite_spans", s,
-                     k_composite_spans<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+                     launch_after(k_composite_spans, (unsigned)((threads + 255) / 256), 256, 0, s, 
                          reinterpret_cast<const uint32_t*>(res.span_xy), res.span_width, res.n_spans, nullptr,
                          res.raster_span_off, in->n_rasters, w, h, cov));
     }
@@ -697,7 +705,7 @@ int ochre_gpu_l2_loss(ochre_gpu_ctx* ctx, const float* cov, const float* target,
     OCHRE_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(double), s));
     if (n == 0) return OCHRE_OK;
     int blocks = (int)std::min<uint64_t>((n + 255) / 256, 152u * 16u);
-    OCHRE_LAUNCH(ctx, "l2_loss", s, k_l2<<<blocks, 256, 0, s>>>(cov, target, n, loss, dl_dcov));
+    OCHRE_LAUNCH(ctx, "l2_loss", s, launch_after(k_l2, blocks, 256, 0, s, cov, target, n, loss, dl_dcov));
     OCHRE_CUDA_TRY(cudaGetLastError());
     collect_timings(ctx, s);
     return OCHRE_OK;
@@ -744,28 +752,28 @@ int ochre_gpu_fill_backward(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t 
     if (res.n_tiles) {
         const uint64_t threads = (uint64_t)res.n_tiles * 64;
         OCHRE_LAUNCH(ctx, "grad_sigma", s,
-                     k_gsigma<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(
+                     launch_after(k_gsigma, (unsigned)((threads + 255) / 256), 256, 0, s, 
                          reinterpret_cast<const uint32_t*>(res.tile_xy), res.tile_cov, res.n_tiles, nullptr,
                          res.raster_tile_off, R, w, h, dl_dcov, gsig));
     }
     const uint64_t rows = (uint64_t)R * h;
     OCHRE_LAUNCH(ctx, "grad_row_suffix", s,
-                 k_row_suffix<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, s>>>(
+                 launch_after(k_row_suffix, (unsigned)((rows * 32 + 255) / 256), 256, 0, s, 
                      gsig, rows, w, ctx->grad_gs.as<float>(), ctx->grad_left.as<float>()));
     OCHRE_LAUNCH(ctx, "grad_lines", s,
-                 k_line_grad<<<(L + 127) / 128, 128, 0, s>>>(ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(),
+                 launch_after(k_line_grad, (L + 127) / 128, 128, 0, s, ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(),
                                                              L, nullptr, w, h, gsig, ctx->grad_gs.as<float>(),
                                                              ctx->grad_left.as<float>(), ctx->grad_line.as<LineGrad>()));
     OCHRE_CUDA_TRY(cudaMemsetAsync(ctx->grad_pts.p, 0, in->n_floats * 4, s));
     const BatchView b = view_of(ctx, in);
     const unsigned cb = (unsigned)((in->n_cmds + 127) / 128);
     OCHRE_LAUNCH(ctx, "grad_commands", s,
-                 k_cmd_grad<<<cb, 128, 0, s>>>(b, ctx->cmd_line_off.as<uint32_t>(), L, nullptr, nullptr,
+                 launch_after(k_cmd_grad, cb, 128, 0, s, b, ctx->cmd_line_off.as<uint32_t>(), L, nullptr, nullptr,
                                                ctx->grad_line.as<LineGrad>(),
                                                ctx->grad_pts.as<float>(), w, h, gsig, ctx->grad_gs.as<float>(),
                                                ctx->grad_left.as<float>()));
     OCHRE_LAUNCH(ctx, "grad_fills", s,
-                 k_fill_grad<<<cb, 128, 0, s>>>(b, ctx->grad_pts.as<float>(), dl_dpts, dl_dxf));
+                 launch_after(k_fill_grad, cb, 128, 0, s, b, ctx->grad_pts.as<float>(), dl_dpts, dl_dxf));
     OCHRE_CUDA_TRY(cudaGetLastError());
     ctx->stats.n_launches = ctx->launches;
     collect_timings(ctx, s);

@@ -102,6 +102,7 @@ template <int BLOCK, int ITEMS, class T, class Op, class In, class Out>
 __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_dev, In in, Out out, Op op,
                                                  T identity, ScanStatus<T>* status, uint32_t* ticket,
                                                  uint32_t ticket_base, uint32_t tag, T* total, uint32_t* err) {
+    dependent_start();
     constexpr int WARPS = BLOCK / 32;
     __shared__ uint32_t s_tile;
     __shared__ T s_warp[WARPS];
@@ -210,10 +211,10 @@ cudaError_t launch_scan(ochre_gpu_ctx* ctx, uint64_t n, In in, Out out, Op op, T
     auto* status = reinterpret_cast<ScanStatus<T>*>(sp.status);
     uint32_t* err = &dev_scalars(ctx)->err;
     if (few)
-        k_scan<SCAN_BLOCK, SCAN_ITEMS_FEW, T, Op, In, Out><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(
+        launch_after(k_scan<SCAN_BLOCK, SCAN_ITEMS_FEW, T, Op, In, Out>, (unsigned)tiles, SCAN_BLOCK, 0, stream, 
             n, n_dev, in, out, op, identity, status, sp.ticket, sp.ticket_base, sp.tag, total, err);
     else
-        k_scan<SCAN_BLOCK, SCAN_ITEMS, T, Op, In, Out><<<(unsigned)tiles, SCAN_BLOCK, 0, stream>>>(
+        launch_after(k_scan<SCAN_BLOCK, SCAN_ITEMS, T, Op, In, Out>, (unsigned)tiles, SCAN_BLOCK, 0, stream, 
             n, n_dev, in, out, op, identity, status, sp.ticket, sp.ticket_base, sp.tag, total, err);
     return cudaGetLastError();
 }

@@ -45,6 +45,7 @@ template <class K, int RB>
 __global__ void __launch_bounds__(256) k_sort_hist(const K* __restrict__ keys, uint64_t n, const uint32_t* n_dev,
                                                    SortPlan plan, uint32_t* hist, uint32_t* __restrict__ off,
                                                    uint32_t* done) {
+    dependent_start();
     constexpr int RADIX = 1 << RB;
     constexpr int MAXP = (64 + RB - 1) / RB;
     constexpr int PER = RADIX / 256;   // consecutive digits per thread
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, RB <= 8 ? 3 : 2) k_onesweep(
     const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, uint64_t n, const uint32_t* n_dev, int shift, uint32_t mask,
     const uint32_t* __restrict__ digit_off, uint32_t* lookback, uint32_t* ticket, uint32_t* err) {
+    dependent_start();
     constexpr int RADIX = 1 << RB;
     constexpr int PER = RADIX / SORT_BLOCK;   // digits per thread in the offset phase
     extern __shared__ __align__(16) unsigned char smem[];
@@ -321,7 +323,7 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         int blocks = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)std::max(sms, 1) * 8);
-        OCHRE_LAUNCH(ctx, "sort_hist", s, k_sort_hist<K, RB><<<blocks, 256, 0, s>>>(
+        OCHRE_LAUNCH(ctx, "sort_hist", s, launch_after(k_sort_hist<K, RB>, blocks, 256, 0, s, 
             kin, n, n_dev, plan, hist, off, shared ? tickets : tickets + TICKETS - 1));
         OCHRE_CUDA_TRY(cudaGetLastError());
     }
@@ -334,7 +336,7 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
             OCHRE_CUDA_TRY(cudaMemsetAsync(lookback, 0, rows * 4, s));
             OCHRE_CUDA_TRY(cudaMemsetAsync(ticket, 0, 4, s));
         }
-        OCHRE_LAUNCH(ctx, "sort_onesweep", s, k_onesweep<K, RB><<<(unsigned)tiles, SORT_BLOCK, smem, s>>>(
+        OCHRE_LAUNCH(ctx, "sort_onesweep", s, launch_after(k_onesweep<K, RB>, (unsigned)tiles, SORT_BLOCK, smem, s, 
             kin, vin, kout, vout, n, n_dev, plan.shift[p], (1u << plan.width[p]) - 1u, off + p * RADIX, lookback,
             ticket, &ds->err));
         OCHRE_CUDA_TRY(cudaGetLastError());

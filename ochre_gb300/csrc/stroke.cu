@@ -100,6 +100,7 @@ struct PairIn {
 template <class Count>
 __global__ void __launch_bounds__(128) k_pair_count(uint64_t n, const uint32_t* n_dev, Count count,
                                                     uint32_t* __restrict__ out_n, uint32_t* __restrict__ out_nf) {
+    dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= dev_count(n, n_dev)) return;
     const Pair p = count(i);
@@ -112,6 +113,7 @@ __global__ void k_poly_emit(const uint8_t* __restrict__ verbs, const float* __re
                             uint64_t n_cmds, const uint32_t* __restrict__ cmd_foff, const uint32_t* __restrict__ cmd_ep,
                             const uint32_t* __restrict__ poly_off, const uint32_t* __restrict__ poly_foff,
                             uint8_t* __restrict__ pverbs, float* __restrict__ ppts, uint32_t p_cap, uint32_t pf_cap) {
+    dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= n_cmds) return;
     const uint32_t c = (uint32_t)i;
@@ -220,6 +222,7 @@ struct OffOutU32 {
 __global__ void k_first_close(const uint8_t* __restrict__ pverbs, uint64_t n_poly, const uint32_t* n_dev,
                               const uint32_t* __restrict__ pfill_off, uint32_t n_fills, const uint8_t* __restrict__ flags,
                               uint32_t* __restrict__ first_close) {
+    dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= dev_count(n_poly, n_dev) || pverbs[i] != V_CLOSE) return;
     const uint32_t f = upper_bound_u32(pfill_off, n_fills + 1, (uint32_t)i) - 1u;
@@ -229,6 +232,7 @@ __global__ void k_first_close(const uint8_t* __restrict__ pverbs, uint64_t n_pol
 __global__ void k_fill_init(uint32_t* __restrict__ first_close, const uint32_t* __restrict__ fill_off,
                             const uint32_t* __restrict__ poly_off, uint64_t n_cmds, uint32_t n_poly,
                             const uint32_t* n_poly_dev, uint32_t n_fills, uint32_t* __restrict__ pfill_off) {
+    dependent_start();
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f > n_fills) return;
     const uint32_t np = (uint32_t)dev_count(n_poly, n_poly_dev);
@@ -368,6 +372,7 @@ __global__ void __launch_bounds__(128) k_out_count(uint32_t n_units, const uint3
                                                    const uint32_t* __restrict__ first_close,
                                                    const float* __restrict__ width, uint32_t* __restrict__ out_n,
                                                    uint32_t* __restrict__ out_nf) {
+    dependent_start();
     const uint64_t u = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     if (u >= dev_count(n_units, n_dev)) return;   // whole warps
     const uint32_t lane = threadIdx.x & 31u;
@@ -401,6 +406,7 @@ __global__ void __launch_bounds__(128) k_out_emit(uint32_t n_units, const uint32
                                                   const float* __restrict__ width, const uint32_t* __restrict__ out_off,
                                                   const uint32_t* __restrict__ out_foff, uint8_t* __restrict__ overbs,
                                                   float* __restrict__ opts, uint32_t* __restrict__ unit_fill) {
+    dependent_start();
     const uint64_t u = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     if (u >= dev_count(n_units, n_dev)) return;   // whole warps
     const uint32_t lane = threadIdx.x & 31u;
@@ -446,6 +452,7 @@ __global__ void k_out_fill_off(const uint32_t* __restrict__ unit_fill, uint32_t 
                                const uint32_t* __restrict__ out_off, uint32_t total, const uint32_t* total_dev,
                                uint32_t pad_end, uint32_t n_fills, uint32_t* __restrict__ ofill_off,
                                const uint8_t* __restrict__ flags, uint8_t* __restrict__ oflags) {
+    dependent_start();
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f > n_fills) return;
     n_units = (uint32_t)dev_count(n_units, units_dev);
@@ -466,6 +473,7 @@ __global__ void k_out_fill_off(const uint32_t* __restrict__ unit_fill, uint32_t 
 // then re-plans).
 __global__ void k_stroke_cap(uint32_t* a, uint32_t cap_a, uint32_t* b, uint32_t cap_b, uint32_t* also,
                              uint32_t* err) {
+    dependent_start();
     if (*a > cap_a || *b > cap_b) {
         *a = 0u;
         *b = 0u;
@@ -507,7 +515,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     wait_inputs(ctx, s);   // path-space flatten counts read points
     OCHRE_CUDA_TRY(ctx->sk_poly_off.ensure((n + 1) * 4));
     OCHRE_CUDA_TRY(ctx->sk_poly_foff.ensure((n + 1) * 4));
-    OCHRE_LAUNCH(ctx, "stroke_poly_count", s, k_pair_count<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "stroke_poly_count", s, launch_after(k_pair_count<PolyCount>, (unsigned)((n + 127) / 128), 128, 0, s, 
         n, nullptr,
         PolyCount{in->verbs, in->pts, in->fill_cmd_off, F, in->fill_flags, ctx->sk_cmd_foff.as<uint32_t>(),
                   ctx->sk_cmd_ep.as<uint32_t>(), &ds->err},
@@ -523,7 +531,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
         P = plan->stroke_poly;
         PF = plan->stroke_poly_floats;
         OCHRE_LAUNCH(ctx, "plan_stroke_poly", s,
-                     k_stroke_cap<<<1, 1, 0, s>>>(&ds->n_lines, P, &ds->n_line_ent, PF, &ds->n_tiles, &ds->err));
+                     launch_after(k_stroke_cap, 1, 1, 0, s, &ds->n_lines, P, &ds->n_line_ent, PF, &ds->n_tiles, &ds->err));
         OCHRE_CUDA_TRY(cudaGetLastError());
     } else {
         st = read_scalars(ctx, s);
@@ -543,11 +551,11 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     OCHRE_CUDA_TRY(ctx->sk_pfill_off.ensure(((size_t)F + 1) * 4));
     OCHRE_CUDA_TRY(ctx->sk_first_close.ensure((size_t)F * 4));
     const unsigned cb = (unsigned)((n + 255) / 256);
-    OCHRE_LAUNCH(ctx, "stroke_poly_emit", s, k_poly_emit<<<cb, 256, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "stroke_poly_emit", s, launch_after(k_poly_emit, cb, 256, 0, s, 
         in->verbs, in->pts, in->fill_cmd_off, F, in->fill_flags, n, ctx->sk_cmd_foff.as<uint32_t>(),
         ctx->sk_cmd_ep.as<uint32_t>(), ctx->sk_poly_off.as<uint32_t>(), ctx->sk_poly_foff.as<uint32_t>(),
         ctx->sk_pverbs.as<uint8_t>(), ctx->sk_ppts.as<float>(), P, PF));
-    OCHRE_LAUNCH(ctx, "stroke_fill_init", s, k_fill_init<<<(F + 256) / 256, 256, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "stroke_fill_init", s, launch_after(k_fill_init, (F + 256) / 256, 256, 0, s, 
         ctx->sk_first_close.as<uint32_t>(), in->fill_cmd_off, ctx->sk_poly_off.as<uint32_t>(), n, P, p_dev, F,
         ctx->sk_pfill_off.as<uint32_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());
@@ -564,7 +572,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     OCHRE_LAUNCH(ctx, "stroke_pfoff_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
         ctx, P, PolyFloats{ctx->sk_pverbs.as<uint8_t>()}, OffOutU32{ctx->sk_pfoff.as<uint32_t>()}, OpSumU32{}, 0u,
         static_cast<uint32_t*>(nullptr), s, p_dev)));
-    OCHRE_LAUNCH(ctx, "stroke_first_close", s, k_first_close<<<(P + 255) / 256, 256, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "stroke_first_close", s, launch_after(k_first_close, (P + 255) / 256, 256, 0, s, 
         ctx->sk_pverbs.as<uint8_t>(), P, p_dev, ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
         ctx->sk_first_close.as<uint32_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());
@@ -591,7 +599,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     // the output totals: a scan that covers no unit writes none
     OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->n_lines, 0, 8, s));
     if (U) {
-        OCHRE_LAUNCH(ctx, "stroke_out_count", s, k_out_count<<<(unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s>>>(
+        OCHRE_LAUNCH(ctx, "stroke_out_count", s, launch_after(k_out_count, (unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s, 
             U, u_dev, ctx->sk_unit_start.as<uint32_t>(), ctx->sk_pverbs.as<uint8_t>(), ctx->sk_ppts.as<float>(),
             ctx->sk_pfoff.as<uint32_t>(), ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
             ctx->sk_first_close.as<uint32_t>(), in->fill_width, ctx->sk_out_off.as<uint32_t>(),
@@ -607,7 +615,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
         ON = plan->stroke_cmds;
         OF = plan->stroke_floats;
         OCHRE_LAUNCH(ctx, "plan_stroke_out", s,
-                     k_stroke_cap<<<1, 1, 0, s>>>(&ds->n_lines, ON, &ds->n_line_ent, OF, &ds->n_tiles, &ds->err));
+                     launch_after(k_stroke_cap, 1, 1, 0, s, &ds->n_lines, ON, &ds->n_line_ent, OF, &ds->n_tiles, &ds->err));
         OCHRE_CUDA_TRY(cudaGetLastError());
     } else {
         st = read_scalars(ctx, s);
@@ -627,13 +635,13 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     // planned: every output command past the true total is a Close
     if (plan) OCHRE_CUDA_TRY(cudaMemsetAsync(ctx->sk_overbs.p, V_CLOSE, ON, s));
     if (U)
-        OCHRE_LAUNCH(ctx, "stroke_out_emit", s, k_out_emit<<<(unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s>>>(
+        OCHRE_LAUNCH(ctx, "stroke_out_emit", s, launch_after(k_out_emit, (unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s, 
             U, u_dev, ctx->sk_unit_start.as<uint32_t>(), ctx->sk_pverbs.as<uint8_t>(), ctx->sk_ppts.as<float>(),
             ctx->sk_pfoff.as<uint32_t>(), ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
             ctx->sk_first_close.as<uint32_t>(), in->fill_width, ctx->sk_out_off.as<uint32_t>(),
             ctx->sk_out_foff.as<uint32_t>(), ctx->sk_overbs.as<uint8_t>(), ctx->sk_opts.as<float>(),
             ctx->sk_unit_fill.as<uint32_t>()));
-    OCHRE_LAUNCH(ctx, "stroke_fill_off", s, k_out_fill_off<<<(F + 256) / 256, 256, 0, s>>>(
+    OCHRE_LAUNCH(ctx, "stroke_fill_off", s, launch_after(k_out_fill_off, (F + 256) / 256, 256, 0, s, 
         ctx->sk_unit_fill.as<uint32_t>(), U, u_dev, ctx->sk_out_off.as<uint32_t>(), ON, plan ? &ds->n_lines : nullptr,
         plan ? ON : 0u, F, ctx->sk_ofill_off.as<uint32_t>(), in->fill_flags, ctx->sk_oflags.as<uint8_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());

@@ -103,6 +103,7 @@ template <class K, int HEAD_ITEMS>
 __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__ keys, HeadArgs A,
                                                            ScanStatus<HeadScan>* status, uint32_t* ticket,
                                                            uint32_t ticket_base, uint32_t tag, uint32_t* err) {
+    dependent_start();
     constexpr int WARPS = HEAD_BLOCK / 32, HEAD_TILE = HEAD_BLOCK * HEAD_ITEMS;
     constexpr uint32_t FULL = 0xffffffffu;
     __shared__ uint32_t s_tile, s_rows;
@@ -248,6 +249,7 @@ __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__
 // Graph replays: the tile count against its capacity; above it there is no
 // tile, no row and no span to work on.
 __global__ void k_plan_tiles(DevScalars* ds, uint32_t cap) {
+    dependent_start();
     if (ds->n_tiles > cap) {
         ds->n_tiles = 0u;
         ds->n_rows = 0u;
@@ -382,6 +384,7 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
     TileView tiles, uint32_t n_tiles, const uint32_t* n_dev, TileBlockState* state, uint32_t* ticket,
     uint32_t* __restrict__ out_xy, uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov, uint32_t* err,
     bool cov_signed) {
+    dependent_start();
     constexpr int WARPS = 4;
     // device-held count (graph replays): blocks past it end before publishing
     n_tiles = (uint32_t)dev_count(n_tiles, n_dev);
@@ -576,6 +579,7 @@ __global__ void __launch_bounds__(128) k_tile_cov(
     const uint32_t* __restrict__ vals, const BinRec* __restrict__ bins, const float2* __restrict__ incs,
     TileView tiles, uint32_t n_tiles, const uint32_t* n_dev, uint32_t* ticket, uint32_t* __restrict__ out_xy,
     uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov, const uint32_t* err, bool cov_signed) {
+    dependent_start();
     constexpr int WARPS = 4;
     // an earlier wait of the run gave up: the tile data is not valid
     if (run_aborted(err)) return;
@@ -740,14 +744,14 @@ static void launch_tile_cov(ochre_gpu_ctx* ctx, const TileView& tiles, uint32_t 
     if (row_form) {
         // no more warps than rows, nor than the GPU keeps resident (16 CTAs of 4 warps per SM)
         const uint32_t ctas = (uint32_t)std::min<uint64_t>(((uint64_t)n_rows + 3) / 4, (uint64_t)sms * 16);
-        k_tile_cov<TPW><<<ctas, 128, 0, s>>>(
+        launch_after(k_tile_cov<TPW>, ctas, 128, 0, s, 
             ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), tiles, T, t_dev,
             &ds->ticket, ctx->out_tile_xy.as<uint32_t>(), ctx->out_tile_alpha.as<uint8_t>(), cov,
             &ds->err, ctx->cov_signed);
     } else {
         const uint32_t blocks = (T + TPW - 1) / TPW;
         cudaMemsetAsync(ctx->tile_state.p, 0, (size_t)blocks * sizeof(TileBlockState), s);
-        k_tile_cov_blocks<TPW><<<(blocks + 3) / 4, 128, 0, s>>>(
+        launch_after(k_tile_cov_blocks<TPW>, (blocks + 3) / 4, 128, 0, s, 
             ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), tiles, T, t_dev,
             ctx->tile_state.as<TileBlockState>(), &ds->ticket, ctx->out_tile_xy.as<uint32_t>(),
             ctx->out_tile_alpha.as<uint8_t>(), cov, &ds->err, ctx->cov_signed);
@@ -784,16 +788,16 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
                         &ds->n_rows};
     auto* status = reinterpret_cast<ScanStatus<HeadScan>*>(sp.status);
     if (steps == 4)
-        OCHRE_LAUNCH(ctx, "tile_heads", s, k_tile_heads<K, 4><<<blocks, HEAD_BLOCK, 0, s>>>(
+        OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 4>, blocks, HEAD_BLOCK, 0, s, 
             ctx->keys.as<K>(), args, status, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
     else
-        OCHRE_LAUNCH(ctx, "tile_heads", s, k_tile_heads<K, 16><<<blocks, HEAD_BLOCK, 0, s>>>(
+        OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 16>, blocks, HEAD_BLOCK, 0, s, 
             ctx->keys.as<K>(), args, status, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
     int st = OCHRE_OK;
     uint32_t T, n_rows;
     if (plan) {
-        OCHRE_LAUNCH(ctx, "plan_tiles", s, k_plan_tiles<<<1, 1, 0, s>>>(ds, plan->tiles));
+        OCHRE_LAUNCH(ctx, "plan_tiles", s, launch_after(k_plan_tiles, 1, 1, 0, s, ds, plan->tiles));
         OCHRE_CUDA_TRY(cudaGetLastError());
         T = plan->tiles;
         n_rows = plan->rows;
