@@ -98,19 +98,6 @@ __device__ uint32_t count_cmd(const CmdCtx& k, bool* capped) {
     return n;
 }
 
-// Line counts folded straight into the line-offset scan.
-struct CountIn {
-    BatchView b;
-    uint32_t* err;
-    __device__ __forceinline__ uint32_t operator()(uint64_t i) const {
-        const CmdCtx k = load_cmd(b, (uint32_t)i);
-        if (!k.ok) { atomicOr(err, ERR_INVALID); return 0u; }
-        bool capped = false;
-        const uint32_t n = count_cmd(k, &capped);
-        if (capped) atomicOr(err, ERR_LIMIT);
-        return n;
-    }
-};
 struct OffOut {
     uint32_t* off;
     __device__ __forceinline__ void operator()(uint64_t i, uint32_t ex, uint32_t) const { off[i] = ex; }
@@ -120,16 +107,24 @@ struct Load32 {
     __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return v[i]; }
 };
 
-// One thread per command: the line counts of a batch with few commands
-// (a scan would give each of a handful of threads eight serial t loops).
-template <class In>
-__global__ void __launch_bounds__(128) k_count_each(uint64_t n, In in, uint32_t* __restrict__ out) {
+// Line counts, one thread per command, then a scan of them (a scan that counted
+// as it read gave each thread eight serial t loops, one after the other: 161
+// against 108 us for the 2.0 M commands of 20,000 uneven paths).
+__global__ void __launch_bounds__(128) k_cmd_count(BatchView b, uint32_t* __restrict__ counts, uint32_t* err) {
     dependent_start();
-    const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (i < n) out[i] = in(i);
+    const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    if (c >= b.n_cmds) return;
+    const CmdCtx k = load_cmd(b, (uint32_t)c);
+    uint32_t n = 0;
+    if (!k.ok) {
+        atomicOr(err, ERR_INVALID);
+    } else {
+        bool capped = false;
+        n = count_cmd(k, &capped);
+        if (capped) atomicOr(err, ERR_LIMIT);
+    }
+    counts[c] = n;
 }
-// Below this many scan tiles the counts get their own kernel.
-constexpr uint64_t SPLIT_COUNT_TILES = 256;
 
 // Lines of more than long_cells cells (walk_cells) are also queued for the
 // long-line emit walk of the DDA stage (long_cells 0: none are).
@@ -181,18 +176,13 @@ int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uin
     BatchView b{in->verbs, in->pts, in->fill_cmd_off, in->fill_xf, in->fill_flags, in->raster_fill_off,
                 in->n_fills, in->n_rasters, n, ctx->cmd_foff.as<uint32_t>(), ctx->cmd_mv.as<uint32_t>(),
                 ctx->cmd_ep.as<uint32_t>(), in->n_floats};
-    if (scan_tiles(n) < SPLIT_COUNT_TILES) {
-        // counts first (one thread per command), then the offsets in place
-        OCHRE_LAUNCH(ctx, "flatten_count", s, launch_after(k_count_each<CountIn>, (unsigned)((n + 127) / 128), 128, 0, s, 
-            n, CountIn{b, &ds->err}, ctx->cmd_line_off.as<uint32_t>()));
-        OCHRE_CUDA_TRY(cudaGetLastError());
-        OCHRE_LAUNCH(ctx, "flatten_count_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-            ctx, n, Load32{ctx->cmd_line_off.as<uint32_t>()}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u,
-            &ds->n_lines, s)));
-    } else {
-        OCHRE_LAUNCH(ctx, "flatten_count_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-            ctx, n, CountIn{b, &ds->err}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u, &ds->n_lines, s)));
-    }
+    // counts first, then the offsets in place
+    OCHRE_LAUNCH(ctx, "flatten_count", s, launch_after(k_cmd_count, (unsigned)((n + 127) / 128), 128, 0, s, b,
+                                                       ctx->cmd_line_off.as<uint32_t>(), &ds->err));
+    OCHRE_CUDA_TRY(cudaGetLastError());
+    OCHRE_LAUNCH(ctx, "flatten_count_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
+        ctx, n, Load32{ctx->cmd_line_off.as<uint32_t>()}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u,
+        &ds->n_lines, s)));
     uint32_t L;
     if (plan) {
         // the line count stays on the device; above the plan it is zeroed

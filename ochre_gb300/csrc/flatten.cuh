@@ -81,9 +81,17 @@ __device__ __forceinline__ uint32_t fill_of(const BatchView& b, uint32_t c) {
     return upper_bound_u32(b.fill_off, b.n_fills + 1, c) - 1u;
 }
 
+// The fill of command j at or before fill f's commands: f, the fill before, or
+// (behind empty fills) searched for.
+__device__ __forceinline__ uint32_t fill_near(const BatchView& b, uint32_t j, uint32_t f) {
+    if (j >= __ldg(b.fill_off + f)) return f;
+    if (f > 0 && j >= __ldg(b.fill_off + f - 1u)) return f - 1u;
+    return fill_of(b, j);
+}
+
 // The transformed end point of command j (a non-Close command).
 __device__ __forceinline__ V2 endpoint_of(const BatchView& b, uint32_t j, uint32_t f_hint) {
-    const uint32_t f = j >= __ldg(b.fill_off + f_hint) ? f_hint : fill_of(b, j);
+    const uint32_t f = fill_near(b, j, f_hint);
     const uint8_t v = __ldg(b.verbs + j);
     const float* fp = b.pts + __ldg(b.cmd_foff + j) + endpoint_float(v);
     V2 p = v2(__ldg(fp), __ldg(fp + 1));
@@ -124,7 +132,7 @@ __device__ inline CmdCtx load_cmd(const BatchView& b, uint32_t c) {
     k.last = ep > rc0 ? endpoint_of(b, ep - 1u, f) : v2(0.0f, 0.0f);
     if (mv > rc0) {
         const uint32_t m = mv - 1u;
-        const uint32_t fm = m >= __ldg(b.fill_off + f) ? f : fill_of(b, m);
+        const uint32_t fm = fill_near(b, m, f);
         const float* fp = b.pts + __ldg(b.cmd_foff + m);
         V2 p = v2(__ldg(fp), __ldg(fp + 1));
         const bool raw = b.fill_flags != nullptr && (__ldg(b.fill_flags + fm) & OCHRE_FILL_RAW);
