@@ -326,8 +326,11 @@ int run_device(ochre_gpu_ctx* ctx, const ochre_batch* in_orig, ochre_result* out
         uint32_t bits = 0;
         st = stage_bin(ctx, in, L, s, &E, &bits);
         if (st != OCHRE_OK) return st;
-        uint32_t passes = 0;
-        st = stage_sort(ctx, E, bits, s, &passes);
+        uint32_t passes = 1;
+        if (L && sort_local_wanted(ctx) && host_scalars(ctx)->n_sort[2] == 0u)
+            st = stage_sort_local(ctx, in, s);
+        else
+            st = stage_sort(ctx, E, bits, s, &passes);
         if (st != OCHRE_OK) return st;
         st = stage_tiles(ctx, in, E, s, &T, &N);
         if (st != OCHRE_OK) return st;
@@ -446,7 +449,7 @@ std::vector<DevBuf*> device_buffers(ochre_gpu_ctx* ctx) {
     return {&ctx->in_verbs, &ctx->in_pts, &ctx->in_fill_off, &ctx->in_fill_xf, &ctx->in_fill_flags,
                      &ctx->in_raster_off, &ctx->cmd_foff, &ctx->cmd_mv, &ctx->cmd_ep, &ctx->cmd_line_off,
                      &ctx->lines, &ctx->line_raster, &ctx->line_ent_off, &ctx->line_inc_off, &ctx->long_lines, &ctx->incs, &ctx->raster_bbox, &ctx->raster_keybase,
-                     &ctx->raster_empty, &ctx->raster_wsum, &ctx->raster_wbase, &ctx->keys, &ctx->vals, &ctx->keys_alt, &ctx->vals_alt, &ctx->bins,
+                     &ctx->raster_empty, &ctx->raster_run, &ctx->raster_wsum, &ctx->raster_wbase, &ctx->keys, &ctx->vals, &ctx->keys_alt, &ctx->vals_alt, &ctx->bins,
                      &ctx->sort_hist, &ctx->sort_lookback, &ctx->tile_head, &ctx->tile_xy, &ctx->tile_rf, &ctx->tile_state,
                      &ctx->scan_status, &ctx->scalars, &ctx->fused_chain, &ctx->fused_stage,
                      &ctx->grad_g, &ctx->grad_gs, &ctx->grad_left, &ctx->grad_line, &ctx->grad_pts,

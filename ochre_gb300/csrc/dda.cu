@@ -454,20 +454,49 @@ struct RasterScan {
     uint64_t ks;
     uint32_t ne;
     int32_t w;   // crossing signs of the rasters so far
+    uint32_t by_size[3];   // rasters sorted by the middle and the large block of stage_sort_local, and by neither
+    uint32_t begin, n;     // (of one raster alone) its entries
+    uint32_t pad;
 };
 struct OpRaster {
     __device__ __forceinline__ RasterScan operator()(RasterScan a, RasterScan b) const {
-        return RasterScan{a.ks + b.ks, a.ne + b.ne, a.w + b.w};
+        return RasterScan{a.ks + b.ks, a.ne + b.ne, a.w + b.w,
+                          {a.by_size[0] + b.by_size[0], a.by_size[1] + b.by_size[1], a.by_size[2] + b.by_size[2]}, 0u, 0u, 0u};
+    }
+};
+// First entry of raster r's lines (r = n_rasters: their end).
+struct RasterEntries {
+    const uint32_t* cmd_line_off;
+    uint64_t n_cmds;
+    const uint32_t* fill_off;
+    const uint32_t* raster_off;   // or null: one fill per raster
+    const uint32_t* line_ent_off;
+    uint32_t n_lines;
+    const uint32_t* line_ent_total;
+    __device__ __forceinline__ uint32_t operator()(uint32_t r) const {
+        const uint32_t c = fill_off[raster_off ? raster_off[r] : r];
+        const uint32_t l = c < n_cmds ? cmd_line_off[c] : n_lines;
+        return l < n_lines ? line_ent_off[l] : *line_ent_total;
     }
 };
 struct RasterIn {
     const int4* bbox;
     const int* wsum;
+    RasterEntries first;
+    bool sizes;   // the rasters are listed by size
     __device__ __forceinline__ RasterScan operator()(uint64_t r) const {
         const int4 b = bbox[r];
-        if (b.x > b.z) return RasterScan{2ull, 1u, wsum[r]};
+        const uint32_t e = sizes ? first((uint32_t)r) : 0u;
+        if (b.x > b.z) return RasterScan{2ull, 1u, wsum[r], {0u, 0u, 0u}, e, 0u, 0u};
         const uint64_t w = (uint64_t)(b.z - b.x + 1), h = (uint64_t)(b.w - b.y + 1);
-        return RasterScan{w * h * 2ull, 0u, wsum[r]};
+        RasterScan v{w * h * 2ull, 0u, wsum[r], {0u, 0u, 0u}, e, 0u, 0u};
+        if (sizes) {
+            v.n = first((uint32_t)r + 1u) - e;
+            if (v.n > LOCAL_SORT_LARGE || v.ks > (1ull << LOCAL_SORT_KEY_BITS)) v.by_size[2] = 1u;
+            else if (v.n > LOCAL_SORT_MIDDLE) v.by_size[1] = 1u;
+            else if (v.n > LOCAL_SORT_SMALL) v.by_size[0] = 1u;
+        }
+        return v;
     }
 };
 struct RasterOut {
@@ -475,15 +504,19 @@ struct RasterOut {
     uint64_t* key_base;
     uint32_t* empty;   // 0: has increments; else 1 + rank among empty rasters
     int* wbase;        // crossing signs of all earlier rasters
+    RasterRun* run;    // (or null) small from the front, middle from n_rasters - 1 down, large from n_rasters on
+    uint32_t n_rasters;
     __device__ __forceinline__ void operator()(uint64_t r, RasterScan ex, RasterScan v) const {
         key_base[r] = ex.ks;
         wbase[r] = ex.w;
-        if (v.ne) {
-            bbox[r] = make_int4(0, 0, 0, 0);
-            empty[r] = ex.ne + 1u;
-        } else {
-            empty[r] = 0u;
+        empty[r] = v.ne ? ex.ne + 1u : 0u;
+        if (run != nullptr && !v.by_size[2]) {
+            const uint32_t at = v.by_size[0]   ? n_rasters - 1u - ex.by_size[0]
+                                : v.by_size[1] ? n_rasters + ex.by_size[1]
+                                               : (uint32_t)r - ex.by_size[0] - ex.by_size[1] - ex.by_size[2];
+            run[at] = RasterRun{(uint32_t)r, v.begin, v.n, v.begin + ex.ne};
         }
+        if (v.ne) bbox[r] = make_int4(0, 0, 0, 0);
     }
 };
 
@@ -880,9 +913,15 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
     const uint32_t* queue = long_cells ? ctx->long_lines.as<uint32_t>() : nullptr;
     // graph replays: n_lines is the capacity, the count is on the device
     const GraphPlan* plan = ctx->plan;
+    if (n_lines) OCHRE_CUDA_TRY(ctx->line_ent_off.ensure((size_t)n_lines * 4));
+    const bool sizes = n_lines != 0 && sort_local_wanted(ctx);
+    if (sizes) OCHRE_CUDA_TRY(ctx->raster_run.ensure((size_t)R * 2 * sizeof(RasterRun)));
+    static_assert(sizeof(RasterScan) == 40 && offsetof(DevScalars, n_sort) == offsetof(DevScalars, keyspace) + 16,
+                  "layout");
+    const RasterEntries first{ctx->cmd_line_off.as<uint32_t>(), in->n_cmds, in->fill_cmd_off, in->raster_fill_off,
+                              ctx->line_ent_off.as<uint32_t>(), n_lines, &ds->line_ent_total};
     const uint32_t* lines_dev = plan ? &ds->n_lines : nullptr;
     if (n_lines) {
-        OCHRE_CUDA_TRY(ctx->line_ent_off.ensure((size_t)n_lines * 4));
         OCHRE_CUDA_TRY(ctx->line_inc_off.ensure((size_t)n_lines * 4));
         unsigned count_grid = 1;
         uint32_t groups = 1;
@@ -901,10 +940,10 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
             LinePair{0u, 0u}, reinterpret_cast<LinePair*>(&ds->line_ent_total), s, lines_dev)));
     }
     OCHRE_LAUNCH(ctx, "raster_key_scan", s, OCHRE_CUDA_TRY(launch_scan<RasterScan>(
-        ctx, R, RasterIn{ctx->raster_bbox.as<int4>(), ctx->raster_wsum.as<int>()},
+        ctx, R, RasterIn{ctx->raster_bbox.as<int4>(), ctx->raster_wsum.as<int>(), first, sizes},
         RasterOut{ctx->raster_bbox.as<int4>(), ctx->raster_keybase.as<uint64_t>(), ctx->raster_empty.as<uint32_t>(),
-                  ctx->raster_wbase.as<int>()},
-        OpRaster{}, RasterScan{0, 0, 0}, reinterpret_cast<RasterScan*>(&ds->keyspace), s)));
+                  ctx->raster_wbase.as<int>(), sizes ? ctx->raster_run.as<RasterRun>() : nullptr, R},
+        OpRaster{}, RasterScan{0, 0, 0, {0, 0, 0}, 0, 0, 0}, reinterpret_cast<RasterScan*>(&ds->keyspace), s)));
     uint64_t E;
     uint32_t bits;
     uint32_t first_entry = 0;

@@ -57,19 +57,15 @@ struct DevScalars {
     uint32_t n_entries;    // all sort entries: n_line_ent + n_empty
     uint64_t keyspace;     // total key space (raster scan .ks)
     uint32_t n_empty;      // rasters without increments (raster scan .ne)
-    uint32_t pad1;
+    uint32_t pad1;         // (raster scan .w)
+    uint32_t n_sort[3];    // rasters whose entries a larger block sorts, the largest block, none (.by_size)
+    uint32_t pad3[3];
     uint32_t n_tiles;      // tiles                         }
     int32_t head_wind;     // sum of all crossing signs     } (HeadScan layout)
     uint32_t n_rows;       // tile rows (raster, tile_y)
-    uint32_t pad2;
     uint32_t n_spans;
-    uint32_t sort_ticket;
-    uint32_t fused_fallback;  // fused path: some raster did not fit
-    uint32_t fused_tiles;     // fused path totals
-    uint32_t fused_spans;
-    uint32_t pad1b;
     uint32_t spin_log2;       // poll limit of the run's bounded waits, log2 (0: SPIN_LIMIT)
-    uint32_t pad3;
+    uint32_t pad2;
     uint32_t line_ent_total;  // chain: sort entries the lines produce   } (line scan
     uint32_t n_incs;          // chain: pixel-cell increments of the lines } pair total)
     uint64_t inc_total;       // the same increment count summed in 64 bits (the pair
@@ -80,6 +76,10 @@ struct DevScalars {
     uint32_t pad4;
     uint32_t line_ticket;     // line windows handed out in the count walk
     uint32_t pad5;
+    uint32_t sort_ticket;
+    uint32_t fused_fallback;  // fused path: some raster did not fit
+    uint32_t fused_tiles;     // fused path totals
+    uint32_t fused_spans;
 };
 // The waits find spin_log2 from the error word's address (common.cuh).
 static_assert(offsetof(DevScalars, spin_log2) - offsetof(DevScalars, err) == 4 * 22,
@@ -125,6 +125,13 @@ struct GraphPlan {
     // a differentiable step: after the chain (signed coverage), its render,
     // loss and backward, their counts on the device
     const DiffStep* diff;
+};
+
+// A raster's entries: n of them from `begin` among the emitted ones (line by
+// line, the lines in raster order, then one entry per raster without
+// increments, whose n is 0), from `out` on in sorted order.
+struct alignas(16) RasterRun {
+    uint32_t raster, begin, n, out;
 };
 
 // Entry value tag for tile-row crossings: 1 | raster (23 bits) | sign byte.
@@ -176,6 +183,7 @@ struct ochre_gpu_ctx {
     ochre::DevBuf incs;
     // per raster
     ochre::DevBuf raster_bbox, raster_keybase, raster_empty;
+    ochre::DevBuf raster_run;   // RasterRun, by the block size that sorts the entries (stage_sort_local)
     // per raster: sum of its tile-row crossing signs, and the sum over earlier rasters
     ochre::DevBuf raster_wsum, raster_wbase;
     // sort entries
@@ -291,6 +299,14 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
 // Sorts by key bits first_bit .. first_bit + key_bits - 1.
 int stage_sort(ochre_gpu_ctx* ctx, uint64_t n_entries, uint32_t key_bits, cudaStream_t s, uint32_t* passes,
                uint32_t first_bit = 0);
+// The same order by one block per raster, when every raster's entries fit one.
+// Limits: entries of a raster for the three block sizes, and bits of its keys.
+constexpr uint32_t LOCAL_SORT_SMALL = 1024, LOCAL_SORT_MIDDLE = 4096, LOCAL_SORT_LARGE = 8192;
+constexpr int LOCAL_SORT_IDX_BITS = 13, LOCAL_SORT_KEY_BITS = 32 - LOCAL_SORT_IDX_BITS;
+// May the context's run sort that way (then stage_bin lists the rasters by
+// block size and the host sees whether all fit)?
+inline bool sort_local_wanted(const ochre_gpu_ctx* ctx);
+int stage_sort_local(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s);
 int stage_tiles(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t n_entries, cudaStream_t s, uint32_t* n_tiles,
                 uint32_t* n_spans);
 // Rewrites stroked fills into plain fills (stroke.cu); *out views device memory.
@@ -338,6 +354,11 @@ int copy_scalars_async(ochre_gpu_ctx* ctx, cudaStream_t s);
 // Every device buffer of a context (release on destroy; a graph capture
 // checks that none of them moved).
 std::vector<DevBuf*> device_buffers(ochre_gpu_ctx* ctx);
+// Not in a captured chain (its largest raster is not known) nor in an arena
+// (which has no room for the list), nor when 11-bit digits were asked for.
+inline bool sort_local_wanted(const ochre_gpu_ctx* ctx) {
+    return ctx->plan == nullptr && ctx->scan_status.arena == nullptr && ctx->tune_sort_digit_bits == 8;
+}
 inline DevScalars* dev_scalars(ochre_gpu_ctx* ctx) { return ctx->scalars.as<DevScalars>(); }
 inline DevScalars* host_scalars(ochre_gpu_ctx* ctx) { return ctx->h_scalars.as<DevScalars>(); }
 int check_device_error(ochre_gpu_ctx* ctx);

@@ -363,4 +363,219 @@ int stage_sort(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStream_t s
                        : sort_impl<uint32_t, 8>(ctx, n, key_bits, s, passes, first_bit);
 }
 
+// ---- one block per raster ----
+// The entries were emitted raster by raster and a raster's keys are its key
+// base plus a number below its own key space, so the order asked for is each
+// raster's entries sorted by that number.  Where every raster's entries fit
+// one block's shared memory, a block reads their keys once, ranks them there
+// (8 bits a pass, as in k_onesweep: lanes with equal digits by ballots, warps
+// in entry order, so it is stable) and writes the
+// entries once.  An entry is one word, its number and its place among the
+// raster's entries; its value is fetched when it is written.  That is one
+// launch and 16 bytes an entry, where the device-wide passes move 16 bytes an
+// entry each, as many passes as all rasters' key spaces together have digits.
+// Bound by the latency of a block's few serial phases, so blocks come in three
+// sizes (128, 256 and 512 threads), each raster to the smallest that holds it.
+// 1,000 shapes of 2,785 entries (23 key bits, 13 of them within a raster): 124
+// us for three passes and their histogram, 40 here; 20,000 strokes of 957: 620
+// and 287.
+// The lanes of the warp whose digit equals this lane's, among those with
+// `valid` set: one ballot per digit bit.  (Here 6 us shorter than
+// __match_any_sync for 1,000 shapes; in k_onesweep it is the longer way.)
+template <int BITS>
+__device__ __forceinline__ uint32_t same_digit(uint32_t d, bool valid) {
+    uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < BITS; b++) {
+        const bool set = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, set);
+        peers &= set ? m : ~m;
+    }
+    return peers;
+}
+
+struct LocalSortArgs {
+    const RasterRun* run;       // the rasters: small from the front, middle from n_rasters - 1 down, large from n_rasters on
+    uint32_t n_rasters, middle, large;
+    uint32_t first;             // of the launch, in the order large, middle, small
+    const int4* bbox;
+    const uint64_t* key_base;
+    const uint32_t* line_ent_total;
+};
+template <int THREADS, int ITEMS>
+constexpr size_t local_sort_smem() {
+    return (size_t)THREADS * ITEMS * 4 + (size_t)(THREADS / 32) * 256 * 4 + 256 * 4;
+}
+template <class K, int THREADS, int ITEMS, int BLOCKS>
+__global__ void __launch_bounds__(THREADS, BLOCKS) k_sort_local(const K* __restrict__ keys_in,
+                                                                const uint32_t* __restrict__ vals_in,
+                                                                K* __restrict__ keys_out,
+                                                                uint32_t* __restrict__ vals_out, LocalSortArgs A) {
+    dependent_start();
+    constexpr int WARPS = THREADS / 32;
+    constexpr uint32_t FULL = 0xffffffffu;
+    constexpr int IDX = LOCAL_SORT_IDX_BITS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint32_t* s_word = reinterpret_cast<uint32_t*>(smem);    // [THREADS * ITEMS]
+    uint32_t* s_cnt = s_word + THREADS * ITEMS;              // [WARPS][256]
+    uint32_t* s_dig = s_cnt + WARPS * 256;                   // [256]
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t q = A.first + blockIdx.x;
+    const RasterRun run = A.run[q < A.large              ? A.n_rasters + q
+                                : q < A.large + A.middle ? A.n_rasters - 1u - (q - A.large)
+                                                         : q - A.large - A.middle];
+    const uint32_t r = run.raster, e0 = run.begin, out = run.out;
+    const K base = (K)A.key_base[r];
+    if (run.n == 0u) {   // no increments: its one entry comes after the lines' entries
+        if (tid == 0) {
+            const uint32_t at = *A.line_ent_total + (out - e0);
+            keys_out[out] = keys_in[at];
+            vals_out[out] = vals_in[at];
+        }
+        return;
+    }
+    const uint32_t n = min(run.n, (uint32_t)(THREADS * ITEMS));   // (listed by size: it fits)
+    const int4 bb = A.bbox[r];
+    const uint32_t space = (uint32_t)(bb.z - bb.x + 1) * (uint32_t)(bb.w - bb.y + 1) * 2u;
+    const int bits = 32 - __clz(space - 1u);
+    const int passes = (bits + 7) / 8;
+    const int width = (bits + passes - 1) / passes;
+    const uint32_t mask = (1u << width) - 1u;
+    // a warp owns `steps` times 32 consecutive entries
+    const int steps = (int)((n + THREADS - 1) / THREADS);
+    const uint32_t first = warp * 32u * (uint32_t)steps + lane;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t word[ITEMS], rank[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const uint32_t i = first + 32u * k;
+        word[k] = k < steps && i < n ? (uint32_t)(keys_in[e0 + i] - base) << IDX | i : 0u;
+    }
+    for (int p = 0; p < passes; p++) {
+        const int shift = IDX + p * width;
+        for (uint32_t d = lane; d <= mask; d += 32) s_cnt[warp * 256u + d] = 0u;
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            if (k >= steps) break;
+            const bool valid = first + 32u * k < n;
+            const uint32_t d = (word[k] >> shift) & mask;
+            const uint32_t peers = same_digit<8>(d, valid);
+            const int leader = valid ? __ffs(peers) - 1 : (int)lane;
+            uint32_t b = 0;
+            if ((int)lane == leader && valid) {
+                b = s_cnt[warp * 256u + d];
+                s_cnt[warp * 256u + d] = b + (uint32_t)__popc(peers);
+            }
+            rank[k] = __shfl_sync(FULL, b, leader) + (uint32_t)__popc(peers & lt);
+            __syncwarp();
+        }
+        __syncthreads();
+        // per digit: the warps' starts, then the digits' starts
+        for (uint32_t d = tid; d < 256u; d += THREADS) {
+            uint32_t run = 0;
+            if (d <= mask) {
+#pragma unroll
+                for (int w = 0; w < WARPS; w++) {
+                    const uint32_t c = s_cnt[w * 256u + d];
+                    s_cnt[w * 256u + d] = run;
+                    run += c;
+                }
+            }
+            s_dig[d] = run;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t v[8], sum = 0;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                v[q] = s_dig[lane * 8u + q];
+                sum += v[q];
+            }
+            uint32_t inc = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= (uint32_t)o) inc += t;
+            }
+            uint32_t run = inc - sum;
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                s_dig[lane * 8u + q] = run;
+                run += v[q];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            if (k < steps && first + 32u * k < n) {
+                const uint32_t d = (word[k] >> shift) & mask;
+                s_word[s_dig[d] + s_cnt[warp * 256u + d] + rank[k]] = word[k];
+            }
+        }
+        __syncthreads();
+        if (p + 1 < passes) {
+#pragma unroll
+            for (int k = 0; k < ITEMS; k++) {
+                const uint32_t i = first + 32u * k;
+                if (k < steps && i < n) word[k] = s_word[i];
+            }
+        }
+    }
+    for (uint32_t i = tid; i < n; i += THREADS) {
+        const uint32_t w = s_word[i];
+        keys_out[out + i] = base + (K)(w >> IDX);
+        vals_out[out + i] = vals_in[e0 + (w & ((1u << IDX) - 1u))];
+    }
+}
+
+template <class K, int THREADS, int ITEMS, int BLOCKS>
+static int launch_sort_local(ochre_gpu_ctx* ctx, LocalSortArgs a, uint32_t first, uint32_t rasters, cudaStream_t s) {
+    if (rasters == 0) return OCHRE_OK;
+    constexpr size_t smem = local_sort_smem<THREADS, ITEMS>();
+    if (smem > 48 * 1024)
+        OCHRE_CUDA_TRY(cudaFuncSetAttribute(k_sort_local<K, THREADS, ITEMS, BLOCKS>,
+                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    a.first = first;
+    OCHRE_LAUNCH(ctx, "sort_local", s, launch_after(
+        k_sort_local<K, THREADS, ITEMS, BLOCKS>, rasters, THREADS, smem, s, ctx->keys.as<K>(),
+        ctx->vals.as<uint32_t>(), ctx->keys_alt.as<K>(), ctx->vals_alt.as<uint32_t>(), a));
+    OCHRE_CUDA_TRY(cudaGetLastError());
+    return OCHRE_OK;
+}
+// Few rasters go in one launch, all to the size the largest of them needs
+// (three short launches one after the other took 53 us for a document of 415
+// paths, one 16; the device-wide sort 47).
+constexpr uint32_t LOCAL_SORT_FEW = 1024;
+template <class K>
+static int sort_local(ochre_gpu_ctx* ctx, const LocalSortArgs& a, cudaStream_t s) {
+    const uint32_t R = a.n_rasters, few = R <= LOCAL_SORT_FEW;
+    uint32_t large = a.large, middle = a.middle;
+    if (few && large) {
+        large = R;
+        middle = 0;
+    } else if (few && middle) {
+        middle = R;
+    }
+    int st = launch_sort_local<K, 512, 16, 2>(ctx, a, 0u, large, s);
+    if (st == OCHRE_OK) st = launch_sort_local<K, 256, 16, 4>(ctx, a, large, middle, s);
+    if (st == OCHRE_OK) st = launch_sort_local<K, 128, 8, 8>(ctx, a, large + middle, R - middle - large, s);
+    return st;
+}
+static_assert(LOCAL_SORT_SMALL == 128 * 8 && LOCAL_SORT_MIDDLE == 256 * 16 && LOCAL_SORT_LARGE == 512 * 16 &&
+                  LOCAL_SORT_LARGE <= 1u << LOCAL_SORT_IDX_BITS,
+              "block sizes");
+
+int stage_sort_local(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s) {
+    const DevScalars* hs = host_scalars(ctx);
+    const LocalSortArgs a{ctx->raster_run.as<RasterRun>(), in->n_rasters, hs->n_sort[0], hs->n_sort[1], 0u,
+                          ctx->raster_bbox.as<int4>(), ctx->raster_keybase.as<uint64_t>(),
+                          &dev_scalars(ctx)->line_ent_total};
+    const int st = ctx->keys64 ? sort_local<uint64_t>(ctx, a, s) : sort_local<uint32_t>(ctx, a, s);
+    if (st != OCHRE_OK) return st;
+    std::swap(ctx->keys, ctx->keys_alt);
+    std::swap(ctx->vals, ctx->vals_alt);
+    return OCHRE_OK;
+}
+
 }  // namespace ochre
