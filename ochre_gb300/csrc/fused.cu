@@ -527,9 +527,8 @@ __global__ void __launch_bounds__(THREADS, fused_min_ctas(THREADS)) k_raster_fus
                     const float cov0 = fabsf(acc0 + a0);
                     const float cov1 = fabsf((acc0 + h0) + a1);
                     const size_t t = stage0 + lo + i;
-                    const uint32_t al0 = f2u8(rmin(cov0 * 256.0f, 255.0f));
-                    const uint32_t al1 = f2u8(rmin(cov1 * 256.0f, 255.0f));
-                    reinterpret_cast<uint16_t*>(A.stage_alpha + t * 64)[lane] = (uint16_t)(al0 | (al1 << 8));
+                    reinterpret_cast<uint16_t*>(A.stage_alpha + t * 64)[lane] =
+                        (uint16_t)__byte_perm(alpha_bits(cov0), alpha_bits(cov1), 0x0040);
                     if (A.out_cov) reinterpret_cast<float2*>(A.stage_cov + t * 64)[lane] = make_float2(cov0, cov1);
                 }
                 __syncthreads();

@@ -269,17 +269,19 @@ __device__ __forceinline__ void add_chunk_increments(const uint32_t* __restrict_
                                                      const uint32_t* s_head, int nt, float (*acc)[ACC_STRIDE],
                                                      BinStage& st) {
     const int lane = threadIdx.x & 31;
+    const uint32_t le_mask = 0xffffffffu >> (31 - lane);
+    const uint32_t my_head = lane > 0 && lane < nt ? s_head[lane] : 0xffffffffu;   // of the chunk's later tiles
     for (uint32_t eb = e0; eb < e1; eb += 32) {
         const uint32_t e = eb + lane;
         uint32_t n = 0, inc = 0, xy = 0, meta = 0;
+        // an entry's tile: the heads before the batch and those up to it
+        const int slots_before = __popc(__ballot_sync(0xffffffffu, my_head < eb));
+        const uint32_t heads_in = __reduce_or_sync(0xffffffffu, my_head - eb < 32u ? 1u << (my_head - eb) : 0u);
         if (e < e1) {
             const uint32_t v = vals[e];
             if (!(v & CROSS_TAG)) {
                 const BinRec rec = bins[v];
-                int slot = 0;
-#pragma unroll
-                for (int i = 1; i < CH; i++)
-                    if (i < nt && s_head[i] <= e) slot = i;
+                const int slot = slots_before + __popc(heads_in & le_mask);
                 n = rec.n;
                 inc = rec.inc;
                 xy = (uint32_t)(uint16_t)rec.x | ((uint32_t)(uint16_t)rec.y << 16);
@@ -528,18 +530,17 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
         if (valid) {
             const uint32_t t = t0 + i;
             float accum = carry;
-            uint32_t lo = 0, hi = 0;
+            uint32_t al[8];
             float cv[8];
 #pragma unroll
             for (int c = 0; c < 8; c++) {
                 const float sum = accum + a[c];
-                const float cov = fabsf(sum);
-                cv[c] = cov_signed ? sum : cov;
-                const uint32_t al = f2u8(rmin(cov * 256.0f, 255.0f));
-                if (c < 4) lo |= al << (8 * c); else hi |= al << (8 * (c - 4));
+                cv[c] = cov_signed ? sum : fabsf(sum);
+                al[c] = alpha_bits(sum);
                 accum = accum + h[c];
             }
-            reinterpret_cast<uint2*>(out_alpha + (size_t)t * 64)[y] = make_uint2(lo, hi);
+            reinterpret_cast<uint2*>(out_alpha + (size_t)t * 64)[y] =
+                make_uint2(pack_bytes(al[0], al[1], al[2], al[3]), pack_bytes(al[4], al[5], al[6], al[7]));
             if (out_cov) {
                 float4* o = reinterpret_cast<float4*>(out_cov + (size_t)t * 64 + 8 * y);
                 o[0] = make_float4(cv[0], cv[1], cv[2], cv[3]);
@@ -640,18 +641,17 @@ __global__ void __launch_bounds__(128) k_tile_cov(
                     if (valid) {
                         const uint32_t t = t0 + i;
                         float accum = carry;
-                        uint32_t lo = 0, hi = 0;
+                        uint32_t al[8];
                         float cv[8];
 #pragma unroll
                         for (int c = 0; c < 8; c++) {
                             const float sum = accum + a[c];
-                            const float cov = fabsf(sum);
-                            cv[c] = cov_signed ? sum : cov;
-                            const uint32_t al = f2u8(rmin(cov * 256.0f, 255.0f));
-                            if (c < 4) lo |= al << (8 * c); else hi |= al << (8 * (c - 4));
+                            cv[c] = cov_signed ? sum : fabsf(sum);
+                            al[c] = alpha_bits(sum);
                             accum = accum + h[c];
                         }
-                        reinterpret_cast<uint2*>(out_alpha + (size_t)t * 64)[y] = make_uint2(lo, hi);
+                        reinterpret_cast<uint2*>(out_alpha + (size_t)t * 64)[y] =
+                            make_uint2(pack_bytes(al[0], al[1], al[2], al[3]), pack_bytes(al[4], al[5], al[6], al[7]));
                         if (out_cov) {
                             float4* o = reinterpret_cast<float4*>(out_cov + (size_t)t * 64 + 8 * y);
                             o[0] = make_float4(cv[0], cv[1], cv[2], cv[3]);
