@@ -85,7 +85,7 @@ __device__ __forceinline__ uint32_t pack_bytes(uint32_t a, uint32_t b, uint32_t 
 // bits.  A float-to-integer conversion runs at a quarter of an add's rate;
 // eight of them a row, with their range checks, and the entries' tiles by a
 // search instead of by bits (tiles.cu) were a tenth of the coverage kernel:
-// 9.05 ms -> 8.07 ms for 8 million tiles.
+// 9.05 ms -> 8.07 ms for 70 million tiles.
 __device__ __forceinline__ uint32_t alpha_bits(float sum) {
     return __float_as_uint(__fadd_rd(fminf(__fmul_rn(fabsf(sum), 256.0f), 255.0f), 8388608.0f));
 }

@@ -123,84 +123,58 @@ __device__ __forceinline__ void lb_publish(const FusedArgs& A, uint32_t r, uint3
 __device__ __forceinline__ void lb_resolve(const FusedArgs& A, uint32_t r, uint32_t a0, uint32_t a1, uint32_t& p0,
                                            uint32_t& p1) {
     const int lane = threadIdx.x & 31;
-    const uint32_t b = r / LB_BLOCK, b0 = b * LB_BLOCK;
+    const uint32_t b = r / LB_BLOCK;
     long long spins = 0;
     const long long poll_limit = spin_limit(A.err);
     p0 = 0;
     p1 = 0;
-    // level 1: the rasters of this block before r, nearest first (q = k * 32 + lane)
-    bool done = false;
+    // Level 1: the rasters of this block before r; then level 2: whole blocks
+    // before it.  Nearest first, LB_BLOCK words a round (q = k * 32 + lane),
+    // one copy of the round for both.
+    const uint64_t* inc = A.r_inc;
+    const uint64_t* agg = A.r_agg;
+    int64_t top = (int64_t)r - 1, bottom = (int64_t)(b * LB_BLOCK);
+    bool rasters = true;
+#pragma unroll 1
     for (;;) {
         uint64_t wa[LB_PER_LANE], wi[LB_PER_LANE];
 #pragma unroll
         for (int k = 0; k < LB_PER_LANE; k++) {
-            const int64_t j = (int64_t)r - 1 - (k * 32 + lane);
-            const bool in = j >= (int64_t)b0;
-            wi[k] = in ? ld_relaxed64(A.r_inc + j) : 0ull;
-            wa[k] = in ? ld_relaxed64(A.r_agg + j) : CH_AGG;
+            const int64_t j = top - (k * 32 + lane);
+            const bool in = j >= bottom;
+            wi[k] = in ? ld_relaxed64(inc + j) : rasters ? 0ull : CH_INC;   // before block 0: an inclusive zero
+            wa[k] = in ? ld_relaxed64(agg + j) : CH_AGG;
         }
-        int q_inc = LB_BLOCK;   // nearest predecessor of the block already placed
+        int q_inc = LB_BLOCK;   // nearest predecessor already placed
+        bool missing = false;
 #pragma unroll
         for (int k = LB_PER_LANE - 1; k >= 0; k--) {
             const uint32_t m = __ballot_sync(0xffffffffu, ch_flag(wi[k]) == 2u);
             if (m) q_inc = k * 32 + __ffs(m) - 1;
         }
-        bool missing = false;
+        uint32_t v0 = 0, v1 = 0;
 #pragma unroll
-        for (int k = 0; k < LB_PER_LANE; k++)
-            if (k * 32 + lane < q_inc && ch_flag(wa[k]) == 0u) missing = true;
+        for (int k = 0; k < LB_PER_LANE; k++) {
+            const int q = k * 32 + lane;
+            const uint64_t w = q < q_inc ? wa[k] : q == q_inc ? wi[k] : CH_AGG;
+            missing = missing || ch_flag(w) == 0u;
+            v0 += ch_t(w);
+            v1 += ch_s(w);
+        }
         if (__any_sync(0xffffffffu, missing)) {
             if (wait_give_up_warp(spins, poll_limit, A.err)) return;
             if (spins > 16) __nanosleep(64);
             continue;
         }
-        uint32_t v0 = 0, v1 = 0;
-#pragma unroll
-        for (int k = 0; k < LB_PER_LANE; k++) {
-            const int q = k * 32 + lane;
-            if (q < q_inc) {
-                v0 += ch_t(wa[k]);
-                v1 += ch_s(wa[k]);
-            } else if (q == q_inc) {
-                v0 += ch_t(wi[k]);
-                v1 += ch_s(wi[k]);
-            }
-        }
-        p0 = __reduce_add_sync(0xffffffffu, v0);
-        p1 = __reduce_add_sync(0xffffffffu, v1);
-        done = q_inc < LB_BLOCK;
-        break;
-    }
-    // level 2: whole blocks before this one, nearest first, 32 per round
-    int64_t top = (int64_t)b - 1;
-    while (!done && top >= 0) {
-        const int64_t j = top - lane;
-        uint64_t bi = 0, ba = CH_AGG;
-        if (j >= 0) {
-            bi = ld_relaxed64(A.b_inc + j);
-            ba = ld_relaxed64(A.b_agg + j);
-        } else {
-            bi = CH_INC;   // before block 0: an inclusive zero
-        }
-        const uint32_t m = __ballot_sync(0xffffffffu, ch_flag(bi) == 2u);
-        const int q_inc = m ? __ffs(m) - 1 : 32;
-        if (__any_sync(0xffffffffu, lane < q_inc && ch_flag(ba) == 0u)) {
-            if (wait_give_up_warp(spins, poll_limit, A.err)) return;
-            if (spins > 16) __nanosleep(64);
-            continue;
-        }
-        uint32_t v0 = 0, v1 = 0;
-        if (lane < q_inc) {
-            v0 = ch_t(ba);
-            v1 = ch_s(ba);
-        } else if (lane == q_inc) {
-            v0 = ch_t(bi);
-            v1 = ch_s(bi);
-        }
         p0 += __reduce_add_sync(0xffffffffu, v0);
         p1 += __reduce_add_sync(0xffffffffu, v1);
-        if (m) break;
-        top -= 32;
+        if (q_inc < (int)LB_BLOCK) break;
+        top = rasters ? (int64_t)b - 1 : top - LB_BLOCK;
+        if (top < 0) break;
+        bottom = 0;
+        inc = A.b_inc;
+        agg = A.b_agg;
+        rasters = false;
     }
     p0 = min(p0, CH_MAX);
     p1 = min(p1, CH_MAX);
