@@ -129,32 +129,36 @@ __device__ __forceinline__ LineCount count_line(V2 a, V2 p, uint32_t* err) {
     return n;
 }
 
-// Block-local work order by walk length: the BLOCK items of a block are
-// grouped by log2 of their cell count (unstable within a group), so each
-// warp walks lines of about the same length and a warp of short lines does
-// not run as long as the longest line of a random 32.  Returns the item
-// (0..BLOCK-1 within the block) this thread walks.  Every thread of the
-// block calls it.
-template <int BLOCK>
-__device__ __forceinline__ uint32_t order_by_length(uint32_t cells, uint32_t* s_cnt, uint16_t* s_item) {
-    constexpr int GROUPS = 17;
-    const uint32_t g = min(31u - (uint32_t)__clz(max(cells, 1u)), (uint32_t)GROUPS - 1u);
-    if (threadIdx.x < GROUPS) s_cnt[threadIdx.x] = 0u;
+// Block-local work order by walk length: the items of a block are grouped by
+// log2 of their cell count (unstable within a group), so each warp walks
+// lines of about the same length and a warp of short lines does not run as
+// long as the longest of a random 32.  Not finer: neighbours in a group are
+// neighbours in memory, and what their lanes write lies together (groups of
+// one cell count, eight an octave from 32 on: 7.45 ms instead of 7.20 for the 60 M
+// lines of 20,000 uneven paths).  Returns this thread's place in that order; items without a
+// walk (cells 0) come last, from *n_walks on.  Every thread of the block calls
+// it.
+constexpr int LENGTH_GROUPS = 17;
+__device__ __forceinline__ uint32_t order_by_length(uint32_t cells, uint32_t* s_cnt, uint32_t* n_walks) {
+    const uint32_t g = cells == 0u ? (uint32_t)LENGTH_GROUPS - 1u : 31u - (uint32_t)__clz(cells);
+    if (threadIdx.x < LENGTH_GROUPS) s_cnt[threadIdx.x] = 0u;
     __syncthreads();
     const uint32_t k = atomicAdd(&s_cnt[g], 1u);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0;
-        for (int q = 0; q < GROUPS; q++) {
-            const uint32_t c = s_cnt[q];
-            s_cnt[q] = run;
-            run += c;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        const uint32_t c = lane < LENGTH_GROUPS ? s_cnt[lane] : 0u;
+        uint32_t inc = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += o;
         }
+        if (lane < LENGTH_GROUPS) s_cnt[lane] = inc - c;
     }
     __syncthreads();
-    s_item[s_cnt[g] + k] = (uint16_t)threadIdx.x;
-    __syncthreads();
-    return s_item[threadIdx.x];
+    *n_walks = s_cnt[LENGTH_GROUPS - 1];
+    return s_cnt[g] + k;
 }
 
 // The next window of a warp (lane 0 takes the ticket).
@@ -171,29 +175,6 @@ __device__ __forceinline__ void box_grow(int4* d, int x0, int y0, int x1, int y1
     if (y0 < cur.y) atomicMin(&d->y, y0);
     if (x1 > cur.z) atomicMax(&d->z, x1);
     if (y1 > cur.w) atomicMax(&d->w, y1);
-}
-
-// The rest of a line's walk from its current state: walk_line's loop with
-// the job's callbacks, then job.end.
-template <class Job>
-__device__ __forceinline__ void walk_one(const Walk& w, WalkState& s, Job& job) {
-    int ty_prev = div8(s.y);
-    bool capped = false;
-    for (uint32_t it = 0;;) {
-        job.cell(w, s);
-        const bool done = walk_step(w, s);
-        const int ty = div8(s.y);
-        if (ty != ty_prev) {
-            job.cross(div8(s.x), min(ty_prev, ty), (int)(int8_t)(int16_t)(ty - ty_prev));
-            ty_prev = ty;
-        }
-        if (done) break;
-        if (++it >= WALK_CAP) {
-            capped = true;
-            break;
-        }
-    }
-    job.end(capped);
 }
 
 // ---------------------------------------------------------------------
@@ -520,110 +501,8 @@ struct RasterOut {
     }
 };
 
-template <class K>
-__device__ __forceinline__ K make_key(uint64_t base, const int4& bb, int tx, int ty, uint32_t kind) {
-    const uint64_t w = (uint64_t)(bb.z - bb.x + 1);
-    return (K)(base + (((uint64_t)(ty - bb.y) * w + (uint64_t)(tx - bb.x)) << 1) + kind);
-}
-
-// Entries and increments of the emit pass (see k_line_emit) for one line.
-template <class K>
-struct EmitJob {
-    const float4* lines;
-    const uint32_t* line_raster;
-    const uint32_t* ent_off;
-    const uint32_t* inc_off;
-    const int4* bbox;
-    const uint64_t* key_base;
-    K* keys;
-    uint32_t* vals;
-    BinRec* bins;
-    float2* incs;
-    // the line's raster (kept while the lane stays in it)
-    uint32_t r;
-    int4 bb;
-    uint64_t base;
-    // the line
-    uint32_t e, q;   // next entry, next stored increment
-    float2 pend;     // increments leave in 16-byte pairs; the first of a pair waits here
-    bool has_pend;
-    int btx, bty, prev_x;   // open bin
-    uint32_t bcount, bentry;
-    BinRec rec;
-
-    __device__ __forceinline__ void flush_bin() {
-        if (bcount) {
-            rec.n = (uint8_t)bcount;
-            *reinterpret_cast<uint4*>(bins + bentry) = *reinterpret_cast<const uint4*>(&rec);
-            keys[bentry] = make_key<K>(base, bb, btx, bty, 1u);
-            vals[bentry] = bentry;
-        }
-    }
-    __device__ __forceinline__ bool begin(uint32_t i, Walk& w, WalkState& s) {
-        const float4 l = lines[i];
-        const V2 a = v2(l.x, l.y), p = v2(l.z, l.w);
-        if (veq(a, p)) return false;
-        const uint32_t ri = line_raster[i];
-        if (ri != r) {
-            r = ri;
-            bb = bbox[ri];
-            base = key_base[ri];
-        }
-        e = ent_off[i];
-        q = inc_off[i];
-        has_pend = false;
-        btx = bty = 0x7fffffff;
-        prev_x = 0;
-        bcount = 0;
-        walk_setup(a, p, w, s);
-        return true;
-    }
-    __device__ __forceinline__ void cell(const Walk& w, const WalkState& s) {
-        float area, height;
-        walk_increment(w, s, area, height);
-        const int tx = div8(s.x), ty = div8(s.y);
-        if (tx != btx || ty != bty || bcount == BIN_MAX_CELLS) {
-            flush_bin();
-            btx = tx;
-            bty = ty;
-            bcount = 0;
-            bentry = e++;
-            rec.inc = q;
-            rec.raster = r;
-            rec.x = (int16_t)s.x;
-            rec.y = (int16_t)s.y;
-            rec.steps = 0;
-            rec.dirs = (uint8_t)((w.x_dir < 0 ? 1u : 0u) | (w.y_dir < 0 ? 2u : 0u));
-        } else if (s.x != prev_x) {
-            rec.steps = (uint16_t)(rec.steps | (1u << (bcount - 1)));   // the step into this cell moved in x
-        }
-        const float2 v = make_float2(area, height);
-        if ((q & 1u) == 0u) {
-            pend = v;
-            has_pend = true;
-        } else if (has_pend) {
-            reinterpret_cast<float4*>(incs)[q >> 1] = make_float4(pend.x, pend.y, v.x, v.y);
-            has_pend = false;
-        } else {
-            incs[q] = v;   // the line's first increment at an odd index
-        }
-        q++;
-        prev_x = s.x;
-        bcount++;
-    }
-    __device__ __forceinline__ void cross(int tx, int ty, int sign) {
-        const uint32_t c = e++;
-        keys[c] = make_key<K>(base, bb, tx, ty, 0u);
-        vals[c] = CROSS_TAG | (r << 8) | ((uint32_t)sign & 0xffu);
-    }
-    __device__ __forceinline__ void end(bool) {
-        flush_bin();
-        if (has_pend) incs[q - 1] = pend;
-    }
-};
-
-// Entries and increments of queued lines (see k_line_emit and EmitJob, whose
-// entries in the same order these are).
+// Entries and increments of queued lines (see k_line_emit, whose entries in
+// the same order these are).
 template <int G, class K>
 __device__ __forceinline__ void emit_long(const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster,
                                           const uint32_t* __restrict__ ent_off, const uint32_t* __restrict__ inc_off,
@@ -766,43 +645,166 @@ __global__ void __launch_bounds__(LONG_THREADS) k_line_emit_long(
         emit_long<32, K>(lines, line_raster, ent_off, inc_off, bbox, key_base, keys, vals, bins, incs, queue, n, ticket);
 }
 
+// Four increments, one aligned 32-byte store (sm_100 and later).
+__device__ __forceinline__ void store_increments(float2* o, float2 a, float2 b, float2 c, float2 d) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o), "f"(a.x), "f"(a.y), "f"(b.x),
+                 "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y)
+                 : "memory");
+}
+
 // Every thread walks one line, the lines of a block in order of length
 // (order_by_length) so a warp's lanes walk lines of about the same length.
 // Lines of more than long_cells cells are left to k_line_emit_long (default
 // 96: on 20,000 strokes a call takes 4.93 / 4.84 / 4.79 / 4.79 / 4.84 ms at 48 /
 // 64 / 96 / 128 / 192, a document of 415 paths 0.824 .. 0.828 ms up to 96 and
 // 0.852 at 192; one path, shapes and the uneven mix do not care).
+//
+// Bound by the writes: a lane writes its own line's increments, bins and
+// entries, so nearly every store is a request of its own (840 M of 4 to 16
+// bytes for 139 M bins and 689 M increments), and more lanes in flight make it
+// slower (20,000 uneven paths: 5.9 ms alone with 16 to 32 warps an SM, 7.4 ms with 40, 10.4 ms
+// with 64).  So increments leave four at a time, a whole 32-byte sector in one
+// store, offsets and lines are read coalesced before the block orders them,
+// keys are one multiply-add of the key's own width, a cell starts where the
+// one before ended, and a bin, its crossing and the next bin's opening are one
+// branch.  20,000 uneven paths (60 M lines; the long lines beside): 7.86 ms -> 6.37 ms; 1,000
+// shapes 128 -> 110 us; 128 dense scenes (14 M lines of two cells) 388 -> 364 us.
+constexpr int EMIT_BLOCK = 128;
+constexpr int EMIT_CARVEOUT = 28;          // percent shared: room for the blocks that fit by registers
 template <class K>
-__global__ void __launch_bounds__(256) k_line_emit(const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster,
-                            const uint32_t* __restrict__ ent_off, const uint32_t* __restrict__ inc_off, uint64_t n_cap,
-                            const uint32_t* n_dev, const int4* __restrict__ bbox, const uint64_t* __restrict__ key_base,
-                            K* __restrict__ keys, uint32_t* __restrict__ vals, BinRec* __restrict__ bins,
-                            float2* __restrict__ incs, uint32_t long_cells) {
+__global__ void __launch_bounds__(EMIT_BLOCK) k_line_emit(
+    const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster, const uint32_t* __restrict__ ent_off,
+    const uint32_t* __restrict__ inc_off, uint64_t n_cap, const uint32_t* n_dev, const int4* __restrict__ bbox,
+    const uint64_t* __restrict__ key_base, K* __restrict__ keys, uint32_t* __restrict__ vals,
+    BinRec* __restrict__ bins, float2* __restrict__ incs, uint32_t long_cells) {
     dependent_start();
-    __shared__ uint32_t s_cnt[17];
-    __shared__ uint16_t s_item[256];
+    __shared__ uint32_t s_cnt[LENGTH_GROUPS];
+    __shared__ float4 s_line[EMIT_BLOCK];
+    __shared__ uint4 s_off[EMIT_BLOCK];   // first entry, first increment, raster, twice the raster's tile columns
+    __shared__ K s_key0[EMIT_BLOCK];      // key of tile (0, 0)
     const uint64_t n_lines = dev_count(n_cap, n_dev);
-    const uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x;
+    const uint64_t i0 = blockIdx.x * (uint64_t)EMIT_BLOCK;
     if (i0 >= n_lines) return;
-    const uint32_t cells = i0 + threadIdx.x < n_lines ? walk_cells(lines[i0 + threadIdx.x]) : 0u;
-    const uint64_t i = i0 + order_by_length<256>(cells, s_cnt, s_item);
-    if (i >= n_lines) return;
-    if (long_cells && walk_cells(lines[i]) > long_cells) return;
-    EmitJob<K> job;
-    job.lines = lines;
-    job.line_raster = line_raster;
-    job.ent_off = ent_off;
-    job.inc_off = inc_off;
-    job.bbox = bbox;
-    job.key_base = key_base;
-    job.keys = keys;
-    job.vals = vals;
-    job.bins = bins;
-    job.incs = incs;
-    job.r = 0xffffffffu;
+    {
+        const uint64_t i = i0 + threadIdx.x;
+        uint32_t cells = 0;
+        float4 l = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        uint4 off = make_uint4(0u, 0u, 0u, 0u);
+        K key0 = 0;
+        if (i < n_lines) {
+            l = lines[i];
+            off = make_uint4(ent_off[i], inc_off[i], line_raster[i], 0u);
+            cells = walk_cells(l);
+            if ((l.x == l.z && l.y == l.w) || (long_cells && cells > long_cells)) cells = 0;
+            if (cells) {
+                const int4 bb = bbox[off.z];
+                const K cols = (K)(bb.z - bb.x + 1);
+                key0 = (K)key_base[off.z] - (((K)(int64_t)bb.y * cols + (K)(int64_t)bb.x) << 1);
+                off.w = (uint32_t)cols << 1;
+            }
+        }
+        uint32_t n_walks;
+        const uint32_t at = order_by_length(cells, s_cnt, &n_walks);
+        s_line[at] = l;
+        s_off[at] = off;
+        s_key0[at] = key0;
+        __syncthreads();
+        if (threadIdx.x >= n_walks) return;
+    }
+    const float4 l = s_line[threadIdx.x];
+    const uint4 off = s_off[threadIdx.x];
+    const K key0 = s_key0[threadIdx.x];
+    const K cols2 = (K)off.w;
+    const uint32_t r = off.z;
     Walk w;
     WalkState s;
-    if (job.begin((uint32_t)i, w, s)) walk_one(w, s, job);
+    walk_setup(v2(l.x, l.y), v2(l.z, l.w), w, s);
+    // A cell's start parameter is the larger of the two axes' last steps,
+    // which is the step into the cell, so its start point is the end point of
+    // the cell before.  Before both axes have stepped 0 takes part, which
+    // matters to a step below 0 (cells at the i16 limits).
+    const bool below = rmin(s.row_t1, s.col_t1) < 0.0f;
+    bool row_moved = false, col_moved = false;
+    V2 p0 = w.a;
+    uint32_t e = off.x, q = off.y;   // next entry, next increment
+    const uint32_t q_cap = q + WALK_CAP;
+    // increments leave in fours, a whole 32-byte sector; three wait here
+    float2 h0 = make_float2(0.0f, 0.0f), h1 = h0, h2 = h0;
+    bool held = false;
+    // the open bin: entry, tile, cells, steps and first cell
+    uint32_t bin = e++, b_n = 0, b_steps = 0, b_inc = q;
+    int btx = div8(s.x), bty = div8(s.y);
+    uint32_t b_xy = (uint32_t)(uint16_t)s.x | ((uint32_t)(uint16_t)s.y << 16);
+    const uint32_t dirs = (w.x_dir < 0 ? 1u << 24 : 0u) | (w.y_dir < 0 ? 2u << 24 : 0u);
+    for (;;) {
+        // walk_increment (rasterizer.rs:98-106)
+        const bool row = s.row_t1 < s.col_t1;
+        const float t1 = row ? s.row_t1 : s.col_t1;
+        const V2 p1 = vlerp(t1, w.a, w.p);
+        const float height = __fsub_rn(p1.y, p0.y);
+        const float right = (float)wrap16(s.x + 1);
+        const float2 v = make_float2(
+            __fmul_rn(__fmul_rn(0.5f, height), __fadd_rn(__fsub_rn(right, p0.x), __fsub_rn(right, p1.x))), height);
+        if ((q & 3u) == 3u && held) {
+            store_increments(incs + (q - 3u), h0, h1, h2, v);
+            held = false;
+        } else if (held || (q & 3u) == 0u) {
+            if ((q & 3u) == 0u) h0 = v;
+            if ((q & 3u) == 1u) h1 = v;
+            if ((q & 3u) == 2u) h2 = v;
+            held = true;
+        } else {
+            incs[q] = v;   // before the line's first whole sector
+        }
+        q++;
+        b_n++;
+        // walk_step (rasterizer.rs:108-121)
+        p0 = p1;
+        if (below) {
+            if (row) row_moved = true; else col_moved = true;
+            if (t1 < 0.0f && !(row_moved && col_moved)) p0 = w.a;
+        }
+        if (row) {
+            s.row_t1 = rmin(__fadd_rn(s.row_t1, w.y_step), 1.0f);
+            s.y = wrap16(s.y + w.y_dir);
+        } else {
+            s.col_t1 = rmin(__fadd_rn(s.col_t1, w.x_step), 1.0f);
+            s.x = wrap16(s.x + w.x_dir);
+        }
+        const bool snap = t1 == 1.0f;
+        if (snap) {
+            s.x = w.end_x;
+            s.y = w.end_y;
+        }
+        const bool done = snap || q == q_cap;
+        const int tx = div8(s.x), ty = div8(s.y);
+        if (tx != btx || ty != bty || done) {
+            *reinterpret_cast<uint4*>(bins + bin) = make_uint4(b_inc, r, b_xy, b_steps | (b_n << 16) | dirs);
+            keys[bin] = key0 + (K)(int64_t)bty * cols2 + ((K)(int64_t)btx << 1) + (K)1;
+            vals[bin] = bin;
+            if (ty != bty) {
+                keys[e] = key0 + (K)(int64_t)min(bty, ty) * cols2 + ((K)(int64_t)tx << 1);
+                vals[e] = CROSS_TAG | (r << 8) | ((uint32_t)(ty - bty) & 0xffu);
+                e++;
+            }
+            if (done) break;
+            bin = e++;
+            btx = tx;
+            bty = ty;
+            b_n = 0;
+            b_steps = 0;
+            b_inc = q;
+            b_xy = (uint32_t)(uint16_t)s.x | ((uint32_t)(uint16_t)s.y << 16);
+        } else if (!row) {
+            b_steps |= 1u << (b_n - 1u);   // the step into the next cell moves in x
+        }
+    }
+    if (held) {
+        float2* o = incs + (q & ~3u);
+        o[0] = h0;
+        if ((q & 3u) >= 2u) o[1] = h1;
+        if ((q & 3u) == 3u) o[2] = h2;
+    }
 }
 
 template <class K>
@@ -986,25 +988,25 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
         cudaStream_t side = s;
         if (long_blocks) OCHRE_CUDA_TRY(fork_walks(ctx, s, &side));
         if (long_blocks && ctx->keys64)
-            OCHRE_LAUNCH(ctx, "dda_emit_long", side, k_line_emit_long<uint64_t><<<long_blocks, LONG_THREADS, 0, side>>>(
+            OCHRE_LAUNCH(ctx, "dda_emit_long", side, launch_beside(EMIT_CARVEOUT, k_line_emit_long<uint64_t>, long_blocks, LONG_THREADS, 0, side,
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint64_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), queue, &ds->n_long, &ds->walk_ticket));
         else if (long_blocks)
-            OCHRE_LAUNCH(ctx, "dda_emit_long", side, k_line_emit_long<uint32_t><<<long_blocks, LONG_THREADS, 0, side>>>(
+            OCHRE_LAUNCH(ctx, "dda_emit_long", side, launch_beside(EMIT_CARVEOUT, k_line_emit_long<uint32_t>, long_blocks, LONG_THREADS, 0, side,
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), queue, &ds->n_long, &ds->walk_ticket));
         if (ctx->keys64)
-            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint64_t>, (unsigned)((n_lines + 255) / 256), 256, 0, s, 
+            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint64_t>, (unsigned)((n_lines + EMIT_BLOCK - 1) / EMIT_BLOCK), EMIT_BLOCK, 0, s,
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint64_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), long_cells));
         else
-            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint32_t>, (unsigned)((n_lines + 255) / 256), 256, 0, s, 
+            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint32_t>, (unsigned)((n_lines + EMIT_BLOCK - 1) / EMIT_BLOCK), EMIT_BLOCK, 0, s, 
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),

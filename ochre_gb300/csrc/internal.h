@@ -395,6 +395,25 @@ cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
 }
+// A launch that another one, on another stream, is to run beside: an SM takes
+// blocks of two kernels only where both ask for the same split of its memory
+// between L1 and shared memory (`carveout`, percent shared), so a kernel that
+// uses none has to ask for its neighbour's.
+template <class... Params, class... Args>
+cudaError_t launch_beside(int carveout, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                          Args&&... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute a{};
+    a.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    a.val.sharedMemCarveout = (unsigned)carveout;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+}
 
 #define OCHRE_CUDA_TRY(expr)                                   \
     do {                                                       \
