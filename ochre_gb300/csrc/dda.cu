@@ -396,7 +396,9 @@ __global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restr
     if (lane == 0 && crosses) atomicAdd(n_cross, crosses);
 }
 // Entry and increment offsets of every line, one scan of the pair (in place:
-// every count is read by the thread that writes its offset).
+// every count is read by the thread that writes its offset).  Bound by memory
+// requests: with a thread's 8 items in 16-byte accesses (load_all, store_all) 60
+// M lines take 326 us, item by item 686 (14 M lines 84 and 176).
 struct LinePair {
     uint32_t ent, inc;
 };
@@ -409,6 +411,15 @@ struct LinePairIn {
     const uint32_t* ent;
     const uint32_t* inc;
     __device__ __forceinline__ LinePair operator()(uint64_t i) const { return LinePair{ent[i], inc[i]}; }
+    using takes_all = void;
+    template <int N>
+    __device__ __forceinline__ void load_all(uint64_t i, LinePair (&v)[N]) const {
+        uint32_t e[N], q[N];
+        load_words(ent + i, e);
+        load_words(inc + i, q);
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = LinePair{e[k], q[k]};
+    }
 };
 struct LinePairOut {
     uint32_t* ent;
@@ -416,6 +427,19 @@ struct LinePairOut {
     __device__ __forceinline__ void operator()(uint64_t i, LinePair ex, LinePair) const {
         ent[i] = ex.ent;
         inc[i] = ex.inc;
+    }
+    using takes_all = void;
+    template <int N>
+    __device__ __forceinline__ void store_all(uint64_t i, LinePair run, const LinePair (&v)[N]) const {
+        uint32_t e[N], q[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            e[k] = run.ent;
+            q[k] = run.inc;
+            run = OpLinePair{}(run, v[k]);
+        }
+        store_words(ent + i, e);
+        store_words(inc + i, q);
     }
 };
 

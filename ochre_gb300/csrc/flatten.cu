@@ -98,13 +98,14 @@ __device__ uint32_t count_cmd(const CmdCtx& k, bool* capped) {
     return n;
 }
 
-struct OffOut {
-    uint32_t* off;
-    __device__ __forceinline__ void operator()(uint64_t i, uint32_t ex, uint32_t) const { off[i] = ex; }
-};
 struct Load32 {
     const uint32_t* v;
     __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return v[i]; }
+    using takes_all = void;
+    template <int N>
+    __device__ __forceinline__ void load_all(uint64_t i, uint32_t (&w)[N]) const {
+        load_words(v + i, w);
+    }
 };
 
 // Line counts, one thread per command, then a scan of them (a scan that counted
@@ -181,7 +182,7 @@ int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uin
                                                        ctx->cmd_line_off.as<uint32_t>(), &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
     OCHRE_LAUNCH(ctx, "flatten_count_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-        ctx, n, Load32{ctx->cmd_line_off.as<uint32_t>()}, OffOut{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u,
+        ctx, n, Load32{ctx->cmd_line_off.as<uint32_t>()}, ScanOff{ctx->cmd_line_off.as<uint32_t>()}, OpSumU32{}, 0u,
         &ds->n_lines, s)));
     uint32_t L;
     if (plan) {

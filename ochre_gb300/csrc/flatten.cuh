@@ -7,6 +7,7 @@
 
 #include "common.cuh"
 #include "internal.h"
+#include "scan.cuh"
 
 namespace ochre {
 
@@ -65,6 +66,20 @@ struct CmdIn {
         const uint32_t id = (uint32_t)i + 1u;
         return CmdScan{floats_per_verb(v), v == V_MOVE ? id : 0u, v <= V_CONIC ? id : 0u};
     }
+    using takes_all = void;
+    template <int N>
+    __device__ __forceinline__ void load_all(uint64_t i, CmdScan (&v)[N]) const {
+        uint32_t b[N];
+        load_bytes(verbs + i, b);
+        uint32_t top = 0;
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            top = max(top, b[k]);
+            const uint32_t id = (uint32_t)i + k + 1u;
+            v[k] = CmdScan{floats_per_verb((uint8_t)b[k]), b[k] == V_MOVE ? id : 0u, b[k] <= V_CONIC ? id : 0u};
+        }
+        if (top > V_CLOSE) atomicOr(err, ERR_INVALID);
+    }
 };
 struct CmdOut {
     uint32_t* foff;
@@ -74,6 +89,21 @@ struct CmdOut {
         foff[i] = ex.foff;
         mv[i] = ex.mv;
         ep[i] = ex.ep;
+    }
+    using takes_all = void;
+    template <int N>
+    __device__ __forceinline__ void store_all(uint64_t i, CmdScan run, const CmdScan (&v)[N]) const {
+        uint32_t f[N], m[N], e[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            f[k] = run.foff;
+            m[k] = run.mv;
+            e[k] = run.ep;
+            run = OpCmd{}(run, v[k]);
+        }
+        store_words(foff + i, f);
+        store_words(mv + i, m);
+        store_words(ep + i, e);
     }
 };
 

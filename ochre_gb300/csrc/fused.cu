@@ -802,15 +802,6 @@ static int fused_shape(ochre_gpu_ctx* ctx, const FusedArgs* a, int* grid, cudaSt
 #undef OCHRE_FUSED_CASE
 }
 
-struct VerbFloats {
-    const uint8_t* verbs;
-    __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return floats_per_verb(__ldg(verbs + i)); }
-};
-struct FloatOff {
-    uint32_t* off;
-    __device__ __forceinline__ void operator()(uint64_t i, uint32_t ex, uint32_t) const { off[i] = ex; }
-};
-
 // Runs the fused kernel over the whole batch.  *handled is false when some
 // raster does not fit (the caller then runs the general chain).
 static int run_fused(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, bool* handled, uint32_t* n_tiles,
@@ -866,7 +857,7 @@ static int run_fused(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, 
         OCHRE_CUDA_TRY(reset_scalars(ctx, s));
         if (n_cmds)
             OCHRE_LAUNCH(ctx, "fused_float_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-                ctx, n_cmds, VerbFloats{in->verbs}, FloatOff{ctx->cmd_foff.as<uint32_t>()}, OpSumU32{}, 0u,
+                ctx, n_cmds, VerbFloats{in->verbs}, ScanOff{ctx->cmd_foff.as<uint32_t>()}, OpSumU32{}, 0u,
                 &ds->n_floats, s, nullptr,
                 ctx->test_skip_first_ticket ? 1u : 0u)));
         FusedArgs a{};

@@ -8,6 +8,8 @@
 // and a timeout sets ERR_TIMEOUT instead of hanging.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "internal.h"
 
@@ -98,6 +100,57 @@ __device__ __forceinline__ T scan_lookback(uint32_t tile, const T& tile_agg, Op 
     return prefix;
 }
 
+// Functors over whole arrays of words may take a thread's items at once, in
+// 8- and 16-byte accesses (load_all(i, v), store_all(i, run, v, op) for the
+// ITEMS items from i on): item by item a warp's access touches a sector for
+// every 8 items and each of them ITEMS times.
+template <class F, class = void>
+struct takes_all : std::false_type {};
+template <class F>
+struct takes_all<F, std::void_t<typename F::takes_all>> : std::true_type {};
+// N consecutive words (N 2 or 8; the address a multiple of 8 or 16 bytes).
+template <int N>
+__device__ __forceinline__ void load_words(const uint32_t* p, uint32_t (&w)[N]) {
+    static_assert(N == 2 || N % 4 == 0, "pairs or fours");
+    if constexpr (N == 2) {
+        const uint2 q = *reinterpret_cast<const uint2*>(p);
+        w[0] = q.x;
+        w[1] = q.y;
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k += 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(p + k);
+            w[k] = q.x;
+            w[k + 1] = q.y;
+            w[k + 2] = q.z;
+            w[k + 3] = q.w;
+        }
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_words(uint32_t* p, const uint32_t (&w)[N]) {
+    static_assert(N == 2 || N % 4 == 0, "pairs or fours");
+    if constexpr (N == 2) {
+        *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[1]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k += 4) *reinterpret_cast<uint4*>(p + k) = make_uint4(w[k], w[k + 1], w[k + 2], w[k + 3]);
+    }
+}
+
+// N consecutive bytes, as words (a caller's array may lie anywhere).
+template <int N>
+__device__ __forceinline__ void load_bytes(const uint8_t* p, uint32_t (&b)[N]) {
+    if (N == 8 && (reinterpret_cast<uintptr_t>(p) & 7u) == 0u) {
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+#pragma unroll
+        for (int k = 0; k < N; k++) b[k] = ((k < 4 ? q.x : q.y) >> (8 * (k & 3))) & 0xffu;
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) b[k] = __ldg(p + k);
+    }
+}
+
 template <int BLOCK, int ITEMS, class T, class Op, class In, class Out>
 __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_dev, In in, Out out, Op op,
                                                  T identity, ScanStatus<T>* status, uint32_t* ticket,
@@ -123,12 +176,21 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
 
     T v[ITEMS];
     T acc = identity;
-#pragma unroll
-    for (int k = 0; k < ITEMS; k++) {
-        const uint64_t i = base + k;
-        v[k] = i < n ? in(i) : identity;
-        acc = op(acc, v[k]);
+    const bool whole = base + ITEMS <= n;
+    bool loaded = false;
+    if constexpr (takes_all<In>::value) {
+        if (whole) in.load_all(base, v);
+        loaded = whole;
     }
+    if (!loaded) {
+#pragma unroll
+        for (int k = 0; k < ITEMS; k++) {
+            const uint64_t i = base + k;
+            v[k] = i < n ? in(i) : identity;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) acc = op(acc, v[k]);
     // warp inclusive scan of per-thread aggregates
     T inc = acc;
 #pragma unroll
@@ -161,6 +223,12 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
     T ex_lane = shfl_up_T(inc, 1);
     if (lane == 0) ex_lane = identity;
     T run = op(op(s_prefix, s_warp[warp]), ex_lane);
+    if constexpr (takes_all<Out>::value) {
+        if (whole) {
+            out.store_all(base, run, v);
+            return;
+        }
+    }
 #pragma unroll
     for (int k = 0; k < ITEMS; k++) {
         const uint64_t i = base + k;
@@ -171,6 +239,36 @@ __global__ void __launch_bounds__(BLOCK) k_scan(uint64_t n, const uint32_t* n_de
 
 struct OpSumU32 {
     __device__ __forceinline__ uint32_t operator()(uint32_t a, uint32_t b) const { return a + b; }
+};
+
+// Floats of every command.
+struct VerbFloats {
+    const uint8_t* verbs;
+    __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return floats_per_verb(__ldg(verbs + i)); }
+    using takes_all = void;
+    template <int N>
+    __device__ __forceinline__ void load_all(uint64_t i, uint32_t (&v)[N]) const {
+        uint32_t b[N];
+        load_bytes(verbs + i, b);
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = floats_per_verb((uint8_t)b[k]);
+    }
+};
+// Every item's exclusive prefix.
+struct ScanOff {
+    uint32_t* off;
+    __device__ __forceinline__ void operator()(uint64_t i, uint32_t ex, uint32_t) const { off[i] = ex; }
+    using takes_all = void;
+    template <int N>
+    __device__ __forceinline__ void store_all(uint64_t i, uint32_t run, const uint32_t (&v)[N]) const {
+        uint32_t o[N];
+#pragma unroll
+        for (int k = 0; k < N; k++) {
+            o[k] = run;
+            run += v[k];
+        }
+        store_words(off + i, o);
+    }
 };
 
 constexpr int SCAN_BLOCK = 256;

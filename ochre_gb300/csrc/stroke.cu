@@ -210,15 +210,6 @@ struct UnitOut {
     }
 };
 
-struct PolyFloats {
-    const uint8_t* v;
-    __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return floats_per_verb(v[i]); }
-};
-struct OffOutU32 {
-    uint32_t* off;
-    __device__ __forceinline__ void operator()(uint64_t i, uint32_t ex, uint32_t) const { off[i] = ex; }
-};
-
 __global__ void k_first_close(const uint8_t* __restrict__ pverbs, uint64_t n_poly, const uint32_t* n_dev,
                               const uint32_t* __restrict__ pfill_off, uint32_t n_fills, const uint8_t* __restrict__ flags,
                               uint32_t* __restrict__ first_close) {
@@ -570,7 +561,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     }
     // float offset of every polyline command: an exclusive scan of its float counts
     OCHRE_LAUNCH(ctx, "stroke_pfoff_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
-        ctx, P, PolyFloats{ctx->sk_pverbs.as<uint8_t>()}, OffOutU32{ctx->sk_pfoff.as<uint32_t>()}, OpSumU32{}, 0u,
+        ctx, P, VerbFloats{ctx->sk_pverbs.as<uint8_t>()}, ScanOff{ctx->sk_pfoff.as<uint32_t>()}, OpSumU32{}, 0u,
         static_cast<uint32_t*>(nullptr), s, p_dev)));
     OCHRE_LAUNCH(ctx, "stroke_first_close", s, launch_after(k_first_close, (P + 255) / 256, 256, 0, s, 
         ctx->sk_pverbs.as<uint8_t>(), P, p_dev, ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
