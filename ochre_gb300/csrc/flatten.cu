@@ -25,56 +25,14 @@
 namespace ochre {
 
 
-// Runs the flattening of one command, calling line(a, b) for each line_to
-// in order.  Returns false when a cap was hit.
-template <class Line>
-__device__ bool flatten_cmd(const CmdCtx& k, Line line) {
-    bool capped = false;
-    V2 prev = k.last;
-    auto to = [&](V2 p) { line(prev, p); prev = p; };
-    switch (k.verb) {
-    case V_MOVE:
-        if (!veq(k.last, k.first)) line(k.last, k.first);
-        break;
-    case V_LINE:
-        to(k.pt[0]);
-        break;
-    case V_QUAD: {
-        const float dt = quad_dt(k.last, k.pt[0], k.pt[1]);
-        float t = 0.0f;
-        uint32_t n = 0;
-        while (t < 1.0f) {
-            t = rmin(__fadd_rn(t, dt), 1.0f);
-            to(quad_point(t, k.last, k.pt[0], k.pt[1]));
-            if (++n >= FLATTEN_CAP) { capped = true; break; }
-        }
-        break;
-    }
-    case V_CUBIC: {
-        const float dt = cubic_dt(k.last, k.pt[0], k.pt[1], k.pt[2]);
-        float t = 0.0f;
-        uint32_t n = 0;
-        while (t < 1.0f) {
-            t = rmin(__fadd_rn(t, dt), 1.0f);
-            to(cubic_point(t, k.last, k.pt[0], k.pt[1], k.pt[2]));
-            if (++n >= FLATTEN_CAP) { capped = true; break; }
-        }
-        break;
-    }
-    case V_CONIC:
-        conic_flatten(k.last, k.pt[0], k.pt[1], k.w, &capped, to);
-        break;
-    default:
-        break;
-    }
-    if (k.last_of_raster) {
-        // finish(): line_to(first) when last != first (rasterizer.rs:181-183)
-        const V2 last_end = k.verb == V_CLOSE ? k.last : k.verb == V_CUBIC ? k.pt[2]
-                          : k.verb == V_MOVE || k.verb == V_LINE ? k.pt[0] : k.pt[1];
-        const V2 first_end = k.verb == V_MOVE ? k.pt[0] : k.first;
-        if (!veq(last_end, first_end)) line(last_end, first_end);
-    }
-    return !capped;
+// The line finish() adds after a raster's last command, if any
+// (rasterizer.rs:181-183: line_to(first) when last != first).
+__device__ __forceinline__ bool closing_line(const CmdCtx& k, V2* from, V2* to) {
+    if (!k.last_of_raster) return false;
+    *from = k.verb == V_CLOSE ? k.last : k.verb == V_CUBIC ? k.pt[2]
+          : k.verb == V_MOVE || k.verb == V_LINE ? k.pt[0] : k.pt[1];
+    *to = k.verb == V_MOVE ? k.pt[0] : k.first;
+    return !veq(*from, *to);
 }
 
 // Line count of one command (the count pass never materialises points for
@@ -89,12 +47,8 @@ __device__ uint32_t count_cmd(const CmdCtx& k, bool* capped) {
     case V_CONIC: conic_flatten(k.last, k.pt[0], k.pt[1], k.w, capped, [&](V2) { n++; }); break;
     default: break;
     }
-    if (k.last_of_raster) {
-        const V2 last_end = k.verb == V_CLOSE ? k.last : k.verb == V_CUBIC ? k.pt[2]
-                          : k.verb == V_MOVE || k.verb == V_LINE ? k.pt[0] : k.pt[1];
-        const V2 first_end = k.verb == V_MOVE ? k.pt[0] : k.first;
-        if (!veq(last_end, first_end)) n++;
-    }
+    V2 from, to;
+    if (closing_line(k, &from, &to)) n++;
     return n;
 }
 
@@ -127,28 +81,148 @@ __global__ void __launch_bounds__(128) k_cmd_count(BatchView b, uint32_t* __rest
     counts[c] = n;
 }
 
+// Lines of a block's commands.  SHARED: a curve's line is one thread's work,
+// as the next line of the same curve is the next thread's; the parameter of a
+// point is the reference's serial sum, which a thread carries from one of its
+// lines to the next, and the line's two points follow from it.  The other
+// commands (and a raster's closing line) are written by the thread that read
+// them, and without SHARED the curves as well.  A thread that writes a whole
+// curve writes line after line, 16 bytes at a time in as many places as there
+// are lanes, which is what bounds it with many lines a command: 2.0 M commands,
+// 60 M lines 1.15 ms, shared 0.71 ms.  With few lines a command a thread's
+// lines lie close together and the sharing costs more than it saves (14 M
+// lines of 2.7 M commands 158 us, shared 207), and with few commands the blocks
+// have too many lines each (33,000 commands, 1.1 M lines 26 us, shared 76).  So:
+// shared from 8 lines a command and 131,072 commands on.  (Blocks of 128
+// commands, a conic's stack out of the curves' way: 190 -> 158 us, strokes 174 ->
+// 150.)
 // Lines of more than long_cells cells (walk_cells) are also queued for the
 // long-line emit walk of the DDA stage (long_cells 0: none are).
-__global__ void k_cmd_emit(BatchView b, const uint32_t* __restrict__ line_off, uint32_t n_lines_cap,
-                           float4* __restrict__ lines, uint32_t* __restrict__ line_raster, uint32_t long_cells,
-                           uint32_t* __restrict__ long_lines, uint32_t* n_long, uint32_t* err) {
+constexpr int FLAT_BLOCK = 128;
+constexpr uint64_t FLAT_SHARED_LINES = 8, FLAT_SHARED_CMDS = 1u << 17;
+template <bool SHARED>
+__global__ void __launch_bounds__(FLAT_BLOCK) k_cmd_emit(BatchView b, const uint32_t* __restrict__ line_off,
+                                                         const uint32_t* n_lines, uint32_t n_lines_cap,
+                                                         float4* __restrict__ lines, uint32_t* __restrict__ line_raster,
+                                                         uint32_t long_cells, uint32_t* __restrict__ long_lines,
+                                                         uint32_t* n_long, uint32_t* err) {
     dependent_start();
-    const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-    if (c >= b.n_cmds) return;
-    const CmdCtx k = load_cmd(b, (uint32_t)c);
-    if (!k.ok) return;
-    uint32_t o = line_off[c];
-    flatten_cmd(k, [&](V2 a, V2 p) {
+    // the curves: last, control points and end; parameter step; 2 or 3 (0: no
+    // curve); raster.  And every command's first line.
+    constexpr int CMDS = FLAT_BLOCK, S = SHARED ? CMDS : 1;
+    __shared__ V2 s_p[4][S];
+    __shared__ float s_dt[S];
+    __shared__ uint8_t s_degree[S];
+    __shared__ uint32_t s_raster[S], s_off[S + 1], s_end[S];
+    const uint64_t c0 = blockIdx.x * (uint64_t)CMDS;
+    const int n = (int)min((uint64_t)CMDS, b.n_cmds - c0);
+    auto put = [&](uint32_t o, V2 a, V2 p, uint32_t raster) {
         if (o < n_lines_cap) {
             const float4 l = make_float4(a.x, a.y, p.x, p.y);
             lines[o] = l;
-            line_raster[o] = k.raster;
+            line_raster[o] = raster;
             if (long_cells && walk_cells(l) > long_cells) long_lines[atomicAdd(n_long, 1u)] = o;
         } else {
             atomicOr(err, ERR_CAPACITY);
         }
-        o++;
-    });
+    };
+    uint8_t degree = 0;
+    if ((int)threadIdx.x < n) {
+        const uint64_t c = c0 + threadIdx.x;
+        const CmdCtx k = load_cmd(b, (uint32_t)c);
+        uint32_t o = line_off[c];
+        // (a line count zeroed on the device, after an overflow of a graph's plan, ends no lines)
+        uint32_t end = max(o, c + 1 < b.n_cmds ? line_off[c + 1] : *n_lines);
+        if (k.ok) {
+            V2 from, to;
+            const bool closes = closing_line(k, &from, &to);
+            if (closes && end > o) put(end - 1u, from, to, k.raster);
+            if (closes && end > o) end--;
+            switch (k.verb) {
+            case V_MOVE:
+                if (!veq(k.last, k.first)) put(o, k.last, k.first, k.raster);
+                break;
+            case V_LINE:
+                put(o, k.last, k.pt[0], k.raster);
+                break;
+            case V_QUAD:
+            case V_CUBIC: {
+                degree = k.verb == V_QUAD ? 2 : 3;
+                const float dt = degree == 2 ? quad_dt(k.last, k.pt[0], k.pt[1]) : cubic_dt(k.last, k.pt[0], k.pt[1], k.pt[2]);
+                if (SHARED) {
+                    s_dt[threadIdx.x] = dt;
+                    break;
+                }
+                V2 prev = k.last;
+                float t = 0.0f;
+                for (; o < end; o++) {
+                    t = rmin(__fadd_rn(t, dt), 1.0f);
+                    const V2 p = degree == 2 ? quad_point(t, k.last, k.pt[0], k.pt[1])
+                                             : cubic_point(t, k.last, k.pt[0], k.pt[1], k.pt[2]);
+                    put(o, prev, p, k.raster);
+                    prev = p;
+                }
+                break;
+            }
+            case V_CONIC: {
+                bool capped = false;
+                V2 prev = k.last;
+                conic_flatten(k.last, k.pt[0], k.pt[1], k.w, &capped, [&](V2 p) {
+                    put(o++, prev, p, k.raster);
+                    prev = p;
+                });
+                break;
+            }
+            default:
+                break;
+            }
+            if (SHARED) {
+                s_p[0][threadIdx.x] = k.last;
+                s_p[1][threadIdx.x] = k.pt[0];
+                s_p[2][threadIdx.x] = k.pt[1];
+                s_p[3][threadIdx.x] = k.pt[2];
+                s_raster[threadIdx.x] = k.raster;
+            }
+        }
+        if (SHARED) {
+            s_off[threadIdx.x] = line_off[c];
+            s_degree[threadIdx.x] = degree;
+            s_end[threadIdx.x] = end;   // of the command's own lines
+            if ((int)threadIdx.x == n - 1) s_off[n] = end;
+        }
+    }
+    if (!SHARED) return;
+    if (!__syncthreads_or(degree != 0)) return;
+    int curve = -1;         // the command of the thread's line before this one,
+    uint32_t done = 0;      // the steps of its parameter taken
+    float t = 0.0f;         // and where they led
+    for (uint32_t o = s_off[0] + threadIdx.x; o < s_off[n]; o += FLAT_BLOCK) {
+        int j = 0;   // the last command with s_off <= o
+#pragma unroll
+        for (int step = CMDS / 2; step > 0; step >>= 1)
+            if (j + step < n && s_off[j + step] <= o) j += step;
+        const int degree = s_degree[j];
+        if (degree == 0 || o >= s_end[j]) continue;
+        const V2 last = s_p[0][j], p0 = s_p[1][j], p1 = s_p[2][j], p2 = s_p[3][j];
+        const float dt = s_dt[j];
+        const uint32_t before = o - s_off[j];
+        if (j != curve) {
+            curve = j;
+            done = 0;
+            t = 0.0f;
+        }
+        for (; done < before; done++) t = rmin(__fadd_rn(t, dt), 1.0f);
+        const float t1 = rmin(__fadd_rn(t, dt), 1.0f);
+        V2 a, p;
+        if (degree == 2) {
+            a = quad_point(t, last, p0, p1);
+            p = quad_point(t1, last, p0, p1);
+        } else {
+            a = cubic_point(t, last, p0, p1, p2);
+            p = cubic_point(t1, last, p0, p1, p2);
+        }
+        put(o, before ? a : last, p, s_raster[j]);
+    }
 }
 
 int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uint32_t* n_lines) {
@@ -204,9 +278,11 @@ int stage_flatten(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, uin
     const uint32_t long_cells = (uint32_t)ctx->tune_chain_long_cells;
     if (long_cells) OCHRE_CUDA_TRY(ctx->long_lines.ensure((size_t)L * 4));
     OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->n_long, 0, 4, s));
-    const unsigned blocks = (unsigned)((n + 255) / 256);
-    OCHRE_LAUNCH(ctx, "flatten_emit", s, launch_after(k_cmd_emit, blocks, 256, 0, s, 
-        b, ctx->cmd_line_off.as<uint32_t>(), L, ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), long_cells,
+    // (planned: L is the plan's capacity)
+    const bool shared = L >= FLAT_SHARED_LINES * n && n >= FLAT_SHARED_CMDS;
+    OCHRE_LAUNCH(ctx, "flatten_emit", s, launch_after(shared ? k_cmd_emit<true> : k_cmd_emit<false>,
+        (unsigned)((n + FLAT_BLOCK - 1) / FLAT_BLOCK), FLAT_BLOCK, 0, s, b, ctx->cmd_line_off.as<uint32_t>(), &ds->n_lines,
+        L, ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), long_cells,
         long_cells ? ctx->long_lines.as<uint32_t>() : nullptr, &ds->n_long, &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
     return OCHRE_OK;
