@@ -64,7 +64,10 @@ __device__ __forceinline__ bool bin_before(const uint32_t* __restrict__ vals, ui
 // metadata gathered by a kernel of its own and a scan for the rows took 3.40
 // ms; 1.33 ms here (the coverage kernel finds the rows itself).  Few entries
 // take 4 steps a warp instead of 16, so that more warps share the gathers'
-// latency: one path's 6,339 entries 16 us at 16 steps, 10 us at 4.
+// latency: one path's 6,339 entries 16 us at 16 steps, 10 us at 4.  The records
+// of eight steps are gathered together (one step after the other, the values
+// kept in indexed registers, which are memory: 1.34 ms; four steps 1.14; eight 1.04;
+// 19 M entries of strokes 162 -> 123 us, one path 10 -> 8 us).
 constexpr int HEAD_BLOCK = 256;
 struct HeadArgs {
     const uint32_t* vals;
@@ -85,6 +88,7 @@ __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__
                                                            ScanStatus<HeadScan>* status, uint32_t* ticket,
                                                            uint32_t ticket_base, uint32_t tag, uint32_t* err) {
     dependent_start();
+    constexpr int HEAD_GATHER = HEAD_ITEMS < 8 ? HEAD_ITEMS : 8;   // steps whose records are gathered together
     constexpr int WARPS = HEAD_BLOCK / 32, HEAD_TILE = HEAD_BLOCK * HEAD_ITEMS;
     constexpr uint32_t FULL = 0xffffffffu;
     __shared__ uint32_t s_tile, s_rows;
@@ -171,56 +175,70 @@ __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__
     uint32_t t0 = s_prefix.heads + s_warp[warp].heads;   // tiles before the step
     int32_t w0 = s_prefix.w + s_warp[warp].w;            // signs before the step
     uint32_t rows = 0;
-#pragma unroll 4
-    for (int k = 0; k < HEAD_ITEMS; k++) {
-        const bool is = (heads >> k) & 1u;
-        const bool cross = (val[k] & CROSS_TAG) != 0u;
-        const int sign = cross ? (int)(int8_t)(val[k] & 0xffu) : 0;
-        const uint32_t hm = __ballot_sync(FULL, is);
-        const uint32_t pos = __ballot_sync(FULL, sign == 1), neg = __ballot_sync(FULL, sign == -1);
-        int wb = __popc(pos & lt) - __popc(neg & lt), wt = __popc(pos) - __popc(neg);
-        if (__any_sync(FULL, sign > 1 || sign < -1)) {
-            int inc = sign;
+    // HEAD_GATHER steps at a time: their values again (out of the cache) and
+    // their records, all in flight before the first is used
+#pragma unroll 1
+    for (int k0 = 0; k0 < HEAD_ITEMS; k0 += HEAD_GATHER) {
+        uint32_t v[HEAD_GATHER], rec_r[HEAD_GATHER], rec_xy[HEAD_GATHER];
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int o = __shfl_up_sync(FULL, inc, d);
-                if (lane >= (uint32_t)d) inc += o;
-            }
-            wb = inc - sign;
-            wt = __shfl_sync(FULL, inc, 31);
+        for (int q = 0; q < HEAD_GATHER; q++) {
+            const uint64_t i = base + (k0 + q) * 32 + lane;
+            v[q] = i < n ? A.vals[i] : CROSS_TAG;
         }
-        if (hm) {
-            uint32_t r = 0;
-            int tx = 0, ty = 0;
-            if (is) {
-                const BinRec rec = A.bins[val[k]];
-                r = rec.raster;
-                tx = div8((int)rec.x);
-                ty = div8((int)rec.y);
+#pragma unroll
+        for (int q = 0; q < HEAD_GATHER; q++) {
+            rec_r[q] = rec_xy[q] = 0u;
+            if (heads >> (k0 + q) & 1u) {
+                const uint4 rec = *reinterpret_cast<const uint4*>(A.bins + v[q]);
+                rec_r[q] = rec.y;
+                rec_xy[q] = rec.z;
             }
-            // the head before: in this step, else the last one so far (or the
-            // last bin before the warp: the same tile as the head before)
-            const uint32_t below = hm & lt;
-            const int src = below ? 31 - __clz(below) : 0;
-            const uint32_t sr = __shfl_sync(FULL, r, src);
-            const int sy = __shfl_sync(FULL, ty, src);
-            const uint32_t pr = below ? sr : prev_r;
-            const int py = below ? sy : prev_ty;
-            const bool row = is && (pr != r || py != ty);
-            if (is) {
-                const uint32_t t = t0 + (uint32_t)__popc(below);
-                A.head[t] = (uint32_t)(base + k * 32 + lane);
-                A.xy[t] = pack_tile(tx, ty);
-                A.rf[t] = r | (w0 + wb != A.raster_wbase[r] ? RF_WIND : 0u) | (row ? RF_ROW : 0u);
-                if (pr != r) A.raster_tile_off[r] = t;
-            }
-            rows += (uint32_t)__popc(__ballot_sync(FULL, row));
-            const int last = 31 - __clz(hm);
-            prev_r = __shfl_sync(FULL, r, last);
-            prev_ty = __shfl_sync(FULL, ty, last);
         }
-        t0 += (uint32_t)__popc(hm);
-        w0 += wt;
+#pragma unroll
+        for (int q = 0; q < HEAD_GATHER; q++) {
+            const bool is = heads >> (k0 + q) & 1u;
+            const bool cross = (v[q] & CROSS_TAG) != 0u;
+            const int sign = cross ? (int)(int8_t)(v[q] & 0xffu) : 0;
+            const uint32_t hm = __ballot_sync(FULL, is);
+            const uint32_t pos = __ballot_sync(FULL, sign == 1), neg = __ballot_sync(FULL, sign == -1);
+            int wb = __popc(pos & lt) - __popc(neg & lt), wt = __popc(pos) - __popc(neg);
+            if (__any_sync(FULL, sign > 1 || sign < -1)) {
+                int inc = sign;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int o = __shfl_up_sync(FULL, inc, d);
+                    if (lane >= (uint32_t)d) inc += o;
+                }
+                wb = inc - sign;
+                wt = __shfl_sync(FULL, inc, 31);
+            }
+            if (hm) {
+                const uint32_t r = rec_r[q], at = rec_xy[q];
+                const int tx = div8(tile_tx(at)), ty = div8(tile_ty(at));
+                // the head before: in this step, else the last one so far (or the
+                // last bin before the warp: the same tile as the head before)
+                const uint32_t below = hm & lt;
+                const int src = below ? 31 - __clz(below) : 0;
+                const uint32_t sr = __shfl_sync(FULL, r, src);
+                const int sy = __shfl_sync(FULL, ty, src);
+                const uint32_t pr = below ? sr : prev_r;
+                const int py = below ? sy : prev_ty;
+                const bool row = is && (pr != r || py != ty);
+                if (is) {
+                    const uint32_t t = t0 + (uint32_t)__popc(below);
+                    A.head[t] = (uint32_t)(base + (k0 + q) * 32 + lane);
+                    A.xy[t] = pack_tile(tx, ty);
+                    A.rf[t] = r | (w0 + wb != A.raster_wbase[r] ? RF_WIND : 0u) | (row ? RF_ROW : 0u);
+                    if (pr != r) A.raster_tile_off[r] = t;
+                }
+                rows += (uint32_t)__popc(__ballot_sync(FULL, row));
+                const int last = 31 - __clz(hm);
+                prev_r = __shfl_sync(FULL, r, last);
+                prev_ty = __shfl_sync(FULL, ty, last);
+            }
+            t0 += (uint32_t)__popc(hm);
+            w0 += wt;
+        }
     }
     if (lane == 0 && rows) atomicAdd(&s_rows, rows);
     __syncthreads();
