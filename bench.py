@@ -88,7 +88,7 @@ def kernel_bytes(name: str, st: dict, batch) -> int:
     if name == "flatten_count":
         return batch.verbs.nbytes + batch.pts.nbytes + 24 * batch.n_fills + C * 12 + C * 4
     if name == "flatten_count_scan":
-        return batch.verbs.nbytes + batch.pts.nbytes + 24 * batch.n_fills + C * 12 + C * 4
+        return C * 8
     if name == "flatten_emit":
         return batch.verbs.nbytes + batch.pts.nbytes + 24 * batch.n_fills + C * 16 + L * 20
     I = st.get("n_incs", 0)
@@ -105,18 +105,16 @@ def kernel_bytes(name: str, st: dict, batch) -> int:
         return 2 * E * (kb + 4)
     if name == "sort_hist":
         return E * kb
-    if name == "tile_head_scan":
-        return E * (kb + 4) + T * 4
-    if name == "tile_info":
-        # head, bin count and winding of the tile (and the next tile's bin
-        # count); value and record of its head and its predecessor's; info out
-        return T * 16 + T * 2 * (4 + 16) + T * 32 + R * 8
+    if name == "sort_local":
+        return 2 * E * (kb + 4) + R * 16
+    if name == "tile_heads":
+        # every entry's key and value; a tile's head, place and raster out
+        return E * (kb + 4) + T * 12 + R * 4
     if name == "tile_coverage":
-        # entries: value 4; bins: record 16; increments 8; tiles: info 32 +
-        # 68 out + 12 span slot
-        return E * 4 + B * 16 + I * 8 + T * (32 + 68 + 12)
+        # entries: value 4; bins: record 16; increments 8; tiles: metadata 12 + 68 out
+        return E * 4 + B * 16 + I * 8 + T * (12 + 68)
     if name == "span_scan":
-        return T * 4 + T * 8 + N * 10 + R * 4
+        return T * 8 + N * 10 + R * 4
     if name == "raster_fused":
         # the whole path in one kernel: compulsory input + output bytes, and
         # the float offset of every command (from the command scan)

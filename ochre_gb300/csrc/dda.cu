@@ -683,12 +683,12 @@ __device__ __forceinline__ void store_increments(float2* o, float2 a, float2 b, 
 // 64 / 96 / 128 / 192, a document of 415 paths 0.824 .. 0.828 ms up to 96 and
 // 0.852 at 192; one path, shapes and the uneven mix do not care).
 //
-// Bound by the writes: a lane writes its own line's increments, bins and
-// entries, so nearly every store is a request of its own (840 M of 4 to 16
-// bytes for 139 M bins and 689 M increments), and more lanes in flight make it
-// slower (20,000 uneven paths: 5.9 ms alone with 16 to 32 warps an SM, 7.4 ms with 40, 10.4 ms
-// with 64).  So increments leave four at a time, a whole 32-byte sector in one
-// store, offsets and lines are read coalesced before the block orders them,
+// Bound by its store requests and by issue (77 % of the slots, 13 of 32 lanes
+// active): a lane writes its own line's increments, bins and entries, so nearly
+// every store is a request of its own (840 M of 4 to 16 bytes for 139 M bins and
+// 689 M increments), and more lanes in flight made it slower (20,000 uneven
+// paths: 5.9 ms alone with 16 to 32 warps an SM, 7.4 ms with 40, 10.4 ms with 64).
+// So increments leave four at a time, a whole 32-byte sector in one store, offsets and lines are read coalesced before the block orders them,
 // keys are one multiply-add of the key's own width, a cell starts where the
 // one before ended, and a bin, its crossing and the next bin's opening are one
 // branch.  20,000 uneven paths (60 M lines; the long lines beside): 7.86 ms -> 6.37 ms; 1,000
