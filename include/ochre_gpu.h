@@ -21,6 +21,10 @@
  *
  * Every function returns OCHRE_OK (0) or an ochre_status code.  A context is
  * bound to one CUDA device and one stream; use one context per host thread.
+ * A call that failed leaves the context usable.  The entries that rasterize or
+ * composite read counts back, so on a stream that is being captured they queue
+ * nothing and return OCHRE_E_CUDA (the capture goes on); ochre_graph_* captures
+ * whole chains.
  * Output buffers returned in ochre_result are owned by the context and stay
  * valid until the next rasterize/finish call on it or ochre_gpu_destroy.
  */

@@ -170,8 +170,8 @@ int read_scalars(ochre_gpu_ctx* ctx, cudaStream_t s) {
     return OCHRE_OK;
 }
 
-// Modes: eager on a context of its own: cleared when the buffer is new (or a
-// wait gave up), else not at all.  In a launch chain captured into a graph the
+// Modes: eager on a context of its own: cleared when the buffer is new, a call
+// failed or a wait gave up, else not at all.  In a launch chain captured into a graph the
 // tag and the tickets are fixed arguments, so every scan clears its words and
 // its own ticket word; in an arena (no allocation) the words lie where
 // anything may have lain, and the ticket is the run's.
@@ -207,7 +207,17 @@ cudaError_t scan_space(ochre_gpu_ctx* ctx, size_t status_bytes, uint32_t tiles, 
     out->tag = ++ctx->scan_tag;
     out->ticket_base = ctx->scan_tickets - first_ticket;
     ctx->scan_tickets += tiles;
+    if (ctx->test_fail_scan && --ctx->test_fail_scan == 0u) return cudaErrorMemoryAllocation;
     return cudaSuccess;
+}
+
+bool stream_captures(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {   // (the legacy stream beside a capture)
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
 }
 
 void prof_begin(ochre_gpu_ctx* ctx, const char* name, cudaStream_t s) {
@@ -264,7 +274,8 @@ static bool non_decreasing(const uint32_t* a, uint64_t n) {
     return bad == 0;
 }
 
-int run_device(ochre_gpu_ctx* ctx, const ochre_batch* in_orig, ochre_result* out, cudaStream_t s, bool remember_miss) {
+static int run_chain(ochre_gpu_ctx* ctx, const ochre_batch* in_orig, ochre_result* out, cudaStream_t s,
+                     bool remember_miss) {
     // the test hooks apply to this run only
     struct HookReset {
         ochre_gpu_ctx* c;
@@ -273,7 +284,6 @@ int run_device(ochre_gpu_ctx* ctx, const ochre_batch* in_orig, ochre_result* out
             c->test_skip_first_ticket = 0;
         }
     } hook_reset{ctx};
-    std::memset(out, 0, sizeof *out);
     ctx->epoch++;
     ctx->stats = ochre_stats{};
     ctx->prof_used = 0;
@@ -354,6 +364,15 @@ int run_device(ochre_gpu_ctx* ctx, const ochre_batch* in_orig, ochre_result* out
     out->raster_tile_off = ctx->out_raster_tile_off.as<uint32_t>();
     out->raster_span_off = ctx->out_raster_span_off.as<uint32_t>();
     return OCHRE_OK;
+}
+
+int run_device(ochre_gpu_ctx* ctx, const ochre_batch* in, ochre_result* out, cudaStream_t s, bool remember_miss) {
+    std::memset(out, 0, sizeof *out);
+    if (reads_back(in) && stream_captures(s)) return OCHRE_E_CUDA;
+    const int st = run_chain(ctx, in, out, s, remember_miss);
+    // wherever it failed, a scan may be counted that never ran
+    if (st != OCHRE_OK) ctx->scan_dirty = true;
+    return st;
 }
 
 }  // namespace ochre
@@ -709,6 +728,9 @@ int ochre_gpu_set_tunable(ochre_gpu_ctx* ctx, const char* name, int value) {
     } else if (!std::strcmp(name, "test_skip_first_ticket")) {
         if (value < 0 || value > 1) return OCHRE_E_INVALID;
         ctx->test_skip_first_ticket = (uint32_t)value;
+    } else if (!std::strcmp(name, "test_fail_scan")) {
+        if (value < 0 || value > 64) return OCHRE_E_INVALID;
+        ctx->test_fail_scan = (uint32_t)value;
     } else {
         return OCHRE_E_INVALID;
     }

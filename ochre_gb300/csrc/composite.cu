@@ -297,22 +297,9 @@ static int composite_pieces(ochre_gpu_ctx* ctx, const PieceItems& items, uint32_
     return OCHRE_OK;
 }
 
-}  // namespace ochre
-
-using namespace ochre;
-
-extern "C" int ochre_gpu_composite(ochre_gpu_ctx* ctx, const ochre_result* res, uint32_t n_rasters,
-                                   const uint8_t* colors, uint32_t w, uint32_t h, uint8_t* canvas, void* stream) {
-    if (!ctx || !res || (n_rasters && !colors) || (w && h && !canvas)) return OCHRE_E_INVALID;
-    if (w > 32768 || h > 32768 || n_rasters > MAX_RASTERS) return OCHRE_E_INVALID;
-    if ((reinterpret_cast<uintptr_t>(canvas) & 3) || (reinterpret_cast<uintptr_t>(colors) & 3)) return OCHRE_E_INVALID;
-    if (cudaSetDevice(ctx->device) != cudaSuccess) return OCHRE_E_CUDA;
-    cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
-    ctx->epoch++;   // the sort below reuses the chain's buffers
-    ctx->prof_used = 0;
-    ctx->launches = 0;
+static int composite(ochre_gpu_ctx* ctx, const ochre_result* res, uint32_t n_rasters, const uint8_t* colors, uint32_t w,
+                     uint32_t h, uint8_t* canvas, cudaStream_t s) {
     const uint32_t T = res->n_tiles, N = res->n_spans;
-    if (w == 0 || h == 0 || n_rasters == 0 || (uint64_t)T + N == 0) return OCHRE_OK;
     const uint32_t w8 = (w + 7) / 8, h8 = (h + 7) / 8;
     uint32_t rbits = 1;
     while (rbits < 32 && ((n_rasters - 1) >> rbits)) rbits++;
@@ -340,4 +327,26 @@ extern "C" int ochre_gpu_composite(ochre_gpu_ctx* ctx, const ochre_result* res, 
     ctx->stats.n_launches = ctx->launches;
     collect_timings(ctx, s);
     return check_device_error(ctx);
+}
+
+}  // namespace ochre
+
+using namespace ochre;
+
+extern "C" int ochre_gpu_composite(ochre_gpu_ctx* ctx, const ochre_result* res, uint32_t n_rasters,
+                                   const uint8_t* colors, uint32_t w, uint32_t h, uint8_t* canvas, void* stream) {
+    if (!ctx || !res || (n_rasters && !colors) || (w && h && !canvas)) return OCHRE_E_INVALID;
+    if (w > 32768 || h > 32768 || n_rasters > MAX_RASTERS) return OCHRE_E_INVALID;
+    if ((reinterpret_cast<uintptr_t>(canvas) & 3) || (reinterpret_cast<uintptr_t>(colors) & 3)) return OCHRE_E_INVALID;
+    if (cudaSetDevice(ctx->device) != cudaSuccess) return OCHRE_E_CUDA;
+    cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : ctx->own_stream;
+    const bool nothing = w == 0 || h == 0 || n_rasters == 0 || (uint64_t)res->n_tiles + res->n_spans == 0;
+    if (!nothing && stream_captures(s)) return OCHRE_E_CUDA;
+    ctx->epoch++;   // the sort reuses the chain's buffers
+    ctx->prof_used = 0;
+    ctx->launches = 0;
+    if (nothing) return OCHRE_OK;
+    const int st = composite(ctx, res, n_rasters, colors, w, h, canvas, s);
+    if (st != OCHRE_OK) ctx->scan_dirty = true;   // a scan may be counted that never ran
+    return st;
 }

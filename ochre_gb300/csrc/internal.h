@@ -193,7 +193,8 @@ struct ochre_gpu_ctx {
     ochre::DevBuf tile_head, tile_xy, tile_rf, tile_state;
     // scan workspace: four ticket words, then look-back words (scan_space).
     // scan_tag: the last eager scan's; scan_tickets: tickets taken so far;
-    // scan_dirty: a wait gave up, so tickets and words may be anything.
+    // scan_dirty: a call failed or a wait gave up, so a counted scan may not
+    // have run and the ticket word may be anything.
     ochre::DevBuf scan_status;
     uint32_t scan_tag = 0, scan_tickets = 0;
     bool scan_dirty = false;
@@ -248,8 +249,11 @@ struct ochre_gpu_ctx {
     // the poll limit of its bounded waits (log2; 0: the default), and, on the
     // fused path, a command scan whose first tile is never taken, so that
     // the waits of the tiles after it cannot finish.
+    // And for any scan of the context: the test_fail_scan-th eager one from here
+    // (0: none) is counted but not launched, and reported as out of memory.
     uint32_t test_spin_log2 = 0;
     uint32_t test_skip_first_ticket = 0;
+    uint32_t test_fail_scan = 0;
 
     // Launch-shape tunables (ochre_gpu_set_tunable; chosen by the autotuner).
     int tune_fused_threads = 64;
@@ -340,6 +344,12 @@ int run_device(ochre_gpu_ctx* ctx, const ochre_batch* in, ochre_result* out, cud
 cudaError_t launch_plan_entries(ochre_gpu_ctx* ctx, uint32_t cap, uint32_t key_bits, uint32_t inc_cap,
                                 cudaStream_t s);
 cudaError_t launch_plan_cap(ochre_gpu_ctx* ctx, uint32_t* count, uint32_t cap, cudaStream_t s);
+
+// The entries that read counts back cannot run on a stream that is being
+// captured: what they queue would go into the capture, and the read-back
+// would then refuse (and end the capture).  They ask before they queue anything.
+bool stream_captures(cudaStream_t s);
+inline bool reads_back(const ochre_batch* in) { return in->n_rasters != 0 || in->fill_width != nullptr; }
 
 // Makes stream s wait for the batch's points if they are still being copied
 // (host-batch entry); every stage calls it before its first read of points.

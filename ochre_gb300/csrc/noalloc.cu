@@ -67,6 +67,7 @@ extern "C" int ochre_gpu_rasterize_noalloc(const ochre_batch* in, ochre_output_b
         return OCHRE_E_INVALID;
     out->n_tiles = 0;
     out->n_spans = 0;
+    if (ochre::reads_back(in) && ochre::stream_captures(static_cast<cudaStream_t>(stream))) return OCHRE_E_CUDA;
     std::lock_guard<std::mutex> lock(g_mutex);
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return OCHRE_E_CUDA;
