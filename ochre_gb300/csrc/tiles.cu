@@ -43,15 +43,25 @@ struct OpHead {
         return HeadScan{a.heads + b.heads, a.w + b.w};
     }
 };
-// The value of the last bin entry before entry i (false: there is none).  The
-// entries between are the crossings of the tile that starts at or after i: its
-// bins are as many, so the search never costs more than they do.
-__device__ __forceinline__ bool bin_before(const uint32_t* __restrict__ vals, uint64_t i, uint32_t& value) {
-    for (int64_t j = (int64_t)i - 1; j >= 0; j--) {
-        value = vals[j];
-        if (!(value & CROSS_TAG)) return true;
+// Beside its look-back words every block publishes its last head: 1 + the
+// entry (0: the block has none), under the scan's flag.  The last one before a
+// block (0: none), by a whole warp, 32 blocks a round.
+__device__ __forceinline__ uint32_t head_before(const uint64_t* last_head, uint32_t block, uint32_t flag, uint32_t* err) {
+    const uint32_t lane = threadIdx.x & 31u;
+    long long spins = 0;
+    const long long poll_limit = spin_limit(err);
+    for (int64_t top = (int64_t)block - 1; top >= 0;) {
+        const int64_t j = top - lane;
+        const uint64_t v = j >= 0 ? ld_relaxed64(last_head + j) : (uint64_t)flag << 32;
+        if (__any_sync(0xffffffffu, (uint32_t)(v >> 32) != flag)) {   // (published before its look-back: on its way)
+            if (wait_give_up_warp(spins, poll_limit, err)) break;
+            continue;
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, (uint32_t)v != 0u);
+        if (m) return __shfl_sync(0xffffffffu, (uint32_t)v, __ffs(m) - 1);
+        top -= 32;
     }
-    return false;
+    return 0u;
 }
 
 // A warp takes HEAD_ITEMS steps of 32 consecutive entries, so every load is
@@ -59,7 +69,11 @@ __device__ __forceinline__ bool bin_before(const uint32_t* __restrict__ vals, ui
 // is the sum of the signs before it (they are +-1 but for walks that snap far,
 // which take a shuffle scan).  Each head then gathers its bin record once; a
 // row starts where raster or tile row differ from the head before, a shuffle
-// away.  Bound by those gathers.  For the 178 M entries and 70 M tiles of
+// away.  For a warp's first head that is the last bin before the warp: one of
+// the 32 entries there, loaded with the warp's own, and where they are all
+// crossings (a tile's crossings may be any number, also of a tile without bins: a
+// line that ends in a tile's corner leaves its crossing where it has no cell)
+// the last head of the warps and blocks before.  Bound by those gathers.  For the 178 M entries and 70 M tiles of
 // 20,000 uneven paths a generic scan (threads own 8 consecutive entries), the
 // metadata gathered by a kernel of its own and a scan for the rows took 3.40
 // ms; 1.33 ms here (the coverage kernel finds the rows itself).  Few entries
@@ -85,14 +99,16 @@ struct HeadArgs {
 };
 template <class K, int HEAD_ITEMS>
 __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__ keys, HeadArgs A,
-                                                           ScanStatus<HeadScan>* status, uint32_t* ticket,
-                                                           uint32_t ticket_base, uint32_t tag, uint32_t* err) {
+                                                           ScanStatus<HeadScan>* status, uint64_t* last_head,
+                                                           uint32_t* ticket, uint32_t ticket_base, uint32_t tag,
+                                                           uint32_t* err) {
     dependent_start();
     constexpr int HEAD_GATHER = HEAD_ITEMS < 8 ? HEAD_ITEMS : 8;   // steps whose records are gathered together
     constexpr int WARPS = HEAD_BLOCK / 32, HEAD_TILE = HEAD_BLOCK * HEAD_ITEMS;
     constexpr uint32_t FULL = 0xffffffffu;
     __shared__ uint32_t s_tile, s_rows;
     __shared__ HeadScan s_warp[WARPS];
+    __shared__ uint32_t s_last[WARPS];   // 1 + the warp's last head (0: none)
     __shared__ HeadScan s_prefix;
     const uint64_t n = dev_count(A.n, A.n_dev);
     if (run_aborted(err)) return;   // a wait of the sort gave up: the values are not valid indices
@@ -112,6 +128,7 @@ __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__
     uint32_t heads = 0;   // bit k: this lane's entry of step k is a head
     int32_t w = 0;
     uint32_t n_heads = 0;
+    const uint32_t near = base > lane && base < n ? A.vals[base - 1 - lane] : CROSS_TAG;   // the entries before the warp
     {
         K key[HEAD_ITEMS];
         K before = 0;     // the key before the warp's first entry
@@ -136,19 +153,21 @@ __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__
         }
     }
     const int32_t warp_w = __reduce_add_sync(FULL, w);
-    if (lane == 0) s_warp[warp] = HeadScan{n_heads, warp_w};
+    const uint32_t last = __reduce_max_sync(FULL, heads ? (uint32_t)base + (31u - (uint32_t)__clz(heads)) * 32u + lane + 1u : 0u);
+    if (lane == 0) {
+        s_warp[warp] = HeadScan{n_heads, warp_w};
+        s_last[warp] = last;
+    }
     // raster and tile row of the last bin before the warp's entries
     uint32_t prev_r = 0xffffffffu;
     int prev_ty = 0;
-    if (lane == 0 && heads + n_heads != 0u && base < n) {
-        uint32_t pv;
-        if (bin_before(A.vals, base, pv)) {
-            prev_r = A.bins[pv].raster;
-            prev_ty = div8((int)A.bins[pv].y);
-        }
-    }
-    prev_r = __shfl_sync(FULL, prev_r, 0);
-    prev_ty = __shfl_sync(FULL, prev_ty, 0);
+    auto previous = [&](uint32_t value) {
+        const BinRec* rec = A.bins + value;
+        prev_r = rec->raster;
+        prev_ty = div8((int)rec->y);
+    };
+    const uint32_t near_bins = __ballot_sync(FULL, !(near & CROSS_TAG));
+    if (n_heads && near_bins) previous(__shfl_sync(FULL, near, __ffs(near_bins) - 1));
     __syncthreads();
     if (warp == 0) {
         HeadScan v = lane < (uint32_t)WARPS ? s_warp[lane] : HeadScan{0u, 0};
@@ -161,6 +180,8 @@ __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__
         if (lane == 0) ex = HeadScan{0u, 0};
         const HeadScan agg = shfl_idx_T(v, WARPS - 1);
         if (lane < (uint32_t)WARPS) s_warp[lane] = ex;
+        const uint32_t block_last = __reduce_max_sync(FULL, lane < (uint32_t)WARPS ? s_last[lane] : 0u);
+        if (lane == 0) st_relaxed64(last_head + tile, (uint64_t)(tag << 2 | SCAN_INC) << 32 | block_last);
         const HeadScan prefix = scan_lookback(tile, agg, OpHead{}, HeadScan{0u, 0}, status, tag, err);
         if (lane == 0) {
             s_prefix = prefix;
@@ -174,6 +195,11 @@ __global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__
     __syncthreads();
     uint32_t t0 = s_prefix.heads + s_warp[warp].heads;   // tiles before the step
     int32_t w0 = s_prefix.w + s_warp[warp].w;            // signs before the step
+    if (n_heads && !near_bins) {
+        uint32_t before = __reduce_max_sync(FULL, lane < warp ? s_last[lane] : 0u);
+        if (!before) before = head_before(last_head, tile, tag << 2 | SCAN_INC, err);
+        if (before) previous(A.vals[before - 1u]);
+    }
     uint32_t rows = 0;
     // HEAD_GATHER steps at a time: their values again (out of the cache) and
     // their records, all in flight before the first is used
@@ -848,18 +874,19 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
     const int steps = E < (uint64_t)sms * 2 * HEAD_BLOCK * 16 ? 4 : 16;
     const uint32_t blocks = (uint32_t)((E + HEAD_BLOCK * steps - 1) / (HEAD_BLOCK * steps));
     ScanSpace sp;
-    OCHRE_CUDA_TRY(scan_space(ctx, blocks * sizeof(ScanStatus<HeadScan>), blocks, 0u, s, &sp));
+    OCHRE_CUDA_TRY(scan_space(ctx, blocks * (sizeof(ScanStatus<HeadScan>) + sizeof(uint64_t)), blocks, 0u, s, &sp));
     const HeadArgs args{ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->raster_wbase.as<int32_t>(), E, e_dev, R,
                         ctx->tile_head.as<uint32_t>(), ctx->tile_xy.as<uint32_t>(), ctx->tile_rf.as<uint32_t>(),
                         ctx->out_raster_tile_off.as<uint32_t>(), reinterpret_cast<HeadScan*>(&ds->n_tiles),
                         &ds->n_rows};
     auto* status = reinterpret_cast<ScanStatus<HeadScan>*>(sp.status);
+    auto* last_head = reinterpret_cast<uint64_t*>(status + blocks);
     if (steps == 4)
         OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 4>, blocks, HEAD_BLOCK, 0, s, 
-            ctx->keys.as<K>(), args, status, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
+            ctx->keys.as<K>(), args, status, last_head, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
     else
         OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 16>, blocks, HEAD_BLOCK, 0, s, 
-            ctx->keys.as<K>(), args, status, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
+            ctx->keys.as<K>(), args, status, last_head, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
     int st = OCHRE_OK;
     uint32_t T, n_rows;
