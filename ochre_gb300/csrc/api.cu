@@ -96,7 +96,7 @@ void HostBuf::release() {
     cap = 0;
 }
 
-__global__ void k_copy_words(const uint32_t* __restrict__ src, uint32_t n, uint32_t* dst) {
+__global__ void k_copy_words(const uint32_t* src, uint32_t n, uint32_t* dst) {
     dependent_start();
     const uint32_t i = threadIdx.x;
     if (i < n) dst[i] = src[i];

@@ -53,6 +53,11 @@ constexpr int SPIN_LOG2_WORD = 22;
 // for the kernels before it to finish before it reads or writes anything.  No
 // block of a kernel waits on a block not yet placed: the next kernel's blocks
 // come only when all of this one's have.
+// So a kernel is resident while what it reads is still being written, and reads
+// it by ordinary loads: the read-only path (__ldg, or what the compiler makes
+// of const __restrict__ parameters) wants data that no one writes while the
+// kernel lives, and a load through __restrict__ need not stay behind the wait.
+// Only what a kernel writes and does not read carries __restrict__.
 __device__ __forceinline__ void dependent_start() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -447,7 +452,7 @@ __device__ __forceinline__ uint32_t upper_bound_u32(const uint32_t* a, uint32_t 
     uint32_t lo = 0, hi = n;   // first index with a[i] > v
     while (lo < hi) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(a + mid) <= v) lo = mid + 1; else hi = mid;
+        if (a[mid] <= v) lo = mid + 1; else hi = mid;
     }
     return lo;
 }

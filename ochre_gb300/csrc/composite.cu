@@ -44,12 +44,12 @@ struct PieceItems {
         uint32_t lo = 0, hi = R + 1;   // first raster whose range starts after i
         while (lo < hi) {
             const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(raster_tile_off + mid) + __ldg(raster_span_off + mid) <= i) lo = mid + 1; else hi = mid;
+            if (raster_tile_off[mid] + raster_span_off[mid] <= i) lo = mid + 1; else hi = mid;
         }
         const uint32_t r = lo - 1u;
         if (lo == 0u || r >= R) return it;   // a raster past the caller's count: not drawn
-        const uint32_t t0 = __ldg(raster_tile_off + r), s0 = __ldg(raster_span_off + r);
-        const uint32_t nt = __ldg(raster_tile_off + r + 1) - t0, k = i - t0 - s0;
+        const uint32_t t0 = raster_tile_off[r], s0 = raster_span_off[r];
+        const uint32_t nt = raster_tile_off[r + 1] - t0, k = i - t0 - s0;
         it.raster = r;
         if (k < nt) {
             const uint32_t t = t0 + k;
@@ -86,7 +86,7 @@ struct PieceOff {
 };
 
 template <class K>
-__global__ void k_piece_emit(PieceItems items, uint32_t rbits, const uint32_t* __restrict__ off, K* __restrict__ keys,
+__global__ void k_piece_emit(PieceItems items, uint32_t rbits, const uint32_t* off, K* __restrict__ keys,
                              uint32_t* __restrict__ vals) {
     dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -106,7 +106,7 @@ __global__ void k_piece_emit(PieceItems items, uint32_t rbits, const uint32_t* _
 // per screen tile.
 constexpr uint32_t NO_PIECE = 0xffffffffu;
 template <class K>
-__global__ void k_piece_heads(const K* __restrict__ keys, uint32_t E, uint32_t rbits, uint32_t n_tiles,
+__global__ void k_piece_heads(const K* keys, uint32_t E, uint32_t rbits, uint32_t n_tiles,
                               uint32_t* __restrict__ head, const uint32_t* err) {
     dependent_start();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -185,11 +185,11 @@ __device__ __forceinline__ f32x2 bytes2(uint32_t v) {
 // 28 us where (screen tile, raster) took 58.
 constexpr int BLEND_AHEAD = 4;
 template <class K>
-__global__ void __launch_bounds__(128) k_composite(const K* __restrict__ keys, const uint32_t* __restrict__ vals,
-                                                   uint32_t E, const uint32_t* __restrict__ head, uint32_t rbits,
-                                                   uint32_t T, const uint8_t* __restrict__ tile_alpha,
-                                                   const uint32_t* __restrict__ colors, uint32_t n_rasters, uint32_t w,
-                                                   uint32_t h, uint32_t w8, uint32_t h8, uint32_t* __restrict__ canvas,
+__global__ void __launch_bounds__(128) k_composite(const K* keys, const uint32_t* vals,
+                                                   uint32_t E, const uint32_t* head, uint32_t rbits,
+                                                   uint32_t T, const uint8_t* tile_alpha,
+                                                   const uint32_t* colors, uint32_t n_rasters, uint32_t w,
+                                                   uint32_t h, uint32_t w8, uint32_t h8, uint32_t* canvas,
                                                    float neg_zero, const uint32_t* err) {
     dependent_start();
     const uint32_t st = (uint32_t)((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5);

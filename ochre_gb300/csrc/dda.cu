@@ -325,8 +325,8 @@ constexpr uint32_t LONG_BLOCKS_PER_SM = 2;
 constexpr int COUNT_GROUPS_MAX = 8;
 constexpr int WALK_BLOCK = 128;
 constexpr int BOX_SLOTS = 8;
-__global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* __restrict__ lines,
-                                                           const uint32_t* __restrict__ line_raster, uint32_t n_cap,
+__global__ void __launch_bounds__(WALK_BLOCK) k_line_count(const float4* lines,
+                                                           const uint32_t* line_raster, uint32_t n_cap,
                                                            const uint32_t* n_dev, uint32_t groups, int4* bbox,
                                                            int* raster_wsum, uint32_t* __restrict__ counts,
                                                            uint32_t* __restrict__ inc_counts,
@@ -528,11 +528,11 @@ struct RasterOut {
 // Entries and increments of queued lines (see k_line_emit, whose entries in
 // the same order these are).
 template <int G, class K>
-__device__ __forceinline__ void emit_long(const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster,
-                                          const uint32_t* __restrict__ ent_off, const uint32_t* __restrict__ inc_off,
-                                          const int4* __restrict__ bbox, const uint64_t* __restrict__ key_base,
+__device__ __forceinline__ void emit_long(const float4* lines, const uint32_t* line_raster,
+                                          const uint32_t* ent_off, const uint32_t* inc_off,
+                                          const int4* bbox, const uint64_t* key_base,
                                           K* __restrict__ keys, uint32_t* __restrict__ vals, BinRec* __restrict__ bins,
-                                          float2* __restrict__ incs, const uint32_t* __restrict__ queue,
+                                          float2* __restrict__ incs, const uint32_t* queue,
                                           uint32_t n_queue, uint32_t* ticket) {
     const uint32_t lane = threadIdx.x & 31u, c = lane & (G - 1), gshift = lane & ~(uint32_t)(G - 1);
     constexpr uint32_t ALL = G == 32 ? 0xffffffffu : (1u << G) - 1u;
@@ -653,10 +653,10 @@ __device__ __forceinline__ void emit_long(const float4* __restrict__ lines, cons
 // The queued long lines' entries and increments (see k_line_emit).
 template <class K>
 __global__ void __launch_bounds__(LONG_THREADS) k_line_emit_long(
-    const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster, const uint32_t* __restrict__ ent_off,
-    const uint32_t* __restrict__ inc_off, uint64_t n_cap, const uint32_t* n_dev, const int4* __restrict__ bbox,
-    const uint64_t* __restrict__ key_base, K* __restrict__ keys, uint32_t* __restrict__ vals,
-    BinRec* __restrict__ bins, float2* __restrict__ incs, const uint32_t* __restrict__ queue, const uint32_t* n_queue,
+    const float4* lines, const uint32_t* line_raster, const uint32_t* ent_off,
+    const uint32_t* inc_off, uint64_t n_cap, const uint32_t* n_dev, const int4* bbox,
+    const uint64_t* key_base, K* __restrict__ keys, uint32_t* __restrict__ vals,
+    BinRec* __restrict__ bins, float2* __restrict__ incs, const uint32_t* queue, const uint32_t* n_queue,
     uint32_t* ticket) {
     dependent_start();
     // (a line count zeroed on the device, after an overflow of a graph's
@@ -697,9 +697,9 @@ constexpr int EMIT_BLOCK = 128;
 constexpr int EMIT_CARVEOUT = 28;          // percent shared: room for the blocks that fit by registers
 template <class K>
 __global__ void __launch_bounds__(EMIT_BLOCK) k_line_emit(
-    const float4* __restrict__ lines, const uint32_t* __restrict__ line_raster, const uint32_t* __restrict__ ent_off,
-    const uint32_t* __restrict__ inc_off, uint64_t n_cap, const uint32_t* n_dev, const int4* __restrict__ bbox,
-    const uint64_t* __restrict__ key_base, K* __restrict__ keys, uint32_t* __restrict__ vals,
+    const float4* lines, const uint32_t* line_raster, const uint32_t* ent_off,
+    const uint32_t* inc_off, uint64_t n_cap, const uint32_t* n_dev, const int4* bbox,
+    const uint64_t* key_base, K* __restrict__ keys, uint32_t* __restrict__ vals,
     BinRec* __restrict__ bins, float2* __restrict__ incs, uint32_t long_cells) {
     dependent_start();
     __shared__ uint32_t s_cnt[LENGTH_GROUPS];
@@ -832,9 +832,9 @@ __global__ void __launch_bounds__(EMIT_BLOCK) k_line_emit(
 }
 
 template <class K>
-__global__ void k_empty_emit(const uint32_t* __restrict__ empty, uint32_t n_rasters, uint32_t first_entry,
+__global__ void k_empty_emit(const uint32_t* empty, uint32_t n_rasters, uint32_t first_entry,
                              const uint32_t* first_dev, const uint32_t* n_ent_dev,
-                             const uint64_t* __restrict__ key_base, K* __restrict__ keys,
+                             const uint64_t* key_base, K* __restrict__ keys,
                              uint32_t* __restrict__ vals, BinRec* __restrict__ bins) {
     dependent_start();
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;

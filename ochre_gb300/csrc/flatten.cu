@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128) k_cmd_count(BatchView b, uint32_t* __rest
 constexpr int FLAT_BLOCK = 128;
 constexpr uint64_t FLAT_SHARED_LINES = 8, FLAT_SHARED_CMDS = 1u << 17;
 template <bool SHARED>
-__global__ void __launch_bounds__(FLAT_BLOCK) k_cmd_emit(BatchView b, const uint32_t* __restrict__ line_off,
+__global__ void __launch_bounds__(FLAT_BLOCK) k_cmd_emit(BatchView b, const uint32_t* line_off,
                                                          const uint32_t* n_lines, uint32_t n_lines_cap,
                                                          float4* __restrict__ lines, uint32_t* __restrict__ line_raster,
                                                          uint32_t long_cells, uint32_t* __restrict__ long_lines,
@@ -130,7 +130,8 @@ __global__ void __launch_bounds__(FLAT_BLOCK) k_cmd_emit(BatchView b, const uint
     if ((int)threadIdx.x < n) {
         const uint64_t c = c0 + threadIdx.x;
         const CmdCtx k = load_cmd(b, (uint32_t)c);
-        uint32_t o = line_off[c];
+        const uint32_t first = line_off[c];
+        uint32_t o = first;
         // (a line count zeroed on the device, after an overflow of a graph's plan, ends no lines)
         uint32_t end = max(o, c + 1 < b.n_cmds ? line_off[c + 1] : *n_lines);
         if (k.ok) {
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(FLAT_BLOCK) k_cmd_emit(BatchView b, const uint
             }
         }
         if (SHARED) {
-            s_off[threadIdx.x] = line_off[c];
+            s_off[threadIdx.x] = first;
             s_degree[threadIdx.x] = degree;
             s_end[threadIdx.x] = end;   // of the command's own lines
             if ((int)threadIdx.x == n - 1) s_off[n] = end;

@@ -28,7 +28,7 @@ struct BatchView {
 
 // Command j's floats lie inside the point array.
 __device__ __forceinline__ bool cmd_in_bounds(const BatchView& b, uint32_t j) {
-    return (uint64_t)__ldg(b.cmd_foff + j) + floats_per_verb(__ldg(b.verbs + j)) <= b.n_floats;
+    return (uint64_t)b.cmd_foff[j] + floats_per_verb(b.verbs[j]) <= b.n_floats;
 }
 
 // Everything a command's flattening depends on.
@@ -114,18 +114,18 @@ __device__ __forceinline__ uint32_t fill_of(const BatchView& b, uint32_t c) {
 // The fill of command j at or before fill f's commands: f, the fill before, or
 // (behind empty fills) searched for.
 __device__ __forceinline__ uint32_t fill_near(const BatchView& b, uint32_t j, uint32_t f) {
-    if (j >= __ldg(b.fill_off + f)) return f;
-    if (f > 0 && j >= __ldg(b.fill_off + f - 1u)) return f - 1u;
+    if (j >= b.fill_off[f]) return f;
+    if (f > 0 && j >= b.fill_off[f - 1u]) return f - 1u;
     return fill_of(b, j);
 }
 
 // The transformed end point of command j (a non-Close command).
 __device__ __forceinline__ V2 endpoint_of(const BatchView& b, uint32_t j, uint32_t f_hint) {
     const uint32_t f = fill_near(b, j, f_hint);
-    const uint8_t v = __ldg(b.verbs + j);
-    const float* fp = b.pts + __ldg(b.cmd_foff + j) + endpoint_float(v);
-    V2 p = v2(__ldg(fp), __ldg(fp + 1));
-    const bool raw = b.fill_flags != nullptr && (__ldg(b.fill_flags + f) & OCHRE_FILL_RAW);
+    const uint8_t v = b.verbs[j];
+    const float* fp = b.pts + b.cmd_foff[j] + endpoint_float(v);
+    V2 p = v2(*fp, fp[1]);
+    const bool raw = b.fill_flags != nullptr && (b.fill_flags[f] & OCHRE_FILL_RAW);
     if (!raw) p = xf_apply(b.fill_xf + 6 * (size_t)f, p);
     return p;
 }
@@ -133,22 +133,22 @@ __device__ __forceinline__ V2 endpoint_of(const BatchView& b, uint32_t j, uint32
 __device__ inline CmdCtx load_cmd(const BatchView& b, uint32_t c) {
     CmdCtx k;
     k.ok = true;
-    k.verb = __ldg(b.verbs + c);
+    k.verb = b.verbs[c];
     const uint32_t f = fill_of(b, c);
     uint32_t r, rf0, rf1;
     if (b.raster_off != nullptr) {
         r = upper_bound_u32(b.raster_off, b.n_rasters + 1, f) - 1u;
-        rf0 = __ldg(b.raster_off + r);
-        rf1 = __ldg(b.raster_off + r + 1);
+        rf0 = b.raster_off[r];
+        rf1 = b.raster_off[r + 1];
     } else {
         r = f;
         rf0 = f;
         rf1 = f + 1;
     }
     k.raster = r;
-    const uint32_t rc0 = __ldg(b.fill_off + rf0), rc1 = __ldg(b.fill_off + rf1);
+    const uint32_t rc0 = b.fill_off[rf0], rc1 = b.fill_off[rf1];
     k.last_of_raster = c + 1 == rc1;
-    const uint32_t ep = __ldg(b.cmd_ep + c), mv = __ldg(b.cmd_mv + c);
+    const uint32_t ep = b.cmd_ep[c], mv = b.cmd_mv[c];
     k.fill = f;
     k.last_ref = ep > rc0 ? (int64_t)(ep - 1u) : -1;
     k.first_ref = mv > rc0 ? (int64_t)(mv - 1u) : -1;
@@ -163,21 +163,21 @@ __device__ inline CmdCtx load_cmd(const BatchView& b, uint32_t c) {
     if (mv > rc0) {
         const uint32_t m = mv - 1u;
         const uint32_t fm = fill_near(b, m, f);
-        const float* fp = b.pts + __ldg(b.cmd_foff + m);
-        V2 p = v2(__ldg(fp), __ldg(fp + 1));
-        const bool raw = b.fill_flags != nullptr && (__ldg(b.fill_flags + fm) & OCHRE_FILL_RAW);
+        const float* fp = b.pts + b.cmd_foff[m];
+        V2 p = v2(*fp, fp[1]);
+        const bool raw = b.fill_flags != nullptr && (b.fill_flags[fm] & OCHRE_FILL_RAW);
         k.first = raw ? p : xf_apply(b.fill_xf + 6 * (size_t)fm, p);
     } else {
         k.first = v2(0.0f, 0.0f);
     }
-    const bool raw = b.fill_flags != nullptr && (__ldg(b.fill_flags + f) & OCHRE_FILL_RAW);
+    const bool raw = b.fill_flags != nullptr && (b.fill_flags[f] & OCHRE_FILL_RAW);
     const float* xf = b.fill_xf + 6 * (size_t)f;
-    const float* fp = b.pts + __ldg(b.cmd_foff + c);
+    const float* fp = b.pts + b.cmd_foff[c];
     const int np = k.verb == V_MOVE || k.verb == V_LINE ? 1 : k.verb == V_QUAD || k.verb == V_CONIC ? 2
                  : k.verb == V_CUBIC ? 3 : 0;
     for (int q = 0; q < 3; q++) {
         if (q < np) {
-            V2 p = v2(__ldg(fp + 2 * q), __ldg(fp + 2 * q + 1));
+            V2 p = v2(fp[2 * q], fp[2 * q + 1]);
             if (!raw) p = xf_apply(xf, p);   // PathCmd::transform (path.rs:16-37)
             if (!finite2(p)) k.ok = false;
             k.pt[q] = p;
@@ -185,7 +185,7 @@ __device__ inline CmdCtx load_cmd(const BatchView& b, uint32_t c) {
             k.pt[q] = v2(0.0f, 0.0f);
         }
     }
-    k.w = k.verb == V_CONIC ? __ldg(fp + 4) : 0.0f;
+    k.w = k.verb == V_CONIC ? fp[4] : 0.0f;
     if (k.verb == V_CONIC && !isfinite(k.w)) k.ok = false;
     return k;
 }

@@ -204,9 +204,9 @@ __global__ void __launch_bounds__(THREADS, fused_min_ctas(THREADS)) k_raster_fus
         if (r < A.n_rasters) {
             f0 = r;
             f1 = r + 1;
-            if (A.raster_off) { f0 = __ldg(A.raster_off + r); f1 = __ldg(A.raster_off + r + 1); }
-            c0 = __ldg(A.fill_off + f0);
-            c1 = __ldg(A.fill_off + f1);
+            if (A.raster_off) { f0 = A.raster_off[r]; f1 = A.raster_off[r + 1]; }
+            c0 = A.fill_off[f0];
+            c1 = A.fill_off[f1];
         }
         S.next = r;
         S.next_f0 = f0;
@@ -314,13 +314,13 @@ __global__ void __launch_bounds__(THREADS, fused_min_ctas(THREADS)) k_raster_fus
         V2 last_end = v2(0, 0), first_end = v2(0, 0);
         if (!bail) {
             const bool active = tid < n_cmd;
-            verb = active ? __ldg(A.verbs + c0 + tid) : V_CLOSE;
-            const uint32_t foff = active ? __ldg(A.cmd_foff + c0 + tid) : 0u;
+            verb = active ? A.verbs[c0 + tid] : V_CLOSE;
+            const uint32_t foff = active ? A.cmd_foff[c0 + tid] : 0u;
             bool ok = true;
             if (active) {
                 uint32_t f = f0;
                 if (f1 - f0 > 1) f = upper_bound_u32(A.fill_off, A.n_fills + 1, c0 + tid) - 1u;
-                const bool raw = A.fill_flags != nullptr && (__ldg(A.fill_flags + f) & OCHRE_FILL_RAW);
+                const bool raw = A.fill_flags != nullptr && (A.fill_flags[f] & OCHRE_FILL_RAW);
                 const float* xf = A.fill_xf + 6 * (size_t)f;
                 const float* fp = A.pts + foff;
                 const int np = verb == V_MOVE || verb == V_LINE ? 1 : verb == V_QUAD || verb == V_CONIC ? 2
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(THREADS, fused_min_ctas(THREADS)) k_raster_fus
                 }
                 if (!finite2(pt0) || !finite2(pt1) || !finite2(pt2)) ok = false;
                 if (verb == V_CONIC && ok) {
-                    wgt = __ldg(fp + 4);
+                    wgt = fp[4];
                     if (!isfinite(wgt)) ok = false;
                 }
                 S.u.early.ep[tid] = verb == V_CUBIC ? pt2 : (verb == V_QUAD || verb == V_CONIC) ? pt1 : pt0;

@@ -70,7 +70,7 @@ struct FusedArgs {
     float* stage_cov;
 };
 
-__device__ __forceinline__ V2 load_pt(const float* p) { return v2(__ldg(p), __ldg(p + 1)); }
+__device__ __forceinline__ V2 load_pt(const float* p) { return v2(*p, p[1]); }
 
 // Publishes raster r's counts (one warp); the raster that completes its
 // block also publishes the block's aggregate.

@@ -49,15 +49,15 @@ __device__ __forceinline__ int tile_y_of(uint32_t xy) { return (int)(int16_t)(xy
 // 140 and 168 us with a thread and a search per pixel, 44 and 59 now.
 // First pixel of a tile's row in the images, and how many of its eight lie on
 // the canvas (0: none; tiles start at multiples of 8, so none straddles x = 0).
-__device__ __forceinline__ int tile_row(const uint32_t* __restrict__ xy, const uint32_t* __restrict__ rf, uint32_t t,
+__device__ __forceinline__ int tile_row(const uint32_t* xy, const uint32_t* rf, uint32_t t,
                                         int y8, uint32_t W, uint32_t H, size_t& at) {
     const int x = 8 * tile_tx(xy[t]), y = 8 * tile_ty(xy[t]) + y8;
     if (x < 0 || y < 0 || x >= (int)W || y >= (int)H) return 0;
     at = (size_t)(rf[t] & RF_RASTER) * W * H + (size_t)y * W + (size_t)x;
     return min(8, (int)W - x);
 }
-__global__ void k_composite_tiles(const uint32_t* __restrict__ xy, const uint32_t* __restrict__ rf,
-                                  const float* __restrict__ tile_sum, uint32_t T, const uint32_t* t_dev, uint32_t W,
+__global__ void k_composite_tiles(const uint32_t* xy, const uint32_t* rf,
+                                  const float* tile_sum, uint32_t T, const uint32_t* t_dev, uint32_t W,
                                   uint32_t H, bool vec, float* __restrict__ cov) {
     dependent_start();
     const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -81,8 +81,8 @@ __global__ void k_composite_tiles(const uint32_t* __restrict__ xy, const uint32_
     }
 }
 
-__global__ void k_composite_spans(const uint32_t* __restrict__ span_xy, const uint16_t* __restrict__ span_w,
-                                  uint32_t N, const uint32_t* n_dev, const uint32_t* __restrict__ raster_span_off,
+__global__ void k_composite_spans(const uint32_t* span_xy, const uint16_t* span_w,
+                                  uint32_t N, const uint32_t* n_dev, const uint32_t* raster_span_off,
                                   uint32_t R, uint32_t W, uint32_t H, float* __restrict__ cov) {
     dependent_start();
     const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -104,7 +104,7 @@ __global__ void k_composite_spans(const uint32_t* __restrict__ span_xy, const ui
 // does not grow with the count: FP64 arithmetic per pixel would bound this
 // kernel by the GPU's FP64 rate instead of HBM), one double per thread into
 // the block reduction.  16-byte accesses when all three arrays allow.
-__global__ void k_l2(const float* __restrict__ cov, const float* __restrict__ target, uint64_t n,
+__global__ void k_l2(const float* cov, const float* target, uint64_t n,
                      double* __restrict__ loss, float* __restrict__ dl) {
     dependent_start();
     float sum = 0.0f, comp = 0.0f;
@@ -153,9 +153,9 @@ __global__ void k_l2(const float* __restrict__ cov, const float* __restrict__ ta
 }
 
 // ---- backward 1: dL/dS at boundary-tile pixels ----
-__global__ void k_gsigma(const uint32_t* __restrict__ xy, const uint32_t* __restrict__ rf,
-                         const float* __restrict__ tile_sum, uint32_t T, const uint32_t* t_dev, uint32_t W, uint32_t H,
-                         bool vec, const float* __restrict__ dl_dcov, float* __restrict__ gsig) {
+__global__ void k_gsigma(const uint32_t* xy, const uint32_t* rf,
+                         const float* tile_sum, uint32_t T, const uint32_t* t_dev, uint32_t W, uint32_t H,
+                         bool vec, const float* dl_dcov, float* __restrict__ gsig) {
     dependent_start();
     const uint64_t idx = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint32_t t = (uint32_t)(idx >> 3), y8 = (uint32_t)(idx & 7u);
@@ -181,7 +181,7 @@ __global__ void k_gsigma(const uint32_t* __restrict__ xy, const uint32_t* __rest
 
 // ---- backward 2: exclusive suffix sums of dL/dS along every canvas row ----
 // Writes (dL/dS, suffix sum) pairs: the adjoint of a cell reads both at once.
-__global__ void k_row_suffix(const float* __restrict__ gsig, uint64_t rows, uint32_t W, float2* __restrict__ gG,
+__global__ void k_row_suffix(const float* gsig, uint64_t rows, uint32_t W, float2* __restrict__ gG,
                              float* __restrict__ row_total) {
     dependent_start();
     const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -284,10 +284,10 @@ __device__ __forceinline__ float div_by(float a, float b, float r) {
 // lines cancel, and single gradients then moved by 0.3 % of their rms; as it
 // is every operation rounds as it did.  14.4 M lines (27.9 M cells) of 128
 // dense scenes: 567 us with both sides and all divisions on their own, 373 now.
-__global__ void __launch_bounds__(128) k_line_grad(const float4* __restrict__ lines,
-                                                   const uint32_t* __restrict__ line_raster, uint32_t L,
+__global__ void __launch_bounds__(128) k_line_grad(const float4* lines,
+                                                   const uint32_t* line_raster, uint32_t L,
                                                    const uint32_t* l_dev, uint32_t W, uint32_t H,
-                                                   const float2* __restrict__ gG, const float* __restrict__ row_total,
+                                                   const float2* gG, const float* row_total,
                                                    LineGrad* __restrict__ out) {
     dependent_start();
     const uint32_t l = blockIdx.x * blockDim.x + threadIdx.x;
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__(128) k_line_grad(const float4* __restrict__ li
 // ---- backward 4: per command, through the flattening to device-space points ----
 __device__ __forceinline__ void add_point(float* gp, const BatchView& b, int64_t cmd, int q, V2 g) {
     if (cmd < 0) return;
-    const uint32_t f = __ldg(b.cmd_foff + cmd) + 2u * (uint32_t)q;
+    const uint32_t f = b.cmd_foff[cmd] + 2u * (uint32_t)q;
     atomicAdd(gp + f, g.x);
     atomicAdd(gp + f + 1, g.y);
 }
@@ -427,9 +427,9 @@ __device__ __forceinline__ V2 mul2(float s, V2 a) { return v2(s * a.x, s * a.y);
 
 // (`err`: a planned run's error word; when a count of the run outgrew its
 // capacity the lines and offsets are not all there, and nothing is read)
-__global__ void k_cmd_grad(BatchView b, const uint32_t* __restrict__ line_off, uint32_t L, const uint32_t* l_dev,
-                           const uint32_t* err, const LineGrad* __restrict__ lg, float* __restrict__ gp, uint32_t W,
-                           uint32_t H, const float2* __restrict__ gG, const float* __restrict__ row_total) {
+__global__ void k_cmd_grad(BatchView b, const uint32_t* line_off, uint32_t L, const uint32_t* l_dev,
+                           const uint32_t* err, const LineGrad* lg, float* __restrict__ gp, uint32_t W,
+                           uint32_t H, const float2* gG, const float* row_total) {
     dependent_start();
     const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (c >= b.n_cmds) return;
@@ -447,7 +447,7 @@ __global__ void k_cmd_grad(BatchView b, const uint32_t* __restrict__ line_off, u
     const bool final_close = k.last_of_raster && !veq(last_end, first_end);
     const int n_own = (int)(o1 - o0) - (final_close ? 1 : 0);
     auto add_last = [&](V2 g) {
-        if (k.last_ref >= 0) add_point(gp, b, k.last_ref, endpoint_index(__ldg(b.verbs + k.last_ref)), g);
+        if (k.last_ref >= 0) add_point(gp, b, k.last_ref, endpoint_index(b.verbs[k.last_ref]), g);
     };
     auto add_first = [&](V2 g) { add_point(gp, b, k.first_ref, 0, g); };
     switch (k.verb) {
@@ -575,7 +575,7 @@ __global__ void k_cmd_grad(BatchView b, const uint32_t* __restrict__ line_off, u
         add_last(g0);
         add_point(gp, b, self, 0, g1);
         add_point(gp, b, self, 1, g2);
-        atomicAdd(gp + __ldg(b.cmd_foff + c) + 4, gw);   // the weight (not transformed)
+        atomicAdd(gp + b.cmd_foff[c] + 4, gw);   // the weight (not transformed)
         break;
     }
     default:
@@ -601,7 +601,7 @@ __global__ void k_cmd_grad(BatchView b, const uint32_t* __restrict__ line_off, u
 }
 
 // ---- backward 5: device-space point gradients -> input points and transforms ----
-__global__ void k_fill_grad(BatchView b, const float* __restrict__ gp, float* __restrict__ dl_dpts,
+__global__ void k_fill_grad(BatchView b, const float* gp, float* __restrict__ dl_dpts,
                             float* __restrict__ dl_dxf) {
     dependent_start();
     const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -611,10 +611,10 @@ __global__ void k_fill_grad(BatchView b, const float* __restrict__ gp, float* __
     uint32_t f = 0xffffffffu;
     if (valid) {
         f = fill_of(b, (uint32_t)c);
-        const uint8_t v = __ldg(b.verbs + c);
-        const uint32_t fo = __ldg(b.cmd_foff + c);
+        const uint8_t v = b.verbs[c];
+        const uint32_t fo = b.cmd_foff[c];
         const int np = v == V_MOVE || v == V_LINE ? 1 : v == V_QUAD || v == V_CONIC ? 2 : v == V_CUBIC ? 3 : 0;
-        const bool raw = b.fill_flags != nullptr && (__ldg(b.fill_flags + f) & OCHRE_FILL_RAW);
+        const bool raw = b.fill_flags != nullptr && (b.fill_flags[f] & OCHRE_FILL_RAW);
         const float* m = b.fill_xf + 6 * (size_t)f;
         for (int q = 0; q < np; q++) {
             const float gx = gp[fo + 2 * q], gy = gp[fo + 2 * q + 1];
@@ -622,9 +622,9 @@ __global__ void k_fill_grad(BatchView b, const float* __restrict__ gp, float* __
                 dl_dpts[fo + 2 * q] = gx;
                 dl_dpts[fo + 2 * q + 1] = gy;
             } else {
-                const float vx = __ldg(b.pts + fo + 2 * q), vy = __ldg(b.pts + fo + 2 * q + 1);
-                dl_dpts[fo + 2 * q] = __ldg(m + 0) * gx + __ldg(m + 2) * gy;
-                dl_dpts[fo + 2 * q + 1] = __ldg(m + 1) * gx + __ldg(m + 3) * gy;
+                const float vx = b.pts[fo + 2 * q], vy = b.pts[fo + 2 * q + 1];
+                dl_dpts[fo + 2 * q] = m[0] * gx + m[2] * gy;
+                dl_dpts[fo + 2 * q + 1] = m[1] * gx + m[3] * gy;
                 acc[0] += gx * vx;
                 acc[1] += gx * vy;
                 acc[2] += gy * vx;

@@ -142,12 +142,12 @@ __device__ __forceinline__ void store_words(uint32_t* p, const uint32_t (&w)[N])
 template <int N>
 __device__ __forceinline__ void load_bytes(const uint8_t* p, uint32_t (&b)[N]) {
     if (N == 8 && (reinterpret_cast<uintptr_t>(p) & 7u) == 0u) {
-        const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+        const uint2 q = *reinterpret_cast<const uint2*>(p);
 #pragma unroll
         for (int k = 0; k < N; k++) b[k] = ((k < 4 ? q.x : q.y) >> (8 * (k & 3))) & 0xffu;
     } else {
 #pragma unroll
-        for (int k = 0; k < N; k++) b[k] = __ldg(p + k);
+        for (int k = 0; k < N; k++) b[k] = p[k];
     }
 }
 
@@ -244,7 +244,7 @@ struct OpSumU32 {
 // Floats of every command.
 struct VerbFloats {
     const uint8_t* verbs;
-    __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return floats_per_verb(__ldg(verbs + i)); }
+    __device__ __forceinline__ uint32_t operator()(uint64_t i) const { return floats_per_verb(verbs[i]); }
     using takes_all = void;
     template <int N>
     __device__ __forceinline__ void load_all(uint64_t i, uint32_t (&v)[N]) const {

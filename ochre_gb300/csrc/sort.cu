@@ -42,7 +42,7 @@ struct SortPlan {
 // Histograms of every pass's digits; the block that adds its counts last turns
 // them into each digit's first output place (`done` counts the blocks).
 template <class K, int RB>
-__global__ void __launch_bounds__(256) k_sort_hist(const K* __restrict__ keys, uint64_t n, const uint32_t* n_dev,
+__global__ void __launch_bounds__(256) k_sort_hist(const K* keys, uint64_t n, const uint32_t* n_dev,
                                                    SortPlan plan, uint32_t* hist, uint32_t* __restrict__ off,
                                                    uint32_t* done) {
     dependent_start();
@@ -110,9 +110,9 @@ constexpr size_t onesweep_smem() {
 // digits are held to two by their shared memory.
 template <class K, int RB>
 __global__ void __launch_bounds__(SORT_BLOCK, RB <= 8 ? 3 : 2) k_onesweep(
-    const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
+    const K* keys_in, const uint32_t* vals_in, K* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, uint64_t n, const uint32_t* n_dev, int shift, uint32_t mask,
-    const uint32_t* __restrict__ digit_off, uint32_t* lookback, uint32_t* ticket, uint32_t* err) {
+    const uint32_t* digit_off, uint32_t* lookback, uint32_t* ticket, uint32_t* err) {
     dependent_start();
     constexpr int RADIX = 1 << RB;
     constexpr int PER = RADIX / SORT_BLOCK;   // digits per thread in the offset phase
@@ -407,8 +407,8 @@ constexpr size_t local_sort_smem() {
     return (size_t)THREADS * ITEMS * 4 + (size_t)(THREADS / 32) * 256 * 4 + 256 * 4;
 }
 template <class K, int THREADS, int ITEMS, int BLOCKS>
-__global__ void __launch_bounds__(THREADS, BLOCKS) k_sort_local(const K* __restrict__ keys_in,
-                                                                const uint32_t* __restrict__ vals_in,
+__global__ void __launch_bounds__(THREADS, BLOCKS) k_sort_local(const K* keys_in,
+                                                                const uint32_t* vals_in,
                                                                 K* __restrict__ keys_out,
                                                                 uint32_t* __restrict__ vals_out, LocalSortArgs A) {
     dependent_start();
@@ -522,10 +522,22 @@ __global__ void __launch_bounds__(THREADS, BLOCKS) k_sort_local(const K* __restr
             }
         }
     }
-    for (uint32_t i = tid; i < n; i += THREADS) {
-        const uint32_t w = s_word[i];
-        keys_out[out + i] = base + (K)(w >> IDX);
-        vals_out[out + i] = vals_in[e0 + (w & ((1u << IDX) - 1u))];
+    // every value is on its way before the first is written
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const uint32_t i = tid + k * THREADS;
+        if (i < n) {
+            word[k] = s_word[i];
+            rank[k] = vals_in[e0 + (word[k] & ((1u << IDX) - 1u))];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < ITEMS; k++) {
+        const uint32_t i = tid + k * THREADS;
+        if (i < n) {
+            keys_out[out + i] = base + (K)(word[k] >> IDX);
+            vals_out[out + i] = rank[k];
+        }
     }
 }
 

@@ -27,7 +27,7 @@
 namespace ochre {
 
 __device__ __forceinline__ bool is_stroke(const uint8_t* flags, uint32_t f) {
-    return flags != nullptr && (__ldg(flags + f) & OCHRE_FILL_STROKE);
+    return flags != nullptr && (flags[f] & OCHRE_FILL_STROKE);
 }
 
 // Path-space `last` of command c in fill f: the end point of the most recent
@@ -35,10 +35,10 @@ __device__ __forceinline__ bool is_stroke(const uint8_t* flags, uint32_t f) {
 __device__ __forceinline__ V2 path_last(const uint8_t* verbs, const float* pts, const uint32_t* cmd_foff,
                                         const uint32_t* cmd_ep, const uint32_t* fill_off, uint32_t f, uint32_t c) {
     const uint32_t ep = cmd_ep[c];
-    if (ep == 0 || ep - 1u < __ldg(fill_off + f)) return v2(0.0f, 0.0f);
+    if (ep == 0 || ep - 1u < fill_off[f]) return v2(0.0f, 0.0f);
     const uint32_t j = ep - 1u;
-    const float* fp = pts + cmd_foff[j] + endpoint_float(__ldg(verbs + j));
-    return v2(__ldg(fp), __ldg(fp + 1));
+    const float* fp = pts + cmd_foff[j] + endpoint_float(verbs[j]);
+    return v2(*fp, fp[1]);
 }
 
 // ---- 2. polyline sizes ----
@@ -60,7 +60,7 @@ struct PolyCount {
     uint32_t* err;
     __device__ Pair operator()(uint64_t i) const {
         const uint32_t c = (uint32_t)i;
-        const uint8_t v = __ldg(verbs + c);
+        const uint8_t v = verbs[c];
         const uint32_t f = upper_bound_u32(fill_off, n_fills + 1, c) - 1u;
         if (!is_stroke(flags, f)) return Pair{1u, floats_per_verb(v)};
         if (v == V_MOVE || v == V_LINE) return Pair{1u, 2u};
@@ -108,16 +108,16 @@ __global__ void __launch_bounds__(128) k_pair_count(uint64_t n, const uint32_t* 
     out_nf[i] = p.nf;
 }
 
-__global__ void k_poly_emit(const uint8_t* __restrict__ verbs, const float* __restrict__ pts,
-                            const uint32_t* __restrict__ fill_off, uint32_t n_fills, const uint8_t* __restrict__ flags,
-                            uint64_t n_cmds, const uint32_t* __restrict__ cmd_foff, const uint32_t* __restrict__ cmd_ep,
-                            const uint32_t* __restrict__ poly_off, const uint32_t* __restrict__ poly_foff,
+__global__ void k_poly_emit(const uint8_t* verbs, const float* pts,
+                            const uint32_t* fill_off, uint32_t n_fills, const uint8_t* flags,
+                            uint64_t n_cmds, const uint32_t* cmd_foff, const uint32_t* cmd_ep,
+                            const uint32_t* poly_off, const uint32_t* poly_foff,
                             uint8_t* __restrict__ pverbs, float* __restrict__ ppts, uint32_t p_cap, uint32_t pf_cap) {
     dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     if (i >= n_cmds) return;
     const uint32_t c = (uint32_t)i;
-    const uint8_t v = __ldg(verbs + c);
+    const uint8_t v = verbs[c];
     const uint32_t f = upper_bound_u32(fill_off, n_fills + 1, c) - 1u;
     uint32_t o = poly_off[c], fo = poly_foff[c];
     const float* fp = pts + cmd_foff[c];
@@ -131,7 +131,7 @@ __global__ void k_poly_emit(const uint8_t* __restrict__ verbs, const float* __re
     };
     if (!is_stroke(flags, f)) {
         verb(o, v);
-        for (uint32_t k = 0; k < floats_per_verb(v); k++) flt(fo + k, __ldg(fp + k));
+        for (uint32_t k = 0; k < floats_per_verb(v); k++) flt(fo + k, fp[k]);
         return;
     }
     auto line = [&](V2 p) {
@@ -143,8 +143,8 @@ __global__ void k_poly_emit(const uint8_t* __restrict__ verbs, const float* __re
     case V_MOVE:
     case V_LINE:
         verb(o, v);
-        flt(fo, __ldg(fp));
-        flt(fo + 1, __ldg(fp + 1));
+        flt(fo, *fp);
+        flt(fo + 1, fp[1]);
         break;
     case V_CLOSE:
         verb(o, V_CLOSE);
@@ -200,7 +200,7 @@ struct UnitIn {
         if (!is_stroke(flags, f)) return 1u;
         const uint8_t v = pverbs[p];
         if (v == V_CLOSE) return 0u;
-        return (v == V_MOVE || p == __ldg(pfill_off + f) || pverbs[p - 1] == V_CLOSE) ? 1u : 0u;
+        return (v == V_MOVE || p == pfill_off[f] || pverbs[p - 1] == V_CLOSE) ? 1u : 0u;
     }
 };
 struct UnitOut {
@@ -210,8 +210,8 @@ struct UnitOut {
     }
 };
 
-__global__ void k_first_close(const uint8_t* __restrict__ pverbs, uint64_t n_poly, const uint32_t* n_dev,
-                              const uint32_t* __restrict__ pfill_off, uint32_t n_fills, const uint8_t* __restrict__ flags,
+__global__ void k_first_close(const uint8_t* pverbs, uint64_t n_poly, const uint32_t* n_dev,
+                              const uint32_t* pfill_off, uint32_t n_fills, const uint8_t* flags,
                               uint32_t* __restrict__ first_close) {
     dependent_start();
     const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -220,14 +220,14 @@ __global__ void k_first_close(const uint8_t* __restrict__ pverbs, uint64_t n_pol
     if (is_stroke(flags, f)) atomicMin(first_close + f, (uint32_t)i);
 }
 
-__global__ void k_fill_init(uint32_t* __restrict__ first_close, const uint32_t* __restrict__ fill_off,
-                            const uint32_t* __restrict__ poly_off, uint64_t n_cmds, uint32_t n_poly,
+__global__ void k_fill_init(uint32_t* __restrict__ first_close, const uint32_t* fill_off,
+                            const uint32_t* poly_off, uint64_t n_cmds, uint32_t n_poly,
                             const uint32_t* n_poly_dev, uint32_t n_fills, uint32_t* __restrict__ pfill_off) {
     dependent_start();
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f > n_fills) return;
     const uint32_t np = (uint32_t)dev_count(n_poly, n_poly_dev);
-    const uint32_t c = __ldg(fill_off + f);
+    const uint32_t c = fill_off[f];
     pfill_off[f] = c < n_cmds ? min(poly_off[c], np) : np;
     if (f < n_fills) first_close[f] = 0xffffffffu;
 }
@@ -244,7 +244,7 @@ __global__ void k_fill_init(uint32_t* __restrict__ first_close, const uint32_t* 
 // joins' point counts (1 or 2) gives each point its place.  emit(k, point)
 // receives the side's k-th point; every lane returns the side's point count.
 template <class Emit>
-__device__ uint32_t stroke_side_warp(const float* __restrict__ P, uint32_t len, bool closed, bool reverse, float width,
+__device__ uint32_t stroke_side_warp(const float* P, uint32_t len, bool closed, bool reverse, float width,
                                      Emit emit) {
     const uint32_t lane = threadIdx.x & 31u;
     auto pt = [&](uint32_t k) { return v2(P[2 * k], P[2 * k + 1]); };
@@ -336,7 +336,7 @@ __device__ __forceinline__ UnitGeom unit_geom_warp(uint32_t u, const uint32_t* u
         g.closed = 2;
         return g;
     }
-    const uint32_t pe = __ldg(pfill_off + g.fill + 1);
+    const uint32_t pe = pfill_off[g.fill + 1];
     uint32_t e = g.p0 + 1;
     for (;;) {
         const uint32_t k = e + lane;
@@ -355,13 +355,13 @@ __device__ __forceinline__ UnitGeom unit_geom_warp(uint32_t u, const uint32_t* u
 
 // Output commands and floats of every unit, one warp per unit.
 __global__ void __launch_bounds__(128) k_out_count(uint32_t n_units, const uint32_t* n_dev,
-                                                   const uint32_t* __restrict__ unit_start,
-                                                   const uint8_t* __restrict__ pverbs, const float* __restrict__ ppts,
-                                                   const uint32_t* __restrict__ poly_foff_of,
-                                                   const uint32_t* __restrict__ pfill_off, uint32_t n_fills,
-                                                   const uint8_t* __restrict__ flags,
-                                                   const uint32_t* __restrict__ first_close,
-                                                   const float* __restrict__ width, uint32_t* __restrict__ out_n,
+                                                   const uint32_t* unit_start,
+                                                   const uint8_t* pverbs, const float* ppts,
+                                                   const uint32_t* poly_foff_of,
+                                                   const uint32_t* pfill_off, uint32_t n_fills,
+                                                   const uint8_t* flags,
+                                                   const uint32_t* first_close,
+                                                   const float* width, uint32_t* __restrict__ out_n,
                                                    uint32_t* __restrict__ out_nf) {
     dependent_start();
     const uint64_t u = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(128) k_out_count(uint32_t n_units, const uint3
         return;
     }
     const float* P = ppts + poly_foff_of[g.p0];
-    const float w = __ldg(width + g.fill);
+    const float w = width[g.fill];
     auto none = [](uint32_t, V2) {};
     const uint32_t n = stroke_side_warp(P, g.len, g.closed != 0, false, w, none) +
                        stroke_side_warp(P, g.len, g.closed != 0, true, w, none);
@@ -388,14 +388,14 @@ __global__ void __launch_bounds__(128) k_out_count(uint32_t n_units, const uint3
 
 // Every unit's output commands and points (path.rs:214-274), one warp per unit.
 __global__ void __launch_bounds__(128) k_out_emit(uint32_t n_units, const uint32_t* n_dev,
-                                                  const uint32_t* __restrict__ unit_start,
-                                                  const uint8_t* __restrict__ pverbs, const float* __restrict__ ppts,
-                                                  const uint32_t* __restrict__ poly_foff_of,
-                                                  const uint32_t* __restrict__ pfill_off, uint32_t n_fills,
-                                                  const uint8_t* __restrict__ flags,
-                                                  const uint32_t* __restrict__ first_close,
-                                                  const float* __restrict__ width, const uint32_t* __restrict__ out_off,
-                                                  const uint32_t* __restrict__ out_foff, uint8_t* __restrict__ overbs,
+                                                  const uint32_t* unit_start,
+                                                  const uint8_t* pverbs, const float* ppts,
+                                                  const uint32_t* poly_foff_of,
+                                                  const uint32_t* pfill_off, uint32_t n_fills,
+                                                  const uint8_t* flags,
+                                                  const uint32_t* first_close,
+                                                  const float* width, const uint32_t* out_off,
+                                                  const uint32_t* out_foff, uint8_t* __restrict__ overbs,
                                                   float* __restrict__ opts, uint32_t* __restrict__ unit_fill) {
     dependent_start();
     const uint64_t u = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(128) k_out_emit(uint32_t n_units, const uint32
         return;
     }
     if (lane == 0) unit_fill[u] = g.fill;
-    const float w = __ldg(width + g.fill);
+    const float w = width[g.fill];
     const bool closed = g.closed != 0;
     // forward side: its first point becomes a Move (path.rs:249-250)
     const uint32_t nf = stroke_side_warp(P, g.len, closed, false, w, [&](uint32_t k, V2 p) {
@@ -439,10 +439,10 @@ __global__ void __launch_bounds__(128) k_out_emit(uint32_t n_units, const uint32
 
 // A planned run (pad_end > 0) ends the last fill at pad_end: the output
 // commands from the true total up to it are Close commands.
-__global__ void k_out_fill_off(const uint32_t* __restrict__ unit_fill, uint32_t n_units, const uint32_t* units_dev,
-                               const uint32_t* __restrict__ out_off, uint32_t total, const uint32_t* total_dev,
+__global__ void k_out_fill_off(const uint32_t* unit_fill, uint32_t n_units, const uint32_t* units_dev,
+                               const uint32_t* out_off, uint32_t total, const uint32_t* total_dev,
                                uint32_t pad_end, uint32_t n_fills, uint32_t* __restrict__ ofill_off,
-                               const uint8_t* __restrict__ flags, uint8_t* __restrict__ oflags) {
+                               const uint8_t* flags, uint8_t* __restrict__ oflags) {
     dependent_start();
     const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f > n_fills) return;
@@ -455,7 +455,7 @@ __global__ void k_out_fill_off(const uint32_t* __restrict__ unit_fill, uint32_t 
         if (unit_fill[mid] < f) lo = mid + 1; else hi = mid;
     }
     ofill_off[f] = f == n_fills && pad_end ? pad_end : lo < n_units ? min(out_off[lo], total) : total;
-    if (f < n_fills) oflags[f] = flags ? (uint8_t)(__ldg(flags + f) & ~OCHRE_FILL_STROKE) : 0u;
+    if (f < n_fills) oflags[f] = flags ? (uint8_t)(flags[f] & ~OCHRE_FILL_STROKE) : 0u;
 }
 
 // A planned run (CUDA graph): a count pair above its capacities zeroes the

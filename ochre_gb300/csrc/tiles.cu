@@ -98,7 +98,7 @@ struct HeadArgs {
     uint32_t* n_rows;        // zero before the launch
 };
 template <class K, int HEAD_ITEMS>
-__global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* __restrict__ keys, HeadArgs A,
+__global__ void __launch_bounds__(HEAD_BLOCK) k_tile_heads(const K* keys, HeadArgs A,
                                                            ScanStatus<HeadScan>* status, uint64_t* last_head,
                                                            uint32_t* ticket, uint32_t ticket_base, uint32_t tag,
                                                            uint32_t* err) {
@@ -309,7 +309,7 @@ constexpr int CELL_UNROLL = 4;
 // staged, then the warp's lanes take equal contiguous ranges of their cells,
 // so every lane has cells whatever the bins' lengths; a cell's place follows
 // from its bin's first cell and steps.
-__device__ __forceinline__ void add_increments(bool bin, uint4 rec, int slot, const float2* __restrict__ incs, float* acc,
+__device__ __forceinline__ void add_increments(bool bin, uint4 rec, int slot, const float2* incs, float* acc,
                                                BinStage& st) {
     const int lane = threadIdx.x & 31;
     const uint32_t n = bin ? (rec.w >> 16) & 0xffu : 0u;
@@ -403,7 +403,7 @@ struct EntryRun {
     }
     // Adds the entries up to e1, the end of a chunk of tiles (my_head: see
     // entry_slot; crossing entries in between are skipped).
-    __device__ __forceinline__ void add_to(uint32_t e1, uint32_t my_head, const float2* __restrict__ incs, float* acc,
+    __device__ __forceinline__ void add_to(uint32_t e1, uint32_t my_head, const float2* incs, float* acc,
                                            BinStage& st) {
         for (;;) {
             const bool bin = eb + (threadIdx.x & 31) < e1 && !(v & CROSS_TAG);
@@ -458,7 +458,7 @@ __device__ __forceinline__ void shade_row(const float* a, const float* h, float 
 // (382,000 tiles, 16 million bins) 546 -> 532 us, 256 shapes 36 -> 32 us.
 template <int CH>
 __global__ void __launch_bounds__(128) k_tile_cov_blocks(
-    const uint32_t* __restrict__ vals, const BinRec* __restrict__ bins, const float2* __restrict__ incs,
+    const uint32_t* vals, const BinRec* bins, const float2* incs,
     TileView tiles, uint32_t n_tiles, const uint32_t* n_dev, TileBlockState* state, uint32_t* ticket,
     uint32_t* __restrict__ out_xy, uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov, uint32_t* err,
     bool cov_signed) {
@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(128) k_tile_cov_blocks(
 constexpr uint32_t ROW_RANGE = 32;   // tiles per ticket, and per window of metadata
 template <int CH>
 __global__ void __launch_bounds__(128, CH == 8 ? 9 : 1) k_tile_cov(
-    const uint32_t* __restrict__ vals, const BinRec* __restrict__ bins, const float2* __restrict__ incs,
+    const uint32_t* vals, const BinRec* bins, const float2* incs,
     TileView tiles, uint32_t n_tiles, const uint32_t* n_dev, uint32_t* ticket, uint32_t* __restrict__ out_xy,
     uint8_t* __restrict__ out_alpha, float* __restrict__ out_cov, const uint32_t* err, bool cov_signed) {
     dependent_start();
