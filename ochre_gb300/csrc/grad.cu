@@ -357,8 +357,10 @@ __global__ void __launch_bounds__(128) k_line_grad(const float4* lines,
         const float h = p1.y - p0.y;
         const float right = (float)(x + 1);
         const float m = 0.5f * ((right - p0.x) + (right - p1.x));
-        // dL/dp0 = (dx, -dy) and dL/dp1 = (dx, dy) of a = h m and h
-        const float dx = -0.5f * h * g, dy = m * g + G;
+        // dL/dp0 = (dx, -dy) and dL/dp1 = (dx, dy) of a = h m and h (nothing
+        // where no pixel sees the cell: its h and m may have overflowed)
+        const bool seen = g != 0.0f || G != 0.0f;
+        const float dx = seen ? -0.5f * h * g : 0.0f, dy = seen ? m * g + G : 0.0f;
         if (first) {
             d.ax += dx;
             d.ay -= dy;
