@@ -257,11 +257,15 @@ __device__ __forceinline__ void cell_grads(int x, int y, uint32_t r, uint32_t W,
 // a / b for r = 1 / b rounded to nearest: the product with the reciprocal and
 // one residual correction give the rounded quotient (Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", 1990, for
-// quotients in the normal range); beyond it, where r is no finite number, the
-// division itself.
+// quotients in the normal range).  Beyond it the division itself: where the
+// product is no number below 1e38, as it never is with a reciprocal that does
+// not serve (reciprocal_for).
+__device__ __forceinline__ float reciprocal_for(float r) {
+    return fabsf(r) > 1e30f ? __int_as_float(0x7f800000) : r;
+}
 __device__ __forceinline__ float div_by(float a, float b, float r) {
-    if (fabsf(r) > 1e30f) return a / b;
     const float q = __fmul_rn(a, r);
+    if (!(fabsf(q) < 1e38f)) return a / b;
     return __fmaf_rn(__fmaf_rn(-b, q, a), r, q);
 }
 
@@ -283,7 +287,7 @@ __device__ __forceinline__ float div_by(float a, float b, float r) {
 // before they go to A and B would save more, but the terms of steep and flat
 // lines cancel, and single gradients then moved by 0.3 % of their rms; as it
 // is every operation rounds as it did.  14.4 M lines (27.9 M cells) of 128
-// dense scenes: 567 us with both sides and all divisions on their own, 373 now.
+// dense scenes: 567 us with both sides and all divisions on their own, 383 now.
 __global__ void __launch_bounds__(128) k_line_grad(const float4* lines,
                                                    const uint32_t* line_raster, uint32_t L,
                                                    const uint32_t* l_dev, uint32_t W, uint32_t H,
@@ -307,7 +311,8 @@ __global__ void __launch_bounds__(128) k_line_grad(const float4* lines,
     WalkState s;
     walk_setup(A, B, w, s);
     const float D = B.x - A.x, E = B.y - A.y;
-    const float rD = w.x_dir < 0 ? -w.x_step : w.x_step, rE = w.y_dir < 0 ? -w.y_step : w.y_step;   // 1 / D, 1 / E
+    const float rD = reciprocal_for(w.x_dir < 0 ? -w.x_step : w.x_step);   // 1 / D
+    const float rE = reciprocal_for(w.y_dir < 0 ? -w.y_step : w.y_step);   // 1 / E
     // p.y on the vertical pixel boundary x = X, as a function of A and B
     // (dL/d(p.y) from one cell, then from the other)
     auto vertical = [&](float X, float gy, float gy2) {

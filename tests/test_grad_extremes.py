@@ -1,5 +1,5 @@
 """The backward on inputs far from any picture: what no pixel sees has gradient
-0 however far away it lies."""
+0 however far away it lies, and a gradient past the largest number is infinite."""
 import numpy as np
 import pytest
 
@@ -36,3 +36,17 @@ def test_far_lines_have_no_gradient(far):
     assert np.array_equal(p[6:], np.zeros(4, np.float32)), p
     # (the same terms, their atomic adds in any order)
     assert np.allclose(p[:6], near, rtol=1e-5, atol=1e-5 * np.abs(near).max()), (p, near)
+
+
+def test_products_past_the_largest_number_are_infinite():
+    """One pixel's gradient on a line, where the line crosses from one pixel column
+    to the next: gradient * height and gradient * width overflow, each with one
+    sign, and no infinity meets another or a 0."""
+    w, h = 80, 320
+    b = BatchBuilder().begin_raster().fill([0, 1, 1], [2.5, 2.5, 66.5, 302.5, 70.25, 150.5], raw=True).build()
+    # the line goes from column 18 to column 19 at y = 79.84
+    dl = np.zeros((1, h, w), np.float32)
+    dl[0, 79, 18] = 1e38
+    p, _ = _gradients(b, w, h, dl)
+    assert not np.isnan(p).any(), p
+    assert np.isinf(p[:2]).all() and np.isfinite(p[2:]).all(), p
