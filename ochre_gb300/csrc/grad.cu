@@ -153,6 +153,22 @@ __global__ void k_l2(const float* cov, const float* target, uint64_t n,
 }
 
 // ---- backward 1: dL/dS at boundary-tile pixels ----
+// An image row of W values stands at the front of the row's W pairs, where the
+// next kernel leaves (dL/dS, suffix sum): one image of pairs is all the
+// backward keeps, 8 bytes a pixel.  A warp clears a row's values (cudaMemset2D
+// takes 15 us longer for the 65,536 rows of 128 dense scenes).
+__global__ void k_clear_rows(uint64_t rows, uint32_t W, bool vec, float* __restrict__ gsig) {
+    dependent_start();
+    const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (row >= rows) return;
+    float* g = gsig + 2 * row * W;
+    if (vec) {
+        for (uint32_t i = lane; i < W / 4; i += 32) reinterpret_cast<float4*>(g)[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    } else {
+        for (uint32_t i = lane; i < W; i += 32) g[i] = 0.0f;
+    }
+}
 __global__ void k_gsigma(const uint32_t* xy, const uint32_t* rf,
                          const float* tile_sum, uint32_t T, const uint32_t* t_dev, uint32_t W, uint32_t H,
                          bool vec, const float* dl_dcov, float* __restrict__ gsig) {
@@ -167,7 +183,7 @@ __global__ void k_gsigma(const uint32_t* xy, const uint32_t* rf,
     const float s[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
     auto dsig = [](float v, float g) { return fabsf(v) < 1.0f ? (v > 0.0f ? g : v < 0.0f ? -g : 0.0f) : 0.0f; };
     const float* d = dl_dcov + at;
-    float* o = gsig + at;
+    float* o = gsig + (2 * at - (size_t)(8 * tile_tx(xy[t])));
     if (vec && n == 8) {
         const float4 g = reinterpret_cast<const float4*>(d)[0], h = reinterpret_cast<const float4*>(d)[1];
         reinterpret_cast<float4*>(o)[0] = make_float4(dsig(s[0], g.x), dsig(s[1], g.y), dsig(s[2], g.z), dsig(s[3], g.w));
@@ -180,15 +196,16 @@ __global__ void k_gsigma(const uint32_t* xy, const uint32_t* rf,
 }
 
 // ---- backward 2: exclusive suffix sums of dL/dS along every canvas row ----
-// Writes (dL/dS, suffix sum) pairs: the adjoint of a cell reads both at once.
-__global__ void k_row_suffix(const float* gsig, uint64_t rows, uint32_t W, float2* __restrict__ gG,
-                             float* __restrict__ row_total) {
+// Writes (dL/dS, suffix sum) pairs over the row's values: the adjoint of a cell
+// reads both at once.  In place: a step's pairs lie at or past twice its first
+// value's place, and every value not yet read lies before that one.
+__global__ void k_row_suffix(uint64_t rows, uint32_t W, float2* gG, float* __restrict__ row_total) {
     dependent_start();
     const uint64_t row = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (row >= rows) return;
-    const float* g = gsig + row * W;
     float2* o = gG + row * W;
+    const float* g = reinterpret_cast<const float*>(o);
     float carry = 0.0f;
     int base = (int)((W - 1) / 32) * 32;
     float next = base + lane < (int)W ? g[base + lane] : 0.0f;
@@ -731,27 +748,26 @@ static int launch_backward(ochre_gpu_ctx* ctx, const ochre_batch* in, const Forw
     if (in->n_floats) OCHRE_CUDA_TRY(cudaMemsetAsync(dl_dpts, 0, in->n_floats * sizeof(float), s));
     if (in->n_fills) OCHRE_CUDA_TRY(cudaMemsetAsync(dl_dxf, 0, (size_t)in->n_fills * 6 * sizeof(float), s));
     if (R == 0 || in->n_cmds == 0 || n.lines == 0 || npx == 0) return OCHRE_OK;
-    OCHRE_CUDA_TRY(ctx->grad_g.ensure(npx * 4));
     OCHRE_CUDA_TRY(ctx->grad_gs.ensure(npx * sizeof(float2)));
     OCHRE_CUDA_TRY(ctx->grad_left.ensure((size_t)R * h * 4));
     OCHRE_CUDA_TRY(ctx->grad_line.ensure((size_t)n.lines * sizeof(LineGrad)));
     OCHRE_CUDA_TRY(ctx->grad_pts.ensure(in->n_floats * 4));
-    float* gsig = ctx->grad_g.as<float>();
     float2* gG = ctx->grad_gs.as<float2>();
+    float* gsig = ctx->grad_gs.as<float>();   // (a row's values at the front of its pairs)
     float* row_total = ctx->grad_left.as<float>();
     LineGrad* lg = ctx->grad_line.as<LineGrad>();
     float* gp = ctx->grad_pts.as<float>();
-    OCHRE_CUDA_TRY(cudaMemsetAsync(gsig, 0, npx * 4, s));
     OCHRE_CUDA_TRY(cudaMemsetAsync(gp, 0, in->n_floats * 4, s));
+    const uint64_t rows = (uint64_t)R * h;
+    const unsigned row_warps = (unsigned)((rows * 32 + 255) / 256);
+    OCHRE_LAUNCH(ctx, "grad_clear", s, launch_after(k_clear_rows, row_warps, 256, 0, s, rows, w,
+                                                    rows_aligned(gsig, gsig, w), gsig));
     if (n.tiles)
         OCHRE_LAUNCH(ctx, "grad_sigma", s, launch_after(
             k_gsigma, (unsigned)(((uint64_t)n.tiles * 8 + 255) / 256), 256, 0, s, ctx->tile_xy.as<uint32_t>(),
             ctx->tile_rf.as<uint32_t>(), ctx->out_tile_cov.as<float>(), n.tiles, n.tiles_dev, w, h,
             rows_aligned(dl_dcov, gsig, w), dl_dcov, gsig));
-    const uint64_t rows = (uint64_t)R * h;
-    OCHRE_LAUNCH(ctx, "grad_row_suffix", s,
-                 launch_after(k_row_suffix, (unsigned)((rows * 32 + 255) / 256), 256, 0, s, gsig, rows, w, gG,
-                              row_total));
+    OCHRE_LAUNCH(ctx, "grad_row_suffix", s, launch_after(k_row_suffix, row_warps, 256, 0, s, rows, w, gG, row_total));
     OCHRE_LAUNCH(ctx, "grad_lines", s, launch_after(
         k_line_grad, (n.lines + 127) / 128, 128, 0, s, ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(),
         n.lines, n.lines_dev, w, h, gG, row_total, lg));

@@ -224,7 +224,7 @@ struct ochre_gpu_ctx {
 
     bool cov_signed = false;   // tile_cov holds accum + area (signed) instead of |accum + area|
     // differentiable path scratch
-    ochre::DevBuf grad_g, grad_gs, grad_left, grad_line, grad_pts;
+    ochre::DevBuf grad_gs, grad_left, grad_line, grad_pts;
     // Bumped by every call that rewrites the chain's buffers (run_device,
     // compositing).  The chain structure left by ochre_gpu_render_coverage
     // (lines, per-command line offsets, tiles with signed coverage) stays

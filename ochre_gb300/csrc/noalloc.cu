@@ -103,7 +103,7 @@ extern "C" int ochre_gpu_rasterize_noalloc(const ochre_batch* in, ochre_output_b
                                  &ctx.keys_alt, &ctx.vals_alt, &ctx.bins, &ctx.sort_hist, &ctx.sort_lookback,
                                  &ctx.tile_head, &ctx.tile_xy, &ctx.tile_rf, &ctx.tile_state,
                                  &ctx.scan_status, &ctx.scalars, &ctx.fused_chain, &ctx.fused_stage, &ctx.out_tile_cov,
-                                 &ctx.grad_g, &ctx.grad_gs, &ctx.grad_left, &ctx.grad_line, &ctx.grad_pts,
+                                 &ctx.grad_gs, &ctx.grad_left, &ctx.grad_line, &ctx.grad_pts,
                                  &ctx.sk_cmd_foff, &ctx.sk_cmd_mv, &ctx.sk_cmd_ep, &ctx.sk_poly_off,
                                  &ctx.sk_poly_foff, &ctx.sk_pverbs, &ctx.sk_ppts, &ctx.sk_pfoff, &ctx.sk_pfill_off,
                                  &ctx.sk_first_close, &ctx.sk_unit_start, &ctx.sk_out_off, &ctx.sk_out_foff,
