@@ -30,6 +30,7 @@ constexpr int SORT_TILE = SORT_BLOCK * SORT_ITEMS;
 constexpr uint32_t LB_AGG = 1u << 30, LB_INC = 2u << 30, LB_MASK = (1u << 30) - 1u;
 constexpr int LB_WINDOW = 8;      // predecessor tiles one digit's look-back reads per round
 constexpr int SORT_MAX_PASSES = 8;
+constexpr size_t SORT_APART = (size_t)64 << 20;   // bytes that look-back words of passes of their own may take
 
 // The digits of a sort: pass p takes `width[p]` bits from bit `shift[p]`
 // (widths balanced over the key bits, at most the digit width RB).
@@ -294,14 +295,16 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
     const int passes = plan.passes;
     const uint64_t tiles = (n + SORT_TILE - 1) / SORT_TILE;
     // The counts, the tickets and every pass's look-back words lie together
-    // and are cleared once.  In an arena (no allocation) the passes share one
-    // pass's words, cleared before each, so that the sort takes no more of it.
+    // and are cleared once.  In an arena (no allocation), and where a long sort's
+    // passes would take more than SORT_APART bytes beyond one pass's words, the
+    // passes share those, cleared before each (a clear and a late launch, some 5
+    // us of passes that take 500 there).
     // No count is read back: a pass whose digit is the same in all keys runs
     // like any other (the read-back that found it out took longer than most
     // calls' passes: 15 to 20 us of every call).
-    const bool shared = ctx->sort_lookback.arena != nullptr;
-    constexpr size_t TICKETS = 16;   // one per pass, the last one counts k_sort_hist's blocks
     const size_t rows = (size_t)tiles * RADIX;
+    const bool shared = ctx->sort_lookback.arena != nullptr || (size_t)(passes - 1) * rows * 4 > SORT_APART;
+    constexpr size_t TICKETS = 16;   // one per pass, the last one counts k_sort_hist's blocks
     OCHRE_CUDA_TRY(ctx->sort_hist.ensure((size_t)passes * RADIX * 4 * 2));
     const size_t head = shared ? 0 : (size_t)passes * RADIX + TICKETS;
     const size_t words = head + rows * (shared ? 1 : passes);
