@@ -313,11 +313,7 @@ static int run_chain(ochre_gpu_ctx* ctx, const ochre_batch* in_orig, ochre_resul
     // a batch that did not fit the fused kernel last time (same arrays and
     // counts) goes to the chain directly; the results are the same either way
     const bool known_miss = remember_miss && ctx->fused_miss_valid && same_batch(ctx->fused_miss, *in_orig);
-    // more commands than the fused kernel takes for every raster: some raster
-    // has too many, and the attempt (which costs up to 0.4 ms: the rasters taken
-    // before the first misfit do their whole work) is not made
-    const bool too_many = in->n_cmds > (uint64_t)R * (uint32_t)ctx->tune_fused_threads;
-    if (!(ctx->flags & OCHRE_CTX_CHAIN_ONLY) && !known_miss && !too_many) {
+    if (!(ctx->flags & OCHRE_CTX_CHAIN_ONLY) && !known_miss) {
         st = stage_fused(ctx, in, s, &handled, &T, &N);
         if (st != OCHRE_OK) return st;
         if (remember_miss) {

@@ -932,6 +932,13 @@ int stage_fused(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, bool*
                 uint32_t* n_spans) {
     *handled = false;
     if (in->n_rasters == 0) return OCHRE_OK;
+    int grid = 0;
+    const int st = fused_shape(ctx, nullptr, &grid, s);   // (a shape that is not built is refused)
+    if (st != OCHRE_OK) return st;
+    // more commands than the kernel takes for every raster: some raster has too
+    // many, and the attempt (which costs up to 0.4 ms: the rasters taken before
+    // the first misfit do their whole work) is not made
+    if (in->n_cmds > (uint64_t)in->n_rasters * (uint32_t)ctx->tune_fused_threads) return OCHRE_OK;
     return run_fused(ctx, in, s, handled, n_tiles, n_spans);
 }
 
