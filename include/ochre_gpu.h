@@ -305,7 +305,10 @@ int ochre_gpu_get_tunable(const ochre_gpu_ctx *ctx, const char *name, int *value
  * the RGBA8 canvas (w * h * 4 bytes, device, row-major, read and written):
  * fragment = colour * (1, 1, 1, mask / 255), blended SRC_ALPHA,
  * ONE_MINUS_SRC_ALPHA on all channels and quantised to 8 bits after every
- * quad.  colors and canvas are 4-byte aligned device pointers. */
+ * quad.  colors and canvas are 4-byte aligned device pointers.  Returns with the
+ * drawing queued on the stream.  Should a bounded wait of its sort give up, the
+ * canvas is left as it was, and the context's next call that rasterizes or
+ * composites returns OCHRE_E_TIMEOUT in its place. */
 int ochre_gpu_composite(ochre_gpu_ctx *ctx, const ochre_result *res, uint32_t n_rasters, const uint8_t *colors,
                         uint32_t w, uint32_t h, uint8_t *canvas, void *stream);
 

@@ -155,7 +155,9 @@ int copy_scalars_async(ochre_gpu_ctx* ctx, cudaStream_t s) {
 }
 
 cudaError_t reset_scalars(ochre_gpu_ctx* ctx, cudaStream_t s) {
-    cudaError_t e = cudaMemsetAsync(ctx->scalars.p, 0, sizeof(DevScalars), s);
+    // (in an arena anything may have lain there, and no call returns early)
+    const size_t bytes = ctx->scalars.arena != nullptr ? sizeof(DevScalars) : offsetof(DevScalars, late_err);
+    cudaError_t e = cudaMemsetAsync(ctx->scalars.p, 0, bytes, s);
     if (e == cudaSuccess && ctx->test_spin_log2 != 0u)
         e = cudaMemcpyAsync(&dev_scalars(ctx)->spin_log2, &ctx->test_spin_log2, sizeof(uint32_t),
                             cudaMemcpyHostToDevice, s);
@@ -167,6 +169,10 @@ int read_scalars(ochre_gpu_ctx* ctx, cudaStream_t s) {
     if (st != OCHRE_OK) return st;
     OCHRE_CUDA_TRY(cudaStreamSynchronize(s));
     if (host_scalars(ctx)->err & ERR_TIMEOUT) ctx->scan_dirty = true;   // blocks left without taking tickets
+    if (host_scalars(ctx)->late_err) {
+        OCHRE_CUDA_TRY(cudaMemsetAsync(&dev_scalars(ctx)->late_err, 0, sizeof(uint32_t), s));
+        return OCHRE_E_TIMEOUT;
+    }
     return OCHRE_OK;
 }
 
@@ -401,7 +407,9 @@ int ochre_gpu_create(ochre_gpu_ctx** out, int device, uint32_t flags) {
     ctx->flags = flags;
     if (cudaSetDevice(device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        ctx->scalars.ensure(sizeof(DevScalars)) != cudaSuccess) {
+        ctx->scalars.ensure(sizeof(DevScalars)) != cudaSuccess ||
+        cudaMemsetAsync(ctx->scalars.p, 0, sizeof(DevScalars), ctx->own_stream) != cudaSuccess ||
+        cudaStreamSynchronize(ctx->own_stream) != cudaSuccess) {
         ochre_gpu_destroy(ctx);
         return OCHRE_E_CUDA;
     }
@@ -727,6 +735,9 @@ int ochre_gpu_set_tunable(ochre_gpu_ctx* ctx, const char* name, int value) {
     } else if (!std::strcmp(name, "test_fail_scan")) {
         if (value < 0 || value > 64) return OCHRE_E_INVALID;
         ctx->test_fail_scan = (uint32_t)value;
+    } else if (!std::strcmp(name, "test_skip_sort_ticket")) {
+        if (value < 0 || value > 1) return OCHRE_E_INVALID;
+        ctx->test_skip_sort_ticket = (uint32_t)value;
     } else {
         return OCHRE_E_INVALID;
     }

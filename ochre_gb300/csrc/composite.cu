@@ -107,10 +107,14 @@ __global__ void k_piece_emit(PieceItems items, uint32_t rbits, const uint32_t* o
 constexpr uint32_t NO_PIECE = 0xffffffffu;
 template <class K>
 __global__ void k_piece_heads(const K* keys, uint32_t E, uint32_t rbits, uint32_t n_tiles,
-                              uint32_t* __restrict__ head, const uint32_t* err) {
+                              uint32_t* __restrict__ head, const uint32_t* err, uint32_t* late_err) {
     dependent_start();
     const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= E || run_aborted(err)) return;   // a wait of the sort gave up: the sorted pieces are not valid
+    if (e >= E) return;
+    if (run_aborted(err)) {   // a wait of the sort gave up: the sorted pieces are not valid
+        if (e == 0) atomicOr(late_err, ERR_TIMEOUT);   // (the call will have returned)
+        return;
+    }
     const K st = keys[e] >> rbits;
     if ((e == 0 || (keys[e - 1] >> rbits) != st) && st < (K)n_tiles) head[st] = e;
 }
@@ -287,7 +291,7 @@ static int composite_pieces(ochre_gpu_ctx* ctx, const PieceItems& items, uint32_
     uint32_t* head = ctx->tile_head.as<uint32_t>();
     OCHRE_CUDA_TRY(cudaMemsetAsync(head, 0xff, (size_t)screen * 4, s));
     OCHRE_LAUNCH(ctx, "composite_heads", s, launch_after(k_piece_heads<K>, (E + 255) / 256, 256, 0, s, 
-        ctx->keys.as<K>(), E, rbits, screen, head, &ds->err));
+        ctx->keys.as<K>(), E, rbits, screen, head, &ds->err, &ds->late_err));
     OCHRE_CUDA_TRY(cudaGetLastError());
     OCHRE_LAUNCH(ctx, "composite", s, launch_after(k_composite<K>, (unsigned)(((uint64_t)screen * 32 + 127) / 128), 128, 0, s, 
         ctx->keys.as<K>(), ctx->vals.as<uint32_t>(), E, head, rbits, items.T, tile_alpha,
@@ -326,7 +330,7 @@ static int composite(ochre_gpu_ctx* ctx, const ochre_result* res, uint32_t n_ras
     if (st != OCHRE_OK) return st;
     ctx->stats.n_launches = ctx->launches;
     collect_timings(ctx, s);
-    return check_device_error(ctx);
+    return OCHRE_OK;
 }
 
 }  // namespace ochre
@@ -347,6 +351,7 @@ extern "C" int ochre_gpu_composite(ochre_gpu_ctx* ctx, const ochre_result* res, 
     ctx->launches = 0;
     if (nothing) return OCHRE_OK;
     const int st = composite(ctx, res, n_rasters, colors, w, h, canvas, s);
+    ctx->test_spin_log2 = 0;   // (this call's)
     if (st != OCHRE_OK) ctx->scan_dirty = true;   // a scan may be counted that never ran
     return st;
 }

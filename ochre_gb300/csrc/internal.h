@@ -80,6 +80,9 @@ struct DevScalars {
     uint32_t fused_fallback;  // fused path: some raster did not fit
     uint32_t fused_tiles;     // fused path totals
     uint32_t fused_spans;
+    // What a call that returned before its last kernels did not see (ERR_*
+    // bits): reset_scalars leaves it, the context's next read-back reports it.
+    uint32_t late_err;
 };
 // The waits find spin_log2 from the error word's address (common.cuh).
 static_assert(offsetof(DevScalars, spin_log2) - offsetof(DevScalars, err) == 4 * 22,
@@ -254,6 +257,8 @@ struct ochre_gpu_ctx {
     uint32_t test_spin_log2 = 0;
     uint32_t test_skip_first_ticket = 0;
     uint32_t test_fail_scan = 0;
+    // The first pass of the next radix sort never takes its first tile.
+    uint32_t test_skip_sort_ticket = 0;
 
     // Launch-shape tunables (ochre_gpu_set_tunable; chosen by the autotuner).
     int tune_fused_threads = 64;
@@ -355,7 +360,7 @@ inline bool reads_back(const ochre_batch* in) { return in->n_rasters != 0 || in-
 // (host-batch entry); every stage calls it before its first read of points.
 void wait_inputs(ochre_gpu_ctx* ctx, cudaStream_t s);
 
-// Zeroes the device scalars of a run (and applies the poll-limit test hook).
+// Zeroes the device scalars of a run but late_err (and applies the poll-limit test hook).
 cudaError_t reset_scalars(ochre_gpu_ctx* ctx, cudaStream_t s);
 // Read the device scalars into ctx->h_scalars (synchronises the stream).
 int read_scalars(ochre_gpu_ctx* ctx, cudaStream_t s);
