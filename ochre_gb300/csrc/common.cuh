@@ -271,17 +271,6 @@ __device__ __forceinline__ void walk_setup(V2 a, V2 p, Walk& w, WalkState& s) {
     w.end_y = f2i16(floorf(p.y));
 }
 
-// The increment pushed for the current cell (rasterizer.rs:98-106).
-__device__ __forceinline__ void walk_increment(const Walk& w, const WalkState& s, float& area, float& height) {
-    const float t0 = rmax(s.row_t0, s.col_t0);
-    const float t1 = rmin(s.row_t1, s.col_t1);
-    const V2 p0 = vlerp(t0, w.a, w.p);
-    const V2 p1 = vlerp(t1, w.a, w.p);
-    height = __fsub_rn(p1.y, p0.y);
-    const float right = (float)wrap16(s.x + 1);
-    area = __fmul_rn(__fmul_rn(0.5f, height), __fadd_rn(__fsub_rn(right, p0.x), __fsub_rn(right, p1.x)));
-}
-
 // One step (rasterizer.rs:108-121).  Returns true when the walk ends; the
 // cell is then the snapped end cell, which receives no increment.
 __device__ __forceinline__ bool walk_step(const Walk& w, WalkState& s) {

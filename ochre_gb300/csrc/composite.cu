@@ -282,7 +282,7 @@ static int composite_pieces(ochre_gpu_ctx* ctx, const PieceItems& items, uint32_
     OCHRE_CUDA_TRY(ctx->keys_alt.ensure((size_t)E * sizeof(K)));
     OCHRE_CUDA_TRY(ctx->vals_alt.ensure((size_t)E * 4));
     OCHRE_CUDA_TRY(ctx->tile_head.ensure((size_t)screen * 4));
-    OCHRE_LAUNCH(ctx, "composite_pieces", s, launch_after(k_piece_emit<K>, (unsigned)((S + 255) / 256), 256, 0, s, 
+    OCHRE_LAUNCH(ctx, "composite_pieces", s, launch_after(k_piece_emit<K>, (unsigned)((S + 255) / 256), 256, 0, s,
         items, rbits, ctx->line_ent_off.as<uint32_t>(), ctx->keys.as<K>(), ctx->vals.as<uint32_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());
     uint32_t passes = 0;
@@ -290,10 +290,10 @@ static int composite_pieces(ochre_gpu_ctx* ctx, const PieceItems& items, uint32_
     if (st != OCHRE_OK) return st;
     uint32_t* head = ctx->tile_head.as<uint32_t>();
     OCHRE_CUDA_TRY(cudaMemsetAsync(head, 0xff, (size_t)screen * 4, s));
-    OCHRE_LAUNCH(ctx, "composite_heads", s, launch_after(k_piece_heads<K>, (E + 255) / 256, 256, 0, s, 
+    OCHRE_LAUNCH(ctx, "composite_heads", s, launch_after(k_piece_heads<K>, (E + 255) / 256, 256, 0, s,
         ctx->keys.as<K>(), E, rbits, screen, head, &ds->err, &ds->late_err));
     OCHRE_CUDA_TRY(cudaGetLastError());
-    OCHRE_LAUNCH(ctx, "composite", s, launch_after(k_composite<K>, (unsigned)(((uint64_t)screen * 32 + 127) / 128), 128, 0, s, 
+    OCHRE_LAUNCH(ctx, "composite", s, launch_after(k_composite<K>, (unsigned)(((uint64_t)screen * 32 + 127) / 128), 128, 0, s,
         ctx->keys.as<K>(), ctx->vals.as<uint32_t>(), E, head, rbits, items.T, tile_alpha,
         reinterpret_cast<const uint32_t*>(colors), items.R, (uint32_t)items.w, (uint32_t)items.h, w8, h8,
         reinterpret_cast<uint32_t*>(canvas), -0.0f, &ds->err));

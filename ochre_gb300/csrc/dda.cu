@@ -577,7 +577,7 @@ __device__ __forceinline__ void emit_long(const float4* lines, const uint32_t* l
         GroupCell q;
         group_round<G>(L, q);
         if (q.valid) {
-            // walk_increment (rasterizer.rs:98-106)
+            // the cell's increment (rasterizer.rs:98-106)
             const V2 p0 = vlerp(q.t0, L.a, L.p), p1 = vlerp(q.t1, L.a, L.p);
             const float height = __fsub_rn(p1.y, p0.y);
             const float right = (float)wrap16(q.x + 1);
@@ -761,7 +761,7 @@ __global__ void __launch_bounds__(EMIT_BLOCK) k_line_emit(
     uint32_t b_xy = (uint32_t)(uint16_t)s.x | ((uint32_t)(uint16_t)s.y << 16);
     const uint32_t dirs = (w.x_dir < 0 ? 1u << 24 : 0u) | (w.y_dir < 0 ? 2u << 24 : 0u);
     for (;;) {
-        // walk_increment (rasterizer.rs:98-106)
+        // the cell's increment (rasterizer.rs:98-106)
         const bool row = s.row_t1 < s.col_t1;
         const float t1 = row ? s.row_t1 : s.col_t1;
         const V2 p1 = vlerp(t1, w.a, w.p);
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(EMIT_BLOCK) k_line_emit(
         }
         q++;
         b_n++;
-        // walk_step (rasterizer.rs:108-121)
+        // the step out of it (rasterizer.rs:108-121)
         p0 = p1;
         if (below) {
             if (row) row_moved = true; else col_moved = true;
@@ -952,7 +952,7 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
         unsigned count_grid = 1;
         uint32_t groups = 1;
         count_shape(ctx, n_lines, &count_grid, &groups);
-        OCHRE_LAUNCH(ctx, "dda_count", s, launch_after(k_line_count, count_grid, WALK_BLOCK, 0, s, 
+        OCHRE_LAUNCH(ctx, "dda_count", s, launch_after(k_line_count, count_grid, WALK_BLOCK, 0, s,
             ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), n_lines, lines_dev, groups,
             ctx->raster_bbox.as<int4>(),
             ctx->raster_wsum.as<int>(), ctx->line_ent_off.as<uint32_t>(), ctx->line_inc_off.as<uint32_t>(),
@@ -1030,7 +1030,7 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint64_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), long_cells));
         else
-            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint32_t>, (unsigned)((n_lines + EMIT_BLOCK - 1) / EMIT_BLOCK), EMIT_BLOCK, 0, s, 
+            OCHRE_LAUNCH(ctx, "dda_emit", s, launch_after(k_line_emit<uint32_t>, (unsigned)((n_lines + EMIT_BLOCK - 1) / EMIT_BLOCK), EMIT_BLOCK, 0, s,
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),
@@ -1042,12 +1042,12 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
         const uint32_t* first_dev = plan ? &ds->line_ent_total : nullptr;
         const uint32_t* ent_dev = plan ? &ds->n_entries : nullptr;
         if (ctx->keys64)
-            OCHRE_LAUNCH(ctx, "empty_emit", s, launch_after(k_empty_emit<uint64_t>, (R + 255) / 256, 256, 0, s, 
+            OCHRE_LAUNCH(ctx, "empty_emit", s, launch_after(k_empty_emit<uint64_t>, (R + 255) / 256, 256, 0, s,
                 ctx->raster_empty.as<uint32_t>(), R, first_entry, first_dev, ent_dev,
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint64_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>()));
         else
-            OCHRE_LAUNCH(ctx, "empty_emit", s, launch_after(k_empty_emit<uint32_t>, (R + 255) / 256, 256, 0, s, 
+            OCHRE_LAUNCH(ctx, "empty_emit", s, launch_after(k_empty_emit<uint32_t>, (R + 255) / 256, 256, 0, s,
                 ctx->raster_empty.as<uint32_t>(), R, first_entry, first_dev, ent_dev,
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<uint32_t>(), ctx->vals.as<uint32_t>(),
                 ctx->bins.as<BinRec>()));

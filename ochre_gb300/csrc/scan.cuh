@@ -280,7 +280,6 @@ constexpr int SCAN_ITEMS = 8;
 // look-back words take no more of it.
 constexpr int SCAN_ITEMS_FEW = 2;
 constexpr uint64_t SCAN_FEW = 1u << 16;
-inline uint64_t scan_tiles(uint64_t n) { return (n + SCAN_BLOCK * SCAN_ITEMS - 1) / (SCAN_BLOCK * SCAN_ITEMS); }
 
 // Look-back memory of one scan (scan_space, api.cu).  An eager scan clears
 // nothing: its flags carry a tag no earlier scan of the context used, and its
@@ -309,10 +308,10 @@ cudaError_t launch_scan(ochre_gpu_ctx* ctx, uint64_t n, In in, Out out, Op op, T
     auto* status = reinterpret_cast<ScanStatus<T>*>(sp.status);
     uint32_t* err = &dev_scalars(ctx)->err;
     if (few)
-        launch_after(k_scan<SCAN_BLOCK, SCAN_ITEMS_FEW, T, Op, In, Out>, (unsigned)tiles, SCAN_BLOCK, 0, stream, 
+        launch_after(k_scan<SCAN_BLOCK, SCAN_ITEMS_FEW, T, Op, In, Out>, (unsigned)tiles, SCAN_BLOCK, 0, stream,
             n, n_dev, in, out, op, identity, status, sp.ticket, sp.ticket_base, sp.tag, total, err);
     else
-        launch_after(k_scan<SCAN_BLOCK, SCAN_ITEMS, T, Op, In, Out>, (unsigned)tiles, SCAN_BLOCK, 0, stream, 
+        launch_after(k_scan<SCAN_BLOCK, SCAN_ITEMS, T, Op, In, Out>, (unsigned)tiles, SCAN_BLOCK, 0, stream,
             n, n_dev, in, out, op, identity, status, sp.ticket, sp.ticket_base, sp.tag, total, err);
     return cudaGetLastError();
 }

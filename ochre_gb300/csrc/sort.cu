@@ -326,7 +326,7 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
         int blocks = (int)std::min<uint64_t>((n + 255) / 256, (uint64_t)std::max(sms, 1) * 8);
-        OCHRE_LAUNCH(ctx, "sort_hist", s, launch_after(k_sort_hist<K, RB>, blocks, 256, 0, s, 
+        OCHRE_LAUNCH(ctx, "sort_hist", s, launch_after(k_sort_hist<K, RB>, blocks, 256, 0, s,
             kin, n, n_dev, plan, hist, off, shared ? tickets : tickets + TICKETS - 1));
         OCHRE_CUDA_TRY(cudaGetLastError());
     }
@@ -343,7 +343,7 @@ static int sort_impl(ochre_gpu_ctx* ctx, uint64_t n, uint32_t key_bits, cudaStre
             ctx->test_skip_sort_ticket = 0;
             OCHRE_CUDA_TRY(cudaMemsetAsync(ticket, 1, 1, s));   // (its low byte)
         }
-        OCHRE_LAUNCH(ctx, "sort_onesweep", s, launch_after(k_onesweep<K, RB>, (unsigned)tiles, SORT_BLOCK, smem, s, 
+        OCHRE_LAUNCH(ctx, "sort_onesweep", s, launch_after(k_onesweep<K, RB>, (unsigned)tiles, SORT_BLOCK, smem, s,
             kin, vin, kout, vout, n, n_dev, plan.shift[p], (1u << plan.width[p]) - 1u, off + p * RADIX, lookback,
             ticket, &ds->err));
         OCHRE_CUDA_TRY(cudaGetLastError());

@@ -506,7 +506,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     wait_inputs(ctx, s);   // path-space flatten counts read points
     OCHRE_CUDA_TRY(ctx->sk_poly_off.ensure((n + 1) * 4));
     OCHRE_CUDA_TRY(ctx->sk_poly_foff.ensure((n + 1) * 4));
-    OCHRE_LAUNCH(ctx, "stroke_poly_count", s, launch_after(k_pair_count<PolyCount>, (unsigned)((n + 127) / 128), 128, 0, s, 
+    OCHRE_LAUNCH(ctx, "stroke_poly_count", s, launch_after(k_pair_count<PolyCount>, (unsigned)((n + 127) / 128), 128, 0, s,
         n, nullptr,
         PolyCount{in->verbs, in->pts, in->fill_cmd_off, F, in->fill_flags, ctx->sk_cmd_foff.as<uint32_t>(),
                   ctx->sk_cmd_ep.as<uint32_t>(), &ds->err},
@@ -542,11 +542,11 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     OCHRE_CUDA_TRY(ctx->sk_pfill_off.ensure(((size_t)F + 1) * 4));
     OCHRE_CUDA_TRY(ctx->sk_first_close.ensure((size_t)F * 4));
     const unsigned cb = (unsigned)((n + 255) / 256);
-    OCHRE_LAUNCH(ctx, "stroke_poly_emit", s, launch_after(k_poly_emit, cb, 256, 0, s, 
+    OCHRE_LAUNCH(ctx, "stroke_poly_emit", s, launch_after(k_poly_emit, cb, 256, 0, s,
         in->verbs, in->pts, in->fill_cmd_off, F, in->fill_flags, n, ctx->sk_cmd_foff.as<uint32_t>(),
         ctx->sk_cmd_ep.as<uint32_t>(), ctx->sk_poly_off.as<uint32_t>(), ctx->sk_poly_foff.as<uint32_t>(),
         ctx->sk_pverbs.as<uint8_t>(), ctx->sk_ppts.as<float>(), P, PF));
-    OCHRE_LAUNCH(ctx, "stroke_fill_init", s, launch_after(k_fill_init, (F + 256) / 256, 256, 0, s, 
+    OCHRE_LAUNCH(ctx, "stroke_fill_init", s, launch_after(k_fill_init, (F + 256) / 256, 256, 0, s,
         ctx->sk_first_close.as<uint32_t>(), in->fill_cmd_off, ctx->sk_poly_off.as<uint32_t>(), n, P, p_dev, F,
         ctx->sk_pfill_off.as<uint32_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());
@@ -563,7 +563,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     OCHRE_LAUNCH(ctx, "stroke_pfoff_scan", s, OCHRE_CUDA_TRY(launch_scan<uint32_t>(
         ctx, P, VerbFloats{ctx->sk_pverbs.as<uint8_t>()}, ScanOff{ctx->sk_pfoff.as<uint32_t>()}, OpSumU32{}, 0u,
         static_cast<uint32_t*>(nullptr), s, p_dev)));
-    OCHRE_LAUNCH(ctx, "stroke_first_close", s, launch_after(k_first_close, (P + 255) / 256, 256, 0, s, 
+    OCHRE_LAUNCH(ctx, "stroke_first_close", s, launch_after(k_first_close, (P + 255) / 256, 256, 0, s,
         ctx->sk_pverbs.as<uint8_t>(), P, p_dev, ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
         ctx->sk_first_close.as<uint32_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());
@@ -590,7 +590,7 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     // the output totals: a scan that covers no unit writes none
     OCHRE_CUDA_TRY(cudaMemsetAsync(&ds->n_lines, 0, 8, s));
     if (U) {
-        OCHRE_LAUNCH(ctx, "stroke_out_count", s, launch_after(k_out_count, (unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s, 
+        OCHRE_LAUNCH(ctx, "stroke_out_count", s, launch_after(k_out_count, (unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s,
             U, u_dev, ctx->sk_unit_start.as<uint32_t>(), ctx->sk_pverbs.as<uint8_t>(), ctx->sk_ppts.as<float>(),
             ctx->sk_pfoff.as<uint32_t>(), ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
             ctx->sk_first_close.as<uint32_t>(), in->fill_width, ctx->sk_out_off.as<uint32_t>(),
@@ -626,13 +626,13 @@ int stage_stroke(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s, ochr
     // planned: every output command past the true total is a Close
     if (plan) OCHRE_CUDA_TRY(cudaMemsetAsync(ctx->sk_overbs.p, V_CLOSE, ON, s));
     if (U)
-        OCHRE_LAUNCH(ctx, "stroke_out_emit", s, launch_after(k_out_emit, (unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s, 
+        OCHRE_LAUNCH(ctx, "stroke_out_emit", s, launch_after(k_out_emit, (unsigned)(((uint64_t)U * 32 + 127) / 128), 128, 0, s,
             U, u_dev, ctx->sk_unit_start.as<uint32_t>(), ctx->sk_pverbs.as<uint8_t>(), ctx->sk_ppts.as<float>(),
             ctx->sk_pfoff.as<uint32_t>(), ctx->sk_pfill_off.as<uint32_t>(), F, in->fill_flags,
             ctx->sk_first_close.as<uint32_t>(), in->fill_width, ctx->sk_out_off.as<uint32_t>(),
             ctx->sk_out_foff.as<uint32_t>(), ctx->sk_overbs.as<uint8_t>(), ctx->sk_opts.as<float>(),
             ctx->sk_unit_fill.as<uint32_t>()));
-    OCHRE_LAUNCH(ctx, "stroke_fill_off", s, launch_after(k_out_fill_off, (F + 256) / 256, 256, 0, s, 
+    OCHRE_LAUNCH(ctx, "stroke_fill_off", s, launch_after(k_out_fill_off, (F + 256) / 256, 256, 0, s,
         ctx->sk_unit_fill.as<uint32_t>(), U, u_dev, ctx->sk_out_off.as<uint32_t>(), ON, plan ? &ds->n_lines : nullptr,
         plan ? ON : 0u, F, ctx->sk_ofill_off.as<uint32_t>(), in->fill_flags, ctx->sk_oflags.as<uint8_t>()));
     OCHRE_CUDA_TRY(cudaGetLastError());

@@ -837,14 +837,14 @@ static void launch_tile_cov(ochre_gpu_ctx* ctx, const TileView& tiles, uint32_t 
     if (row_form) {
         // no more warps than rows, nor than the GPU keeps resident (16 CTAs of 4 warps per SM)
         const uint32_t ctas = (uint32_t)std::min<uint64_t>(((uint64_t)n_rows + 3) / 4, (uint64_t)sms * 16);
-        launch_after(k_tile_cov<TPW>, ctas, 128, 0, s, 
+        launch_after(k_tile_cov<TPW>, ctas, 128, 0, s,
             ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), tiles, T, t_dev,
             &ds->ticket, ctx->out_tile_xy.as<uint32_t>(), ctx->out_tile_alpha.as<uint8_t>(), cov,
             &ds->err, ctx->cov_signed);
     } else {
         const uint32_t blocks = (T + TPW - 1) / TPW;
         cudaMemsetAsync(ctx->tile_state.p, 0, (size_t)blocks * sizeof(TileBlockState), s);
-        launch_after(k_tile_cov_blocks<TPW>, (blocks + 3) / 4, 128, 0, s, 
+        launch_after(k_tile_cov_blocks<TPW>, (blocks + 3) / 4, 128, 0, s,
             ctx->vals.as<uint32_t>(), ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), tiles, T, t_dev,
             ctx->tile_state.as<TileBlockState>(), &ds->ticket, ctx->out_tile_xy.as<uint32_t>(),
             ctx->out_tile_alpha.as<uint8_t>(), cov, &ds->err, ctx->cov_signed);
@@ -882,10 +882,10 @@ static int tiles_impl(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t E, cud
     auto* status = reinterpret_cast<ScanStatus<HeadScan>*>(sp.status);
     auto* last_head = reinterpret_cast<uint64_t*>(status + blocks);
     if (steps == 4)
-        OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 4>, blocks, HEAD_BLOCK, 0, s, 
+        OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 4>, blocks, HEAD_BLOCK, 0, s,
             ctx->keys.as<K>(), args, status, last_head, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
     else
-        OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 16>, blocks, HEAD_BLOCK, 0, s, 
+        OCHRE_LAUNCH(ctx, "tile_heads", s, launch_after(k_tile_heads<K, 16>, blocks, HEAD_BLOCK, 0, s,
             ctx->keys.as<K>(), args, status, last_head, sp.ticket, sp.ticket_base, sp.tag, &ds->err));
     OCHRE_CUDA_TRY(cudaGetLastError());
     int st = OCHRE_OK;
