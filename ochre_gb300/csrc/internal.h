@@ -5,6 +5,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 #include "../../include/ochre_gpu.h"
@@ -395,9 +396,10 @@ void collect_timings(ochre_gpu_ctx* ctx, cudaStream_t s);
 // stream ends (it waits in dependent_start, common.cuh).  What that hides is 1
 // to 2 us a launch, a good part of a short call: a document of 415 paths (43
 // launches) 510 -> 442 us, a differentiable step of 256 shapes (25) 324 -> 286.
+// Not `early`: an ordinary launch.
 template <class... Params, class... Args>
-cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                         Args&&... args) {
+cudaError_t launch_kernel(bool early, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                          Args&&... args) {
     cudaLaunchConfig_t c{};
     c.gridDim = grid;
     c.blockDim = block;
@@ -407,8 +409,13 @@ cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_
     a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     a.val.programmaticStreamSerializationAllowed = 1;
     c.attrs = &a;
-    c.numAttrs = 1;
+    c.numAttrs = early ? 1 : 0;
     return cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);
+}
+template <class... Params, class... Args>
+cudaError_t launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                         Args&&... args) {
+    return launch_kernel(true, kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 // A launch that another one, on another stream, is to run beside: an SM takes
 // blocks of two kernels only where both ask for the same split of its memory
