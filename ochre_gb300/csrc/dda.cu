@@ -311,6 +311,16 @@ __device__ __forceinline__ bool long_lines_share(uint32_t n_queue) {
 
 constexpr int LONG_THREADS = 128;
 constexpr uint32_t LONG_BLOCKS_PER_SM = 2;
+// The walkers are for few long lines among many.  Where an eighth of all lines
+// and more are long, and they are many enough to occupy the GPU by themselves,
+// the per-line kernel takes them too: its warps then walk long lines side by
+// side, and a lane does less for a cell than a group does.  The call, walkers
+// against none: 20,000 rasters of 100 lines (1.36 M of the 2.0 M long, 168 cells on
+// average) 8.9 -> 5.8 ms, its replay 15.4 -> 6.8; 50,000 lines of 4,000 cells 7.95 ->
+// 6.97 and 12.7 -> 7.0 ms; 40,000 of 160 cells 0.46 -> 0.40 and 0.70 -> 0.43 ms.
+bool long_lines_apart(uint64_t n_long, uint64_t n_lines) {
+    return n_long * 8 < n_lines || n_long < (1u << 15);
+}
 
 // Entry counts per line (written in place of the offsets, then scanned)
 // and the raster tile boxes.  Counting is a separate kernel, not folded into
@@ -1015,8 +1025,10 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
     // of 20,000 strokes 5.92 -> 5.36).
     if (n_lines) {
         // long-line walkers: persistent, their groups take lines from the queue
+        const bool apart = long_cells != 0 &&
+                           (plan ? plan->long_apart : long_lines_apart(host_scalars(ctx)->n_long, n_lines));
         uint32_t long_blocks = 0;
-        if (long_cells) {
+        if (apart) {
             int sms = 152;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
             long_blocks = (uint32_t)sms * LONG_BLOCKS_PER_SM;
@@ -1038,7 +1050,7 @@ int stage_bin(ochre_gpu_ctx* ctx, const ochre_batch* in, uint32_t n_lines, cudaS
                 ctx->lines.as<float4>(), ctx->line_raster.as<uint32_t>(), ctx->line_ent_off.as<uint32_t>(),
                 ctx->line_inc_off.as<uint32_t>(), n_lines, lines_dev, ctx->raster_bbox.as<int4>(),
                 ctx->raster_keybase.as<uint64_t>(), ctx->keys.as<K>(), ctx->vals.as<uint32_t>(),
-                ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), long_cells));
+                ctx->bins.as<BinRec>(), ctx->incs.as<float2>(), apart ? long_cells : 0u));
         };
         if (ctx->keys64) emit(uint64_t{}); else emit(uint32_t{});
         OCHRE_CUDA_TRY(cudaGetLastError());

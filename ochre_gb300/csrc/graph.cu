@@ -159,6 +159,7 @@ int build(ochre_graph* g) {
         if (es.key_bits <= 32 && kb > 32) kb = 32;
         p.key_bits = kb;
         p.rows = std::max<uint32_t>(host_scalars(ctx)->n_rows, 1u);
+        p.long_apart = long_lines_apart(host_scalars(ctx)->n_long, es.n_lines);
     }
     p.diff = g->is_diff ? &g->diff : nullptr;
     // stroked fills: the stroke stage's counts of the planning run

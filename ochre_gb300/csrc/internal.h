@@ -118,6 +118,7 @@ struct GraphPlan {
     uint32_t key_bits;   // sort key bits; keys are 64-bit above 32
     uint32_t incs;       // general chain: stored pixel-cell increments
     uint32_t rows;       // tile rows of the planning run (coverage form and grid)
+    bool long_apart;     // long_lines_apart of the planning run
     // Stroked fills (planned on the general chain): polyline commands and
     // floats, output commands and floats of the stroke stage.  Its units
     // never outnumber the polyline commands.  The output is padded to
@@ -317,6 +318,8 @@ constexpr int LOCAL_SORT_IDX_BITS = 13, LOCAL_SORT_KEY_BITS = 32 - LOCAL_SORT_ID
 // block size and the host sees whether all fit)?
 inline bool sort_local_wanted(const ochre_gpu_ctx* ctx);
 int stage_sort_local(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s);
+// Are the queued long lines walked by kernels of their own (dda.cu)?
+bool long_lines_apart(uint64_t n_long, uint64_t n_lines);
 int stage_tiles(ochre_gpu_ctx* ctx, const ochre_batch* in, uint64_t n_entries, cudaStream_t s, uint32_t* n_tiles,
                 uint32_t* n_spans);
 // Rewrites stroked fills into plain fills (stroke.cu); *out views device memory.
