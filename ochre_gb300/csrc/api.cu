@@ -339,7 +339,7 @@ static int run_chain(ochre_gpu_ctx* ctx, const ochre_batch* in_orig, ochre_resul
         st = stage_bin(ctx, in, L, s, &E, &bits);
         if (st != OCHRE_OK) return st;
         uint32_t passes = 1;
-        if (L && sort_local_wanted(ctx) && host_scalars(ctx)->n_sort[2] == 0u)
+        if (L && sort_local_wanted(ctx) && host_scalars(ctx)->n_sort[2] == 0u && sort_local_pays(R, E))
             st = stage_sort_local(ctx, in, s);
         else
             st = stage_sort(ctx, E, bits, s, &passes);

@@ -317,6 +317,15 @@ constexpr int LOCAL_SORT_IDX_BITS = 13, LOCAL_SORT_KEY_BITS = 32 - LOCAL_SORT_ID
 // May the context's run sort that way (then stage_bin lists the rasters by
 // block size and the host sees whether all fit)?
 inline bool sort_local_wanted(const ochre_gpu_ctx* ctx);
+// Does it pay?  A block costs 2.8 ns whatever it sorts, the device-wide passes 30
+// us and 30 ps an entry: with R rasters that is 96 entries a raster, less what
+// the 30 us are worth.  Measured, one block a raster against the passes: 300,000
+// rasters of 14 entries 839 and 147 us, of 85 897 and 817, of 169 1,021 and 1,508;
+// 20,000 of 3 entries 53 and 30, of 37 55 and 65, of 404 124 and 243; 3,000 of 3
+// entries 14 and 29.
+inline bool sort_local_pays(uint64_t n_rasters, uint64_t n_entries) {
+    return n_entries + (1u << 20) >= 96 * n_rasters;
+}
 int stage_sort_local(ochre_gpu_ctx* ctx, const ochre_batch* in, cudaStream_t s);
 // Are the queued long lines walked by kernels of their own (dda.cu)?
 bool long_lines_apart(uint64_t n_long, uint64_t n_lines);
