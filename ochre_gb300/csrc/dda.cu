@@ -3,14 +3,16 @@
 // Reference: Rasterizer::line_to (rasterizer.rs:72-140) and the run-length
 // binning of finish (rasterizer.rs:185-208).
 //
-// Every line is walked by one thread with the reference's exact serial
-// recurrence.  Invariant used to make lines independent: at the start of
+// The count takes a line's row and column recurrences one after the other,
+// without its cells.  The emission walks the cells with the reference's exact
+// serial recurrence: one thread a line, or a group of lanes a long line, all
+// of which run both recurrences alike.  Invariant used to make lines independent: at the start of
 // every line_to, tile_y_prev == div_euclid(floor(last.y) as i16, 8) — move_to
 // sets it that way (rasterizer.rs:68) and every walk ends by snapping to
 // floor(point) and updating tile_y_prev for that cell (rasterizer.rs:118-131).
 //
-// A walk stores the increment (area, height) of every cell it visits once,
-// line by line (the count pass gives each line its offset), and produces two
+// The emission stores the increment (area, height) of every cell once, line
+// by line (the count gives each line its offset), and produces two
 // kinds of sort entries:
 //   * a *bin* per run of consecutive increment cells in one tile
 //     (value = entry index; the BinRec at that index holds the run's first
